@@ -306,6 +306,53 @@ int spgt_spectral_conv2d_fwd(const float* x, const float* wr, const float* br, c
                              const void* tables, void* workspace, size_t workspace_bytes, float* y,
                              int B, int r, int C, int m, int act, spgt_stream_t stream);
 
+/* ---------------------------------------------------------------------------------------------
+ * The whole Darcy forward as one call (reference: network/sp_model.py:91-113)
+ * ------------------------------------------------------------------------------------------- */
+
+#define SPGT_MAX_LAYERS 32
+
+/* One encoder layer (network/sp_layer.py:94-104): weights as the single-op entry points above take them. */
+typedef struct {
+    const void* wqkv;                                        /* spgt_tc_weight_prepare of Wq | Wk | Wv [128, 384] */
+    const float *bq, *bk, *bv, *lnwk, *lnbk, *lnwv, *lnbv;
+    const void* wfc; const float* bfc;                       /* [128 + 4 d_pos, 128] */
+    const void* w1; const float* b1;                         /* [128, 256] */
+    const void* w2; const float* b2;                         /* [256, 128] */
+} spgt_encoder_weights;
+
+/* One spectral layer: as spgt_spectral_conv2d_fwd takes them. */
+typedef struct { const float *wr, *br, *fw0, *fw1; } spgt_spectral_weights;
+
+/* Sizes, constants and device pointers of a Darcy Galerkin transformer of width 128 with 4 heads, feed-forward width 256
+ * and decoder width 32 (a host struct; the library keeps no copy).  r, mid, ra: fine grid, grid of the scalers' convolutions,
+ * attention grid.  c1 + c2 + c3 = 128: output channels of the three concatenated down-scaler convolutions, whose prepared
+ * weights and biases are zero-padded to multiples of 4 channels. */
+typedef struct {
+    int r, mid, ra, d_pos, n_encoder, n_decoder, modes, c1, c2, c3;
+    int act_down, act_up, act_ffn, act_dec, dirichlet;
+    float eps, b2, scale, shift;
+    const float *conv0_w, *conv0_b;                          /* [9, 128], [128] */
+    const void* conv_w[3]; const float* conv_b[3];
+    const void* up_w; const float* up_b;                     /* 3x3, 128 -> 128 */
+    const void* fcx_w; const float *fcg_w, *fc_b;            /* spatial fc: prepared [128, 32], [d_pos = 2, 32], [32] */
+    const void* tables;                                      /* spgt_spectral_tables_init(r, modes) */
+    const void* head_w1; const float *head_b1, *head_w2;     /* prepared [32, 128], [128], [128] */
+    const float *scale_map, *shift_map;                      /* NULL or [r * r] */
+    spgt_encoder_weights encoder[SPGT_MAX_LAYERS];
+    spgt_spectral_weights decoder[SPGT_MAX_LAYERS];
+} spgt_darcy_model;
+
+/* Bytes of scratch one forward of B samples needs (0: unsupported sizes). */
+size_t spgt_darcy_workspace_bytes(const spgt_darcy_model* model, int B);
+/* Kernels one forward of B samples launches. */
+int spgt_darcy_launches(const spgt_darcy_model* model, int B);
+/* node [B,r,r,1], position [B,ra*ra,d_pos], grid [B,r,r,2] -> out [B,r,r,1].  taps, when not NULL: n_encoder + 2 device pointers,
+ * each NULL or a buffer that receives a copy of the down-scaler output [B,ra,ra,128], of every encoder layer's output, and of
+ * the up-scaler output before its last interpolation [B,mid,mid,128].  Every launch goes to `stream`; nothing synchronises. */
+int spgt_darcy_forward(const spgt_darcy_model* model, const float* node, const float* position, const float* grid, float* out,
+                       int B, float* const* taps, void* workspace, size_t workspace_bytes, spgt_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

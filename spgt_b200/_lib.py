@@ -23,6 +23,28 @@ _fl = C.c_float
 _sz = C.c_size_t
 _st = C.c_void_p     # cudaStream_t
 
+
+MAX_LAYERS = 32
+
+
+class EncoderWeights(C.Structure):          # spgt_encoder_weights
+    _fields_ = [(n, _f) for n in ('wqkv', 'bq', 'bk', 'bv', 'lnwk', 'lnbk', 'lnwv', 'lnbv', 'wfc', 'bfc', 'w1', 'b1', 'w2', 'b2')]
+
+
+class SpectralWeights(C.Structure):         # spgt_spectral_weights
+    _fields_ = [(n, _f) for n in ('wr', 'br', 'fw0', 'fw1')]
+
+
+class DarcyModel(C.Structure):              # spgt_darcy_model
+    _fields_ = ([(n, _i) for n in ('r', 'mid', 'ra', 'd_pos', 'n_encoder', 'n_decoder', 'modes', 'c1', 'c2', 'c3', 'act_down', 'act_up',
+                                   'act_ffn', 'act_dec', 'dirichlet')]
+                + [(n, _fl) for n in ('eps', 'b2', 'scale', 'shift')]
+                + [('conv0_w', _f), ('conv0_b', _f), ('conv_w', _f * 3), ('conv_b', _f * 3)]
+                + [(n, _f) for n in ('up_w', 'up_b', 'fcx_w', 'fcg_w', 'fc_b', 'tables', 'head_w1', 'head_b1', 'head_w2', 'scale_map',
+                                     'shift_map')]
+                + [('encoder', EncoderWeights * MAX_LAYERS), ('decoder', SpectralWeights * MAX_LAYERS)])
+
+
 SIGNATURES = {
     'spgt_error_string': (C.c_char_p, [_i]),
     'spgt_last_cuda_error': (_i, []),
@@ -68,6 +90,9 @@ SIGNATURES = {
     'spgt_spectral_workspace_bytes': (_sz, [_i, _i, _i, _i]),
     'spgt_spectral_chunk_samples': (_i, [_i]),
     'spgt_spectral_launches': (_i, [_i, _i, _i]),
+    'spgt_darcy_workspace_bytes': (_sz, [_f, _i]),
+    'spgt_darcy_launches': (_i, [_f, _i]),
+    'spgt_darcy_forward': (_i, [_f] * 5 + [_i, _f, _f, _sz, _st]),
     'spgt_spectral_conv2d_fwd': (_i, [_f, _f, _f, _f, _f, _f, _f, _sz, _f, _i, _i, _i, _i, _i, _st]),
 }
 

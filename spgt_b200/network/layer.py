@@ -13,12 +13,35 @@ from torch import Tensor
 from .. import ops
 
 
+class ParameterWatch:
+    """Tells when a module's parameters are not the ones seen before: tag() differs after a parameter has been written to
+    (an optimizer step bumps the version counters), moved, or replaced, or a submodule has been exchanged.  The tree is walked
+    once, not on every call (Module.parameters() takes longer than the launch it would guard)."""
+
+    def __init__(self):
+        self.tree = None         # (no reference to the module itself: a cycle would keep its memory until a garbage collection)
+
+    def tag(self, module: torch.nn.Module) -> tuple:
+        if self.tree is None or any(len(d) != n for d, n in self.sizes) or any(d[k] is not c for d, k, c in self.tree):
+            modules = list(module.modules())
+            self.sizes = [(d, len(d)) for m in modules for d in (m._modules, m._parameters)]
+            self.tree = [(m._modules, k, c) for m in modules for k, c in m._modules.items()]
+            self.slots = [(m._parameters, k) for m in modules for k, p in m._parameters.items() if p is not None]
+        params = [d[k] for d, k in self.slots]
+        return tuple([p._version for p in params] + [p.data_ptr() for p in params])
+
+    def hold(self) -> list:
+        """Aliases of the parameters' storages: while they are kept, no other tensor can come to lie at these addresses."""
+        return [d[k].detach() for d, k in self.slots]
+
+
 class _KernelWeights(torch.nn.Module):
     """Caches derived weight layouts; the cache is dropped whenever parameters are (re)loaded or moved."""
 
     def __init__(self):
         super().__init__()
         self._kw = {}
+        self._watch = ParameterWatch()
         self.register_load_state_dict_post_hook(lambda module, incompatible: module._kw.clear())
 
     def _apply(self, fn, *args, **kwargs):
@@ -26,13 +49,12 @@ class _KernelWeights(torch.nn.Module):
         return super()._apply(fn, *args, **kwargs)
 
     def _cached(self, key, make):
-        """Derived layout of the module's weights, rebuilt when a parameter has been modified in place since it was
-        made (an optimizer step bumps the parameters' version counters)."""
-        tag = sum(p._version for p in self.parameters())
+        """Derived layout of the module's weights, rebuilt when a parameter is not the one it was made from."""
+        tag = self._watch.tag(self)
         hit = self._kw.get(key)
         if hit is None or hit[0] != tag:
             with torch.no_grad():
-                hit = (tag, make())
+                hit = (tag, make(), self._watch.hold())
             self._kw[key] = hit
         return hit[1]
 
@@ -88,11 +110,13 @@ class ConvResBlock2D(_KernelWeights):
         return ops.conv3x3(X, cin_off, w.shape[1], self.kernel_weight(), self.conv_layer.bias.detach(), out, cout_off,
                            w.shape[0], self.activation if act is None else act)
 
+    def tc_weight(self, cin_pad: int, cout_pad: int):
+        return self._cached(('tc', cin_pad, cout_pad), lambda: _conv_tc(self.conv_layer.weight, self.conv_layer.bias, cin_pad, cout_pad))
+
     def forward_tc(self, X: Tensor, cin_pad: int, cout_pad: int, act=None) -> Tensor:
         """tcgen05 path: X [N,H,W,cin_pad] (channels beyond in_dim must be finite; their weights are zero) ->
         new tensor [N,H,W,cout_pad] whose channels beyond out_dim hold act(0)."""
-        wt, b = self._cached(('tc', cin_pad, cout_pad),
-                             lambda: _conv_tc(self.conv_layer.weight, self.conv_layer.bias, cin_pad, cout_pad))
+        wt, b = self.tc_weight(cin_pad, cout_pad)
         out = torch.empty(*X.shape[:3], cout_pad, device=X.device, dtype=X.dtype)
         return ops.conv3x3_tc(X, 0, cin_pad, wt, b, out, 0, cout_pad, self.activation if act is None else act)
 
@@ -113,10 +137,12 @@ class FeedForward(_KernelWeights):
         self.layer2 = torch.nn.Linear(dim_hidden, out_dim)
         self.fused = True        # one kernel for both GEMMs when the shape is 128 -> 256 -> 128
 
+    def tc_weights(self):
+        return self._cached('w1', lambda: _linear_tc(self.layer1.weight)), self._cached('w2', lambda: _linear_tc(self.layer2.weight))
+
     def forward(self, X: Tensor, residual: Tensor = None) -> Tensor:
         """X [..., in_dim] -> [..., out_dim] (+ residual when given, fused into the second GEMM)."""
-        w1 = self._cached('w1', lambda: _linear_tc(self.layer1.weight))
-        w2 = self._cached('w2', lambda: _linear_tc(self.layer2.weight))
+        w1, w2 = self.tc_weights()
         if self.fused and w1.K == 128 and w1.N == 256 and w2.N == 128:
             return ops.ffn_tc(X, w1, self.layer1.bias.detach(), w2, self.layer2.bias.detach(), self.activation, residual)
         h = ops.linear_tc(X, w1, self.layer1.bias.detach(), self.activation)

@@ -28,11 +28,13 @@ class DownScaler2D(_KernelWeights):
         self.conv2 = ConvResBlock2D(out_dim1, out_dim2, 3, 1, droprate, activation)
         self.conv3 = ConvResBlock2D(out_dim2, out_dim3, 3, 1, droprate, activation)
 
+    def kernel_weight0(self):
+        return self._cached('w0', lambda: self.conv0.conv_layer.weight.detach().reshape(-1, 9).t().contiguous())
+
     def forward(self, X: Tensor) -> Tensor:
         N, r, _, _ = X.shape
         mid, ra = self.resolution_size[1], self.resolution_size[2]
-        w0 = self._cached('w0', lambda: self.conv0.conv_layer.weight.detach().reshape(-1, 9).t().contiguous())
-        X = ops.conv0_down(X.reshape(N, r, r), w0, self.conv0.conv_layer.bias.detach(), mid[0], mid[1], self.activation)
+        X = ops.conv0_down(X.reshape(N, r, r), self.kernel_weight0(), self.conv0.conv_layer.bias.detach(), mid[0], mid[1], self.activation)
         d1, d2, d3 = self.dims
         pad4 = lambda c: (c + 3) // 4 * 4          # the tcgen05 implicit GEMM wants channel counts that are multiples of 4
         X1 = self.conv1.forward_tc(X, X.shape[3], pad4(d1))

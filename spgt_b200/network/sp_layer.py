@@ -46,16 +46,21 @@ class Sp_GalerkinAttention(_KernelWeights):
             torch.nn.init.ones_(lnw)
             torch.nn.init.zeros_(lnb)
 
+    def qkv_weight(self):
+        return self._cached('wqkv', lambda: ops.TcWeight(
+            torch.cat([self.weight_Q.detach(), self.weight_K.detach(), self.weight_V.detach()], dim=1).contiguous()))
+
+    def fc_weight(self):
+        return self._cached('fc', lambda: _linear_tc(self.fc_layer.weight))
+
     def forward(self, Q: Tensor, K: Tensor, V: Tensor, position: Tensor, residual: Tensor = None) -> Tensor:
         """Q,K,V [N,S,D], position [N,S,d_pos] -> [N,S,D] (+ residual, fused into the output projection).
         When Q, K and V are the same tensor (self-attention) all three projections run in one launch."""
         d = lambda t: t.detach()
         H, dh, dp = self.num_head, self.dim_head, self.dim_position
         if Q is K and K is V and self.dim_hidden == 128:
-            wqkv = self._cached('wqkv', lambda: ops.TcWeight(
-                torch.cat([d(self.weight_Q), d(self.weight_K), d(self.weight_V)], dim=1).contiguous()))
             q, k, v = ops.projpos_qkv_tc(
-                Q, wqkv, d(self.bias_Q), d(self.bias_K), d(self.bias_V), d(self.ln_weight_K), d(self.ln_bias_K),
+                Q, self.qkv_weight(), d(self.bias_Q), d(self.bias_K), d(self.bias_V), d(self.ln_weight_K), d(self.ln_bias_K),
                 d(self.ln_weight_V), d(self.ln_bias_V), self.norm_eps, position, H, dh, dp)
         elif Q is K and K is V:
             q, k, v = ops.projpos_qkv(
@@ -69,8 +74,7 @@ class Sp_GalerkinAttention(_KernelWeights):
             v = ops.projpos_lnorm(V, d(self.weight_V), d(self.bias_V), d(self.ln_weight_V), d(self.ln_bias_V), position,
                                   self.norm_eps, H, dh, dp)
         X = ops.galerkin_attention(q, k, v, merged_heads=True)          # [N, S, H*(d_pos+d_head)]
-        wfc = self._cached('fc', lambda: _linear_tc(self.fc_layer.weight))
-        return ops.linear_tc(X, wfc, d(self.fc_layer.bias), None, residual)
+        return ops.linear_tc(X, self.fc_weight(), d(self.fc_layer.bias), None, residual)
 
 
 def _attention_forward_train(self, Q: Tensor, K: Tensor, V: Tensor, position: Tensor) -> Tensor:
@@ -101,6 +105,15 @@ class Sp_EncoderLayer(torch.nn.Module):
             dim_hidden, num_head, dim_position, norm_eps, attn_droprate, fc_droprate, xavier, diagonal, symmetric)
         self.ffn_layer = FeedForward(dim_hidden, dim_hidden, ffn_dim_hidden, ffn_droprate, ffn_activation)
 
+    def fill_native(self, w, ptr) -> None:
+        """Device pointers of this layer's weights into a spgt_encoder_weights; `ptr` keeps what it is given alive."""
+        a, f = self.attention_layer, self.ffn_layer
+        w.wqkv, w.wfc, w.bfc = ptr(a.qkv_weight()), ptr(a.fc_weight()), ptr(a.fc_layer.bias.detach())
+        w.bq, w.bk, w.bv = (ptr(b.detach()) for b in (a.bias_Q, a.bias_K, a.bias_V))
+        w.lnwk, w.lnbk, w.lnwv, w.lnbv = (ptr(t.detach()) for t in (a.ln_weight_K, a.ln_bias_K, a.ln_weight_V, a.ln_bias_V))
+        w1, w2 = f.tc_weights()
+        w.w1, w.b1, w.w2, w.b2 = ptr(w1), ptr(f.layer1.bias.detach()), ptr(w2), ptr(f.layer2.bias.detach())
+
     def forward(self, X: Tensor, position: Tensor) -> Tensor:
         """X [N,S,D], position [N,S,d_pos] -> X + attention(X) then + ffn(.)  (network/sp_layer.py:94-104)."""
         X = self.attention_layer(X, X, X, position, residual=X)
@@ -128,10 +141,17 @@ class Sp_SpectralConv2D(_KernelWeights):
         for param in self.fourier_weight:
             torch.nn.init.xavier_normal_(param, gain=1.0 / (in_dim * out_dim) * math.sqrt(in_dim + out_dim))
 
+    def residual_weight(self):
+        return self._cached('wr', lambda: _linear_kn(self.residual_layer.weight))
+
+    def fill_native(self, w, ptr) -> None:
+        w.wr, w.br = ptr(self.residual_weight()), ptr(self.residual_layer.bias.detach())
+        w.fw0, w.fw1 = (ptr(p.detach()) for p in self.fourier_weight)
+
     def forward(self, X: Tensor) -> Tensor:
         N, r, _, in_dim = X.shape
         m, out_dim = self.mode, self.out_dim
-        wr = self._cached('wr', lambda: _linear_kn(self.residual_layer.weight))
+        wr = self.residual_weight()
         br = self.residual_layer.bias.detach()
         fw0, fw1 = self.fourier_weight[0].detach(), self.fourier_weight[1].detach()
         if self.structure == 'fused':

@@ -7,7 +7,8 @@ import torch
 from torch import Tensor
 
 from .. import ops
-from .layer import FeedForward, _KernelWeights, _linear_kn, _linear_tc
+from .._lib import MAX_LAYERS, DarcyModel
+from .layer import FeedForward, ParameterWatch, _KernelWeights, _linear_kn, _linear_tc
 from .model import DownScaler2D, UpScaler2D
 from .sp_layer import Sp_EncoderLayer, Sp_SpectralConv2D
 
@@ -48,17 +49,21 @@ class Sp_DecoderRegressor(_KernelWeights):
         dim_ffn_hidden = 2 * dim_position * dim_spatial_hidden
         self.ffn_layer = FeedForward(dim_spatial_hidden, out_dim, dim_ffn_hidden, droprate, activation)
 
+    def head_weights(self):
+        """(first weight as its kernel takes it, second weight [hidden], second bias) of the decoder head."""
+        f = self.ffn_layer
+        make = _linear_tc if f.layer1.out_features == 128 else _linear_kn
+        return (self._cached('w1', lambda: make(f.layer1.weight)), self._cached('w2', lambda: f.layer2.weight.detach().reshape(-1).contiguous()),
+                self._cached('b2', lambda: float(f.layer2.bias.detach().reshape(-1)[0])))
+
     def _spectral_and_head(self, X: Tensor, scale, shift, dirichlet, scale_map=None, shift_map=None) -> Tensor:
         for layer in self.layers:
             X = layer(X)
         f = self.ffn_layer
-        w2 = self._cached('w2', lambda: f.layer2.weight.detach().reshape(-1).contiguous())
-        b2 = self._cached('b2', lambda: float(f.layer2.bias.detach().reshape(-1)[0]))
+        w1, w2, b2 = self.head_weights()
         if f.layer1.out_features == 128:
-            w1 = self._cached('w1tc', lambda: _linear_tc(f.layer1.weight))
             return ops.decoder_head_tc(X, w1, f.layer1.bias.detach(), w2, b2, scale, shift, dirichlet, self.activation,
                                        scale_map, shift_map)
-        w1 = self._cached('w1', lambda: _linear_kn(f.layer1.weight))
         return ops.decoder_head(X, w1, f.layer1.bias.detach(), w2, b2, scale, shift, dirichlet, self.activation,
                                 scale_map, shift_map)
 
@@ -135,6 +140,7 @@ class Sp_GalerkinTransformer2D(torch.nn.Module):
             cfg['num_decoder_layer'], cfg['dim_hidden'], cfg['dim_target'], cfg['dim_position'], cfg['dim_spatial_hidden'],
             cfg['num_frequence_mode'], cfg['drop_decoder_layer'], cfg['acti_decoder_layer'])
         self._affine = None
+        self._plan, self._watch = None, ParameterWatch()
 
     def forward(self, X: Tensor, position: Tensor, grid: Tensor, taps: dict = None) -> Tensor:
         """X [N,r,r,1], position [N,r_attn,r_attn,2], grid [N,r,r,2] -> [N,r,r,1]; CUDA fp32 contiguous tensors.
@@ -159,9 +165,82 @@ class Sp_GalerkinTransformer2D(torch.nn.Module):
         return X
 
     def _forward_fused(self, X: Tensor, position: Tensor, grid: Tensor, taps: dict = None) -> Tensor:
+        plan = self._native_plan(X)
+        if plan is None:
+            return self._forward_modules(X, position, grid, taps)
+        return ops.darcy_forward(plan, X, position, grid, taps)
+
+    def _native_plan(self, X: Tensor):
+        """The model as the one-call forward takes it, rebuilt when the parameters, the grid or the device are not the ones it was
+        made for; None for widths that forward does not cover."""
+        tag = (X.shape[1], X.device, self.normalizer, self.boundary_condition, self._watch.tag(self))
+        if self._plan is None or self._plan[0] != tag:
+            self._plan = (tag, self._build_plan(X), self._watch.hold())
+        return self._plan[1]
+
+    def _apply(self, fn, *args, **kwargs):
+        self._plan = self._affine = None
+        return super()._apply(fn, *args, **kwargs)
+
+    def _build_plan(self, X: Tensor):
+        r, down, up, dec = X.shape[1], self.down_scaler, self.up_scaler, self.decoder_regressor
+        enc = list(self.encoder_mixer.layers)
+        if sum(down.dims) != 128 or not self._native_widths() or max(len(enc), len(dec.layers)) > MAX_LAYERS:
+            return None
+        size = down.resolution_size
+        if size[0] != (r, r) or size[4] != (r, r) or size[3] != size[1] or any(a != b for a, b in size):
+            return None
+        if self._affine is None or self._affine[0] != (r, X.device, self.normalizer):
+            self._affine = ((r, X.device, self.normalizer), _normalizer_affine(self.normalizer, r, X.device))
+        scale, shift, scale_map, shift_map = self._affine[1]
+        keep = []
+
+        def ptr(t):
+            if t is None:
+                return None
+            keep.append(t)
+            return t.data_ptr()
+        m = DarcyModel()
+        m.r, m.mid, m.ra, m.n_encoder, m.n_decoder = r, size[1][0], size[2][0], len(enc), len(dec.layers)
+        m.d_pos = enc[0].attention_layer.dim_position if enc else dec.dim_position
+        m.modes = dec.layers[0].mode if len(dec.layers) else 1
+        m.c1, m.c2, m.c3 = down.dims
+        m.act_down, m.act_dec = ops.act_code(down.activation), ops.act_code(dec.activation)
+        m.act_up = ops.act_code('silu2' if up.activation == 'silu' else 'relu')
+        m.act_ffn = ops.act_code(enc[0].ffn_layer.activation) if enc else 0
+        m.eps = enc[0].attention_layer.norm_eps if enc else 0.0
+        m.dirichlet = int(self.boundary_condition == 'dirichlet')
+        m.scale, m.shift, m.scale_map, m.shift_map = scale, shift, ptr(scale_map), ptr(shift_map)
+        m.conv0_w, m.conv0_b = ptr(down.kernel_weight0()), ptr(down.conv0.conv_layer.bias.detach())
+        cin = 128
+        for i, (conv, c) in enumerate(zip((down.conv1, down.conv2, down.conv3), down.dims)):
+            w, b = conv.tc_weight(cin, (c + 3) // 4 * 4)
+            m.conv_w[i], m.conv_b[i], cin = ptr(w), ptr(b), (c + 3) // 4 * 4
+        for i, layer in enumerate(enc):
+            layer.fill_native(m.encoder[i], ptr)
+        w, b = up.conv.tc_weight(128, 128)
+        m.up_w, m.up_b = ptr(w), ptr(b)
+        wx, wg = dec._split_fc()
+        m.fcx_w, m.fcg_w, m.fc_b = ptr(wx), ptr(wg), ptr(dec.spatial_fc_layer.bias.detach())
+        for i, layer in enumerate(dec.layers):
+            layer.fill_native(m.decoder[i], ptr)
+        m.tables = ptr(ops.spectral_tables(r, m.modes, X.device)) if len(dec.layers) else None
+        w1, w2, m.b2 = dec.head_weights()
+        m.head_w1, m.head_b1, m.head_w2 = ptr(w1), ptr(dec.ffn_layer.layer1.bias.detach()), ptr(w2)
+        return ops.DarcyPlan(m, keep)
+
+    def _native_widths(self) -> bool:
+        enc, dec, up = self.encoder_mixer.layers, self.decoder_regressor, self.up_scaler
+        return (all(a.dim_hidden == 128 and a.num_head == 4 and f.layer1.out_features == 256 and f.layer1.in_features == 128
+                    and f.layer2.out_features == 128 for a, f in ((l.attention_layer, l.ffn_layer) for l in enc))
+                and up.conv.conv_layer.in_channels == 128 and up.conv.conv_layer.out_channels == 128 and dec.in_dim == 128
+                and dec.dim_position == 2 and dec.spatial_fc_layer.out_features == 32 and dec.ffn_layer.layer1.out_features == 128
+                and all(l.structure == 'fused' and l.in_dim == 32 and l.out_dim == 32 for l in dec.layers))
+
+    def _forward_modules(self, X: Tensor, position: Tensor, grid: Tensor, taps: dict = None) -> Tensor:
         r = X.shape[1]
-        if self._affine is None or self._affine[0] != (r, X.device):
-            self._affine = ((r, X.device), _normalizer_affine(self.normalizer, r, X.device))
+        if self._affine is None or self._affine[0] != (r, X.device, self.normalizer):
+            self._affine = ((r, X.device, self.normalizer), _normalizer_affine(self.normalizer, r, X.device))
         scale, shift, scale_map, shift_map = self._affine[1]
         X = self.down_scaler(X)
         if taps is not None:

@@ -28,6 +28,26 @@ def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
+class _device:
+    """torch.cuda.device(tensor.device) for kernels about to be launched, at the cost of one query when that device is already
+    the current one (the usual case)."""
+    __slots__ = ('want', 'back')
+
+    def __init__(self, device):
+        self.want, self.back = device.index, None
+
+    def __enter__(self):
+        current = torch.cuda.current_device()
+        if self.want is not None and self.want != current:
+            torch.cuda.set_device(self.want)
+            self.back = current
+
+    def __exit__(self, *exc):
+        if self.back is not None:
+            torch.cuda.set_device(self.back)
+        return False
+
+
 # kernels launched by one call of each entry point (everything else launches one)
 _KERNELS_PER_CALL = {'spgt_batched_skinny_gemm': 2, 'spgt_galerkin_attn_bwd': 2, 'spgt_projpos_bwd_elementwise': 2}
 LAUNCHES = 0          # running count of kernels launched through this module
@@ -99,7 +119,7 @@ def projpos(x: Tensor, weight: Tensor, bias: Optional[Tensor], position: Tensor,
         _chk(bias, 'bias')
     B, S, D = x.shape
     out = torch.empty(B, num_head, dim_position + dim_head, S, device=x.device, dtype=x.dtype)
-    with torch.cuda.device(x.device):
+    with _device(x.device):
         _call('spgt_projpos_fwd', x.data_ptr(), weight.data_ptr(), _p(bias), position.data_ptr(), out.data_ptr(),
                                    B, S, D, num_head, dim_head, dim_position, _stream())
     return out
@@ -114,7 +134,7 @@ def projpos_lnorm(x: Tensor, weight: Tensor, bias: Optional[Tensor], ln_weight: 
     B, S, D = x.shape
     out = torch.empty(B, num_head, dim_position + dim_head, S, device=x.device, dtype=x.dtype)
     inv = torch.empty(B, num_head, S, device=x.device, dtype=x.dtype) if return_invsigma else None
-    with torch.cuda.device(x.device):
+    with _device(x.device):
         _call('spgt_projpos_lnorm_fwd', x.data_ptr(), weight.data_ptr(), _p(bias), ln_weight.data_ptr(), ln_bias.data_ptr(),
                                          float(norm_eps), position.data_ptr(), out.data_ptr(), _p(inv),
                                          B, S, D, num_head, dim_head, dim_position, _stream())
@@ -126,7 +146,7 @@ def projpos_qkv(x, wq, bq, wk, bk, wv, bv, lnwk, lnbk, lnwv, lnbv, eps, position
         _chk(t, n)
     B, S, D = x.shape
     q, k, v = (torch.empty(B, num_head, dim_position + dim_head, S, device=x.device, dtype=x.dtype) for _ in range(3))
-    with torch.cuda.device(x.device):
+    with _device(x.device):
         _call('spgt_projpos_qkv_fwd', x.data_ptr(), wq.data_ptr(), _p(bq), wk.data_ptr(), _p(bk), wv.data_ptr(), _p(bv),
                                        lnwk.data_ptr(), lnbk.data_ptr(), lnwv.data_ptr(), lnbv.data_ptr(), float(eps),
                                        position.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(),
@@ -142,7 +162,7 @@ def galerkin_attention(Q: Tensor, K: Tensor, V: Tensor, merged_heads: bool = Fal
     shape = (B, S, H * dpk) if merged_heads else (B, H, S, dpk)
     out = torch.empty(shape, device=Q.device, dtype=Q.dtype)
     T = torch.empty(B, H, dpk, dpk, device=Q.device, dtype=Q.dtype) if return_kv else None
-    with torch.cuda.device(Q.device):
+    with _device(Q.device):
         _call('spgt_galerkin_attn_fwd', Q.data_ptr(), K.data_ptr(), V.data_ptr(), out.data_ptr(), _p(T),
                                          B, H, dpk, S, int(merged_heads), _stream())
     return (out, T) if return_kv else out
@@ -165,7 +185,7 @@ def projpos_backward(x: Tensor, weight: Tensor, bias: Optional[Tensor], ln_weigh
     dlnb = torch.empty(D, device=x.device, dtype=x.dtype) if ln_weight is not None else None
     need = int(lib.spgt_projpos_bwd_workspace_bytes(B, S, num_head))
     ws = torch.empty(max(need, 16), dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
+    with _device(x.device):
         _call('spgt_projpos_bwd_elementwise', grad_out.data_ptr(), _p(h), _p(ln_weight), float(norm_eps), dh.data_ptr(), db.data_ptr(),
               _p(dlnw), _p(dlnb), B, S, num_head, dim_head, dim_position, ws.data_ptr(), need, _stream())
     dx = linear_tc(dh, TcWeight(weight.t().contiguous()), None).view(B, S, D)
@@ -185,7 +205,7 @@ def galerkin_attention_backward(Q: Tensor, K: Tensor, V: Tensor, grad_out: Tenso
     need = int(lib.spgt_galerkin_attn_bwd_workspace_bytes(B, H, dpk, S))
     ws = torch.empty(max(need, 16), dtype=torch.uint8, device=Q.device)
     dQ, dK, dV = torch.empty_like(Q), torch.empty_like(Q), torch.empty_like(Q)
-    with torch.cuda.device(Q.device):
+    with _device(Q.device):
         _call('spgt_galerkin_attn_bwd', Q.data_ptr(), K.data_ptr(), V.data_ptr(), grad_out.data_ptr(), dQ.data_ptr(), dK.data_ptr(),
               dV.data_ptr(), B, H, dpk, S, ws.data_ptr(), need, _stream())
     return dQ, dK, dV
@@ -237,7 +257,7 @@ def batched_skinny_gemm(A: Tensor, Bm: Tensor, alpha: float = 1.0, workspace: Op
     need = skinny_gemm_workspace_bytes(M, N, K, batch)
     if workspace is None:
         workspace = torch.empty(need, device=A.device, dtype=torch.uint8)
-    with torch.cuda.device(A.device):
+    with _device(A.device):
         _call('spgt_batched_skinny_gemm', A.data_ptr(), Bm.data_ptr(), Cm.data_ptr(), float(alpha), M, N, K, batch,
                                            workspace.data_ptr(), workspace.numel() * workspace.element_size(), _stream())
     return Cm
@@ -252,7 +272,7 @@ def batched_transpose(X: Tensor, batch_list: Sequence[int], M_list: Sequence[int
     if X.numel() != b * M * N:
         raise ValueError('X does not have prod(batch)*prod(M)*prod(N) elements')
     out = torch.empty(*batch_list, *N_list, *M_list, device=X.device, dtype=X.dtype)
-    with torch.cuda.device(X.device):
+    with _device(X.device):
         _call('spgt_batched_transpose', X.data_ptr(), out.data_ptr(), M, N, b, _stream())
     return out
 
@@ -264,7 +284,7 @@ def transpose_gather_dual(src: Tensor, dim_list, H_all, W_all, H_low, W_low, hb1
         raise ValueError('src does not have prod(dim)*H_all*W_all elements')
     o1 = torch.empty(H_low, W_low, *dim_list, device=src.device, dtype=src.dtype)
     o2 = torch.empty_like(o1)
-    with torch.cuda.device(src.device):
+    with _device(src.device):
         _call('spgt_transpose_gather_dual', src.data_ptr(), o1.data_ptr(), o2.data_ptr(), dim, H_all, W_all, H_low, W_low,
                                              hb1, wb1, hb2, wb2, _stream())
     return o1, o2
@@ -276,7 +296,7 @@ def transpose_scatter_dual(src1: Tensor, src2: Tensor, dim_list, H_all, W_all, H
     if src1.numel() != dim * H_low * W_low or src2.numel() != src1.numel():
         raise ValueError('src1/src2 do not have H_low*W_low*prod(dim) elements')
     out = torch.empty(*dim_list, H_all, W_all, device=src1.device, dtype=src1.dtype)
-    with torch.cuda.device(src1.device):
+    with _device(src1.device):
         _call('spgt_transpose_scatter_dual', src1.data_ptr(), src2.data_ptr(), out.data_ptr(), dim, H_all, W_all,
                                               H_low, W_low, hb1, wb1, hb2, wb2, _stream())
     return out
@@ -308,7 +328,7 @@ def linear(x: Tensor, w_kn: Tensor, bias: Optional[Tensor], N: int, act=None, re
         out = torch.empty(*x.shape[:-1], N, device=x.device, dtype=x.dtype)
     if residual is not None:
         _chk(residual, 'residual')
-    with torch.cuda.device(x.device):
+    with _device(x.device):
         _call('spgt_linear_fwd', x.data_ptr(), K, w_kn.data_ptr(), w_kn.shape[1], _p(bias), _p(residual), N,
                                   out.data_ptr(), N, rows, K, N, act_code(act), _stream())
     return out
@@ -320,7 +340,7 @@ def conv3x3(x: Tensor, cin_off: int, Cin: int, w_kn: Tensor, bias: Tensor, y: Te
     B, Hh, Ww, cp = x.shape
     if y.shape[:3] != x.shape[:3]:
         raise ValueError('x and y must share [B, H, W]')
-    with torch.cuda.device(x.device):
+    with _device(x.device):
         _call('spgt_conv3x3_fwd', x.data_ptr(), cp, cin_off, Cin, w_kn.data_ptr(), w_kn.shape[1], bias.data_ptr(),
                                    y.data_ptr(), y.shape[3], cout_off, Cout, B, Hh, Ww, act_code(act), _stream())
     return y
@@ -330,7 +350,7 @@ def bilinear(x: Tensor, Ho: int, Wo: int, act=None) -> Tensor:
     _chk(x, 'x')
     B, Hi, Wi, Cc = x.shape
     y = torch.empty(B, Ho, Wo, Cc, device=x.device, dtype=x.dtype)
-    with torch.cuda.device(x.device):
+    with _device(x.device):
         _call('spgt_bilinear_fwd', x.data_ptr(), y.data_ptr(), B, Hi, Wi, Ho, Wo, Cc, act_code(act), _stream())
     return y
 
@@ -340,7 +360,7 @@ def bilinear_concat3(x1: Tensor, x2: Tensor, x3: Tensor, c1: int, c2: int, c3: i
     _chk(x1, 'x1'); _chk(x2, 'x2'); _chk(x3, 'x3')
     B, Hi, Wi, _ = x1.shape
     y = torch.empty(B, Ho, Wo, c1 + c2 + c3, device=x1.device, dtype=x1.dtype)
-    with torch.cuda.device(x1.device):
+    with _device(x1.device):
         _call('spgt_bilinear_concat3_fwd', x1.data_ptr(), x2.data_ptr(), x3.data_ptr(), x1.shape[3], x2.shape[3], x3.shape[3],
               c1, c2, c3, y.data_ptr(), B, Hi, Wi, Ho, Wo, act_code(act), _stream())
     return y
@@ -352,7 +372,7 @@ def conv0_down(node: Tensor, w9: Tensor, bias: Tensor, Ho: int, Wo: int, act) ->
     B, Hi, Wi = node.shape
     Cout = w9.shape[1]
     y = torch.empty(B, Ho, Wo, Cout, device=node.device, dtype=node.dtype)
-    with torch.cuda.device(node.device):
+    with _device(node.device):
         _call('spgt_conv0_down_fwd', node.data_ptr(), w9.data_ptr(), bias.data_ptr(), y.data_ptr(), B, Hi, Wi, Ho, Wo, Cout,
                                       act_code(act), _stream())
     return y
@@ -362,7 +382,7 @@ def upsample_grid(uw: Tensor, grid: Tensor, wg: Tensor, bias: Tensor, Ho: int, W
     _chk(uw, 'uw'); _chk(grid, 'grid'); _chk(wg, 'wg'); _chk(bias, 'bias')
     B, Hi, Wi, Cc = uw.shape
     y = torch.empty(B, Ho, Wo, Cc, device=uw.device, dtype=uw.dtype)
-    with torch.cuda.device(uw.device):
+    with _device(uw.device):
         _call('spgt_upsample_grid_fwd', uw.data_ptr(), grid.data_ptr(), wg.data_ptr(), bias.data_ptr(), y.data_ptr(),
                                          B, Hi, Wi, Ho, Wo, Cc, _stream())
     return y
@@ -375,7 +395,7 @@ def decoder_head(x: Tensor, w1_kn: Tensor, b1: Tensor, w2: Tensor, b2: float, sc
     _chk(x, 'x'); _chk(w1_kn, 'w1'); _chk(b1, 'b1'); _chk(w2, 'w2')
     B, Hh, Ww, K = x.shape
     out = torch.empty(B, Hh, Ww, 1, device=x.device, dtype=x.dtype)
-    with torch.cuda.device(x.device):
+    with _device(x.device):
         _call('spgt_decoder_head_fwd', x.data_ptr(), w1_kn.data_ptr(), b1.data_ptr(), w2.data_ptr(), float(b2), float(scale),
                                         float(shift), _p(scale_map), _p(shift_map), int(dirichlet), out.data_ptr(), B, Hh, Ww, K, w1_kn.shape[1],
                                         act_code(act), _stream())
@@ -393,7 +413,7 @@ class TcWeight:
         self.K, self.N = w_kn.shape
         n = int(lib.spgt_tc_weight_bytes(self.K, self.N))
         self.buf = torch.empty(n, dtype=torch.uint8, device=w_kn.device)
-        with torch.cuda.device(w_kn.device):
+        with _device(w_kn.device):
             _call('spgt_tc_weight_prepare', w_kn.data_ptr(), w_kn.shape[1], self.K, self.N, self.buf.data_ptr(), n, _stream())
 
     def data_ptr(self) -> int:
@@ -423,7 +443,7 @@ def linear_tc(x: Tensor, w: TcWeight, bias: Optional[Tensor], act=None, residual
     out = torch.empty(*x.shape[:-1], w.N, device=x.device, dtype=x.dtype)
     if residual is not None:
         _chk(residual, 'residual')
-    with torch.cuda.device(x.device):
+    with _device(x.device):
         _call('spgt_linear_tc_fwd', x.data_ptr(), K, w.data_ptr(), _p(bias), _p(residual), w.N, out.data_ptr(), w.N,
               rows, K, w.N, act_code(act), _stream())
     return out
@@ -439,7 +459,7 @@ def ffn_tc(x: Tensor, w1: TcWeight, b1: Tensor, w2: TcWeight, b2: Optional[Tenso
     out = torch.empty_like(x)
     if residual is not None:
         _chk(residual, 'residual')
-    with torch.cuda.device(x.device):
+    with _device(x.device):
         _call('spgt_ffn_tc_fwd', x.data_ptr(), D, w1.data_ptr(), b1.data_ptr(), w2.data_ptr(), _p(b2), _p(residual), D,
               out.data_ptr(), D, rows, D, w1.N, act_code(act), _stream())
     return out
@@ -450,7 +470,7 @@ def conv3x3_tc(x: Tensor, cin_off: int, Cin: int, w: TcWeight, bias: Tensor, y: 
     B, Hh, Ww, cp = x.shape
     if w.K != 9 * Cin or w.N != Cout:
         raise ValueError('prepared weight does not match [9*Cin, Cout]')
-    with torch.cuda.device(x.device):
+    with _device(x.device):
         _call('spgt_conv3x3_tc_fwd', x.data_ptr(), cp, cin_off, Cin, w.data_ptr(), bias.data_ptr(), y.data_ptr(), y.shape[3],
               cout_off, Cout, B, Hh, Ww, act_code(act), _stream())
     return y
@@ -460,7 +480,7 @@ def projpos_qkv_tc(x, wqkv: TcWeight, bq, bk, bv, lnwk, lnbk, lnwv, lnbv, eps, p
     _chk(x, 'x'); _chk(position, 'position')
     B, S, D = x.shape
     q, k, v = (torch.empty(B, num_head, dim_position + dim_head, S, device=x.device, dtype=x.dtype) for _ in range(3))
-    with torch.cuda.device(x.device):
+    with _device(x.device):
         _call('spgt_projpos_qkv_tc_fwd', x.data_ptr(), wqkv.data_ptr(), _p(bq), _p(bk), _p(bv), lnwk.data_ptr(), lnbk.data_ptr(),
               lnwv.data_ptr(), lnbv.data_ptr(), float(eps), position.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(),
               B, S, D, num_head, dim_head, dim_position, _stream())
@@ -472,7 +492,7 @@ def decoder_head_tc(x: Tensor, w1: TcWeight, b1: Tensor, w2: Tensor, b2: float, 
     _chk(x, 'x'); _chk(b1, 'b1'); _chk(w2, 'w2')
     B, Hh, Ww, K = x.shape
     out = torch.empty(B, Hh, Ww, 1, device=x.device, dtype=x.dtype)
-    with torch.cuda.device(x.device):
+    with _device(x.device):
         _call('spgt_decoder_head_tc_fwd', x.data_ptr(), w1.data_ptr(), b1.data_ptr(), w2.data_ptr(), float(b2), float(scale),
               float(shift), _p(scale_map), _p(shift_map), int(dirichlet), out.data_ptr(), B, Hh, Ww, K, w1.N,
               act_code(act), _stream())
@@ -493,7 +513,7 @@ def spectral_tables(r: int, m: int, device) -> Tensor:
         if n == 0:
             raise ValueError(f'unsupported spectral shape r={r}, m={m}')
         t = torch.empty(n, device=device, dtype=torch.uint8)
-        with torch.cuda.device(device):
+        with _device(torch.device(device)):
             _call('spgt_spectral_tables_init', t.data_ptr(), n, r, m, _stream())
         _TABLES[key] = t
     return _TABLES[key]
@@ -513,9 +533,51 @@ def spectral_conv2d(x: Tensor, wr_kn: Tensor, br: Tensor, fw0: Tensor, fw1: Tens
     if workspace is None:
         workspace = torch.empty(need, device=x.device, dtype=torch.uint8)
     y = torch.empty_like(x)
-    with torch.cuda.device(x.device):
+    with _device(x.device):
         _call('spgt_spectral_conv2d_fwd', x.data_ptr(), wr_kn.data_ptr(), br.data_ptr(), fw0.data_ptr(), fw1.data_ptr(),
                                            tab.data_ptr(), workspace.data_ptr(), workspace.numel(), y.data_ptr(),
                                            B, r, Cc, mode, act_code(act), _stream(),
               kernels=int(lib.spgt_spectral_launches(B, r, mode)))
     return y
+
+
+# ---------------------------------------------------------------------------------------------------------
+# the whole model
+# ---------------------------------------------------------------------------------------------------------
+class DarcyPlan:
+    """A spgt_darcy_model with the tensors it points to."""
+
+    def __init__(self, model, keep):
+        self.model, self.keep, self.address = model, keep, ctypes.addressof(model)
+        self.sizes = {}          # batch -> (workspace bytes, kernels launched)
+
+    def size(self, B: int):
+        hit = self.sizes.get(B)
+        if hit is None:
+            hit = self.sizes[B] = (int(lib.spgt_darcy_workspace_bytes(self.address, B)), int(lib.spgt_darcy_launches(self.address, B)))
+            if hit[0] == 0:
+                raise ValueError(f'unsupported model sizes at batch {B}')
+        return hit
+
+
+def darcy_forward(plan: DarcyPlan, node: Tensor, position: Tensor, grid: Tensor, taps: Optional[dict] = None) -> Tensor:
+    """node [B,r,r,1], position [B,ra,ra,d_pos], grid [B,r,r,2] -> [B,r,r,1]; `taps` receives intermediate tensors."""
+    m = plan.model
+    B, r, S = node.shape[0], m.r, m.ra * m.ra
+    node, position, grid = _chk(node.contiguous(), 'node'), _chk(position.contiguous(), 'position'), _chk(grid.contiguous(), 'grid')
+    if node.numel() != B * r * r or position.numel() != B * S * m.d_pos or grid.numel() != 2 * B * r * r:
+        raise ValueError('node, position and grid do not match the model\'s grids')
+    need, kernels = plan.size(B)
+    with _device(node.device):
+        out = torch.empty(B, r, r, 1, device=node.device, dtype=node.dtype)
+        workspace = torch.empty(need, device=node.device, dtype=torch.uint8)
+        want = None
+        if taps is not None:
+            new = lambda *shape: torch.empty(*shape, device=node.device, dtype=node.dtype)
+            taps['down'] = new(B, m.ra, m.ra, 128)
+            taps.update({f'enc{i}': new(B, S, 128) for i in range(m.n_encoder)}, up_mid=new(B, m.mid, m.mid, 128))
+            ptrs = [taps['down'], *(taps[f'enc{i}'] for i in range(m.n_encoder)), taps['up_mid']]
+            want = (ctypes.c_void_p * len(ptrs))(*(t.data_ptr() for t in ptrs))
+        _call('spgt_darcy_forward', plan.address, node.data_ptr(), position.data_ptr(), grid.data_ptr(), out.data_ptr(), B, want,
+              workspace.data_ptr(), need, _stream(), kernels=kernels)
+    return out
