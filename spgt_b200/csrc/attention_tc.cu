@@ -88,7 +88,7 @@ galerkin_attn_tc_kernel(const float* __restrict__ Q, const float* __restrict__ K
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_mem + 256);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_mem + 264);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = (int)tc_uniform(tid >> 5), lane = tid & 31;
     const uint32_t C = cluster_nctarank();
     const uint32_t rank = cluster_ctarank();
     const int64_t bh = blockIdx.x / C;
@@ -123,7 +123,7 @@ galerkin_attn_tc_kernel(const float* __restrict__ Q, const float* __restrict__ K
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = tc_uniform(*tmem_slot);
     constexpr uint32_t idesc = tc_idesc(AT_NP);
 
     // ============================== phase A: partial T over my columns ==============================
@@ -253,18 +253,19 @@ galerkin_attn_tc_kernel(const float* __restrict__ Q, const float* __restrict__ K
             mbar_arrive(op_full(so));
         }
     } else {
-        // Two issuing warps (one thread issues an MMA only about every 54 cycles; a 128 x 48 x 8 MMA takes 24): warp 8
+        // Two issuing warps: warp 8
         // multiplies k-steps 0-1 of every sub-tile into the accumulator at column 0, warp 9 k-steps 2-3 into the one at
         // column 48; the two partial sums are added when T is read out.
         const int iw = warp - 8;
         const uint32_t d = tmem_base + (uint32_t)(iw * AT_NP);
+        if (tc_elect())
         for (int it = 0; it < nmine; ++it) {
             const uint32_t so = (uint32_t)(it & 1), po = (uint32_t)((it >> 1) & 1);
             if (it > 0 && it % AT_FLUSH == 0 &&
                 !mbar_wait(acc_free, (uint32_t)((it / AT_FLUSH - 1) & 1), abort_flag, 10, &g_attn_status)) break;   // the flushed accumulator has been read
             if (!mbar_wait(op_full(so), po, abort_flag, 3, &g_attn_status)) break;
             tc_fence_after();
-            if (lane == 0) {
+            {
                 const uint32_t vhi = smem_base + AT_OP_OFF + so * (2 * AT_TILE);
                 const uint64_t dbh = tc_smem_desc(vhi), dbl = tc_smem_desc(vhi + AT_TILE);
 #pragma unroll
@@ -279,8 +280,8 @@ galerkin_attn_tc_kernel(const float* __restrict__ Q, const float* __restrict__ K
                 tc_commit(op_empty(so));
                 if (it == nmine - 1 || (it + 1) % AT_FLUSH == 0) tc_commit(t_done);
             }
-            __syncwarp();
         }
+        __syncwarp();
     }
 
     // ============================== reduce T over the cluster ==============================
@@ -461,12 +462,13 @@ galerkin_attn_tc_kernel(const float* __restrict__ Q, const float* __restrict__ K
             __syncwarp();
         }
     } else if (warp == 8) {
+        if (tc_elect())
         for (int it = 0; it < ntile; ++it) {
             const uint32_t sa = (uint32_t)(it & 1), ph = (uint32_t)((it >> 1) & 1);
             if (!mbar_wait(d_empty(sa), ph ^ 1, abort_flag, 7, &g_attn_status)) break;
             if (!mbar_wait(a2_full(sa), ph, abort_flag, 8, &g_attn_status)) break;
             tc_fence_after();
-            if (lane == 0) {
+            {
                 const uint32_t d = tmem_base + sa * AT_NP;
 #pragma unroll
                 for (int k8 = 0; k8 < 5; ++k8) {
@@ -481,8 +483,8 @@ galerkin_attn_tc_kernel(const float* __restrict__ Q, const float* __restrict__ K
                 tc_commit(a2_empty(sa));
                 tc_commit(d_full(sa));
             }
-            __syncwarp();
         }
+        __syncwarp();
     }
     tc_fence_before();
     cluster_sync_all();        // keep Tc alive until every CTA of the cluster has read it; all tensor-memory work is done

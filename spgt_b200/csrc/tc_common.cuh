@@ -64,6 +64,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// Issuing MMAs.  The operands of tcgen05.mma are warp-uniform, and the compiler only keeps them in uniform registers when it can
+// see that: the warp index and the tensor-memory base go through tc_uniform (a shuffle from lane 0), and the whole issue loop
+// runs in one branch guarded by tc_elect.  Measured with operands in tensor memory, cycles per 128 x N x 8 tf32 MMA: N = 48 / 64 /
+// 128 / 256: 24 / 32 / 64 / 128 (N / 2, the tensor pipe's rate) against 66 / 64 / 78 / 140 when a lane chosen by `lane == 0` or by
+// a predicate issues.  With A in shared memory as well: max(N / 2, 32 + N / 4).
+__device__ __forceinline__ uint32_t tc_elect() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p;
+}
+__device__ __forceinline__ uint32_t tc_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -94,35 +105,6 @@ __device__ __forceinline__ void tc_mma_tf32_ts_p(uint32_t d_tmem, uint32_t a_tme
         "mov.b64 bd, {%2, %3};\n\t"
         "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], bd, %4, p;\n\t}"
         ::"r"(d_tmem), "r"(a_tmem), "r"(b_desc_lo), "r"(b_desc_hi), "r"(idesc), "r"(accumulate) : "memory");
-}
-// The same three, executed by a whole warp with one issuing lane: `leader` is non-zero in that lane only.  The warp stays
-// converged around them (the guard is a predicate, not a branch).
-__device__ __forceinline__ void tc_mma_tf32_ts_acc_w(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_desc_lo, uint32_t b_desc_hi, uint32_t idesc,
-                                                     uint32_t leader) {
-    asm volatile(
-        "{\n\t.reg .pred p, g;\n\t.reg .b64 bd;\n\t"
-        "setp.eq.u32 p, 1, 1;\n\t"
-        "setp.ne.b32 g, %5, 0;\n\t"
-        "mov.b64 bd, {%2, %3};\n\t"
-        "@g tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], bd, %4, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "r"(b_desc_lo), "r"(b_desc_hi), "r"(idesc), "r"(leader) : "memory");
-}
-__device__ __forceinline__ void tc_mma_tf32_ts_p_w(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_desc_lo, uint32_t b_desc_hi, uint32_t idesc,
-                                                   uint32_t accumulate, uint32_t leader) {
-    asm volatile(
-        "{\n\t.reg .pred p, g;\n\t.reg .b64 bd;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "setp.ne.b32 g, %6, 0;\n\t"
-        "mov.b64 bd, {%2, %3};\n\t"
-        "@g tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], bd, %4, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "r"(b_desc_lo), "r"(b_desc_hi), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
-}
-__device__ __forceinline__ void tc_commit_w(uint32_t bar, uint32_t leader) {
-    asm volatile(
-        "{\n\t.reg .pred g;\n\t"
-        "setp.ne.b32 g, %1, 0;\n\t"
-        "@g tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-        ::"r"(bar), "r"(leader) : "memory");
 }
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
     uint32_t* u = reinterpret_cast<uint32_t*>(v);

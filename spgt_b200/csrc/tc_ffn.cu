@@ -53,7 +53,7 @@ tc_ffn_kernel(const float* __restrict__ x, int lda, const float* __restrict__ w1
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_mem + 192);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_mem + 200);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = (int)tc_uniform(tid >> 5), lane = tid & 31;
     if (tid == 0) {
         for (int s = 0; s < 2; ++s) { mbar_init(a_full(s), 128); mbar_init(a_empty(s), 1); }
         for (int s = 0; s < FF_NW; ++s) { mbar_init(w_full(s), 1); mbar_init(w_empty(s), 1); }
@@ -71,7 +71,7 @@ tc_ffn_kernel(const float* __restrict__ x, int lda, const float* __restrict__ w1
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = tc_uniform(*tmem_slot);
     const int n_my = ((int)blockIdx.x < n_tiles_m) ? (n_tiles_m - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
 
     if (warp < 4) {
@@ -178,6 +178,7 @@ tc_ffn_kernel(const float* __restrict__ x, int lda, const float* __restrict__ w1
         uint32_t sw = 0, pw = 0;
         bool alive = true;
         auto wadv = [&]() { if (++sw == FF_NW) { sw = 0; pw ^= 1u; } };
+        if (tc_elect())
         for (int ti = 0; ti < n_my && alive; ++ti) {
             const uint32_t tph = (uint32_t)(ti & 1);
             // GEMM1 into D1 (free once the converters have read the previous tile's hidden values)
@@ -191,7 +192,7 @@ tc_ffn_kernel(const float* __restrict__ x, int lda, const float* __restrict__ w1
                 if (!mbar_wait(w_full(s_hi), p_hi, abort_flag, 27, &g_ffn_status)) { alive = false; break; }
                 if (!mbar_wait(w_full(s_lo), p_lo, abort_flag, 27, &g_ffn_status)) { alive = false; break; }
                 tc_fence_after();
-                if (lane == 0) {
+                {
                     const uint64_t dbh = tc_smem_desc(smem_base + s_hi * FF_WSLOT), dbl = tc_smem_desc(smem_base + s_lo * FF_WSLOT);
                     const uint32_t ah0 = tmem_base + FF_A + sa * 64;
 #pragma unroll
@@ -207,7 +208,6 @@ tc_ffn_kernel(const float* __restrict__ x, int lda, const float* __restrict__ w1
                     tc_commit(w_empty(s_lo));
                     if (kb == FF_KB1 - 1) tc_commit(d1_full);
                 }
-                __syncwarp();
             }
             if (!alive) break;
             // GEMM2 into D2 (free once the previous tile's epilogue has read it)
@@ -219,7 +219,7 @@ tc_ffn_kernel(const float* __restrict__ x, int lda, const float* __restrict__ w1
                 const uint32_t s_w = sw, p_w = pw; wadv();
                 if (!mbar_wait(w_full(s_w), p_w, abort_flag, 30, &g_ffn_status)) { alive = false; break; }
                 tc_fence_after();
-                if (lane == 0) {
+                {
                     const uint32_t b_hi = smem_base + s_w * FF_WSLOT;
                     const uint64_t dbh = tc_smem_desc(b_hi), dbl = tc_smem_desc(b_hi + FF_WSLOT / 2);
                     const uint32_t ah0 = tmem_base + FF_A + sa * 64;
@@ -235,9 +235,9 @@ tc_ffn_kernel(const float* __restrict__ x, int lda, const float* __restrict__ w1
                     tc_commit(w_empty(s_w));
                     if (kb == FF_KB2 - 1) tc_commit(d2_full);
                 }
-                __syncwarp();
             }
         }
+        __syncwarp();
     } else {
         // ------------------------------------------ hidden converters + epilogue ------------------------------------------
         const int q = warp & 3, half = (warp - FF_EPI_WARP0) >> 2;

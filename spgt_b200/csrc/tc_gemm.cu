@@ -312,7 +312,7 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_mem + 352);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_mem + 360);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = (int)tc_uniform(tid >> 5), lane = tid & 31;
     const int KB = kpad / TC_BK;
     const int KBA = Loader::CONST_A ? KB - 1 : KB;                   // k-blocks whose A operand passes through the rings
     const bool resident = !Loader::W_PER_UNIT && KB <= SB;          // the whole column tile of W stays in shared memory
@@ -359,7 +359,7 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = tc_uniform(*tmem_slot);
     const uint32_t tmem_a = tmem_base + C::ACC_COLS;
     const uint32_t tmem_c = tmem_a + SA * MT * 64;                   // the constant A k-block, 64 columns (hi|lo) per tile
     if constexpr (Loader::CONST_A) {
@@ -581,10 +581,8 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
         __syncwarp();
     } else if (warp < TC_MMA_WARP + NIWARPS) {
         // ------------------------------------------ MMA issuers ------------------------------------------
-        // One thread issues a tcgen05.mma about every 54 cycles, while a 128 x 64 x 8 tf32 MMA occupies the tensor
-        // pipe for 32 cycles (128 x 128 x 8: 64), so a single issuing thread can starve the pipe.  With two row tiles
-        // per unit (MT == 2) two warps issue concurrently, one tile (its own accumulator) each; both wait on the same
-        // full barriers and the empty / accumulator barriers expect one commit from each.
+        // Two row tiles per unit (MT == 2): two warps, one tile (its own accumulator) each; both wait on the same full barriers
+        // and the empty / accumulator barriers expect one commit from each.
         const int iw = warp - TC_MMA_WARP;
         constexpr int NI = BN;                                              // N of one instruction
         {
@@ -592,10 +590,9 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
         const uint32_t d_off = (MT == 2) ? (uint32_t)(iw * C::ACCW) : (uint32_t)(iw * NI);
         const uint32_t a_off = (MT == 2) ? (uint32_t)(iw * 64) : 0u;
         const uint32_t b_off = (MT == 2) ? 0u : (uint32_t)(iw * NI * 128);   // NI rows of 128 bytes
-        // Only lane 0 runs the loop (waits included): no divergence and reconvergence per k-block.  The B descriptors
-        // differ between stages only in the address field of their low word, so they are advanced with 32-bit adds.
-        {
-            const uint32_t leader = lane == 0 ? 1u : 0u;      // the whole warp runs the loop, this lane issues
+        // One elected thread runs the loop, waits included.  The B descriptors differ between stages only in the address field of
+        // their low word, so they are advanced with 32-bit adds.
+        if (tc_elect()) {
             const uint64_t desc0 = tc_smem_desc(smem_base + b_off);
             const uint32_t desc_hi = (uint32_t)(desc0 >> 32), desc_lo0 = (uint32_t)desc0;
             TcRing ra, rb;
@@ -628,31 +625,31 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
                     if constexpr (C::MERGE) {
                         constexpr uint32_t idesc2 = tc_idesc(2 * NI);           // [W_hi | W_lo] as one operand of twice the rows
                         const int nk8 = (Loader::CONST_A && !a_ring) ? ld.const_ksteps() : TC_BK / 8;   // (zero k-steps of the constant block are skipped)
-                        tc_mma_tf32_ts_p_w(d, ah, bh, desc_hi, idesc2, ki > 0 ? 1u : 0u, leader);
-                        tc_mma_tf32_ts_acc_w(d, al, bh, desc_hi, idesc, leader);
+                        tc_mma_tf32_ts_p(d, ah, bh, desc_hi, idesc2, ki > 0 ? 1u : 0u);
+                        tc_mma_tf32_ts_acc(d, al, bh, desc_hi, idesc);
 #pragma unroll
                         for (int k8 = 1; k8 < TC_BK / 8; ++k8) {
                             if (k8 < nk8) {
-                                tc_mma_tf32_ts_acc_w(d, ah + k8 * 8, bh + k8 * 2, desc_hi, idesc2, leader);
-                                tc_mma_tf32_ts_acc_w(d, al + k8 * 8, bh + k8 * 2, desc_hi, idesc, leader);
+                                tc_mma_tf32_ts_acc(d, ah + k8 * 8, bh + k8 * 2, desc_hi, idesc2);
+                                tc_mma_tf32_ts_acc(d, al + k8 * 8, bh + k8 * 2, desc_hi, idesc);
                             }
                         }
                     } else {
-                    tc_mma_tf32_ts_p_w(d, al, bh, desc_hi, idesc, ki > 0 ? 1u : 0u, leader);
-                    tc_mma_tf32_ts_acc_w(d, ah, bl, desc_hi, idesc, leader);
-                    tc_mma_tf32_ts_acc_w(d, ah, bh, desc_hi, idesc, leader);
+                    tc_mma_tf32_ts_p(d, al, bh, desc_hi, idesc, ki > 0 ? 1u : 0u);
+                    tc_mma_tf32_ts_acc(d, ah, bl, desc_hi, idesc);
+                    tc_mma_tf32_ts_acc(d, ah, bh, desc_hi, idesc);
 #pragma unroll
                     for (int k8 = 1; k8 < TC_BK / 8; ++k8) {          // 32 bytes (2 descriptor units) and 8 TMEM columns per k-step
-                        tc_mma_tf32_ts_acc_w(d, al + k8 * 8, bh + k8 * 2, desc_hi, idesc, leader);
-                        tc_mma_tf32_ts_acc_w(d, ah + k8 * 8, bl + k8 * 2, desc_hi, idesc, leader);
-                        tc_mma_tf32_ts_acc_w(d, ah + k8 * 8, bh + k8 * 2, desc_hi, idesc, leader);
+                        tc_mma_tf32_ts_acc(d, al + k8 * 8, bh + k8 * 2, desc_hi, idesc);
+                        tc_mma_tf32_ts_acc(d, ah + k8 * 8, bl + k8 * 2, desc_hi, idesc);
+                        tc_mma_tf32_ts_acc(d, ah + k8 * 8, bh + k8 * 2, desc_hi, idesc);
                     }
                     }
                     // the A stage (and a streamed W stage) is reusable once every issuer's MMAs have read it
-                    if (a_ring) { tc_commit_w(a_empty(sa), leader); ra.template next<SA>(); }
-                    if (!resident && !tail) { tc_commit_w(b_empty(sb), leader); rb.template next<SBR>(); }
+                    if (a_ring) { tc_commit(a_empty(sa)); ra.template next<SA>(); }
+                    if (!resident && !tail) { tc_commit(b_empty(sb)); rb.template next<SBR>(); }
                 }
-                if (alive) tc_commit_w(acc_full(buf), leader);
+                if (alive) tc_commit(acc_full(buf));
             }
         }
         __syncwarp();
