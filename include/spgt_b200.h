@@ -312,14 +312,26 @@ int spgt_spectral_conv2d_fwd(const float* x, const float* wr, const float* br, c
 
 #define SPGT_MAX_LAYERS 32
 
-/* One encoder layer (network/sp_layer.py:94-104): weights as the single-op entry points above take them. */
+/* One encoder layer of width 128 with 4 heads and two position values (network/sp_layer.py:94-104). */
 typedef struct {
-    const void* wqkv;                                        /* spgt_tc_weight_prepare of Wq | Wk | Wv [128, 384] */
-    const float *bq, *bk, *bv, *lnwk, *lnbk, *lnwv, *lnbv;
-    const void* wfc; const float* bfc;                       /* [128 + 4 d_pos, 128] */
-    const void* w1; const float* b1;                         /* [128, 256] */
-    const void* w2; const float* b2;                         /* [256, 128] */
+    const void* wkv;                 /* spgt_tc_weight_prepare of [128, 256]: Wk heads 0-1 | Wv heads 0-1 | Wk heads 2-3 | Wv heads 2-3,
+                                        every row of a head less its mean over the head's 32 channels */
+    const float* wq;                 /* [128][128], used as [k][n] */
+    const float *bq, *bk, *bv;       /* [128] or NULL */
+    const float *lnwk, *lnbk, *lnwv, *lnbv;
+    const float *wfc, *bfc;          /* output projection as torch keeps it: [128 out][136 in], [128] or NULL */
+    const void* w1; const float* b1; /* prepared [128, 256] */
+    const void* w2; const float* b2; /* prepared [256, 128], [128] or NULL */
 } spgt_encoder_weights;
+
+/* Bytes of scratch a layer of B samples of S grid nodes needs (0: unsupported sizes). */
+size_t spgt_encoder_workspace_bytes(int B, int S);
+/* y = a + (ffn ? act(a w1 + b1) w2 + b2 : 0)  with  a = (residual || ffn ? x : 0) + attention(x, pos) wfc + bfc.
+ * x, y [B,S,128] (y may be x), pos [B,S,2].  Three launches: K / V projection + LayerNorm + T = [pos K]^T [pos V] / S without K or V
+ * reaching memory; T, wq and wfc folded into one 128 x 128 matrix per sample (q is linear in x, so attention(x) wfc is too); x
+ * through that matrix and the feed-forward block.  Replaces Sp_EncoderLayer.forward / Sp_GalerkinAttention.forward. */
+int spgt_encoder_layer_fwd(const spgt_encoder_weights* w, const float* x, const float* pos, float* y, int B, int S, float eps, int act, int ffn,
+                           int residual, void* workspace, size_t workspace_bytes, spgt_stream_t stream);
 
 /* One spectral layer: as spgt_spectral_conv2d_fwd takes them. */
 typedef struct { const float *wr, *br, *fw0, *fw1; } spgt_spectral_weights;

@@ -28,7 +28,7 @@ MAX_LAYERS = 32
 
 
 class EncoderWeights(C.Structure):          # spgt_encoder_weights
-    _fields_ = [(n, _f) for n in ('wqkv', 'bq', 'bk', 'bv', 'lnwk', 'lnbk', 'lnwv', 'lnbv', 'wfc', 'bfc', 'w1', 'b1', 'w2', 'b2')]
+    _fields_ = [(n, _f) for n in ('wkv', 'wq', 'bq', 'bk', 'bv', 'lnwk', 'lnbk', 'lnwv', 'lnbv', 'wfc', 'bfc', 'w1', 'b1', 'w2', 'b2')]
 
 
 class SpectralWeights(C.Structure):         # spgt_spectral_weights
@@ -90,6 +90,8 @@ SIGNATURES = {
     'spgt_spectral_workspace_bytes': (_sz, [_i, _i, _i, _i]),
     'spgt_spectral_chunk_samples': (_i, [_i]),
     'spgt_spectral_launches': (_i, [_i, _i, _i]),
+    'spgt_encoder_workspace_bytes': (_sz, [_i, _i]),
+    'spgt_encoder_layer_fwd': (_i, [_f] * 4 + [_i, _i, _fl, _i, _i, _i, _f, _sz, _st]),
     'spgt_darcy_workspace_bytes': (_sz, [_f, _i]),
     'spgt_darcy_launches': (_i, [_f, _i]),
     'spgt_darcy_forward': (_i, [_f] * 5 + [_i, _f, _f, _sz, _st]),

@@ -7,26 +7,25 @@ namespace spgt {
 
 static int pad4(int c) { return (c + 3) & ~3; }
 
-// Workspace: two encoder activations that outlive the phases, then one region that the phases (down-scaler, encoder layer,
+// Workspace: the encoder's activations, which outlive the phases, then one region that the phases (down-scaler, encoder layer,
 // up-scaler + decoder) reuse one after the other.  Offsets in floats, each a multiple of 64 floats.
 struct DarcyPlan {
-    size_t xa[2], phase, total;
+    size_t xa, phase, total;
     size_t d0, d1, d2, d3;                      // down-scaler: conv0 output and the three convolution outputs
-    size_t q, k, v, att;                        // encoder layer
+    size_t es, es_bytes;                        // encoder layer scratch
     size_t up, uc, uw, y[2], ws, ws_bytes;      // up-scaler and decoder
 };
 
 static bool darcy_plan(const spgt_darcy_model* m, int B, DarcyPlan& p) {
     if (!m || B <= 0 || m->r <= 0 || m->mid <= 0 || m->ra <= 0 || m->n_encoder < 0 || m->n_decoder < 0) return false;
-    if (m->n_encoder > SPGT_MAX_LAYERS || m->n_decoder > SPGT_MAX_LAYERS || m->d_pos < 0 || m->d_pos > 8) return false;
+    if (m->n_encoder > SPGT_MAX_LAYERS || m->n_decoder > SPGT_MAX_LAYERS || m->d_pos != 2) return false;
     if (m->c1 <= 0 || m->c2 <= 0 || m->c3 <= 0 || m->c1 + m->c2 + m->c3 != 128) return false;
     const size_t b = (size_t)B, S = (size_t)m->ra * m->ra, M = (size_t)m->mid * m->mid, R = (size_t)m->r * m->r;
     p.ws_bytes = m->n_decoder > 0 ? spgt_spectral_workspace_bytes(B, m->r, m->modes, 32) : 0;
     if (m->n_decoder > 0 && p.ws_bytes == 0) return false;
     size_t at = 0;
     auto take = [&](size_t& off, size_t floats) { off = at; at += (floats + 63) & ~(size_t)63; };
-    take(p.xa[0], b * S * 128);
-    take(p.xa[1], b * S * 128);
+    take(p.xa, b * S * 128);
     p.phase = at;
     take(p.d0, b * M * 128);
     take(p.d1, b * M * pad4(m->c1));
@@ -34,8 +33,9 @@ static bool darcy_plan(const spgt_darcy_model* m, int B, DarcyPlan& p) {
     take(p.d3, b * M * pad4(m->c3));
     p.total = at;
     at = p.phase;
-    const size_t heads = b * S * 4 * (32 + m->d_pos);
-    take(p.q, heads); take(p.k, heads); take(p.v, heads); take(p.att, heads);
+    p.es_bytes = spgt_encoder_workspace_bytes(B, (int)S);
+    if (p.es_bytes == 0) return false;
+    take(p.es, (p.es_bytes + 3) / 4);
     if (at > p.total) p.total = at;
     at = p.phase;
     take(p.up, b * M * 128);
@@ -60,7 +60,7 @@ extern "C" size_t spgt_darcy_workspace_bytes(const spgt_darcy_model* m, int B) {
 extern "C" int spgt_darcy_launches(const spgt_darcy_model* m, int B) {
     DarcyPlan p;
     if (!darcy_plan(m, B, p)) return 0;
-    return 5 + 4 * m->n_encoder + 4 + m->n_decoder * spgt_spectral_launches(B, m->r, m->modes) + 1;
+    return 5 + 3 * m->n_encoder + 4 + m->n_decoder * spgt_spectral_launches(B, m->r, m->modes) + 1;
 }
 
 extern "C" int spgt_darcy_forward(const spgt_darcy_model* m, const float* node, const float* position, const float* grid, float* out,
@@ -71,7 +71,7 @@ extern "C" int spgt_darcy_forward(const spgt_darcy_model* m, const float* node, 
     if (workspace_bytes < p.total * sizeof(float)) return SPGT_ERR_WORKSPACE;
     if (!aligned16(workspace)) return SPGT_ERR_ALIGN;
     float* ws = (float*)workspace;
-    const int mid = m->mid, ra = m->ra, r = m->r, S = ra * ra, D = 128, dpk = 32 + m->d_pos;
+    const int mid = m->mid, ra = m->ra, r = m->r, S = ra * ra, D = 128;
     const size_t xa_bytes = (size_t)B * S * D * sizeof(float);
     int rc;
 #define SPGT_TRY(call) if ((rc = (call)) != SPGT_OK) return rc
@@ -87,18 +87,14 @@ extern "C" int spgt_darcy_forward(const spgt_darcy_model* m, const float* node, 
     SPGT_TRY(spgt_conv3x3_tc_fwd(ws + p.d0, D, 0, D, m->conv_w[0], m->conv_b[0], ws + p.d1, p1, 0, p1, B, mid, mid, m->act_down, stream));
     SPGT_TRY(spgt_conv3x3_tc_fwd(ws + p.d1, p1, 0, p1, m->conv_w[1], m->conv_b[1], ws + p.d2, p2, 0, p2, B, mid, mid, m->act_down, stream));
     SPGT_TRY(spgt_conv3x3_tc_fwd(ws + p.d2, p2, 0, p2, m->conv_w[2], m->conv_b[2], ws + p.d3, p3, 0, p3, B, mid, mid, m->act_down, stream));
-    SPGT_TRY(spgt_bilinear_concat3_fwd(ws + p.d1, ws + p.d2, ws + p.d3, p1, p2, p3, m->c1, m->c2, m->c3, ws + p.xa[0], B, mid, mid, ra, ra,
+    SPGT_TRY(spgt_bilinear_concat3_fwd(ws + p.d1, ws + p.d2, ws + p.d3, p1, p2, p3, m->c1, m->c2, m->c3, ws + p.xa, B, mid, mid, ra, ra,
                                        m->act_down, stream));
-    SPGT_TRY(tap(0, ws + p.xa[0], xa_bytes));
+    SPGT_TRY(tap(0, ws + p.xa, xa_bytes));
     // encoder
-    float *x = ws + p.xa[0], *x2 = ws + p.xa[1];
+    float* x = ws + p.xa;
     for (int l = 0; l < m->n_encoder; ++l) {
         const spgt_encoder_weights& w = m->encoder[l];
-        SPGT_TRY(spgt_projpos_qkv_tc_fwd(x, w.wqkv, w.bq, w.bk, w.bv, w.lnwk, w.lnbk, w.lnwv, w.lnbv, m->eps, position, ws + p.q, ws + p.k,
-                                         ws + p.v, B, S, D, 4, 32, m->d_pos, stream));
-        SPGT_TRY(spgt_galerkin_attn_fwd(ws + p.q, ws + p.k, ws + p.v, ws + p.att, nullptr, B, 4, dpk, S, 1, stream));
-        SPGT_TRY(spgt_linear_tc_fwd(ws + p.att, 4 * dpk, w.wfc, w.bfc, x, D, x2, D, B * S, 4 * dpk, D, SPGT_ACT_NONE, stream));
-        SPGT_TRY(spgt_ffn_tc_fwd(x2, D, w.w1, w.b1, w.w2, w.b2, x2, D, x, D, B * S, D, 256, m->act_ffn, stream));
+        SPGT_TRY(spgt_encoder_layer_fwd(&w, x, position, x, B, S, m->eps, m->act_ffn, 1, 1, ws + p.es, p.es_bytes, stream));
         SPGT_TRY(tap(1 + l, x, xa_bytes));
     }
     // up-scaler (its last interpolation is fused with the decoder's spatial fc)

@@ -53,6 +53,22 @@ class Sp_GalerkinAttention(_KernelWeights):
     def fc_weight(self):
         return self._cached('fc', lambda: _linear_tc(self.fc_layer.weight))
 
+    def fill_native(self, w, ptr) -> None:
+        """Device pointers of this layer's weights into a spgt_encoder_weights; `ptr` keeps what it is given alive."""
+        w.wkv, w.wq = ptr(self.kv_weight()), ptr(self.weight_Q.detach())
+        w.wfc, w.bfc = ptr(self.fc_layer.weight.detach()), ptr(self.fc_layer.bias.detach())
+        w.bq, w.bk, w.bv = (ptr(b.detach()) for b in (self.bias_Q, self.bias_K, self.bias_V))
+        w.lnwk, w.lnbk, w.lnwv, w.lnbv = (ptr(t.detach()) for t in (self.ln_weight_K, self.ln_bias_K, self.ln_weight_V, self.ln_bias_V))
+
+    def kv_weight(self):
+        """K and V weights as the fused layer takes them: by head pair K0 K1 V0 V1 | K2 K3 V2 V3, less each head's channel mean (the
+        LayerNorm's subtraction, done once on the weights)."""
+        def make():
+            centred = lambda w: (h := w.detach().view(-1, self.num_head, self.dim_head)) - h.mean(dim=2, keepdim=True)
+            kv = torch.stack([centred(self.weight_K), centred(self.weight_V)], dim=1).view(-1, 2, 2, 64)      # [128, K | V, pair, 64]
+            return ops.TcWeight(kv.transpose(1, 2).reshape(-1, 256).contiguous())
+        return self._cached('wkv', make)
+
     def forward(self, Q: Tensor, K: Tensor, V: Tensor, position: Tensor, residual: Tensor = None) -> Tensor:
         """Q,K,V [N,S,D], position [N,S,d_pos] -> [N,S,D] (+ residual, fused into the output projection).
         When Q, K and V are the same tensor (self-attention) all three projections run in one launch."""
@@ -106,11 +122,8 @@ class Sp_EncoderLayer(torch.nn.Module):
         self.ffn_layer = FeedForward(dim_hidden, dim_hidden, ffn_dim_hidden, ffn_droprate, ffn_activation)
 
     def fill_native(self, w, ptr) -> None:
-        """Device pointers of this layer's weights into a spgt_encoder_weights; `ptr` keeps what it is given alive."""
         a, f = self.attention_layer, self.ffn_layer
-        w.wqkv, w.wfc, w.bfc = ptr(a.qkv_weight()), ptr(a.fc_weight()), ptr(a.fc_layer.bias.detach())
-        w.bq, w.bk, w.bv = (ptr(b.detach()) for b in (a.bias_Q, a.bias_K, a.bias_V))
-        w.lnwk, w.lnbk, w.lnwv, w.lnbv = (ptr(t.detach()) for t in (a.ln_weight_K, a.ln_bias_K, a.ln_weight_V, a.ln_bias_V))
+        a.fill_native(w, ptr)
         w1, w2 = f.tc_weights()
         w.w1, w.b1, w.w2, w.b2 = ptr(w1), ptr(f.layer1.bias.detach()), ptr(w2), ptr(f.layer2.bias.detach())
 
