@@ -271,6 +271,13 @@ int spgt_ffn_tc_fwd(const float* x, int lda, const void* w1prep, const float* b1
 int spgt_conv3x3_tc_fwd(const float* x, int cin_pitch, int cin_off, int Cin, const void* wprep, const float* bias,
                         float* y, int cout_pitch, int cout_off, int Cout, int B, int Hh, int Ww, int act,
                         spgt_stream_t stream);
+/* The same convolution for up to 128 output channels, from weights prepared by spgt_conv3x3_weight_prepare: every input value is
+ * split once per tile instead of once per tap.  w_kn [9 * Cin][ldw], row (ky * 3 + kx) * Cin + c.  bias NULL or [Cout]. */
+size_t spgt_conv3x3_weight_bytes(int Cin, int Cout);
+int spgt_conv3x3_weight_prepare(const float* w_kn, int ldw, int Cin, int Cout, void* out, size_t out_bytes, spgt_stream_t stream);
+int spgt_conv3x3_nhwc_fwd(const float* x, int cin_pitch, int cin_off, int Cin, const void* wprep, const float* bias, float* y, int cout_pitch,
+                          int cout_off, int Cout, int B, int Hh, int Ww, int act, spgt_stream_t stream);
+
 /* As spgt_projpos_qkv_fwd for D == 128, H == 4; wprep_qkv is prepared from the [128, 384] matrix Wq | Wk | Wv. */
 int spgt_projpos_qkv_tc_fwd(const float* x, const void* wprep_qkv, const float* bq, const float* bk, const float* bv,
                             const float* lnwk, const float* lnbk, const float* lnwv, const float* lnbv, float eps,

@@ -84,9 +84,9 @@ extern "C" int spgt_darcy_forward(const spgt_darcy_model* m, const float* node, 
     // down-scaler
     const int p1 = pad4(m->c1), p2 = pad4(m->c2), p3 = pad4(m->c3);
     SPGT_TRY(spgt_conv0_down_fwd(node, m->conv0_w, m->conv0_b, ws + p.d0, B, r, r, mid, mid, D, m->act_down, stream));
-    SPGT_TRY(spgt_conv3x3_tc_fwd(ws + p.d0, D, 0, D, m->conv_w[0], m->conv_b[0], ws + p.d1, p1, 0, p1, B, mid, mid, m->act_down, stream));
-    SPGT_TRY(spgt_conv3x3_tc_fwd(ws + p.d1, p1, 0, p1, m->conv_w[1], m->conv_b[1], ws + p.d2, p2, 0, p2, B, mid, mid, m->act_down, stream));
-    SPGT_TRY(spgt_conv3x3_tc_fwd(ws + p.d2, p2, 0, p2, m->conv_w[2], m->conv_b[2], ws + p.d3, p3, 0, p3, B, mid, mid, m->act_down, stream));
+    SPGT_TRY(spgt_conv3x3_nhwc_fwd(ws + p.d0, D, 0, D, m->conv_w[0], m->conv_b[0], ws + p.d1, p1, 0, p1, B, mid, mid, m->act_down, stream));
+    SPGT_TRY(spgt_conv3x3_nhwc_fwd(ws + p.d1, p1, 0, p1, m->conv_w[1], m->conv_b[1], ws + p.d2, p2, 0, p2, B, mid, mid, m->act_down, stream));
+    SPGT_TRY(spgt_conv3x3_nhwc_fwd(ws + p.d2, p2, 0, p2, m->conv_w[2], m->conv_b[2], ws + p.d3, p3, 0, p3, B, mid, mid, m->act_down, stream));
     SPGT_TRY(spgt_bilinear_concat3_fwd(ws + p.d1, ws + p.d2, ws + p.d3, p1, p2, p3, m->c1, m->c2, m->c3, ws + p.xa, B, mid, mid, ra, ra,
                                        m->act_down, stream));
     SPGT_TRY(tap(0, ws + p.xa, xa_bytes));
@@ -99,7 +99,7 @@ extern "C" int spgt_darcy_forward(const spgt_darcy_model* m, const float* node, 
     }
     // up-scaler (its last interpolation is fused with the decoder's spatial fc)
     SPGT_TRY(spgt_bilinear_fwd(x, ws + p.up, B, ra, ra, mid, mid, D, SPGT_ACT_NONE, stream));
-    SPGT_TRY(spgt_conv3x3_tc_fwd(ws + p.up, D, 0, D, m->up_w, m->up_b, ws + p.uc, D, 0, D, B, mid, mid, m->act_up, stream));
+    SPGT_TRY(spgt_conv3x3_nhwc_fwd(ws + p.up, D, 0, D, m->up_w, m->up_b, ws + p.uc, D, 0, D, B, mid, mid, m->act_up, stream));
     SPGT_TRY(tap(1 + m->n_encoder, ws + p.uc, (size_t)B * mid * mid * D * sizeof(float)));
     // decoder
     SPGT_TRY(spgt_linear_tc_fwd(ws + p.uc, D, m->fcx_w, nullptr, nullptr, 32, ws + p.uw, 32, B * mid * mid, D, 32, SPGT_ACT_NONE, stream));

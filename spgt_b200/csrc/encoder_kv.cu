@@ -34,14 +34,6 @@ constexpr int KV_CHAIN = 4;                                    // tiles whose pr
 // a channel lie 16 lanes apart in one warp's quarter of tensor memory.
 __device__ __forceinline__ constexpr int kv_tile_row(int c, int lo) { return (c >> 4) * 32 + (c & 15) + 16 * lo; }
 
-__device__ __forceinline__ void tc_mma_tf32_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-
 __global__ void __launch_bounds__(KV_THREADS, 1)
 encoder_kv_kernel(const float* __restrict__ x, const float* __restrict__ wkv_img, const float* __restrict__ bk, const float* __restrict__ bv,
                   float eps, const float* __restrict__ pos, float* __restrict__ partial, int S, EncoderSplit sp) {

@@ -1057,6 +1057,7 @@ namespace spgt {
 int attn_tc_status(); int ffn_tc_status();          // attention_tc.cu, tc_ffn.cu
 int attn_tc_status_reset(); int ffn_tc_status_reset();
 int encoder_kv_status(bool reset); int encoder_out_status(bool reset);     // encoder_kv.cu, encoder_out.cu
+int conv_status(bool reset);            // tc_conv.cu
 
 // One warp waits on a barrier that nobody arrives at, with a limit of `limit_us` microseconds instead of the two
 // seconds of the production kernels: the wait gives up, latches `code` in the status word and the kernel returns.
@@ -1084,6 +1085,7 @@ extern "C" int spgt_tc_status(void) {
     if (a != 0) return a > 0 ? 100 + a : a;     // 101..109: a wait of the attention kernel gave up
     if (int e = spgt::encoder_kv_status(false)) return e;       // 40..52: the first half of an encoder layer
     if (int e = spgt::encoder_out_status(false)) return e;      // 60..76: its second half
+    if (int e = spgt::conv_status(false)) return e;             // 80..86: the convolution kernel
     return spgt::ffn_tc_status();               // 21..33: a wait of the fused feed-forward kernel gave up
 }
 
@@ -1093,6 +1095,7 @@ extern "C" int spgt_tc_status_reset(void) {
     if (int e = spgt::attn_tc_status_reset()) return e;
     if (int e = spgt::encoder_kv_status(true)) return e;
     if (int e = spgt::encoder_out_status(true)) return e;
+    if (int e = spgt::conv_status(true)) return e;
     return spgt::ffn_tc_status_reset();
 }
 

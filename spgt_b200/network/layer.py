@@ -83,7 +83,8 @@ def _conv_tc(weight: Tensor, bias: Tensor, cin_pad: int, cout_pad: int):
     w[:cout, :cin] = weight.detach()
     b = torch.zeros(cout_pad, device=weight.device, dtype=weight.dtype)
     b[:cout] = bias.detach()
-    return ops.TcWeight(w.permute(2, 3, 1, 0).reshape(9 * cin_pad, cout_pad).contiguous()), b
+    w = w.permute(2, 3, 1, 0).reshape(9 * cin_pad, cout_pad).contiguous()
+    return (ops.ConvWeight(w, cin_pad) if cout_pad <= 128 else ops.TcWeight(w)), b
 
 
 class ConvResBlock2D(_KernelWeights):

@@ -53,6 +53,11 @@ class Sp_GalerkinAttention(_KernelWeights):
     def fc_weight(self):
         return self._cached('fc', lambda: _linear_tc(self.fc_layer.weight))
 
+    @property
+    def fusable(self) -> bool:
+        """Whether the fused layer kernels cover these widths."""
+        return self.dim_hidden == 128 and self.num_head == 4 and self.dim_position == 2
+
     def fill_native(self, w, ptr) -> None:
         """Device pointers of this layer's weights into a spgt_encoder_weights; `ptr` keeps what it is given alive."""
         w.wkv, w.wq = ptr(self.kv_weight()), ptr(self.weight_Q.detach())
@@ -74,6 +79,9 @@ class Sp_GalerkinAttention(_KernelWeights):
         When Q, K and V are the same tensor (self-attention) all three projections run in one launch."""
         d = lambda t: t.detach()
         H, dh, dp = self.num_head, self.dim_head, self.dim_position
+        if Q is K and K is V and self.fusable and (residual is None or residual is Q):
+            plan = self._cached('native', lambda: ops.EncoderPlan(self.fill_native))
+            return ops.encoder_layer(plan, Q, position, self.norm_eps, None, ffn=False, residual=residual is not None)
         if Q is K and K is V and self.dim_hidden == 128:
             q, k, v = ops.projpos_qkv_tc(
                 Q, self.qkv_weight(), d(self.bias_Q), d(self.bias_K), d(self.bias_V), d(self.ln_weight_K), d(self.ln_bias_K),
@@ -113,7 +121,7 @@ def _attention_forward_train(self, Q: Tensor, K: Tensor, V: Tensor, position: Te
 Sp_GalerkinAttention.forward_train = _attention_forward_train
 
 
-class Sp_EncoderLayer(torch.nn.Module):
+class Sp_EncoderLayer(_KernelWeights):
     def __init__(self, dim_hidden, num_head, dim_position, norm_eps, attn_droprate, fc_droprate, xavier, diagonal,
                  symmetric, ffn_dim_hidden, ffn_droprate, ffn_activation) -> None:
         super().__init__()
@@ -129,8 +137,18 @@ class Sp_EncoderLayer(torch.nn.Module):
 
     def forward(self, X: Tensor, position: Tensor) -> Tensor:
         """X [N,S,D], position [N,S,d_pos] -> X + attention(X) then + ffn(.)  (network/sp_layer.py:94-104)."""
+        f = self.ffn_layer
+        if self.fusable:
+            plan = self._cached('native', lambda: ops.EncoderPlan(self.fill_native))
+            return ops.encoder_layer(plan, X, position, self.attention_layer.norm_eps, f.activation)
         X = self.attention_layer(X, X, X, position, residual=X)
-        return self.ffn_layer(X, residual=X)
+        return f(X, residual=X)
+
+    @property
+    def fusable(self) -> bool:
+        f = self.ffn_layer
+        return (self.attention_layer.fusable and f.layer1.in_features == 128 and f.layer1.out_features == 256
+                and f.layer2.out_features == 128)
 
     def forward_train(self, X: Tensor, position: Tensor) -> Tensor:
         X = X + self.attention_layer.forward_train(X, X, X, position)

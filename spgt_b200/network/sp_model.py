@@ -231,8 +231,7 @@ class Sp_GalerkinTransformer2D(torch.nn.Module):
 
     def _native_widths(self) -> bool:
         enc, dec, up = self.encoder_mixer.layers, self.decoder_regressor, self.up_scaler
-        return (all(a.dim_hidden == 128 and a.num_head == 4 and f.layer1.out_features == 256 and f.layer1.in_features == 128
-                    and f.layer2.out_features == 128 for a, f in ((l.attention_layer, l.ffn_layer) for l in enc))
+        return (all(l.fusable for l in enc)
                 and up.conv.conv_layer.in_channels == 128 and up.conv.conv_layer.out_channels == 128 and dec.in_dim == 128
                 and dec.dim_position == 2 and dec.spatial_fc_layer.out_features == 32 and dec.ffn_layer.layer1.out_features == 128
                 and all(l.structure == 'fused' and l.in_dim == 32 and l.out_dim == 32 for l in dec.layers))

@@ -12,7 +12,7 @@ from typing import Optional, Sequence, Tuple
 import torch
 from torch import Tensor
 
-from ._lib import lib, check
+from ._lib import EncoderWeights, check, lib
 
 ACT = {None: 0, 'none': 0, 'relu': 1, 'silu': 2, 'silu2': 3}
 
@@ -420,6 +420,23 @@ class TcWeight:
         return self.buf.data_ptr()
 
 
+class ConvWeight:
+    """A [9 * Cin, Cout <= 128] weight (row (ky * 3 + kx) * Cin + c) prepared for conv3x3_tc."""
+
+    def __init__(self, w_kn: Tensor, Cin: int):
+        _chk(w_kn, 'weight')
+        if w_kn.shape[0] != 9 * Cin:
+            raise ValueError('weight must be [9 * Cin, Cout]')
+        self.K, self.N = w_kn.shape
+        n = int(lib.spgt_conv3x3_weight_bytes(Cin, self.N))
+        self.buf = torch.empty(n, dtype=torch.uint8, device=w_kn.device)
+        with _device(w_kn.device):
+            _call('spgt_conv3x3_weight_prepare', w_kn.data_ptr(), w_kn.shape[1], Cin, self.N, self.buf.data_ptr(), n, _stream())
+
+    def data_ptr(self) -> int:
+        return self.buf.data_ptr()
+
+
 def tc_status() -> int:
     """0, or the code of the first bounded wait of a tensor-core kernel that gave up since the last reset (synchronises)."""
     return int(lib.spgt_tc_status())
@@ -465,13 +482,14 @@ def ffn_tc(x: Tensor, w1: TcWeight, b1: Tensor, w2: TcWeight, b2: Optional[Tenso
     return out
 
 
-def conv3x3_tc(x: Tensor, cin_off: int, Cin: int, w: TcWeight, bias: Tensor, y: Tensor, cout_off: int, Cout: int, act) -> Tensor:
+def conv3x3_tc(x: Tensor, cin_off: int, Cin: int, w, bias: Tensor, y: Tensor, cout_off: int, Cout: int, act) -> Tensor:
+    """w: a ConvWeight, or a TcWeight (any number of output channels, the general GEMM kernel)."""
     _chk(x, 'x'); _chk(y, 'y'); _chk(bias, 'bias')
     B, Hh, Ww, cp = x.shape
     if w.K != 9 * Cin or w.N != Cout:
         raise ValueError('prepared weight does not match [9*Cin, Cout]')
     with _device(x.device):
-        _call('spgt_conv3x3_tc_fwd', x.data_ptr(), cp, cin_off, Cin, w.data_ptr(), bias.data_ptr(), y.data_ptr(), y.shape[3],
+        _call('spgt_conv3x3_nhwc_fwd' if isinstance(w, ConvWeight) else 'spgt_conv3x3_tc_fwd', x.data_ptr(), cp, cin_off, Cin, w.data_ptr(), bias.data_ptr(), y.data_ptr(), y.shape[3],
               cout_off, Cout, B, Hh, Ww, act_code(act), _stream())
     return y
 
@@ -538,6 +556,39 @@ def spectral_conv2d(x: Tensor, wr_kn: Tensor, br: Tensor, fw0: Tensor, fw1: Tens
                                            tab.data_ptr(), workspace.data_ptr(), workspace.numel(), y.data_ptr(),
                                            B, r, Cc, mode, act_code(act), _stream(),
               kernels=int(lib.spgt_spectral_launches(B, r, mode)))
+    return y
+
+
+# ---------------------------------------------------------------------------------------------------------
+# encoder layer
+# ---------------------------------------------------------------------------------------------------------
+class EncoderPlan:
+    """A spgt_encoder_weights with the tensors it points to; `fill` writes the pointers (ptr(tensor) keeps the tensor)."""
+
+    def __init__(self, fill):
+        self.weights, self.keep, self.need = EncoderWeights(), [], {}
+
+        def ptr(t):
+            self.keep.append(t)
+            return None if t is None else t.data_ptr()
+        fill(self.weights, ptr)
+        self.address = ctypes.addressof(self.weights)
+
+
+def encoder_layer(plan: EncoderPlan, x: Tensor, position: Tensor, eps: float, act=None, ffn: bool = True, residual: bool = True) -> Tensor:
+    """x [B,S,128], position [B,S,2] -> the encoder layer's output (ffn), or the attention layer's (+ x with residual)."""
+    _chk(x, 'x'); _chk(position, 'position')
+    B, S, D = x.shape
+    if D != 128 or position.shape != (B, S, 2):
+        raise ValueError('x must be [B, S, 128] and position [B, S, 2]')
+    need = plan.need.get((B, S))
+    if need is None:
+        need = plan.need[(B, S)] = int(lib.spgt_encoder_workspace_bytes(B, S))
+    with _device(x.device):
+        y = torch.empty_like(x)
+        workspace = torch.empty(need, device=x.device, dtype=torch.uint8)
+        _call('spgt_encoder_layer_fwd', plan.address, x.data_ptr(), position.data_ptr(), y.data_ptr(), B, S, float(eps), act_code(act), int(ffn),
+              int(residual), workspace.data_ptr(), need, _stream(), kernels=3)
     return y
 
 

@@ -1,0 +1,64 @@
+"""The fused encoder-layer kernels and the shared-memory convolution kernel against float64, at the edges of their tiles."""
+import pytest
+import torch
+
+from tests.helpers import rel_l2
+from oracle import gt_oracle as O
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-5          # per layer, as for the single ops
+
+
+def _layer(seed):
+    from spgt_b200.network.sp_layer import Sp_EncoderLayer
+    g = torch.Generator().manual_seed(seed)
+    layer = Sp_EncoderLayer(128, 4, 2, 1e-6, 0.0, 0.0, 1e-2, 1e-2, False, 256, 0.0, 'relu').eval()
+    with torch.no_grad():
+        for name, p in layer.named_parameters():
+            scale = {1: 0.1, 2: p.shape[-1] ** -0.5}[p.dim()] if 'ln_' not in name else 0.1
+            p.copy_(torch.randn(p.shape, generator=g) * scale + (1.0 if 'ln_weight' in name else 0.0))
+    return layer, g
+
+
+# one node, ends of a 128-row tile, one tile more than a sample needs, blocks that work on two samples, more tiles than blocks
+@pytest.mark.parametrize('B,S', [(1, 1), (1, 127), (2, 128), (3, 129), (2, 641), (5, 1849), (80, 130), (64, 2809)])
+def test_encoder_layer_edges(B, S):
+    from spgt_b200 import ops
+    layer, g = _layer(S)
+    x, pos = torch.randn(B, S, 128, generator=g), torch.rand(B, S, 2, generator=g)
+    n = min(B, 3)                                          # (the oracle runs on the first and last samples)
+    idx = sorted({0, B // 2, B - 1})[:n]
+    p = {k: v.detach().double().clone() for k, v in layer.state_dict().items()}
+    cfg = dict(num_head=4, dim_hidden=128, attn_norm_eps=1e-6, acti_encoder_ffn='relu')
+    taps = {}
+    ref = O.encoder_layer(x[idx].double(), pos[idx].double(), p, '', cfg, taps)
+    layer = layer.cuda()
+    xd, pd = x.cuda(), pos.cuda()
+    with torch.no_grad():
+        y = layer(xd, pd)
+        att = layer.attention_layer(xd, xd, xd, pd)
+        res = layer.attention_layer(xd, xd, xd, pd, residual=xd)
+        again = layer(xd, pd)
+    assert ops.tc_status() == 0
+    assert torch.equal(y, again) and torch.isfinite(y).all()
+    assert rel_l2(y[idx], ref) < TOL
+    assert rel_l2(att[idx], taps['fc']) < TOL
+    assert rel_l2(res[idx], taps['post_attn']) < TOL
+
+
+@pytest.mark.parametrize('B,Hh,Ww,Cin,Cout,act', [(1, 1, 1, 4, 4, None), (2, 9, 11, 128, 44, 'relu'), (1, 16, 8, 44, 44, 'silu'), (3, 17, 9, 36, 48, 'relu'),
+                                                   (2, 15, 31, 12, 20, None), (1, 20, 17, 128, 128, 'silu2'), (2, 5, 106, 64, 52, 'silu'),
+                                                   (4, 106, 106, 128, 128, 'silu2'), (20, 77, 77, 128, 44, 'relu')])
+def test_conv3x3_shared_memory_operands(B, Hh, Ww, Cin, Cout, act):
+    from spgt_b200 import ops
+    g = torch.Generator().manual_seed(Hh * Ww + Cout)
+    x, w, b = torch.randn(B, Hh, Ww, Cin + 8, generator=g), torch.randn(Cout, Cin, 3, 3, generator=g) / (9 * Cin) ** 0.5, torch.randn(Cout, generator=g)
+    wt = ops.ConvWeight(w.permute(2, 3, 1, 0).reshape(9 * Cin, Cout).contiguous().cuda(), Cin)
+    y = torch.full((B, Hh, Ww, Cout + 8), float('nan'), device='cuda')
+    ops.conv3x3_tc(x.cuda(), 4, Cin, wt, b.cuda(), y, 4, Cout, act)
+    assert ops.tc_status() == 0
+    ref = torch.nn.functional.conv2d(x[..., 4:4 + Cin].permute(0, 3, 1, 2).double(), w.double(), b.double(), padding=1)
+    silu = torch.nn.functional.silu
+    ref = {None: lambda t: t, 'relu': torch.relu, 'silu': silu, 'silu2': lambda t: silu(silu(t))}[act](ref)
+    assert rel_l2(y[..., 4:4 + Cout], ref.permute(0, 2, 3, 1)) < TOL
+    assert torch.isnan(y[..., :4]).all() and torch.isnan(y[..., 4 + Cout:]).all()
