@@ -131,21 +131,19 @@ encoder_kv_kernel(const float* __restrict__ x, const float* __restrict__ wkv_img
 #pragma unroll
             for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const float4*>(src + roff[j]);
             mbar_arrive(raw_empty(s));
+            uint32_t hi[32], lo[32];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                split_tf32(w[j].x, hi[4 * j], lo[4 * j]); split_tf32(w[j].y, hi[4 * j + 1], lo[4 * j + 1]);
+                split_tf32(w[j].z, hi[4 * j + 2], lo[4 * j + 2]); split_tf32(w[j].w, hi[4 * j + 3], lo[4 * j + 3]);
+            }
             if (!mbar_wait(a_empty(s), ph ^ 1, abort_flag, 43, &g_enc_kv_status)) break;
             tc_fence_after();
             const uint32_t a_hi = tmem_base + lane_addr + KV_A + s * 64;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                uint32_t hi[16], lo[16];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float4 v = w[4 * h + j];
-                    split_tf32(v.x, hi[4 * j], lo[4 * j]); split_tf32(v.y, hi[4 * j + 1], lo[4 * j + 1]);
-                    split_tf32(v.z, hi[4 * j + 2], lo[4 * j + 2]); split_tf32(v.w, hi[4 * j + 3], lo[4 * j + 3]);
-                }
-                tc_st16(a_hi + 16 * h, hi);
-                tc_st16(a_hi + 32 + 16 * h, lo);
-            }
+            tc_st16(a_hi, reinterpret_cast<uint32_t(&)[16]>(hi[0]));
+            tc_st16(a_hi + 16, reinterpret_cast<uint32_t(&)[16]>(hi[16]));
+            tc_st16(a_hi + 32, reinterpret_cast<uint32_t(&)[16]>(lo[0]));
+            tc_st16(a_hi + 48, reinterpret_cast<uint32_t(&)[16]>(lo[16]));
             tc_wait_st();
             tc_fence_before();
             mbar_arrive(a_full(s));

@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(EO_THREADS, 1) encoder_out_kernel(const Encode
     auto tile_index = [&](int ti) { return (int)blockIdx.x + ti * (int)gridDim.x; };
     if (tid == 0) {
         for (int s = 0; s < 2; ++s) {
-            mbar_init(a_full(s), 128); mbar_init(a_empty(s), 1); mbar_init(x_full(s), 1); mbar_init(x_empty(s), 256); mbar_init(d_free(s), 256);
+            mbar_init(a_full(s), 128); mbar_init(a_empty(s), 1); mbar_init(x_full(s), 32); mbar_init(x_empty(s), 256); mbar_init(d_free(s), 256);
         }
         mbar_init(d0_full, 1); mbar_init(d1_full, 1); mbar_init(d2_full, 1); mbar_init(x_go, 1);
         for (int s = 0; s < EO_NW; ++s) { mbar_init(w_full(s), 1); mbar_init(w_empty(s), 1); }
@@ -75,20 +75,23 @@ __global__ void __launch_bounds__(EO_THREADS, 1) encoder_out_kernel(const Encode
     tc_fence_after();
     const uint32_t tmem_base = tc_uniform(*tmem_slot);
 
-    // split 32 values of this thread's row and store them as A stage s
-    auto store_a = [&](uint32_t s, uint32_t lane_addr, const float (&v)[32]) {
+    // Split 32 values of this thread's row and store them as A stage s once its previous use (the stage's `use`-th) is over.  The
+    // split comes before the wait: a stage's turn-around is what paces the short k-blocks.
+    auto store_a = [&](uint32_t s, uint32_t use, uint32_t lane_addr, const float (&v)[32], int code) {
+        uint32_t hi[32], lo[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) split_tf32(v[j], hi[j], lo[j]);
+        if (!mbar_wait(a_empty(s), ((use >> 1) & 1u) ^ 1u, abort_flag, code, &g_enc_out_status)) return false;
+        tc_fence_after();
         const uint32_t a_hi = tmem_base + lane_addr + EO_A + s * 64;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            uint32_t hi[16], lo[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) split_tf32(v[16 * h + j], hi[j], lo[j]);
-            tc_st16(a_hi + 16 * h, hi);
-            tc_st16(a_hi + 32 + 16 * h, lo);
-        }
+        tc_st16(a_hi, reinterpret_cast<uint32_t(&)[16]>(hi[0]));
+        tc_st16(a_hi + 16, reinterpret_cast<uint32_t(&)[16]>(hi[16]));
+        tc_st16(a_hi + 32, reinterpret_cast<uint32_t(&)[16]>(lo[0]));
+        tc_st16(a_hi + 48, reinterpret_cast<uint32_t(&)[16]>(lo[16]));
         tc_wait_st();
         tc_fence_before();
         mbar_arrive(a_full(s));
+        return true;
     };
 
     if (warp < 4) {
@@ -98,8 +101,8 @@ __global__ void __launch_bounds__(EO_THREADS, 1) encoder_out_kernel(const Encode
         for (int ti = 0; ti < n_my && alive; ++ti) {
             const uint32_t buf = (uint32_t)(ti & 1);
             if (!mbar_wait(x_full(buf), (uint32_t)((ti >> 1) & 1), abort_flag, 61, &g_enc_out_status)) break;
-            // The A stages are shared with the other converters; after k-block 5 of the previous tile's GEMM 2 every stage use but
-            // the last two has been consumed, so the parity waits below cannot mistake an older phase for the wanted one.
+            // The A stages are shared with the other converters; after k-block 4 of the previous tile's GEMM 2 only the last use
+            // of each stage may be unconsumed when its parity wait below comes, so it cannot mistake an older phase for the wanted one.
             if (FFN && ti > 0 && !mbar_wait(x_go, (uint32_t)((ti - 1) & 1), abort_flag, 62, &g_enc_out_status)) break;
             const float4* row = reinterpret_cast<const float4*>(smem + EO_OFF_X + buf * EO_XT + (warp * 32 + lane) * (EO_PITCH * 4));
             for (int kb = 0; kb < 4; ++kb) {
@@ -110,9 +113,7 @@ __global__ void __launch_bounds__(EO_THREADS, 1) encoder_out_kernel(const Encode
                     const float4 w = row[kb * 8 + j];
                     v[4 * j] = w.x; v[4 * j + 1] = w.y; v[4 * j + 2] = w.z; v[4 * j + 3] = w.w;
                 }
-                if (!mbar_wait(a_empty(s), ((use >> 1) & 1u) ^ 1u, abort_flag, 63, &g_enc_out_status)) { alive = false; break; }
-                tc_fence_after();
-                store_a(s, lane_addr, v);
+                if (!store_a(s, use, lane_addr, v, 63)) { alive = false; break; }
             }
         }
     } else if (warp < 12) {
@@ -122,6 +123,11 @@ __global__ void __launch_bounds__(EO_THREADS, 1) encoder_out_kernel(const Encode
         const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
         const int r = q * 32 + lane;
         bool alive = true;
+        auto fetch_pos = [&](int ti) {                                  // position values of this row, a tile ahead
+            const int tile = tile_index(ti < n_my ? ti : 0), b = tile / p.tps, row = (tile - b * p.tps) * EN_ROWS + r;
+            return row < p.S ? __ldg(reinterpret_cast<const float2*>(p.pos) + (int64_t)b * p.S + row) : make_float2(0.f, 0.f);
+        };
+        float2 pnext = fetch_pos(0);
         for (int ti = 0; ti < n_my && alive; ++ti) {
             const uint32_t buf = (uint32_t)(ti & 1), tph = (uint32_t)(ti & 1);
             const uint32_t d0 = tmem_base + lane_addr + (buf ? 256u : 0u), d1 = tmem_base + lane_addr + (buf ? 0u : 128u);
@@ -129,7 +135,8 @@ __global__ void __launch_bounds__(EO_THREADS, 1) encoder_out_kernel(const Encode
             const int nrows = p.S - row0;                               // (may exceed the tile)
             float* xrow = reinterpret_cast<float*>(smem + EO_OFF_X + buf * EO_XT) + r * EO_PITCH;
             const float* pc = reinterpret_cast<const float*>(smem + EO_OFF_PC + buf * EO_PC);
-            const float2 ps = r < nrows ? __ldg(reinterpret_cast<const float2*>(p.pos) + (int64_t)b * p.S + row0 + r) : make_float2(0.f, 0.f);
+            const float2 ps = pnext;
+            pnext = fetch_pos(ti + 1);
             // rows of this warp, 32 columns from c0: shared memory -> coalesced stores (one 128-byte line per row)
             auto store_rows = [&](int c0) {
                 __syncwarp();
@@ -161,9 +168,7 @@ __global__ void __launch_bounds__(EO_THREADS, 1) encoder_out_kernel(const Encode
                 }
                 if constexpr (FFN) {
                     const uint32_t use = (uint32_t)(ti * USES + 4 + kb);
-                    if (!mbar_wait(a_empty(g), ((use >> 1) & 1u) ^ 1u, abort_flag, 66, &g_enc_out_status)) { alive = false; break; }
-                    tc_fence_after();
-                    store_a(g, lane_addr, v);
+                    if (!store_a(g, use, lane_addr, v, 66)) { alive = false; break; }
                 } else {
                     store_rows(kb * 32);
                 }
@@ -187,9 +192,7 @@ __global__ void __launch_bounds__(EO_THREADS, 1) encoder_out_kernel(const Encode
 #pragma unroll
                         for (int j = 0; j < 32; ++j) v[j] = apply_act(v[j], p.act);
                     }
-                    if (!mbar_wait(a_empty(g), ((use >> 1) & 1u) ^ 1u, abort_flag, 68, &g_enc_out_status)) { alive = false; break; }
-                    tc_fence_after();
-                    store_a(g, lane_addr, v);
+                    if (!store_a(g, use, lane_addr, v, 68)) { alive = false; break; }
                 }
                 if (!alive) break;
                 if (!mbar_wait(d2_full, tph, abort_flag, 69, &g_enc_out_status)) break;
@@ -211,7 +214,6 @@ __global__ void __launch_bounds__(EO_THREADS, 1) encoder_out_kernel(const Encode
                     store_rows(kb * 32);
                 }
             }
-            fence_proxy_async();                                        // the next tile arrives here by bulk copy
             mbar_arrive(x_empty(buf));
         }
     } else if (warp == 12) {
@@ -221,18 +223,20 @@ __global__ void __launch_bounds__(EO_THREADS, 1) encoder_out_kernel(const Encode
             const int tile = tile_index(ti), b = tile / p.tps, row0 = (tile - b * p.tps) * EN_ROWS;
             const int nrows = p.S - row0 < EN_ROWS ? p.S - row0 : EN_ROWS;
             if (!mbar_wait(x_empty(buf), (uint32_t)((ti >> 1) & 1) ^ 1u, abort_flag, 70, &g_enc_out_status)) break;
-            if (lane == 0)
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(x_full(buf)), "r"(nrows * 512 + EO_PC) : "memory");
-            __syncwarp();
-            const float* src = p.x + ((int64_t)b * p.S + row0) * EN_D;
-            const uint32_t dst = smem_base + EO_OFF_X + buf * EO_XT;
-            for (int r = lane; r < nrows; r += 32)
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                             ::"r"(dst + r * (EO_PITCH * 4)), "l"(src + (int64_t)r * EN_D), "r"(512), "r"(x_full(buf)) : "memory");
-            if (lane == 0)
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                             ::"r"(smem_base + EO_OFF_PC + buf * EO_PC), "l"(p.pc + (int64_t)b * 3 * EN_D), "r"(EO_PC), "r"(x_full(buf)) : "memory");
+            // a row per instruction (bulk copies of 512-byte rows took 5000 cycles longer); rows beyond the sample are zero
+            const float* src = p.x + ((int64_t)b * p.S + row0) * EN_D + lane * 4;
+            const uint32_t dst = smem_base + EO_OFF_X + buf * EO_XT + lane * 16;
+#pragma unroll 16
+            for (int r = 0; r < EN_ROWS; ++r) {
+                const bool ok = r < nrows;
+                const float* from = ok ? src + (int64_t)r * EN_D : p.x;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + r * (EO_PITCH * 4)), "l"(from), "r"(ok ? 16 : 0) : "memory");
+            }
+            for (int i = lane; i < EO_PC / 16; i += 32)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_base + EO_OFF_PC + buf * EO_PC + i * 16), "l"(p.pc + (int64_t)b * 3 * EN_D + i * 4) : "memory");
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(x_full(buf)) : "memory");
         }
+        cp_async_wait_all();
     } else if (warp < 15) {
         // ------------------------------------------ image loaders ------------------------------------------
         // slot g of this block's stream: tile g / SLOTS; M: (k-block, part), W1: (k-block, column tile, part), W2: (k-block, part)
@@ -305,7 +309,7 @@ __global__ void __launch_bounds__(EO_THREADS, 1) encoder_out_kernel(const Encode
                     for (int kb = 0; kb < 8; ++kb, ++use) {
                         if (!stage_ready() || !block(d0, use & 1u, kb == 0)) { alive = false; break; }
                         tc_commit(a_empty(use & 1u));
-                        if (kb == 5) tc_commit(x_go);
+                        if (kb == 4) tc_commit(x_go);
                     }
                     if (!alive) break;
                     tc_commit(d2_full);

@@ -28,7 +28,9 @@ constexpr uint32_t CV_HALF = CV_CH / 4 * CV_LBO, CV_STAGE = 2 * CV_HALF;  // hi 
 constexpr int CV_NA = 2, CV_STAGERS = 256, CV_ITEMS = (CV_PX + CV_STAGERS / 8 - 1) / (CV_STAGERS / 8);
 constexpr int CV_THREADS = CV_STAGERS + 64 + 128, CV_SLOT = 16 * 4 + 16;
 template <int BN> struct CvCfg {
-    static constexpr int W_BLOCK = 2 * BN * CV_CH * 4, NW = BN == 128 ? 3 : 6, ACCW = 2 * BN;
+    // One bulk copy brings the taps of a filter row (the issuing thread needs about 400 cycles per copy and wait whatever the size,
+    // as long as a tap's MMAs for 48 channels take), or one tap of 128 channels.
+    static constexpr int TAPS = BN == 128 ? 1 : 3, W_TAP = 2 * BN * CV_CH * 4, W_BLOCK = TAPS * W_TAP, NW = BN == 128 ? 3 : 2, ACCW = 2 * BN;
     static constexpr int TMEM = 2 * ACCW <= 256 ? 256 : 512;
     static constexpr int OFF_A = NW * W_BLOCK, OFF_STG = OFF_A + CV_NA * CV_STAGE, OFF_BIAS = OFF_STG + 128 * CV_SLOT, OFF_BAR = OFF_BIAS + BN * 4;
     static constexpr size_t BYTES = OFF_BAR + 256;
@@ -136,7 +138,7 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv3x3_kernel(const ConvParams
         // ------------------------------------------ weight blocks ------------------------------------------
         if (lane == 0) {
             uint32_t s = 0, ph = 0;
-            const int blocks = chunks * 9;
+            const int blocks = chunks * (9 / C::TAPS);
             bool alive = true;
             for (int ti = 0; ti < n_my && alive; ++ti)
                 for (int k = 0; k < blocks; ++k) {
@@ -161,22 +163,25 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv3x3_kernel(const ConvParams
                     if (!mbar_wait(a_full(s), ph, abort_flag, 84, &g_conv_status)) { alive = false; break; }
                     const uint32_t a0 = smem_base + C::OFF_A + s * CV_STAGE;
                     const int left = p.cin - chunk * CV_CH, nk8 = left >= CV_CH ? CV_CH / 8 : (left + 7) / 8;
-                    for (int tap = 0; tap < 9; ++tap) {
+                    for (int tap0 = 0; tap0 < 9; tap0 += C::TAPS) {
                         if (!mbar_wait(w_full(ws), wph, abort_flag, 85, &g_conv_status)) { alive = false; break; }
                         tc_fence_after();
-                        const int dy = tap / 3, dx = tap - dy * 3;
-                        const uint64_t ah = cv_a_desc(a0 + (uint32_t)(dy * CV_HX + dx) * 16), al = cv_a_desc(a0 + CV_HALF + (uint32_t)(dy * CV_HX + dx) * 16);
-                        const uint64_t db = tc_smem_desc(smem_base + ws * C::W_BLOCK);
-                        constexpr uint64_t AK = 2 * CV_LBO >> 4;         // two 4-channel chunks per k-step
-                        auto step = [&](int k8) {
-                            tc_mma_tf32_ss(d, ah + k8 * AK, db + k8 * 2, idesc2, (chunk > 0 || tap > 0 || k8 > 0) ? 1u : 0u);
-                            tc_mma_tf32_ss(d, al + k8 * AK, db + k8 * 2, idesc1, 1u);
-                        };
-                        if (nk8 == 4) {
 #pragma unroll
-                            for (int k8 = 0; k8 < 4; ++k8) step(k8);
-                        } else {
-                            for (int k8 = 0; k8 < nk8; ++k8) step(k8);
+                        for (int e = 0; e < C::TAPS; ++e) {
+                            const int tap = tap0 + e, dy = tap / 3, dx = tap - dy * 3;
+                            const uint64_t ah = cv_a_desc(a0 + (uint32_t)(dy * CV_HX + dx) * 16), al = cv_a_desc(a0 + CV_HALF + (uint32_t)(dy * CV_HX + dx) * 16);
+                            const uint64_t db = tc_smem_desc(smem_base + ws * C::W_BLOCK + e * C::W_TAP);
+                            constexpr uint64_t AK = 2 * CV_LBO >> 4;     // two 4-channel chunks per k-step
+                            auto step = [&](int k8) {
+                                tc_mma_tf32_ss(d, ah + k8 * AK, db + k8 * 2, idesc2, (chunk > 0 || tap > 0 || k8 > 0) ? 1u : 0u);
+                                tc_mma_tf32_ss(d, al + k8 * AK, db + k8 * 2, idesc1, 1u);
+                            };
+                            if (nk8 == 4) {
+#pragma unroll
+                                for (int k8 = 0; k8 < 4; ++k8) step(k8);
+                            } else {
+                                for (int k8 = 0; k8 < nk8; ++k8) step(k8);
+                            }
                         }
                         tc_commit(w_empty(ws));
                         if (++ws == (uint32_t)C::NW) { ws = 0; wph ^= 1u; }
