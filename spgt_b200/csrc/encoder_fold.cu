@@ -37,6 +37,7 @@ encoder_fold_kernel(const float* __restrict__ partial, const float* __restrict__
     float* s_g = s_wfc + 4 * 40 * FO_WP;          // G': the 128 channel rows of G
     float* s_gp = s_g + EN_D * FO_GP;             // its position rows [head][2][16]
     float *s_ln = s_gp + 8 * FO_N, *s_bq = s_ln + 128, *s_red = s_bq + 128;
+    pdl_launch_next();
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, fg = lane >> 2, ft = lane & 3, b = blockIdx.x / FO_CL;
     const uint32_t rank = cluster_ctarank();
     const int n0 = (int)rank * FO_N, h = (int)rank >> 1, hh = h & 1, r0 = ((int)rank & 1) * FO_ROWS;      // head, head in its pair, first row of T_h
@@ -62,6 +63,7 @@ encoder_fold_kernel(const float* __restrict__ partial, const float* __restrict__
         s_ln[t] = __ldg(ln + h * 32 + (t & 31));
         s_bq[t] = bq ? __ldg(bq + t) : 0.0f;
     }
+    pdl_wait();
     const int first = sp.owner(b * sp.tps), parts = sp.owner(b * sp.tps + sp.tps - 1) - first + 1;
     static_assert(FO_SUMS % 4 == 0 && FO_SUMS / 4 <= FO_THREADS, "one sum of four values per thread");
     if (t < FO_SUMS / 4) {
@@ -75,7 +77,7 @@ encoder_fold_kernel(const float* __restrict__ partial, const float* __restrict__
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
         for (int k = 0; k < parts; ++k) {
-            const float4 v = __ldg(src + (int64_t)k * (EN_P_FLOATS / 4));
+            const float4 v = __ldca(src + (int64_t)k * (EN_P_FLOATS / 4));
             s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
         }
         *reinterpret_cast<float4*>(s_sum + i) = s;
@@ -187,8 +189,7 @@ encoder_fold_kernel(const float* __restrict__ partial, const float* __restrict__
 int encoder_fold(const float* partial, const spgt_encoder_weights& w, float* m_img, float* pc, int B, int S, const EncoderSplit& sp, cudaStream_t st) {
     static SmemOptIn configured;
     if (int e = smem_opt_in(encoder_fold_kernel, FO_SMEM, configured)) return e;
-    encoder_fold_kernel<<<B * FO_CL, FO_THREADS, FO_SMEM, st>>>(partial, w.wq, w.bq, w.lnwk, w.lnbk, w.lnwv, w.lnbv, w.wfc, w.bfc, m_img, pc, S, sp);
-    return launch_status();
+    return launch_chained(encoder_fold_kernel, B * FO_CL, FO_THREADS, FO_SMEM, st, partial, w.wq, w.bq, w.lnwk, w.lnbk, w.lnwv, w.lnbv, w.wfc, w.bfc, m_img, pc, S, sp);
 }
 
 }  // namespace spgt

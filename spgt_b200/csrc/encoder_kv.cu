@@ -39,6 +39,7 @@ encoder_kv_kernel(const float* __restrict__ x, const float* __restrict__ wkv_img
                   float eps, const float* __restrict__ pos, float* __restrict__ partial, int S, EncoderSplit sp) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t smem_base = smem_u32(smem);
+    pdl_launch_next();
     if (smem_base & 1023u) {                                   // (operand tiles need 1024-byte alignment; dynamic shared memory starts so)
         if (threadIdx.x == 0) atomicCAS(&g_enc_kv_status, 0, 40);
         return;
@@ -89,6 +90,7 @@ encoder_kv_kernel(const float* __restrict__ x, const float* __restrict__ wkv_img
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tc_uniform(*tmem_slot);
+    pdl_wait();
     // a chain of T products ends with the sample, with this block's last tile, or after KV_CHAIN tiles
     auto tile_of = [&](int i) { return (u_begin + i) % sp.tps; };
     auto chain_ends = [&](int i, int len) { return len == KV_CHAIN || i == n_my - 1 || tile_of(i) == sp.tps - 1; };
@@ -381,8 +383,7 @@ int encoder_kv(const float* x, const void* wkv, const float* bk, const float* bv
                const EncoderSplit& sp, cudaStream_t st) {
     static SmemOptIn configured;
     if (int e = smem_opt_in(encoder_kv_kernel, KV_SMEM, configured)) return e;
-    encoder_kv_kernel<<<EN_PAIRS * sp.per_pair, KV_THREADS, KV_SMEM, st>>>(x, (const float*)wkv, bk, bv, eps, pos, partial, S, sp);
-    return launch_status();
+    return launch_chained(encoder_kv_kernel, EN_PAIRS * sp.per_pair, KV_THREADS, KV_SMEM, st, x, (const float*)wkv, bk, bv, eps, pos, partial, S, sp);
 }
 
 int encoder_kv_status(bool reset) {

@@ -25,6 +25,8 @@ __host__ __device__ __forceinline__ Tap make_tap(int dst, int in_size, int out_s
 __global__ void __launch_bounds__(256)
 bilinear_kernel(const float4* __restrict__ x, float4* __restrict__ y, int Hi, int Wi, int Ho, int Wo, int C4, int act,
                 int rows) {
+    pdl_launch_next();
+    pdl_wait();
     const int per_row = Wo * C4;
     const bool fixed_c = (blockDim.x % C4) == 0;          // a thread keeps its channel quad: no division per element
     const int c_fix = threadIdx.x % C4, x_step = blockDim.x / C4;
@@ -39,10 +41,10 @@ bilinear_kernel(const float4* __restrict__ x, float4* __restrict__ y, int Hi, in
             int c = c_fix;
             if (!fixed_c) { xo = e / C4; c = e - xo * C4; }
             const Tap tx = make_tap(xo, Wi, Wo);
-            const float4 v00 = __ldg(r0 + tx.i0 * C4 + c);
-            const float4 v01 = __ldg(r0 + tx.i1 * C4 + c);
-            const float4 v10 = __ldg(r1 + tx.i0 * C4 + c);
-            const float4 v11 = __ldg(r1 + tx.i1 * C4 + c);
+            const float4 v00 = __ldca(r0 + tx.i0 * C4 + c);
+            const float4 v01 = __ldca(r0 + tx.i1 * C4 + c);
+            const float4 v10 = __ldca(r1 + tx.i0 * C4 + c);
+            const float4 v11 = __ldca(r1 + tx.i1 * C4 + c);
             const float w00 = ty.w0 * tx.w0, w01 = ty.w0 * tx.w1, w10 = ty.w1 * tx.w0, w11 = ty.w1 * tx.w1;
             float4 o;
             o.x = apply_act(v00.x * w00 + v01.x * w01 + v10.x * w10 + v11.x * w11, act);
@@ -66,6 +68,8 @@ template <int ACT>
 __global__ void __launch_bounds__(128)
 conv0_down_kernel(const float* __restrict__ node, const float4* __restrict__ w, const float4* __restrict__ bias,
                   float4* __restrict__ y, int Hi, int Wi, int Ho, int Wo, int CQ, int npix) {
+    pdl_launch_next();
+    pdl_wait();
     constexpr int act = ACT;
     __shared__ __align__(16) float patch[C0_PIX][16];
     __shared__ __align__(16) float wt[C0_PIX][4];
@@ -75,8 +79,8 @@ conv0_down_kernel(const float* __restrict__ node, const float4* __restrict__ w, 
     if (fixed_cq) {
         const int cq = threadIdx.x % CQ;
 #pragma unroll
-        for (int k = 0; k < 9; ++k) wk[k] = __ldg(w + k * CQ + cq);
-        bc = __ldg(bias + cq);
+        for (int k = 0; k < 9; ++k) wk[k] = __ldca(w + k * CQ + cq);
+        bc = __ldca(bias + cq);
     }
     for (int p0 = blockIdx.x * C0_PIX; p0 < npix; p0 += gridDim.x * C0_PIX) {
         __syncthreads();                              // the previous group's patch has been consumed
@@ -99,7 +103,7 @@ conv0_down_kernel(const float* __restrict__ node, const float4* __restrict__ w, 
             float v = 0.0f;
             if (p0 + pi < npix) {
                 const int yy = pix_y0[pi] + (e >> 2), xx = pix_x0[pi] + (e & 3);
-                if (yy >= 0 && yy < Hi && xx >= 0 && xx < Wi) v = __ldg(node + ((int64_t)pix_row0[pi] + yy) * Wi + xx);
+                if (yy >= 0 && yy < Hi && xx >= 0 && xx < Wi) v = __ldca(node + ((int64_t)pix_row0[pi] + yy) * Wi + xx);
             }
             patch[pi][e] = v;
         }
@@ -110,8 +114,8 @@ conv0_down_kernel(const float* __restrict__ node, const float4* __restrict__ w, 
             if (p >= npix) break;
             if (!fixed_cq) {
 #pragma unroll
-                for (int k = 0; k < 9; ++k) wk[k] = __ldg(w + k * CQ + cq);
-                bc = __ldg(bias + cq);
+                for (int k = 0; k < 9; ++k) wk[k] = __ldca(w + k * CQ + cq);
+                bc = __ldca(bias + cq);
             }
             float pv[16];
 #pragma unroll
@@ -153,13 +157,15 @@ __global__ void __launch_bounds__(256)
 upsample_grid_kernel(const float4* __restrict__ uw, const float2* __restrict__ grid, const float4* __restrict__ wg,
                      const float4* __restrict__ bias, float4* __restrict__ y, int Hi, int Wi, int Ho, int Wo, int C4,
                      int rows) {
+    pdl_launch_next();
+    pdl_wait();
     const int per_row = Wo * C4;
     // When the block size is a multiple of C4 a thread keeps its channel quad for every element: the three parameter
     // vectors stay in registers and the pixel index advances by a constant, without a division.
     const bool fixed_c = (blockDim.x % C4) == 0;
     const int c_fix = threadIdx.x % C4, x_fix = threadIdx.x / C4, x_step = blockDim.x / C4;
     float4 g0f, g1f, bbf;
-    if (fixed_c) { g0f = __ldg(wg + c_fix); g1f = __ldg(wg + C4 + c_fix); bbf = __ldg(bias + c_fix); }
+    if (fixed_c) { g0f = __ldca(wg + c_fix); g1f = __ldca(wg + C4 + c_fix); bbf = __ldca(bias + c_fix); }
     for (int row = blockIdx.x; row < rows; row += gridDim.x) {
         const int b = row / Ho, yo = row - b * Ho;
         const Tap ty = make_tap(yo, Hi, Ho);
@@ -173,15 +179,15 @@ upsample_grid_kernel(const float4* __restrict__ uw, const float2* __restrict__ g
             float4 g0 = g0f, g1 = g1f, bb = bbf;
             if (!fixed_c) {
                 xo = e / C4; c = e - xo * C4;
-                g0 = __ldg(wg + c); g1 = __ldg(wg + C4 + c); bb = __ldg(bias + c);
+                g0 = __ldca(wg + c); g1 = __ldca(wg + C4 + c); bb = __ldca(bias + c);
             }
             const Tap tx = make_tap(xo, Wi, Wo);
-            const float4 v00 = __ldg(r0 + tx.i0 * C4 + c);
-            const float4 v01 = __ldg(r0 + tx.i1 * C4 + c);
-            const float4 v10 = __ldg(r1 + tx.i0 * C4 + c);
-            const float4 v11 = __ldg(r1 + tx.i1 * C4 + c);
+            const float4 v00 = __ldca(r0 + tx.i0 * C4 + c);
+            const float4 v01 = __ldca(r0 + tx.i1 * C4 + c);
+            const float4 v10 = __ldca(r1 + tx.i0 * C4 + c);
+            const float4 v11 = __ldca(r1 + tx.i1 * C4 + c);
             const float w00 = ty.w0 * tx.w0, w01 = ty.w0 * tx.w1, w10 = ty.w1 * tx.w0, w11 = ty.w1 * tx.w1;
-            const float2 gxy = __ldg(gr + xo);
+            const float2 gxy = __ldca(gr + xo);
             float4 o;
             o.x = v00.x * w00 + v01.x * w01 + v10.x * w10 + v11.x * w11 + gxy.x * g0.x + gxy.y * g1.x + bb.x;
             o.y = v00.y * w00 + v01.y * w01 + v10.y * w10 + v11.y * w11 + gxy.x * g0.y + gxy.y * g1.y + bb.y;
@@ -205,10 +211,12 @@ lerp_staged_kernel(const float4* __restrict__ x, float4* __restrict__ y, int Hi,
                    const float2* __restrict__ grid, const float4* __restrict__ wg, const float4* __restrict__ bias, int G,
                    int groups_per_img, int n_groups) {
     extern __shared__ float4 srow[];                       // the source rows of the current group
+    pdl_launch_next();
     const int row_f4 = Wi * C4, per_row = Wo * C4;
     const int c = threadIdx.x % C4, x0 = threadIdx.x / C4, x_step = blockDim.x / C4;     // blockDim.x % C4 == 0 (host)
     float4 g0 = make_float4(0.f, 0.f, 0.f, 0.f), g1 = g0, bb = g0;
-    if (MODE == 1) { g0 = __ldg(wg + c); g1 = __ldg(wg + C4 + c); bb = __ldg(bias + c); }
+    if (MODE == 1) { g0 = __ldca(wg + c); g1 = __ldca(wg + C4 + c); bb = __ldca(bias + c); }
+    pdl_wait();
     for (int grp = blockIdx.x; grp < n_groups; grp += gridDim.x) {
         const int b = grp / groups_per_img, y0 = (grp - b * groups_per_img) * G;
         const int y1 = y0 + G < Ho ? y0 + G : Ho;
@@ -234,7 +242,7 @@ lerp_staged_kernel(const float4* __restrict__ x, float4* __restrict__ y, int Hi,
                 const float w00 = ty.w0 * tx.w0, w01 = ty.w0 * tx.w1, w10 = ty.w1 * tx.w0, w11 = ty.w1 * tx.w1;
                 float4 o;
                 if (MODE == 1) {
-                    const float2 gxy = __ldg(gr + xo);
+                    const float2 gxy = __ldca(gr + xo);
                     o.x = v00.x * w00 + v01.x * w01 + v10.x * w10 + v11.x * w11 + gxy.x * g0.x + gxy.y * g1.x + bb.x;
                     o.y = v00.y * w00 + v01.y * w01 + v10.y * w10 + v11.y * w11 + gxy.x * g0.y + gxy.y * g1.y + bb.y;
                     o.z = v00.z * w00 + v01.z * w01 + v10.z * w10 + v11.z * w11 + gxy.x * g0.z + gxy.y * g1.z + bb.z;
@@ -285,9 +293,8 @@ static int launch_staged(const StagedPlan& p, const float4* x, float4* y, int B,
     const int per_sm = (int)(200 * 1024 / (p.smem + 1024));
     // few resident blocks (long rows): larger blocks keep enough threads per SM (measured: 512 better above 48 KB, worse below)
     const int threads = (p.smem > 48 * 1024 && LS_THREADS % (2 * C4) == 0) ? LS_THREADS : LS_THREADS / 2;
-    lerp_staged_kernel<MODE><<<grid_for(n_groups, 1, per_sm < 1 ? 1 : (per_sm > 8 ? 8 : per_sm)), threads, p.smem, st>>>(
+    return launch_chained(lerp_staged_kernel<MODE>, grid_for(n_groups, 1, per_sm < 1 ? 1 : (per_sm > 8 ? 8 : per_sm)), threads, p.smem, st,
         x, y, Hi, Wi, Ho, Wo, C4, act, grid, wg, bias, p.G, gpi, (int)n_groups);
-    return launch_status();
 }
 
 // y[b,yo,xo,:] = act(bilinear(concat(x1[..., :c1], x2[..., :c2], x3[..., :c3])))  -- the three sources keep their own
@@ -296,6 +303,8 @@ __global__ void __launch_bounds__(256)
 bilinear_concat3_kernel(const float* __restrict__ x1, const float* __restrict__ x2, const float* __restrict__ x3, int p1,
                         int p2, int p3, int c1, int c2, int c3, float4* __restrict__ y, int Hi, int Wi, int Ho, int Wo,
                         int act, int rows) {
+    pdl_launch_next();
+    pdl_wait();
     const int C4 = (c1 + c2 + c3) / 4;
     const int per_row = Wo * C4;
     for (int row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -316,8 +325,8 @@ bilinear_concat3_kernel(const float* __restrict__ x1, const float* __restrict__ 
                 if (c < c1) { src = x1; pitch = p1; }
                 else if (c < c1 + c2) { src = x2; pitch = p2; c -= c1; }
                 else { src = x3; pitch = p3; c -= c1 + c2; }
-                const float v = __ldg(src + o00 * pitch + c) * w00 + __ldg(src + o01 * pitch + c) * w01 +
-                                __ldg(src + o10 * pitch + c) * w10 + __ldg(src + o11 * pitch + c) * w11;
+                const float v = __ldca(src + o00 * pitch + c) * w00 + __ldca(src + o01 * pitch + c) * w01 +
+                                __ldca(src + o10 * pitch + c) * w10 + __ldca(src + o11 * pitch + c) * w11;
                 o[k] = apply_act(v, act);
             }
             yr[e] = make_float4(o[0], o[1], o[2], o[3]);
@@ -340,9 +349,8 @@ extern "C" int spgt_bilinear_fwd(const float* x, float* y, int B, int Hi, int Wi
     if (plan.G > 0)
         return launch_staged<0>(plan, reinterpret_cast<const float4*>(x), reinterpret_cast<float4*>(y), B, Hi, Wi, Ho, Wo, C / 4, act,
                                 nullptr, nullptr, nullptr, (cudaStream_t)stream);
-    bilinear_kernel<<<grid_for(rows, 1, 8), 256, 0, (cudaStream_t)stream>>>(
+    return launch_chained(bilinear_kernel, grid_for(rows, 1, 8), 256, 0, (cudaStream_t)stream,
         reinterpret_cast<const float4*>(x), reinterpret_cast<float4*>(y), Hi, Wi, Ho, Wo, C / 4, act, (int)rows);
-    return launch_status();
 }
 
 extern "C" int spgt_bilinear_concat3_fwd(const float* x1, const float* x2, const float* x3, int p1, int p2, int p3, int c1,
@@ -354,9 +362,8 @@ extern "C" int spgt_bilinear_concat3_fwd(const float* x1, const float* x2, const
     if (!aligned16(y)) return SPGT_ERR_ALIGN;
     const int64_t rows = (int64_t)B * Ho;
     if (rows > 0x7fffffffLL || (int64_t)Wo * (c1 + c2 + c3) > 0x7fffffffLL) return SPGT_ERR_SHAPE;
-    bilinear_concat3_kernel<<<grid_for(rows, 1, 8), 256, 0, (cudaStream_t)stream>>>(
+    return launch_chained(bilinear_concat3_kernel, grid_for(rows, 1, 8), 256, 0, (cudaStream_t)stream,
         x1, x2, x3, p1, p2, p3, c1, c2, c3, reinterpret_cast<float4*>(y), Hi, Wi, Ho, Wo, act, (int)rows);
-    return launch_status();
 }
 
 extern "C" int spgt_conv0_down_fwd(const float* node, const float* w, const float* bias, float* y, int B, int Hi, int Wi,
@@ -369,16 +376,15 @@ extern "C" int spgt_conv0_down_fwd(const float* node, const float* w, const floa
     if (!aligned16(w) || !aligned16(bias) || !aligned16(y)) return SPGT_ERR_ALIGN;
     const unsigned grid = grid_for(ceil_div(npix, (int64_t)C0_PIX), 1, 16);
     auto launch = [&](auto kern) {
-        kern<<<grid, 128, 0, (cudaStream_t)stream>>>(node, reinterpret_cast<const float4*>(w), reinterpret_cast<const float4*>(bias),
-                                                     reinterpret_cast<float4*>(y), Hi, Wi, Ho, Wo, Cout / 4, (int)npix);
+        return launch_chained(kern, grid, 128, 0, (cudaStream_t)stream, node, reinterpret_cast<const float4*>(w), reinterpret_cast<const float4*>(bias),
+                              reinterpret_cast<float4*>(y), Hi, Wi, Ho, Wo, Cout / 4, (int)npix);
     };
     switch (act) {
-        case SPGT_ACT_RELU: launch(conv0_down_kernel<SPGT_ACT_RELU>); break;
-        case SPGT_ACT_SILU: launch(conv0_down_kernel<SPGT_ACT_SILU>); break;
-        case SPGT_ACT_SILU2: launch(conv0_down_kernel<SPGT_ACT_SILU2>); break;
-        default: launch(conv0_down_kernel<SPGT_ACT_NONE>); break;
+        case SPGT_ACT_RELU: return launch(conv0_down_kernel<SPGT_ACT_RELU>);
+        case SPGT_ACT_SILU: return launch(conv0_down_kernel<SPGT_ACT_SILU>);
+        case SPGT_ACT_SILU2: return launch(conv0_down_kernel<SPGT_ACT_SILU2>);
+        default: return launch(conv0_down_kernel<SPGT_ACT_NONE>);
     }
-    return launch_status();
 }
 
 extern "C" int spgt_upsample_grid_fwd(const float* uw, const float* grid, const float* wg, const float* bias, float* y,
@@ -393,8 +399,7 @@ extern "C" int spgt_upsample_grid_fwd(const float* uw, const float* grid, const 
         return launch_staged<1>(plan, reinterpret_cast<const float4*>(uw), reinterpret_cast<float4*>(y), B, Hi, Wi, Ho, Wo, C / 4, 0,
                                 reinterpret_cast<const float2*>(grid), reinterpret_cast<const float4*>(wg),
                                 reinterpret_cast<const float4*>(bias), (cudaStream_t)stream);
-    upsample_grid_kernel<<<grid_for(rows, 1, 8), 256, 0, (cudaStream_t)stream>>>(
+    return launch_chained(upsample_grid_kernel, grid_for(rows, 1, 8), 256, 0, (cudaStream_t)stream,
         reinterpret_cast<const float4*>(uw), reinterpret_cast<const float2*>(grid), reinterpret_cast<const float4*>(wg),
         reinterpret_cast<const float4*>(bias), reinterpret_cast<float4*>(y), Hi, Wi, Ho, Wo, C / 4, (int)rows);
-    return launch_status();
 }

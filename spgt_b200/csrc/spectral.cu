@@ -120,9 +120,11 @@ __global__ void __launch_bounds__(256)
 spectral_fwd_x_kernel(const float* __restrict__ Y1, const float* __restrict__ tab, float* __restrict__ Zr,
                       float* __restrict__ Zi, int r, int m) {
     extern __shared__ __align__(16) float smem[];
+    pdl_launch_next();
     const SpecTables T = spec_tables(r, m);
     float* gr = smem; float* gi = smem + T.J * r;
-    for (int i = threadIdx.x; i < 2 * T.J * r; i += blockDim.x) smem[i] = __ldg(tab + T.gr + i);
+    for (int i = threadIdx.x; i < 2 * T.J * r; i += blockDim.x) smem[i] = __ldca(tab + T.gr + i);
+    pdl_wait();
     __syncthreads();
     const int ky = blockIdx.x; const int64_t b = blockIdx.y;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -130,8 +132,8 @@ spectral_fwd_x_kernel(const float* __restrict__ Y1, const float* __restrict__ ta
     const float* yb = Y1 + b * (int64_t)r * T.J * SP_C + lane;
 #pragma unroll 8
     for (int x = 0; x < r; ++x) {
-        const float yr = __ldg(yb + ((int64_t)x * T.J + ky) * SP_C);
-        const float yi = __ldg(yb + ((int64_t)x * T.J + m + ky) * SP_C);
+        const float yr = __ldca(yb + ((int64_t)x * T.J + ky) * SP_C);
+        const float yi = __ldca(yb + ((int64_t)x * T.J + m + ky) * SP_C);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int q = warp + 8 * k;
@@ -158,17 +160,19 @@ spectral_mix_kernel(const float* __restrict__ Zr, const float* __restrict__ Zi, 
                     const float* __restrict__ fw1, float* __restrict__ Or, float* __restrict__ Oi, int B, int m,
                     const float* __restrict__ wr, float* __restrict__ wr_img) {
     __shared__ float2 w[SP_C * SP_C];
-    if (blockIdx.x == 0 && wr_img != nullptr)            // W stage image of the residual weight Wr [i][o] for the y-inverse GEMM
-        for (int i = threadIdx.x; i < SP_C * SP_C; i += blockDim.x) tc_img_store(wr_img, SP_C, i % SP_C, i / SP_C, __ldg(wr + i));
+    pdl_launch_next();
     const int q = blockIdx.x / m, ky = blockIdx.x % m;
     const float2* src = reinterpret_cast<const float2*>(q < m ? fw0 : fw1) + ((int64_t)(q < m ? q : q - m) * m + ky) * SP_C * SP_C;
-    for (int i = threadIdx.x; i < SP_C * SP_C; i += blockDim.x) w[i] = __ldg(src + i);
+    for (int i = threadIdx.x; i < SP_C * SP_C; i += blockDim.x) w[i] = __ldca(src + i);
+    pdl_wait();
+    if (blockIdx.x == 0 && wr_img != nullptr)            // W stage image of the residual weight Wr [i][o] for the y-inverse GEMM
+        for (int i = threadIdx.x; i < SP_C * SP_C; i += blockDim.x) tc_img_store(wr_img, SP_C, i % SP_C, i / SP_C, __ldca(wr + i));
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int J = 2 * m;
     for (int b = warp; b < B; b += 8) {
         const int64_t base = (((int64_t)b * J + q) * m + ky) * SP_C;
-        const float zr = __ldg(Zr + base + lane), zi = __ldg(Zi + base + lane);
+        const float zr = __ldca(Zr + base + lane), zi = __ldca(Zi + base + lane);
         float orr = 0.0f, oii = 0.0f;
 #pragma unroll
         for (int i = 0; i < SP_C; ++i) {
@@ -187,9 +191,11 @@ __global__ void __launch_bounds__(256)
 spectral_inv_x_kernel(const float* __restrict__ Or, const float* __restrict__ Oi, const float* __restrict__ tab,
                       float* __restrict__ Pimg, int r, int m) {
     extern __shared__ __align__(16) float smem[];
+    pdl_launch_next();
     const SpecTables T = spec_tables(r, m);
     float* gr = smem; float* gi = smem + T.J * r;
-    for (int i = threadIdx.x; i < 2 * T.J * r; i += blockDim.x) smem[i] = __ldg(tab + T.gr + i);
+    for (int i = threadIdx.x; i < 2 * T.J * r; i += blockDim.x) smem[i] = __ldca(tab + T.gr + i);
+    pdl_wait();
     __syncthreads();
     const int ky = blockIdx.x; const int64_t b = blockIdx.y;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -198,7 +204,7 @@ spectral_inv_x_kernel(const float* __restrict__ Or, const float* __restrict__ Oi
     for (int q = 0; q < 32; ++q) {
         if (q < T.J) {
             const int64_t o = ((b * T.J + q) * m + ky) * SP_C + lane;
-            orr[q] = __ldg(Or + o); oii[q] = __ldg(Oi + o);
+            orr[q] = __ldca(Or + o); oii[q] = __ldca(Oi + o);
         } else { orr[q] = 0.0f; oii[q] = 0.0f; }
     }
     for (int x = warp; x < r; x += 8) {
@@ -235,6 +241,7 @@ __global__ void __launch_bounds__(256)
 spectral_fwd_x_mma_kernel(const float* __restrict__ Y1, const float* __restrict__ tab, float* __restrict__ Zr,
                           float* __restrict__ Zi, int r, int m) {
     extern __shared__ __align__(16) float smem[];
+    pdl_launch_next();
     const SpecTables T = spec_tables(r, m);
     const int J = T.J, M2 = 2 * J, MT = (M2 + 15) / 16;
     const int r8 = (r + 7) / 8 * 8;
@@ -244,6 +251,9 @@ spectral_fwd_x_mma_kernel(const float* __restrict__ Y1, const float* __restrict_
     const int ky = blockIdx.x; const int64_t b = blockIdx.y;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
+    for (int i = tid; i < 16 * MT * GP / 4; i += 256) cp_async_zfill<16>(gs + 4 * i, tab + T.ga + 4 * i, true);   // padded G, as stored
+    cp_async_commit();
+    pdl_wait();
     // Y block: 16 float4 per x (8 from the real row, 8 from the imaginary row)
     const float* yb = Y1 + b * (int64_t)r * J * SP_C;
     for (int i = tid; i < r8 * 16; i += 256) {
@@ -252,8 +262,6 @@ spectral_fwd_x_mma_kernel(const float* __restrict__ Y1, const float* __restrict_
         const float* src = yb + ((int64_t)(ok ? x : 0) * J + (c4 < 8 ? ky : m + ky)) * SP_C + (c4 & 7) * 4;
         cp_async_zfill<16>(ys + x * SP_YP + c4 * 4, src, ok);
     }
-    cp_async_commit();
-    for (int i = tid; i < 16 * MT * GP / 4; i += 256) cp_async_zfill<16>(gs + 4 * i, tab + T.ga + 4 * i, true);   // padded G, as stored
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
@@ -317,6 +325,7 @@ __global__ void __launch_bounds__(256)
 spectral_inv_x_mma_kernel(const float* __restrict__ Or, const float* __restrict__ Oi, const float* __restrict__ tab,
                           float* __restrict__ P, int r, int m) {
     extern __shared__ __align__(16) float smem[];
+    pdl_launch_next();
     const SpecTables T = spec_tables(r, m);
     const int J = T.J, M2 = 2 * J, K8 = (M2 + 7) / 8 * 8;
     const int r16 = (r + 15) / 16 * 16;
@@ -328,14 +337,15 @@ spectral_inv_x_mma_kernel(const float* __restrict__ Or, const float* __restrict_
     const int g = lane >> 2, t = lane & 3;
     for (int i = tid; i < K8 * GP / 4; i += 256) cp_async_zfill<16>(gs + 4 * i, tab + T.gc + 4 * i, true);     // padded G, as stored
     cp_async_commit();
+    pdl_wait();
     for (int i = tid; i < K8 * 64; i += 256) {
         const int k = i >> 6, n = i & 63;
         float v = 0.0f;
         if (k < M2) {
             const int q = k < J ? k : k - J;
             const int64_t o = ((b * J + q) * m + ky) * SP_C + (n & 31);
-            if (k < J) v = n < 32 ? __ldg(Or + o) : __ldg(Oi + o);
-            else v = n < 32 ? __ldg(Oi + o) : -__ldg(Or + o);
+            if (k < J) v = n < 32 ? __ldca(Or + o) : __ldca(Oi + o);
+            else v = n < 32 ? __ldca(Oi + o) : -__ldca(Or + o);
         }
         bs[k * SP_YP + n] = v;
     }
@@ -471,24 +481,23 @@ extern "C" int spgt_spectral_conv2d_fwd(const float* x, const float* wr, const f
             const int MT = ceil_div(2 * (int)J, 16), r8 = ceil_div(r, 8) * 8;
             const size_t smem_a = ((size_t)16 * MT * sp_round_pitch(r8, 4) + (size_t)(r8 > 16 * MT ? r8 : 16 * MT) * SP_YP) * sizeof(float);
             if ((e = smem_opt_in(spectral_fwd_x_mma_kernel, smem_a, cfg_am))) return e;
-            spectral_fwd_x_mma_kernel<<<dim3(m, nb), 256, smem_a, st>>>(Y1, tab, Zr, Zi, r, m);
+            e = launch_chained(spectral_fwd_x_mma_kernel, dim3(m, nb), 256, smem_a, st, Y1, tab, Zr, Zi, r, m);
         } else {
             if ((e = smem_opt_in(spectral_fwd_x_kernel, gsmem, cfg_a))) return e;
-            spectral_fwd_x_kernel<<<dim3(m, nb), 256, gsmem, st>>>(Y1, tab, Zr, Zi, r, m);
+            e = launch_chained(spectral_fwd_x_kernel, dim3(m, nb), 256, gsmem, st, Y1, tab, Zr, Zi, r, m);
         }
-        if ((e = launch_status())) return e;
-        spectral_mix_kernel<<<(unsigned)(J * m), 256, 0, st>>>(Zr, Zi, fw0, fw1, Or, Oi, nb, m, wr, b0 == 0 ? wr_img : nullptr);
-        if ((e = launch_status())) return e;
+        if (e) return e;
+        if ((e = launch_chained(spectral_mix_kernel, (unsigned)(J * m), 256, 0, st, Zr, Zi, fw0, fw1, Or, Oi, nb, m, wr, b0 == 0 ? wr_img : nullptr))) return e;
         if (staged) {
             const int K8 = ceil_div(2 * (int)J, 8) * 8, r16 = ceil_div(r, 16) * 16;
             const size_t smem_c = ((size_t)K8 * sp_round_pitch(r16, 8) + (size_t)K8 * SP_YP) * sizeof(float);
             if ((e = smem_opt_in(spectral_inv_x_mma_kernel, smem_c, cfg_cm))) return e;
-            spectral_inv_x_mma_kernel<<<dim3(m, nb), 256, smem_c, st>>>(Or, Oi, tab, P, r, m);
+            e = launch_chained(spectral_inv_x_mma_kernel, dim3(m, nb), 256, smem_c, st, Or, Oi, tab, P, r, m);
         } else {
             if ((e = smem_opt_in(spectral_inv_x_kernel, gsmem, cfg_c))) return e;
-            spectral_inv_x_kernel<<<dim3(m, nb), 256, gsmem, st>>>(Or, Oi, tab, P, r, m);
+            e = launch_chained(spectral_inv_x_kernel, dim3(m, nb), 256, gsmem, st, Or, Oi, tab, P, r, m);
         }
-        if ((e = launch_status())) return e;
+        if (e) return e;
         if ((e = spectral_inv_y_tc(xc, tab + T.f3, wr_img, P, P, (int)J, br, yc, r, nimg, act, st))) return e;
     }
     return SPGT_OK;

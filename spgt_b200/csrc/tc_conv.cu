@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv3x3_kernel(const ConvParams
     using C = CvCfg<BN>;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t smem_base = smem_u32(smem);
+    pdl_launch_next();
     if (smem_base & 1023u) {
         if (threadIdx.x == 0) atomicCAS(&g_conv_status, 0, 80);
         return;
@@ -86,6 +87,7 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv3x3_kernel(const ConvParams
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tc_uniform(*tmem_slot);
+    pdl_wait();
 
     if (warp < 8) {
         // ------------------------------------------ load and split ------------------------------------------
@@ -112,7 +114,7 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv3x3_kernel(const ConvParams
             const bool in = chunk * CV_CH + c4 * 4 < p.cin;
 #pragma unroll
             for (int k = 0; k < CV_ITEMS; ++k)
-                v[k] = in && src[k] != nullptr ? __ldg(reinterpret_cast<const float4*>(src[k] + chunk * CV_CH)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[k] = in && src[k] != nullptr ? __ldca(reinterpret_cast<const float4*>(src[k] + chunk * CV_CH)) : make_float4(0.f, 0.f, 0.f, 0.f);
         };
         if (n_my > 0) { locate(0); fetch(0); }
         for (int ti = 0; ti < n_my && alive; ++ti)
@@ -271,8 +273,7 @@ template <int BN> static int conv_launch(const ConvParams& p, cudaStream_t st) {
     static SmemOptIn configured;
     if (int e = smem_opt_in(conv3x3_kernel<BN>, CvCfg<BN>::BYTES, configured)) return e;
     const int grid = p.n_tiles < num_sms() ? p.n_tiles : num_sms();
-    conv3x3_kernel<BN><<<grid, CV_THREADS, CvCfg<BN>::BYTES, st>>>(p);
-    return launch_status();
+    return launch_chained(conv3x3_kernel<BN>, grid, CV_THREADS, CvCfg<BN>::BYTES, st, p);
 }
 
 }  // namespace spgt

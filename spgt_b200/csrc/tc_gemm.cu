@@ -293,6 +293,7 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
     constexpr int TC_THREADS = tc_threads(MT, EG), TC_EPI_WARP0 = tc_epi_warp0(MT);
     static_assert(EG == 1 || (EG == 2 && (CS || C::NBUF == 2) && (EPI == EPI_LINEAR || EPI == EPI_HEAD)), "two epilogue groups: one per accumulator buffer, or sharing every unit");
     extern __shared__ uint8_t smem_raw[];
+    pdl_launch_next();
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;          // 1024-aligned for the 128B swizzle
     uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
     uint8_t* staging = smem + C::SB * C::B_BYTES + SR * C::RAW_BYTES;
@@ -390,6 +391,7 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
         tc_fence_after();
     }
 
+    pdl_wait();
     // Work distribution: this CTA keeps one column tile (so a resident W is loaded once) and strides over row units.
     const int sched_id = blockIdx.x, sched_n = gridDim.x;
     const int ctas_per_nt = sched_n / n_tiles;
@@ -683,7 +685,7 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
 #pragma unroll
                 for (int i = 0; i < EP_NIT; ++i) {
                     const int64_t orow = ld.out_row(row0_ + i * EP_RPI);
-                    rres[i] = (col_ < e.N && orow >= 0) ? __ldg(reinterpret_cast<const float4*>(e.residual + orow * e.ldr + col_))
+                    rres[i] = (col_ < e.N && orow >= 0) ? __ldca(reinterpret_cast<const float4*>(e.residual + orow * e.ldr + col_))
                                                         : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
             }
@@ -976,8 +978,7 @@ static int tc_launch(Loader ld, const float* wimg, int kpad, int rows, int n_til
     if (per_nt < 1) per_nt = 1;
     if (per_nt > m_units) per_nt = m_units;
     const int grid = per_nt * n_tiles;
-    kern<<<grid, tc_threads(MT, tc_epi_groups<Loader, MT, BN, EPI>()), TcCfg<BN, MT, Loader, EPI>::BYTES, st>>>(ld, wimg, kpad, rows, n_tiles, m_units, ep);
-    return launch_status();
+    return launch_chained(kern, grid, tc_threads(MT, tc_epi_groups<Loader, MT, BN, EPI>()), TcCfg<BN, MT, Loader, EPI>::BYTES, st, ld, wimg, kpad, rows, n_tiles, m_units, ep);
 }
 
 template <class Loader>
