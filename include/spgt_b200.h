@@ -245,6 +245,14 @@ int spgt_decoder_head_fwd(const float* x, const float* w1, const float* b1, cons
 /* Bytes of a prepared weight for a [K,N] matrix, and the preparation itself (w_kn row-major, pitch ldw). */
 size_t spgt_tc_weight_bytes(int K, int N);
 int spgt_tc_weight_prepare(const float* w_kn, int ldw, int K, int N, void* out, size_t out_bytes, spgt_stream_t stream);
+/* The same from the transposed matrix, w_nk [N][ldw] (a torch Linear weight as it is). */
+int spgt_tc_weight_prepare_t(const float* w_nk, int ldw, int K, int N, void* out, size_t out_bytes, spgt_stream_t stream);
+
+/* C[M, N] = A^T B for row-major A [rows, lda], B [rows, ldb] (weight gradient x^T dy), rows the long dimension; colsum, when not NULL, gets
+ * the column sums of B [N] (bias gradient).  lda, ldb multiples of 4.  Partial results per block in `workspace`, added in block order. */
+size_t spgt_tn_gemm_workspace_bytes(int M, int N, int rows);
+int spgt_tn_gemm(const float* A, int lda, const float* B, int ldb, float* C, int ldc, float* colsum, int M, int N, int rows,
+                 void* workspace, size_t workspace_bytes, spgt_stream_t stream);
 /* 0 if no tensor-core kernel gave up on a bounded wait since the last reset, else the code of the first one that did
  * (GEMM: 1..9; fused feed-forward: 21..34; attention: 101..109; spectral layer: 201..219).  Every wait inside these
  * kernels is bounded by two seconds of wall time; a kernel whose wait expires stops waiting, records the code and

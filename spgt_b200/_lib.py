@@ -83,6 +83,9 @@ SIGNATURES = {
     'spgt_tc_selftest_wait_expiry': (_i, [_i, _i, _f, _st]),
     'spgt_linear_tc_fwd': (_i, [_f, _i, _f, _f, _f, _i, _f, _i, _i, _i, _i, _i, _st]),
     'spgt_conv3x3_tc_fwd': (_i, [_f, _i, _i, _i, _f, _f, _f, _i, _i, _i, _i, _i, _i, _i, _st]),
+    'spgt_tn_gemm_workspace_bytes': (_sz, [_i, _i, _i]),
+    'spgt_tn_gemm': (_i, [_f, _i, _f, _i, _f, _i, _f, _i, _i, _i, _f, _sz, _st]),
+    'spgt_tc_weight_prepare_t': (_i, [_f, _i, _i, _i, _f, _sz, _st]),
     'spgt_conv3x3_weight_bytes': (_sz, [_i, _i]),
     'spgt_conv3x3_weight_prepare': (_i, [_f, _i, _i, _i, _f, _sz, _st]),
     'spgt_conv3x3_nhwc_fwd': (_i, [_f, _i, _i, _i, _f, _f, _f, _i, _i, _i, _i, _i, _i, _i, _st]),

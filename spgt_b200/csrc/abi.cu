@@ -3,6 +3,7 @@
 
 namespace spgt {
 thread_local int g_last_cuda_error = 0;
+thread_local int g_chain = 0;
 }
 
 extern "C" const char* spgt_error_string(int code) {

@@ -1,130 +1,168 @@
 // Backward of the Galerkin attention op  out[s][j] = sum_i Q[i][s] T[i][j],  T[i][j] = (1/S) sum_s K[i][s] V[j][s]
 // (reference: multihead_galerkin_attention_cccr_backward, extension/bind/galerkin_attention.cu:126-173, which runs
-// three split-K and three small-K SGEMMs).  Here two kernels, exact fp32 FMA arithmetic:
-//   reduce  every CTA streams one chunk of the S columns of a (batch, head) once and accumulates the two dpk x dpk
-//           matrices that the gradients need,  T  and  dT[i][j] = sum_s Q[i][s] dOut[s][j],  into its slot of the workspace;
-//   apply   every CTA sums the chunk partials in chunk order (deterministic), then, one grid node per thread,
-//           dQ[i][s] = sum_j T[i][j] dOut[s][j],   dK[i][s] = (1/S) sum_j dT[i][j] V[j][s],   dV[j][s] = (1/S) sum_i dT[i][j] K[i][s].
+// three split-K and three small-K SGEMMs).  Exact fp32 FMA arithmetic:
+//   reduce  T and  dT[i][j] = sum_s Q[i][s] dOut[s][j]:  a block streams a chunk of the S columns of one (batch, head) through
+//           shared memory; a thread owns 6 x 6 entries and a seventh of the columns of every tile;
+//   sum     chunk partials in chunk order (deterministic);
+//   apply   up to four grid nodes per thread:  dQ[i][s] = sum_j T[i][j] dOut[s][j],   dK[i][s] = (1/S) sum_j dT[i][j] V[j][s],
+//           dV[j][s] = (1/S) sum_i dT[i][j] K[i][s].
+// Both are bound by the values shared memory hands to registers (128 bytes per cycle and SM): with 6 x 6 entries twelve 16-byte
+// reads feed 144 FMAs, with four nodes nine feed 144.  Batch 16, 4 heads, S = 4096: 540 us with five single entries and one
+// node per thread.
 // Layouts as in the forward: Q, K, V, dQ, dK, dV [B*H, dpk, S] (S fastest), dOut [B*H, S, dpk].
 #include "common.cuh"
 
 namespace spgt {
 
 constexpr int AB_MAXD = 35, AB_TP = 36;        // dpk <= 35; pitch of the dpk x dpk matrices
-constexpr int AB_COLS = 64;                    // columns per staged tile of the reduce kernel
-constexpr int AB_THREADS = 256;
+constexpr int AB_MAT = AB_TP * AB_TP;
+constexpr int AB_GROUPS = 7, AB_COLS = AB_GROUPS * 16, AB_CP = AB_COLS + 4;      // columns per tile, pitch (an odd number of 16-byte units)
+constexpr int AB_THREADS = 256;                // 7 groups x 36 threads work, all load
 
-// workspace per (bh, chunk): T partial [36*36] | dT partial [36*36]
+// partial [bh][which: T, dT][chunk][36][36]
 __global__ void __launch_bounds__(AB_THREADS)
-attn_bwd_reduce_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
-                       const float* __restrict__ dOut, float* __restrict__ ws, int D, int S, int chunks) {
-    __shared__ float ks[AB_MAXD][AB_COLS + 1], vs[AB_MAXD][AB_COLS + 1], qs[AB_MAXD][AB_COLS + 1], gs[AB_COLS][AB_TP + 1];
-    const int64_t bh = blockIdx.x / chunks;
-    const int chunk = blockIdx.x % chunks;
-    const int64_t base = bh * (int64_t)D * S;
-    const int ncol_tiles = (S + AB_COLS - 1) / AB_COLS;
-    const int t_begin = (int)(((int64_t)chunk * ncol_tiles) / chunks), t_end = (int)(((int64_t)(chunk + 1) * ncol_tiles) / chunks);
-    // each thread owns up to 5 entries e = tid + 256 n of the D x D matrices
-    float accT[5] = {0, 0, 0, 0, 0}, accD[5] = {0, 0, 0, 0, 0};
-    int ei[5], ej[5];
-#pragma unroll
-    for (int n = 0; n < 5; ++n) { const int e = threadIdx.x + AB_THREADS * n; ei[n] = e < D * D ? e / D : -1; ej[n] = e < D * D ? e % D : 0; }
+attn_bwd_reduce_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V, const float* __restrict__ dOut,
+                       float* __restrict__ partial, int D, int S, int chunks) {
+    __shared__ __align__(16) float as[AB_TP * AB_CP], bs[AB_TP * AB_CP];
+    const int t = threadIdx.x, chunk = blockIdx.x % chunks, which = blockIdx.y;
+    const int64_t bh = blockIdx.x / chunks, base = bh * (int64_t)D * S;
+    const int tiles = (S + AB_COLS - 1) / AB_COLS;
+    const int t_begin = (int)(((int64_t)chunk * tiles) / chunks), t_end = (int)(((int64_t)(chunk + 1) * tiles) / chunks);
+    const float* A = (which ? Q : K) + base;
+    const float* B = (which ? dOut : V) + base;
+    const int g = t / 36, tt = t - g * 36, i0 = tt / 6, j0 = tt - i0 * 6;          // entries (i0 + 6 a, j0 + 6 b)
+    for (int i = t; i < (AB_TP - D) * AB_CP; i += AB_THREADS) { as[D * AB_CP + i] = 0.0f; bs[D * AB_CP + i] = 0.0f; }
+    float acc[6][6] = {};
     for (int tile = t_begin; tile < t_end; ++tile) {
-        const int s0 = tile * AB_COLS;
+        const int s0 = tile * AB_COLS, ns = S - s0 < AB_COLS ? S - s0 : AB_COLS;
         __syncthreads();
-        for (int i = threadIdx.x; i < D * AB_COLS; i += AB_THREADS) {
-            const int r = i / AB_COLS, c = i % AB_COLS;
-            const bool ok = s0 + c < S;
-            const int64_t o = base + (int64_t)r * S + s0 + c;
-            ks[r][c] = ok ? __ldg(K + o) : 0.0f;
-            vs[r][c] = ok ? __ldg(V + o) : 0.0f;
-            qs[r][c] = ok ? __ldg(Q + o) : 0.0f;
+#pragma unroll 4
+        for (int i = t; i < D * AB_COLS; i += AB_THREADS) {
+            const int r = i / AB_COLS, c = i - r * AB_COLS;
+            as[r * AB_CP + c] = c < ns ? __ldg(A + (int64_t)r * S + s0 + c) : 0.0f;
+            if (!which) bs[r * AB_CP + c] = c < ns ? __ldg(B + (int64_t)r * S + s0 + c) : 0.0f;
         }
-        for (int i = threadIdx.x; i < AB_COLS * D; i += AB_THREADS) {
-            const int c = i / D, j = i % D;
-            gs[c][j] = (s0 + c < S) ? __ldg(dOut + (bh * S + s0 + c) * (int64_t)D + j) : 0.0f;
-        }
+        if (which)
+#pragma unroll 4
+            for (int i = t; i < D * AB_COLS; i += AB_THREADS) {
+                const int c = i / D, j = i - c * D;
+                bs[j * AB_CP + c] = c < ns ? __ldg(B + (int64_t)s0 * D + i) : 0.0f;
+            }
         __syncthreads();
+        if (g < AB_GROUPS) {
+            const float* pa = as + i0 * AB_CP + g * 16;
+            const float* pb = bs + j0 * AB_CP + g * 16;
 #pragma unroll
-        for (int n = 0; n < 5; ++n) {
-            if (ei[n] >= 0) {
-                float a = accT[n], d = accD[n];
-#pragma unroll 8
-                for (int c = 0; c < AB_COLS; ++c) {
-                    a = fmaf(ks[ei[n]][c], vs[ej[n]][c], a);
-                    d = fmaf(qs[ei[n]][c], gs[c][ej[n]], d);
+            for (int s = 0; s < 16; s += 4) {
+                float4 a[6], b[6];
+#pragma unroll
+                for (int e = 0; e < 6; ++e) {
+                    a[e] = *reinterpret_cast<const float4*>(pa + 6 * e * AB_CP + s);
+                    b[e] = *reinterpret_cast<const float4*>(pb + 6 * e * AB_CP + s);
                 }
-                accT[n] = a; accD[n] = d;
+#pragma unroll
+                for (int e = 0; e < 6; ++e)
+#pragma unroll
+                    for (int f = 0; f < 6; ++f) {
+                        acc[e][f] = fmaf(a[e].x, b[f].x, acc[e][f]); acc[e][f] = fmaf(a[e].y, b[f].y, acc[e][f]);
+                        acc[e][f] = fmaf(a[e].z, b[f].z, acc[e][f]); acc[e][f] = fmaf(a[e].w, b[f].w, acc[e][f]);
+                    }
             }
         }
     }
-    float* w = ws + ((bh * chunks + chunk) * 2) * (int64_t)(AB_TP * AB_TP);
+    // the seven column groups, in order
+    float* out = partial + ((bh * 2 + which) * chunks + chunk) * AB_MAT;
+    float* red = as;
+    for (int k = 0; k < AB_GROUPS; ++k) {
+        __syncthreads();
+        if (g == k)
 #pragma unroll
-    for (int n = 0; n < 5; ++n)
-        if (ei[n] >= 0) {
-            w[ei[n] * AB_TP + ej[n]] = accT[n];
-            w[AB_TP * AB_TP + ei[n] * AB_TP + ej[n]] = accD[n];
-        }
-}
-
-__global__ void __launch_bounds__(128)
-attn_bwd_apply_kernel(const float* __restrict__ K, const float* __restrict__ V, const float* __restrict__ dOut,
-                      const float* __restrict__ ws, float* __restrict__ dQ, float* __restrict__ dK, float* __restrict__ dV,
-                      int D, int S, int chunks, int col_tiles) {
-    __shared__ float T[AB_MAXD][AB_TP], dT[AB_MAXD][AB_TP];
-    __shared__ float gs[128][AB_TP + 1];
-    const int64_t bh = blockIdx.x / col_tiles;
-    const int s0 = (blockIdx.x % col_tiles) * 128;
-    const float inv_s = 1.0f / (float)S;
-    for (int e = threadIdx.x; e < D * D; e += blockDim.x) {
-        const int i = e / D, j = e % D;
-        float a = 0.0f, d = 0.0f;
-        for (int c = 0; c < chunks; ++c) {
-            const float* w = ws + ((bh * chunks + c) * 2) * (int64_t)(AB_TP * AB_TP);
-            a += __ldg(w + i * AB_TP + j);
-            d += __ldg(w + AB_TP * AB_TP + i * AB_TP + j);
-        }
-        T[i][j] = a * inv_s;
-        dT[i][j] = d * inv_s;          // the 1/S of dK and dV folded in
-    }
-    for (int i = threadIdx.x; i < 128 * D; i += blockDim.x) {
-        const int c = i / D, j = i % D;
-        gs[c][j] = (s0 + c < S) ? __ldg(dOut + (bh * S + s0 + c) * (int64_t)D + j) : 0.0f;
+            for (int e = 0; e < 6; ++e)
+#pragma unroll
+                for (int f = 0; f < 6; ++f) {
+                    const int at = (i0 + 6 * e) * AB_TP + j0 + 6 * f;
+                    red[at] = k == 0 ? acc[e][f] : red[at] + acc[e][f];
+                }
     }
     __syncthreads();
-    const int s = s0 + threadIdx.x;
-    if (s >= S) return;
-    const int64_t base = bh * (int64_t)D * S + s;
-    float col[AB_MAXD];
-    // dQ[i][s] = sum_j T[i][j] dOut[s][j]
-    for (int i = 0; i < D; ++i) {
-        float a = 0.0f;
-        for (int j = 0; j < D; ++j) a = fmaf(T[i][j], gs[threadIdx.x][j], a);
-        dQ[base + (int64_t)i * S] = a;
-    }
-    // dK[i][s] = sum_j dT[i][j] V[j][s]
-    for (int j = 0; j < D; ++j) col[j] = __ldg(V + base + (int64_t)j * S);
-    for (int i = 0; i < D; ++i) {
-        float a = 0.0f;
-        for (int j = 0; j < D; ++j) a = fmaf(dT[i][j], col[j], a);
-        dK[base + (int64_t)i * S] = a;
-    }
-    // dV[j][s] = sum_i dT[i][j] K[i][s]
-    for (int i = 0; i < D; ++i) col[i] = __ldg(K + base + (int64_t)i * S);
-    for (int j = 0; j < D; ++j) {
-        float a = 0.0f;
-        for (int i = 0; i < D; ++i) a = fmaf(dT[i][j], col[i], a);
-        dV[base + (int64_t)j * S] = a;
+    for (int i = t; i < AB_MAT; i += AB_THREADS) out[i] = red[i];
+}
+
+// sums [bh][T | dT | dT transposed][36][36]: chunk partials in chunk order, 1 / S included
+__global__ void __launch_bounds__(256)
+attn_bwd_sum_kernel(const float* __restrict__ partial, float* __restrict__ sums, int chunks, float inv_s) {
+    const int64_t bh = blockIdx.x;
+    const int which = blockIdx.y;
+    const float* src = partial + (bh * 2 + which) * chunks * AB_MAT;
+    float* dst = sums + bh * 3 * AB_MAT;
+    for (int i = threadIdx.x; i < AB_MAT; i += blockDim.x) {
+        float s = 0.0f;
+#pragma unroll 8
+        for (int k = 0; k < chunks; ++k) s += __ldg(src + (int64_t)k * AB_MAT + i);
+        s *= inv_s;
+        if (which == 0) dst[i] = s;
+        else { dst[AB_MAT + i] = s; dst[2 * AB_MAT + (i % AB_TP) * AB_TP + i / AB_TP] = s; }
     }
 }
 
+constexpr int AP_THREADS = 128;
+
+template <int AP_NODES>
+__global__ void __launch_bounds__(AP_THREADS, 3)
+attn_bwd_apply_kernel(const float* __restrict__ K, const float* __restrict__ V, const float* __restrict__ dOut, const float* __restrict__ sums,
+                      float* __restrict__ dQ, float* __restrict__ dK, float* __restrict__ dV, int D, int S, int col_tiles) {
+    __shared__ __align__(16) float mats[3 * AB_MAT];       // T | dT | dT transposed
+    const int t = threadIdx.x;
+    const int64_t bh = blockIdx.x / col_tiles, base = bh * (int64_t)D * S;
+    const int s0 = (int)(blockIdx.x % col_tiles) * (AP_THREADS * AP_NODES) + t;
+    for (int i = t; i < 3 * AB_MAT / 4; i += AP_THREADS)
+        reinterpret_cast<float4*>(mats)[i] = __ldg(reinterpret_cast<const float4*>(sums + bh * 3 * AB_MAT) + i);
+    __syncthreads();
+    float x[AB_TP][AP_NODES];
+    auto multiply = [&](const float* m, float* dst) {      // dst[i][s] = sum_j m[i][j] x[j]
+#pragma unroll 1
+        for (int i = 0; i < D; ++i) {
+            const float4* row = reinterpret_cast<const float4*>(m + i * AB_TP);
+            float acc[AP_NODES] = {};
+#pragma unroll
+            for (int j = 0; j < AB_TP / 4; ++j) {
+                const float4 w = row[j];
+#pragma unroll
+                for (int n = 0; n < AP_NODES; ++n) {
+                    acc[n] = fmaf(w.x, x[4 * j][n], acc[n]); acc[n] = fmaf(w.y, x[4 * j + 1][n], acc[n]);
+                    acc[n] = fmaf(w.z, x[4 * j + 2][n], acc[n]); acc[n] = fmaf(w.w, x[4 * j + 3][n], acc[n]);
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < AP_NODES; ++n)
+                if (s0 + n * AP_THREADS < S) dst[base + (int64_t)i * S + s0 + n * AP_THREADS] = acc[n];
+        }
+    };
+    auto load_columns = [&](const float* src) {
+#pragma unroll
+        for (int j = 0; j < AB_TP; ++j)
+#pragma unroll
+            for (int n = 0; n < AP_NODES; ++n)
+                x[j][n] = j < D && s0 + n * AP_THREADS < S ? __ldg(src + base + (int64_t)j * S + s0 + n * AP_THREADS) : 0.0f;
+    };
+    load_columns(V);
+    multiply(mats + AB_MAT, dK);
+    load_columns(K);
+    multiply(mats + 2 * AB_MAT, dV);
+#pragma unroll
+    for (int n = 0; n < AP_NODES; ++n)
+#pragma unroll
+        for (int j = 0; j < AB_TP; ++j)
+            x[j][n] = j < D && s0 + n * AP_THREADS < S ? __ldg(dOut + base + (int64_t)(s0 + n * AP_THREADS) * D + j) : 0.0f;
+    multiply(mats, dQ);
+}
+
+// blocks per (batch, head) and matrix: enough for four per SM
 static int attn_bwd_chunks(int64_t BH, int S) {
     const int tiles = ceil_div(S, AB_COLS);
-    int64_t c = ceil_div((int64_t)num_sms() * 4, BH);
+    int64_t c = ceil_div((int64_t)4 * num_sms(), 2 * BH);
     if (c > tiles) c = tiles;
-    if (c > 64) c = 64;
-    if (c < 1) c = 1;
-    return (int)c;
+    return (int)(c < 1 ? 1 : c);
 }
 
 }  // namespace spgt
@@ -132,23 +170,32 @@ static int attn_bwd_chunks(int64_t BH, int S) {
 using namespace spgt;
 
 extern "C" size_t spgt_galerkin_attn_bwd_workspace_bytes(int B, int H, int dpk, int S) {
-    if (B <= 0 || H <= 0 || S <= 0 || dpk < 1 || dpk > AB_MAXD) return 0;
-    return (size_t)B * H * attn_bwd_chunks((int64_t)B * H, S) * 2 * AB_TP * AB_TP * sizeof(float);
+    if (B <= 0 || H <= 0 || S <= 0 || dpk <= 0 || dpk > AB_MAXD) return 0;
+    const int64_t BH = (int64_t)B * H;
+    return (size_t)BH * (2 * attn_bwd_chunks(BH, S) + 3) * AB_MAT * sizeof(float);
 }
 
 extern "C" int spgt_galerkin_attn_bwd(const float* Q, const float* K, const float* V, const float* d_out, float* dQ, float* dK,
                                       float* dV, int B, int H, int dpk, int S, void* workspace, size_t workspace_bytes,
                                       spgt_stream_t stream) {
     if (!Q || !K || !V || !d_out || !dQ || !dK || !dV) return SPGT_ERR_NULL;
-    if (B <= 0 || H <= 0 || S <= 0 || dpk < 1 || dpk > AB_MAXD) return SPGT_ERR_SHAPE;
+    if (B <= 0 || H <= 0 || S <= 0 || dpk <= 0 || dpk > AB_MAXD) return SPGT_ERR_SHAPE;
     const int64_t BH = (int64_t)B * H;
-    const int chunks = attn_bwd_chunks(BH, S), col_tiles = ceil_div(S, 128);
+    // four nodes per thread where that still makes a block per SM; small problems are bound by the length of one thread's work
+    const int chunks = attn_bwd_chunks(BH, S);
+    int nodes = 4;
+    while (nodes > 1 && BH * ceil_div(S, AP_THREADS * nodes) < num_sms()) nodes >>= 1;
+    const int col_tiles = ceil_div(S, AP_THREADS * nodes);
     if (BH * chunks > 0x7fffffffLL || BH * col_tiles > 0x7fffffffLL) return SPGT_ERR_SHAPE;
     if (!workspace || workspace_bytes < spgt_galerkin_attn_bwd_workspace_bytes(B, H, dpk, S)) return SPGT_ERR_WORKSPACE;
     cudaStream_t st = (cudaStream_t)stream;
-    attn_bwd_reduce_kernel<<<(unsigned)(BH * chunks), AB_THREADS, 0, st>>>(Q, K, V, d_out, (float*)workspace, dpk, S, chunks);
+    float* partial = (float*)workspace;
+    float* sums = partial + BH * 2 * chunks * AB_MAT;
+    attn_bwd_reduce_kernel<<<dim3((unsigned)(BH * chunks), 2), AB_THREADS, 0, st>>>(Q, K, V, d_out, partial, dpk, S, chunks);
     if (int e = launch_status()) return e;
-    attn_bwd_apply_kernel<<<(unsigned)(BH * col_tiles), 128, 0, st>>>(K, V, d_out, (const float*)workspace, dQ, dK, dV, dpk, S,
-                                                                      chunks, col_tiles);
+    attn_bwd_sum_kernel<<<dim3((unsigned)BH, 2), 256, 0, st>>>(partial, sums, chunks, 1.0f / (float)S);
+    if (int e = launch_status()) return e;
+    auto apply = nodes == 4 ? attn_bwd_apply_kernel<4> : nodes == 2 ? attn_bwd_apply_kernel<2> : attn_bwd_apply_kernel<1>;
+    apply<<<(unsigned)(BH * col_tiles), AP_THREADS, 0, st>>>(K, V, d_out, sums, dQ, dK, dV, dpk, S, col_tiles);
     return launch_status();
 }

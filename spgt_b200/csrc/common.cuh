@@ -15,18 +15,27 @@ inline int launch_status() {
     if (e != cudaSuccess) { g_last_cuda_error = (int)e; return SPGT_ERR_LAUNCH; }
     return SPGT_OK;
 }
-// Launch with programmatic stream serialization: the kernel may start while the one before it in the stream is still running, once
-// every block of that one has called pdl_launch_next() (or has ended).  Kernels launched this way call pdl_wait() before they
-// touch anything an earlier kernel writes or reads; what they do before it - barriers, tensor-memory allocation, constants -
-// overlaps the tail of the kernel before, and the launch gap (1.7 us per kernel of a small forward) disappears.  What an earlier
-// kernel of the chain writes is read with __ldca or cp.async, never __ldg: the compiler may move a read-only load ahead of the wait.
+// Launches inside a ChainScope, all but the first, use programmatic stream serialization: the kernel may start while the one
+// before it in the stream is still running, once every block of that one has called pdl_launch_next() (or has ended).  Kernels
+// launched this way call pdl_wait() before they touch anything an earlier kernel of the chain writes or reads; what they do
+// before it - barriers, tensor-memory allocation, constants, parameters - overlaps the tail of the kernel before, and the launch
+// gap (1.7 us per kernel of a small forward) disappears.  pdl_launch_next() comes after pdl_wait(), so whatever ran before the
+// direct predecessor has finished.  What an earlier kernel of the chain writes is read with __ldca or cp.async, never __ldg: the
+// compiler may move a read-only load ahead of the wait.
+extern thread_local int g_chain;                       // 0 outside any scope, 1 before a scope's first launch, 2 after it
+struct ChainScope {
+    const int before = g_chain;
+    ChainScope() { if (before == 0) g_chain = 1; }
+    ~ChainScope() { g_chain = before; }
+};
 template <class... KA, class... A>
 inline int launch_chained(void (*kern)(KA...), dim3 grid, int threads, size_t smem, cudaStream_t st, A&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = dim3((unsigned)threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = g_chain == 2 ? 1 : 0;
+    if (g_chain == 1) g_chain = 2;
     cfg.attrs = attr; cfg.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...);
     if (e != cudaSuccess) { g_last_cuda_error = (int)e; (void)cudaGetLastError(); return SPGT_ERR_LAUNCH; }

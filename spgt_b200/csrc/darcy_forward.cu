@@ -70,6 +70,7 @@ extern "C" int spgt_darcy_forward(const spgt_darcy_model* m, const float* node, 
     if (!darcy_plan(m, B, p)) return SPGT_ERR_SHAPE;
     if (workspace_bytes < p.total * sizeof(float)) return SPGT_ERR_WORKSPACE;
     if (!aligned16(workspace)) return SPGT_ERR_ALIGN;
+    const ChainScope chain;
     float* ws = (float*)workspace;
     const int mid = m->mid, ra = m->ra, r = m->r, S = ra * ra, D = 128;
     const size_t xa_bytes = (size_t)B * S * D * sizeof(float);

@@ -37,6 +37,7 @@ extern "C" int spgt_encoder_layer_fwd(const spgt_encoder_weights* w, const float
     float* m_img = (float*)((char*)workspace + align256((size_t)B * EN_PAIRS * sp.max_parts * EN_P_FLOATS * 4));
     float* pc = m_img + (size_t)B * (2 * EN_D * EN_D);
     const cudaStream_t st = (cudaStream_t)stream;
+    const ChainScope chain;
     if (int e = encoder_kv(x, w->wkv, w->bk, w->bv, eps, pos, partial, S, sp, st)) return e;
     if (int e = encoder_fold(partial, *w, m_img, pc, B, S, sp, st)) return e;
     return encoder_out(x, m_img, pc, pos, w->w1, w->b1, w->w2, w->b2, y, B, S, act, ffn != 0, residual != 0, st);

@@ -37,7 +37,6 @@ encoder_fold_kernel(const float* __restrict__ partial, const float* __restrict__
     float* s_g = s_wfc + 4 * 40 * FO_WP;          // G': the 128 channel rows of G
     float* s_gp = s_g + EN_D * FO_GP;             // its position rows [head][2][16]
     float *s_ln = s_gp + 8 * FO_N, *s_bq = s_ln + 128, *s_red = s_bq + 128;
-    pdl_launch_next();
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, fg = lane >> 2, ft = lane & 3, b = blockIdx.x / FO_CL;
     const uint32_t rank = cluster_ctarank();
     const int n0 = (int)rank * FO_N, h = (int)rank >> 1, hh = h & 1, r0 = ((int)rank & 1) * FO_ROWS;      // head, head in its pair, first row of T_h
@@ -64,6 +63,7 @@ encoder_fold_kernel(const float* __restrict__ partial, const float* __restrict__
         s_bq[t] = bq ? __ldg(bq + t) : 0.0f;
     }
     pdl_wait();
+    pdl_launch_next();
     const int first = sp.owner(b * sp.tps), parts = sp.owner(b * sp.tps + sp.tps - 1) - first + 1;
     static_assert(FO_SUMS % 4 == 0 && FO_SUMS / 4 <= FO_THREADS, "one sum of four values per thread");
     if (t < FO_SUMS / 4) {

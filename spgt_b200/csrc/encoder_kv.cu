@@ -39,7 +39,6 @@ encoder_kv_kernel(const float* __restrict__ x, const float* __restrict__ wkv_img
                   float eps, const float* __restrict__ pos, float* __restrict__ partial, int S, EncoderSplit sp) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t smem_base = smem_u32(smem);
-    pdl_launch_next();
     if (smem_base & 1023u) {                                   // (operand tiles need 1024-byte alignment; dynamic shared memory starts so)
         if (threadIdx.x == 0) atomicCAS(&g_enc_kv_status, 0, 40);
         return;
@@ -91,6 +90,7 @@ encoder_kv_kernel(const float* __restrict__ x, const float* __restrict__ wkv_img
     tc_fence_after();
     const uint32_t tmem_base = tc_uniform(*tmem_slot);
     pdl_wait();
+    pdl_launch_next();
     // a chain of T products ends with the sample, with this block's last tile, or after KV_CHAIN tiles
     auto tile_of = [&](int i) { return (u_begin + i) % sp.tps; };
     auto chain_ends = [&](int i, int len) { return len == KV_CHAIN || i == n_my - 1 || tile_of(i) == sp.tps - 1; };

@@ -35,7 +35,6 @@ __global__ void __launch_bounds__(EO_THREADS, 1) encoder_out_kernel(const Encode
     constexpr int USES = FFN ? 16 : 4, SLOTS = FFN ? 40 : 8;            // A-stage uses and image slots per tile
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t smem_base = smem_u32(smem);
-    pdl_launch_next();
     if (smem_base & 1023u) {
         if (threadIdx.x == 0) atomicCAS(&g_enc_out_status, 0, 60);
         return;
@@ -76,6 +75,7 @@ __global__ void __launch_bounds__(EO_THREADS, 1) encoder_out_kernel(const Encode
     tc_fence_after();
     const uint32_t tmem_base = tc_uniform(*tmem_slot);
     pdl_wait();
+    pdl_launch_next();
 
     // Split 32 values of this thread's row and store them as A stage s once its previous use (the stage's `use`-th) is over.  The
     // split comes before the wait: a stage's turn-around is what paces the short k-blocks.

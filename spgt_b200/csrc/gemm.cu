@@ -5,7 +5,7 @@
 //             bias + per-head LayerNorm + head-major transposed store with the position rows (Q/K/V projection);
 //             bias + activation + dot with a vector + affine + Dirichlet frame (decoder head).
 // CTA tile 128 x BN x 32, 8 warps (4 along rows x 2 along columns), 3-stage cp.async pipeline.
-#include "common.cuh"
+#include "tc_common.cuh"
 
 namespace spgt {
 
@@ -480,6 +480,8 @@ extern "C" int spgt_conv3x3_fwd(const float* x, int cin_pitch, int cin_off, int 
     return dispatch_linear(ld, w, ldw, Cout, 9 * Cin, rows, ep, st);
 }
 
+namespace spgt { int projpos_tc(const float* x, int nproj, const float* const* w, const TcProjEpi& ep, int rows, cudaStream_t st); }      // tc_gemm.cu
+
 static int proj_common(const float* x, int nproj, ProjEpi& ep, int B, int S, int D, int H, int d_head, int d_pos,
                        cudaStream_t st) {
     if (B <= 0 || S <= 0 || D <= 0 || H <= 0) return SPGT_ERR_SHAPE;
@@ -487,6 +489,12 @@ static int proj_common(const float* x, int nproj, ProjEpi& ep, int B, int S, int
     const int64_t rows64 = (int64_t)B * S;
     if (rows64 > 0x7fffffffLL / 2) return SPGT_ERR_SHAPE;
     if (d_pos > 0 && !ep.pos) return SPGT_ERR_NULL;
+    if (D == 128) {                                  // (wider models: the warp-MMA kernel below)
+        TcProjEpi t = {};
+        for (int i = 0; i < nproj; ++i) { t.bias[i] = ep.bias[i]; t.lnw[i] = ep.lnw[i]; t.lnb[i] = ep.lnb[i]; t.out[i] = ep.out[i]; t.invsigma[i] = ep.invsigma[i]; }
+        t.pos = ep.pos; t.eps = ep.eps; t.S = S; t.H = H; t.d_pos = d_pos;
+        return projpos_tc(x, nproj, ep.w, t, (int)rows64, st);
+    }
     static SmemOptIn done;
     if (int e = smem_opt_in(gemm_proj_kernel, GemmSmem<8>::BYTES, done)) return e;
     static_assert(GemmSmem<8>::BYTES >= (size_t)128 * (G_BM + 4) * sizeof(float), "staging tile must fit");

@@ -6,76 +6,106 @@
 //           out[b, h, d_pos + c, s] = y[b*S + s, 32 h + c]  (position rows carry no gradient).
 // This kernel takes grad_out [B, H, d_pos + 32, S] and the recomputed h and produces
 //   dh [rows, D]  (the gradient with respect to h, row-major: the A operand of the two GEMMs dX = dh W^T and dW = x^T dh),
-//   per-block partial sums of  db = sum_rows dh,  dlnw = sum_rows g * hat,  dlnb = sum_rows g   (g = gathered grad_out),
+//   per-block sums of  db = sum_rows dh,  dlnw = sum_rows g * hat,  dlnb = sum_rows g   (g = gathered grad_out),
 // which a second kernel adds up in block order (deterministic).  Without LayerNorm (lnw == nullptr) dh = g.
-// One block = 32 consecutive grid nodes of one sample, all heads; warp w of 4 = head w... for H heads the block has H warps.
+// A warp works on one head, a lane on one grid node with all 32 channels in registers: the LayerNorm sums need no shuffles, and
+// the parameter sums stay in registers until the block's last node (a block of one node per iteration and a warp reduction
+// per row took 44 us for 65536 rows, the serial addition of its 2048 partial sums another 66 us).
 #include "common.cuh"
 
 namespace spgt {
 
-constexpr int PB_ROWS = 32;      // grid nodes per block
+constexpr int PB_ROWS = 32;      // grid nodes per warp and iteration
 
+template <bool LN>
 __global__ void __launch_bounds__(256)
 proj_bwd_kernel(const float* __restrict__ grad_out, const float* __restrict__ h, const float* __restrict__ lnw,
-                float* __restrict__ dh, float* __restrict__ partial, int S, int H, int d_pos, float eps, int blocks_per_sample) {
-    extern __shared__ float tile[];                       // [H*32 channels][33]
-    const int b = blockIdx.x / blocks_per_sample;
-    const int s0 = (blockIdx.x % blocks_per_sample) * PB_ROWS;
+                float* __restrict__ dh, float* __restrict__ partial, int S, int H, int d_pos, float eps, int tiles_per_sample, int tiles) {
+    extern __shared__ float red[];                        // [H][32][33]
     const int D = H * 32, dpk = d_pos + 32;
     const int lane = threadIdx.x & 31, head = threadIdx.x >> 5;
-    // gather: channel c of head hd, node s0 + lane (coalesced along s)
-    for (int c = 0; c < 32; ++c) {
-        const int s = s0 + lane;
-        tile[(head * 32 + c) * 33 + lane] = s < S ? __ldg(grad_out + (((int64_t)b * H + head) * dpk + d_pos + c) * S + s) : 0.0f;
-    }
-    __syncthreads();
-    const int ch = head * 32 + lane;                      // this thread's channel
-    const float w = lnw != nullptr ? __ldg(lnw + ch) : 1.0f;
-    float acc_db = 0.0f, acc_w = 0.0f, acc_b = 0.0f;
-    for (int r = 0; r < PB_ROWS; ++r) {
-        const int s = s0 + r;
-        if (s >= S) break;
+    float w[32], db[32], dw[32], dbt[32];
+#pragma unroll
+    for (int c = 0; c < 32; ++c) { w[c] = LN ? __ldg(lnw + head * 32 + c) : 1.0f; db[c] = dw[c] = dbt[c] = 0.0f; }
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int b = tile / tiles_per_sample, s = (tile - b * tiles_per_sample) * PB_ROWS + lane;
+        if (s >= S) continue;
         const int64_t row = (int64_t)b * S + s;
-        const float g = tile[ch * 33 + r];
-        float d;
-        if (lnw != nullptr) {
-            const float hv = __ldg(h + row * D + ch);
-            float mu = hv;
+        const float* gp = grad_out + (((int64_t)b * H + head) * dpk + d_pos) * S + s;
+        float g[32];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) mu += __shfl_xor_sync(0xffffffffu, mu, o);
-            mu *= (1.0f / 32.0f);
-            const float cen = hv - mu;
-            float var = cen * cen;
+        for (int c = 0; c < 32; ++c) g[c] = __ldg(gp + (int64_t)c * S);              // lanes = consecutive nodes
+        if constexpr (LN) {
+            float v[32], mu = 0.0f, var = 0.0f, m1 = 0.0f, m2 = 0.0f;
+            const float4* hp = reinterpret_cast<const float4*>(h + row * D + head * 32);
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) var += __shfl_xor_sync(0xffffffffu, var, o);
-            const float inv = rsqrtf(var * (1.0f / 32.0f) + eps);
-            const float hat = cen * inv;
-            const float dhat = g * w;
-            float m1 = dhat, m2 = dhat * hat;
+            for (int j = 0; j < 8; ++j) {
+                const float4 q = __ldg(hp + j);
+                v[4 * j] = q.x; v[4 * j + 1] = q.y; v[4 * j + 2] = q.z; v[4 * j + 3] = q.w;
+                mu += (q.x + q.y) + (q.z + q.w);
+            }
+            mu *= 1.0f / 32.0f;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) { m1 += __shfl_xor_sync(0xffffffffu, m1, o); m2 += __shfl_xor_sync(0xffffffffu, m2, o); }
-            d = inv * (dhat - m1 * (1.0f / 32.0f) - hat * m2 * (1.0f / 32.0f));
-            acc_w = fmaf(g, hat, acc_w);
-            acc_b += g;
-        } else {
-            d = g;
+            for (int c = 0; c < 32; ++c) { v[c] -= mu; var = fmaf(v[c], v[c], var); }
+            const float inv = 1.0f / sqrtf(var * (1.0f / 32.0f) + eps);
+#pragma unroll
+            for (int c = 0; c < 32; ++c) {
+                v[c] *= inv;                              // hat
+                dw[c] = fmaf(g[c], v[c], dw[c]);
+                dbt[c] += g[c];
+                g[c] *= w[c];                             // gradient of hat
+                m1 += g[c];
+                m2 = fmaf(g[c], v[c], m2);
+            }
+            m1 *= 1.0f / 32.0f; m2 *= 1.0f / 32.0f;
+#pragma unroll
+            for (int c = 0; c < 32; ++c) g[c] = inv * (g[c] - m1 - v[c] * m2);
         }
-        dh[row * D + ch] = d;
-        acc_db += d;
+        float4* dp = reinterpret_cast<float4*>(dh + row * D + head * 32);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) dp[j] = make_float4(g[4 * j], g[4 * j + 1], g[4 * j + 2], g[4 * j + 3]);
+#pragma unroll
+        for (int c = 0; c < 32; ++c) db[c] += g[c];
     }
-    float* p = partial + (int64_t)blockIdx.x * 3 * D;
-    p[ch] = acc_db; p[D + ch] = acc_w; p[2 * D + ch] = acc_b;
+    // lane sums -> channel sums: through a padded square per warp
+    float* sq = red + head * (32 * 33);
+    float* p = partial + (int64_t)blockIdx.x * 3 * D + head * 32 + lane;
+    auto columns = [&](const float (&v)[32], int which) {
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 32; ++c) sq[lane * 33 + c] = v[c];
+        __syncwarp();
+        float t = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 32; ++k) t += sq[k * 33 + lane];
+        p[which * D] = t;
+    };
+    columns(db, 0);
+    if (LN) { columns(dw, 1); columns(dbt, 2); }
 }
 
+// 32 columns per block, eight threads per column take every eighth partial sum
 __global__ void __launch_bounds__(256)
 proj_bwd_reduce_kernel(const float* __restrict__ partial, float* __restrict__ db, float* __restrict__ dlnw, float* __restrict__ dlnb,
                        int D, int nblocks) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 3 * D) return;
+    __shared__ float red[8][33];
+    const int c = threadIdx.x & 31, k0 = threadIdx.x >> 5, i = blockIdx.x * 32 + c;
     float s = 0.0f;
-    for (int k = 0; k < nblocks; ++k) s += __ldg(partial + (int64_t)k * 3 * D + i);
-    float* dst = i < D ? db : (i < 2 * D ? dlnw : dlnb);
-    if (dst != nullptr) dst[i % D] = s;
+#pragma unroll 8
+    for (int k = k0; k < nblocks; k += 8) s += __ldg(partial + (int64_t)k * 3 * D + i);
+    red[k0][c] = s;
+    __syncthreads();
+    if (k0 == 0) {
+#pragma unroll
+        for (int k = 1; k < 8; ++k) s += red[k][c];
+        float* dst = i < D ? db : (i < 2 * D ? dlnw : dlnb);
+        if (dst != nullptr) dst[i % D] = s;
+    }
+}
+
+static int proj_bwd_blocks(int B, int S, int H) {          // enough warps for eight per SM sub-partition, one tile each at least
+    const int64_t tiles = (int64_t)B * ceil_div(S, PB_ROWS), most = (int64_t)num_sms() * (H <= 4 ? 2 : 1);
+    return (int)(tiles < most ? tiles : most);
 }
 
 }  // namespace spgt
@@ -84,7 +114,7 @@ using namespace spgt;
 
 extern "C" size_t spgt_projpos_bwd_workspace_bytes(int B, int S, int H) {
     if (B <= 0 || S <= 0 || H <= 0 || H > 8) return 0;
-    return (size_t)B * ceil_div(S, PB_ROWS) * 3 * H * 32 * sizeof(float);
+    return (size_t)proj_bwd_blocks(B, S, H) * 3 * H * 32 * sizeof(float);
 }
 
 extern "C" int spgt_projpos_bwd_elementwise(const float* grad_out, const float* h, const float* ln_weight, float eps, float* dh,
@@ -93,16 +123,17 @@ extern "C" int spgt_projpos_bwd_elementwise(const float* grad_out, const float* 
     if (!grad_out || !dh) return SPGT_ERR_NULL;
     if (ln_weight && !h) return SPGT_ERR_NULL;
     if (B <= 0 || S <= 0 || H <= 0 || H > 8 || d_head != 32 || d_pos < 0 || d_pos > 8) return SPGT_ERR_SHAPE;
-    const int bps = ceil_div(S, PB_ROWS);
-    const int64_t nblocks = (int64_t)B * bps;
-    if (nblocks > 0x7fffffffLL) return SPGT_ERR_SHAPE;
+    const int tps = ceil_div(S, PB_ROWS);
+    if ((int64_t)B * tps > 0x7fffffffLL) return SPGT_ERR_SHAPE;
     if (!workspace || workspace_bytes < spgt_projpos_bwd_workspace_bytes(B, S, H)) return SPGT_ERR_WORKSPACE;
+    if ((h && !aligned16(h)) || !aligned16(dh)) return SPGT_ERR_ALIGN;
     cudaStream_t st = (cudaStream_t)stream;
-    const int D = H * 32;
-    proj_bwd_kernel<<<(unsigned)nblocks, H * 32, (size_t)D * 33 * sizeof(float), st>>>(grad_out, h, ln_weight, dh, (float*)workspace,
-                                                                                       S, H, d_pos, eps, bps);
+    const int D = H * 32, blocks = proj_bwd_blocks(B, S, H);
+    auto kern = ln_weight ? proj_bwd_kernel<true> : proj_bwd_kernel<false>;
+    kern<<<(unsigned)blocks, H * 32, (size_t)H * 32 * 33 * sizeof(float), st>>>(grad_out, h, ln_weight, dh, (float*)workspace, S, H, d_pos, eps, tps,
+                                                                             B * tps);
     if (int e = launch_status()) return e;
-    proj_bwd_reduce_kernel<<<ceil_div(3 * D, 256), 256, 0, st>>>((const float*)workspace, db, ln_weight ? dlnw : nullptr,
-                                                                ln_weight ? dlnb : nullptr, D, (int)nblocks);
+    proj_bwd_reduce_kernel<<<(ln_weight ? 3 : 1) * D / 32, 256, 0, st>>>((const float*)workspace, db, ln_weight ? dlnw : nullptr,
+                                                                         ln_weight ? dlnb : nullptr, D, blocks);
     return launch_status();
 }

@@ -25,8 +25,8 @@ __host__ __device__ __forceinline__ Tap make_tap(int dst, int in_size, int out_s
 __global__ void __launch_bounds__(256)
 bilinear_kernel(const float4* __restrict__ x, float4* __restrict__ y, int Hi, int Wi, int Ho, int Wo, int C4, int act,
                 int rows) {
-    pdl_launch_next();
     pdl_wait();
+    pdl_launch_next();
     const int per_row = Wo * C4;
     const bool fixed_c = (blockDim.x % C4) == 0;          // a thread keeps its channel quad: no division per element
     const int c_fix = threadIdx.x % C4, x_step = blockDim.x / C4;
@@ -68,8 +68,8 @@ template <int ACT>
 __global__ void __launch_bounds__(128)
 conv0_down_kernel(const float* __restrict__ node, const float4* __restrict__ w, const float4* __restrict__ bias,
                   float4* __restrict__ y, int Hi, int Wi, int Ho, int Wo, int CQ, int npix) {
-    pdl_launch_next();
     pdl_wait();
+    pdl_launch_next();
     constexpr int act = ACT;
     __shared__ __align__(16) float patch[C0_PIX][16];
     __shared__ __align__(16) float wt[C0_PIX][4];
@@ -157,8 +157,8 @@ __global__ void __launch_bounds__(256)
 upsample_grid_kernel(const float4* __restrict__ uw, const float2* __restrict__ grid, const float4* __restrict__ wg,
                      const float4* __restrict__ bias, float4* __restrict__ y, int Hi, int Wi, int Ho, int Wo, int C4,
                      int rows) {
-    pdl_launch_next();
     pdl_wait();
+    pdl_launch_next();
     const int per_row = Wo * C4;
     // When the block size is a multiple of C4 a thread keeps its channel quad for every element: the three parameter
     // vectors stay in registers and the pixel index advances by a constant, without a division.
@@ -211,12 +211,12 @@ lerp_staged_kernel(const float4* __restrict__ x, float4* __restrict__ y, int Hi,
                    const float2* __restrict__ grid, const float4* __restrict__ wg, const float4* __restrict__ bias, int G,
                    int groups_per_img, int n_groups) {
     extern __shared__ float4 srow[];                       // the source rows of the current group
-    pdl_launch_next();
     const int row_f4 = Wi * C4, per_row = Wo * C4;
     const int c = threadIdx.x % C4, x0 = threadIdx.x / C4, x_step = blockDim.x / C4;     // blockDim.x % C4 == 0 (host)
     float4 g0 = make_float4(0.f, 0.f, 0.f, 0.f), g1 = g0, bb = g0;
     if (MODE == 1) { g0 = __ldca(wg + c); g1 = __ldca(wg + C4 + c); bb = __ldca(bias + c); }
     pdl_wait();
+    pdl_launch_next();
     for (int grp = blockIdx.x; grp < n_groups; grp += gridDim.x) {
         const int b = grp / groups_per_img, y0 = (grp - b * groups_per_img) * G;
         const int y1 = y0 + G < Ho ? y0 + G : Ho;
@@ -303,8 +303,8 @@ __global__ void __launch_bounds__(256)
 bilinear_concat3_kernel(const float* __restrict__ x1, const float* __restrict__ x2, const float* __restrict__ x3, int p1,
                         int p2, int p3, int c1, int c2, int c3, float4* __restrict__ y, int Hi, int Wi, int Ho, int Wo,
                         int act, int rows) {
-    pdl_launch_next();
     pdl_wait();
+    pdl_launch_next();
     const int C4 = (c1 + c2 + c3) / 4;
     const int per_row = Wo * C4;
     for (int row = blockIdx.x; row < rows; row += gridDim.x) {

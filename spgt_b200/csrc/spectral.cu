@@ -120,11 +120,11 @@ __global__ void __launch_bounds__(256)
 spectral_fwd_x_kernel(const float* __restrict__ Y1, const float* __restrict__ tab, float* __restrict__ Zr,
                       float* __restrict__ Zi, int r, int m) {
     extern __shared__ __align__(16) float smem[];
-    pdl_launch_next();
     const SpecTables T = spec_tables(r, m);
     float* gr = smem; float* gi = smem + T.J * r;
     for (int i = threadIdx.x; i < 2 * T.J * r; i += blockDim.x) smem[i] = __ldca(tab + T.gr + i);
     pdl_wait();
+    pdl_launch_next();
     __syncthreads();
     const int ky = blockIdx.x; const int64_t b = blockIdx.y;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -160,11 +160,11 @@ spectral_mix_kernel(const float* __restrict__ Zr, const float* __restrict__ Zi, 
                     const float* __restrict__ fw1, float* __restrict__ Or, float* __restrict__ Oi, int B, int m,
                     const float* __restrict__ wr, float* __restrict__ wr_img) {
     __shared__ float2 w[SP_C * SP_C];
-    pdl_launch_next();
     const int q = blockIdx.x / m, ky = blockIdx.x % m;
     const float2* src = reinterpret_cast<const float2*>(q < m ? fw0 : fw1) + ((int64_t)(q < m ? q : q - m) * m + ky) * SP_C * SP_C;
     for (int i = threadIdx.x; i < SP_C * SP_C; i += blockDim.x) w[i] = __ldca(src + i);
     pdl_wait();
+    pdl_launch_next();
     if (blockIdx.x == 0 && wr_img != nullptr)            // W stage image of the residual weight Wr [i][o] for the y-inverse GEMM
         for (int i = threadIdx.x; i < SP_C * SP_C; i += blockDim.x) tc_img_store(wr_img, SP_C, i % SP_C, i / SP_C, __ldca(wr + i));
     __syncthreads();
@@ -191,11 +191,11 @@ __global__ void __launch_bounds__(256)
 spectral_inv_x_kernel(const float* __restrict__ Or, const float* __restrict__ Oi, const float* __restrict__ tab,
                       float* __restrict__ Pimg, int r, int m) {
     extern __shared__ __align__(16) float smem[];
-    pdl_launch_next();
     const SpecTables T = spec_tables(r, m);
     float* gr = smem; float* gi = smem + T.J * r;
     for (int i = threadIdx.x; i < 2 * T.J * r; i += blockDim.x) smem[i] = __ldca(tab + T.gr + i);
     pdl_wait();
+    pdl_launch_next();
     __syncthreads();
     const int ky = blockIdx.x; const int64_t b = blockIdx.y;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -241,7 +241,6 @@ __global__ void __launch_bounds__(256)
 spectral_fwd_x_mma_kernel(const float* __restrict__ Y1, const float* __restrict__ tab, float* __restrict__ Zr,
                           float* __restrict__ Zi, int r, int m) {
     extern __shared__ __align__(16) float smem[];
-    pdl_launch_next();
     const SpecTables T = spec_tables(r, m);
     const int J = T.J, M2 = 2 * J, MT = (M2 + 15) / 16;
     const int r8 = (r + 7) / 8 * 8;
@@ -254,6 +253,7 @@ spectral_fwd_x_mma_kernel(const float* __restrict__ Y1, const float* __restrict_
     for (int i = tid; i < 16 * MT * GP / 4; i += 256) cp_async_zfill<16>(gs + 4 * i, tab + T.ga + 4 * i, true);   // padded G, as stored
     cp_async_commit();
     pdl_wait();
+    pdl_launch_next();
     // Y block: 16 float4 per x (8 from the real row, 8 from the imaginary row)
     const float* yb = Y1 + b * (int64_t)r * J * SP_C;
     for (int i = tid; i < r8 * 16; i += 256) {
@@ -325,7 +325,6 @@ __global__ void __launch_bounds__(256)
 spectral_inv_x_mma_kernel(const float* __restrict__ Or, const float* __restrict__ Oi, const float* __restrict__ tab,
                           float* __restrict__ P, int r, int m) {
     extern __shared__ __align__(16) float smem[];
-    pdl_launch_next();
     const SpecTables T = spec_tables(r, m);
     const int J = T.J, M2 = 2 * J, K8 = (M2 + 7) / 8 * 8;
     const int r16 = (r + 15) / 16 * 16;
@@ -338,6 +337,7 @@ spectral_inv_x_mma_kernel(const float* __restrict__ Or, const float* __restrict_
     for (int i = tid; i < K8 * GP / 4; i += 256) cp_async_zfill<16>(gs + 4 * i, tab + T.gc + 4 * i, true);     // padded G, as stored
     cp_async_commit();
     pdl_wait();
+    pdl_launch_next();
     for (int i = tid; i < K8 * 64; i += 256) {
         const int k = i >> 6, n = i & 63;
         float v = 0.0f;
@@ -471,6 +471,7 @@ extern "C" int spgt_spectral_conv2d_fwd(const float* x, const float* wr, const f
     // 0 * NaN would still spoil the sum), so the images are cleared first.
     if (!staged && cudaMemsetAsync(P, 0, (size_t)CH * r * SP_IMG * sizeof(float), st) != cudaSuccess) return launch_status();
     int e;
+    const ChainScope chain;
     for (int b0 = 0; b0 < B; b0 += CH) {
         const int nb = B - b0 < CH ? B - b0 : CH;
         const float* xc = x + (size_t)b0 * r * r * C;

@@ -5,6 +5,12 @@
 namespace spgt {
 
 constexpr int TC_BM = 128, TC_BK = 32;
+
+// Parameters of the projection epilogue of tc_gemm.cu.
+struct TcProjEpi {          // column tile p = 0,1,2 -> q, k, v; 128 columns = 4 heads of 32
+    const float* bias[3]; const float* lnw[3]; const float* lnb[3]; float* out[3]; float* invsigma[3]; const float* pos;
+    float eps; int S, H, d_pos;
+};
 constexpr unsigned long long TC_WAIT_LIMIT_NS = 2000000000ull;   // a wait gives up after two seconds of wall time
 
 // ---- mbarrier / tcgen05 primitives -------------------------------------------------------------------------

@@ -53,7 +53,6 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv3x3_kernel(const ConvParams
     using C = CvCfg<BN>;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t smem_base = smem_u32(smem);
-    pdl_launch_next();
     if (smem_base & 1023u) {
         if (threadIdx.x == 0) atomicCAS(&g_conv_status, 0, 80);
         return;
@@ -88,6 +87,7 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv3x3_kernel(const ConvParams
     tc_fence_after();
     const uint32_t tmem_base = tc_uniform(*tmem_slot);
     pdl_wait();
+    pdl_launch_next();
 
     if (warp < 8) {
         // ------------------------------------------ load and split ------------------------------------------

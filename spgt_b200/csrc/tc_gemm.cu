@@ -74,6 +74,10 @@ struct TcLoaderDefaults {
     // With W_CONVERT and two k-blocks: the prepared image of the first k-block is the same for every unit and stays in the
     // last W stage (loaded once), the ring of the other stages carries the converted blocks only.
     static constexpr bool W_TAIL_RESIDENT = false;
+    // W comes as it is, [K][BN] fp32 per column tile, and every block splits it into its resident images itself (w_raw(column tile)):
+    // for entry points that get the weight with the call, where a launch that prepares images would cost more.
+    static constexpr bool W_RAW = false;
+    __device__ __forceinline__ const float* w_raw(int) const { return nullptr; }
     __device__ __forceinline__ const float* const_row(int) const { return nullptr; }
     __device__ __forceinline__ const float* w_plain(int) const { return nullptr; }
     __device__ __forceinline__ int w_plain_rows() const { return 0; }
@@ -93,6 +97,11 @@ struct TcDense : TcLoaderDefaults {
         Kst k; k.kc = kb * TC_BK + chunk * 4; k.ok = k.kc < K; if (!k.ok) k.kc = 0; return k;
     }
     __device__ __forceinline__ const float* ptr(const Row& r, const Kst& k, bool& ok) const { ok = r.ok && k.ok; return r.p + k.kc; }
+};
+struct TcDenseRaw : TcDense {
+    static constexpr bool W_RAW = true;
+    const float* w[3];
+    __device__ __forceinline__ const float* w_raw(int nt) const { return w[nt]; }
 };
 struct TcConv : TcLoaderDefaults {          // 3x3, padding 1, NHWC; k = tap * Cin + c with Cin % 4 == 0
     static constexpr bool EPI_COLSPLIT = true;
@@ -231,10 +240,6 @@ struct TcSpecFwd : TcLoaderDefaults {
 struct TcLinearEpi {
     const float* bias; const float* residual; int ldr; float* y; int ldc; int N; int act;
 };
-struct TcProjEpi {          // column tile p = 0,1,2 -> q, k, v; 128 columns = 4 heads of 32
-    const float* bias[3]; const float* lnw[3]; const float* lnb[3]; float* out[3]; const float* pos;
-    float eps; int S, H, d_pos;
-};
 struct TcHeadEpi {
     const float* b1; const float* w2; float b2, scale, shift; const float* scale_map; const float* shift_map;
     int dirichlet, Hh, Ww, act; float* out;
@@ -293,7 +298,6 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
     constexpr int TC_THREADS = tc_threads(MT, EG), TC_EPI_WARP0 = tc_epi_warp0(MT);
     static_assert(EG == 1 || (EG == 2 && (CS || C::NBUF == 2) && (EPI == EPI_LINEAR || EPI == EPI_HEAD)), "two epilogue groups: one per accumulator buffer, or sharing every unit");
     extern __shared__ uint8_t smem_raw[];
-    pdl_launch_next();
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;          // 1024-aligned for the 128B swizzle
     uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
     uint8_t* staging = smem + C::SB * C::B_BYTES + SR * C::RAW_BYTES;
@@ -392,6 +396,22 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
     }
 
     pdl_wait();
+    pdl_launch_next();
+    if constexpr (Loader::W_RAW) {
+        // item: column n, four consecutive k (lanes read consecutive columns, the 16-byte stores of eight lanes fall into different banks)
+        const float* wr = ld.w_raw(blockIdx.x % n_tiles);
+        for (int i = tid; i < BN * (kpad / 4); i += TC_THREADS) {
+            const int n = i % BN, k4 = i / BN;
+            uint32_t h[4], l[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) split_tf32_rn(__ldg(wr + (k4 * 4 + e) * BN + n), h[e], l[e]);
+            uint8_t* stage = smem + (k4 >> 3) * B_STAGE + tc_swz(n, k4 & 7);
+            *reinterpret_cast<uint4*>(stage) = make_uint4(h[0], h[1], h[2], h[3]);
+            *reinterpret_cast<uint4*>(stage + BN * TC_BK * 4) = make_uint4(l[0], l[1], l[2], l[3]);
+        }
+        fence_proxy_async();
+        __syncthreads();
+    }
     // Work distribution: this CTA keeps one column tile (so a resident W is loaded once) and strides over row units.
     const int sched_id = blockIdx.x, sched_n = gridDim.x;
     const int ctas_per_nt = sched_n / n_tiles;
@@ -564,7 +584,7 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
             }
             cp_async_wait_all();
         } else
-        if (lane == 0 && n_my_units > 0) {
+        if (!Loader::W_RAW && lane == 0 && n_my_units > 0) {
             const uint32_t bytes = C::B_BYTES;
             const int64_t total = resident ? KB : (int64_t)n_my_units * KB;
             TcRing rb;
@@ -617,7 +637,7 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
                     bool oka = true, okb = true;
                     if (a_ring) oka = mbar_wait(a_full(sa), pa, abort_flag, 3, &g_tc_status);
                     if (!oka) { alive = false; break; }
-                    if ((!resident && !tail) || ui == 0) {
+                    if (!Loader::W_RAW && ((!resident && !tail) || ui == 0)) {
                         okb = mbar_wait(b_full(sb), (resident || tail) ? 0u : rb.ph, abort_flag, 7, &g_tc_status);
                         if (!okb) { alive = false; break; }
                     }
@@ -865,6 +885,7 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
                         const float4 bb = c4[j4];
                         v[4 * j4] += bb.x; v[4 * j4 + 1] += bb.y; v[4 * j4 + 2] += bb.z; v[4 * j4 + 3] += bb.w;
                     }
+                    float inv_out = 0.0f;
                     if (lnw != nullptr) {
                         float s = 0.0f;
 #pragma unroll
@@ -874,6 +895,7 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
 #pragma unroll
                         for (int j = 0; j < 32; ++j) { const float d = v[j] - mu; qq += d * d; }
                         const float inv = 1.0f / sqrtf(qq * (1.0f / 32.0f) + e.eps);
+                        inv_out = inv;
 #pragma unroll
                         for (int j4 = 0; j4 < 8; ++j4) {
                             const float4 w = c4[32 + j4], lb = c4[64 + j4];
@@ -883,6 +905,7 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
                             v[4 * j4 + 3] = (v[4 * j4 + 3] - mu) * inv * w.w + lb.w;
                         }
                     }
+                    if (rok && e.invsigma[p] != nullptr) e.invsigma[p][((int64_t)b * e.H + hd) * e.S + s_] = inv_out;
                     if (rok) {
                         float* o = out + (((int64_t)b * e.H + hd) * dpk + e.d_pos) * e.S + s_;
 #pragma unroll
@@ -942,13 +965,15 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
 
 // ---- weight preparation: [K][ldw] row-major fp32 -> per (column tile, k-block) the exact shared-memory image the
 // kernel needs: W_hi then W_lo, each [bn rows (n)][32 k] K-major with the 128-byte swizzle applied, zero padded.
+// T: w is [N][ldw] (the matrix transposed).
+template <bool T>
 __global__ void tc_weight_prepare_kernel(const float* __restrict__ w, int ldw, int K, int N, int kpad, int npad, int bn,
                                          float* __restrict__ img) {
     const int64_t total = (int64_t)npad * kpad;
     const int KB = kpad / TC_BK;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int n = (int)(i / kpad), k = (int)(i % kpad);
-        const float v = (n < N && k < K) ? __ldg(w + (int64_t)k * ldw + n) : 0.0f;
+        const float v = (n < N && k < K) ? __ldg(T ? w + (int64_t)n * ldw + k : w + (int64_t)k * ldw + n) : 0.0f;
         const int nt = n / bn, kb = k / TC_BK;
         tc_img_store(img + ((int64_t)nt * KB + kb) * (2 * bn * TC_BK), bn, n % bn, k % TC_BK, v);
     }
@@ -1000,7 +1025,7 @@ static int tc_dispatch_linear(Loader ld, const float* wprep, int K, int N, int r
 // W image of a [K][N <= 32] matrix (pitch ldw) for 32-wide column tiles: 2 * 32 * ceil(K / 32) * 32 floats.
 int spectral_tc_prepare(const float* w_kn, int ldw, int K, int N, float* img, cudaStream_t st) {
     const int kpad = ceil_div(K, TC_BK) * TC_BK;
-    tc_weight_prepare_kernel<<<ceil_div(32 * kpad, 256), 256, 0, st>>>(w_kn, ldw, K, N, kpad, 32, 32, img);
+    tc_weight_prepare_kernel<false><<<ceil_div(32 * kpad, 256), 256, 0, st>>>(w_kn, ldw, K, N, kpad, 32, 32, img);
     return launch_status();
 }
 // Y1[image row][j][c] = sum_y F1[j][y] X[image row][y][c] for nimg image rows of r x 32 floats; f1_img = image of F1^T.
@@ -1031,6 +1056,14 @@ int spectral_inv_y_tc(const float* x, const float* f3, const float* wr_img, cons
     return tc_launch<32, 2, TcSpecInv, EPI_LINEAR, TcLinearEpi>(ld, wr_img, 64, ld.rows, 1, ep, st);
 }
 
+// Projection (+ per-head LayerNorm) + position rows of width 128 from plain weights [128][128] (called from gemm.cu): nproj of them.
+int projpos_tc(const float* x, int nproj, const float* const* w, const TcProjEpi& ep, int rows, cudaStream_t st) {
+    TcDenseRaw ld;
+    ld.x = x; ld.lda = 128; ld.rows = rows; ld.K = 128;
+    for (int i = 0; i < 3; ++i) ld.w[i] = w[i < nproj ? i : 0];
+    return tc_launch<128, 1, TcDenseRaw, EPI_PROJ, TcProjEpi>(ld, nullptr, 128, rows, nproj, ep, st);
+}
+
 }  // namespace spgt
 
 using namespace spgt;
@@ -1041,16 +1074,21 @@ extern "C" size_t spgt_tc_weight_bytes(int K, int N) {
     return (size_t)2 * (ceil_div(N, bn) * bn) * (ceil_div(K, TC_BK) * TC_BK) * sizeof(float);
 }
 
-extern "C" int spgt_tc_weight_prepare(const float* w_kn, int ldw, int K, int N, void* out, size_t out_bytes,
-                                      spgt_stream_t stream) {
-    if (!w_kn || !out) return SPGT_ERR_NULL;
-    if (K <= 0 || N <= 0 || ldw < N) return SPGT_ERR_SHAPE;
+static int weight_prepare(bool transposed, const float* w, int ldw, int K, int N, void* out, size_t out_bytes, spgt_stream_t stream) {
+    if (!w || !out) return SPGT_ERR_NULL;
+    if (K <= 0 || N <= 0 || ldw < (transposed ? K : N)) return SPGT_ERR_SHAPE;
     if (out_bytes < spgt_tc_weight_bytes(K, N)) return SPGT_ERR_WORKSPACE;
     if (!aligned16(out)) return SPGT_ERR_ALIGN;
     const int bn = tc_bn_for(N, K), kpad = ceil_div(K, TC_BK) * TC_BK, npad = ceil_div(N, bn) * bn;
-    tc_weight_prepare_kernel<<<ceil_div(npad * kpad, 256), 256, 0, (cudaStream_t)stream>>>(w_kn, ldw, K, N, kpad, npad, bn,
-                                                                                         (float*)out);
+    auto kern = transposed ? tc_weight_prepare_kernel<true> : tc_weight_prepare_kernel<false>;
+    kern<<<ceil_div(npad * kpad, 256), 256, 0, (cudaStream_t)stream>>>(w, ldw, K, N, kpad, npad, bn, (float*)out);
     return launch_status();
+}
+extern "C" int spgt_tc_weight_prepare(const float* w_kn, int ldw, int K, int N, void* out, size_t out_bytes, spgt_stream_t stream) {
+    return weight_prepare(false, w_kn, ldw, K, N, out, out_bytes, stream);
+}
+extern "C" int spgt_tc_weight_prepare_t(const float* w_nk, int ldw, int K, int N, void* out, size_t out_bytes, spgt_stream_t stream) {
+    return weight_prepare(true, w_nk, ldw, K, N, out, out_bytes, stream);
 }
 
 
@@ -1058,7 +1096,7 @@ namespace spgt {
 int attn_tc_status(); int ffn_tc_status();          // attention_tc.cu, tc_ffn.cu
 int attn_tc_status_reset(); int ffn_tc_status_reset();
 int encoder_kv_status(bool reset); int encoder_out_status(bool reset);     // encoder_kv.cu, encoder_out.cu
-int conv_status(bool reset);            // tc_conv.cu
+int conv_status(bool reset); int tn_status(bool reset);     // tc_conv.cu, tc_tn.cu
 
 // One warp waits on a barrier that nobody arrives at, with a limit of `limit_us` microseconds instead of the two
 // seconds of the production kernels: the wait gives up, latches `code` in the status word and the kernel returns.
@@ -1087,6 +1125,7 @@ extern "C" int spgt_tc_status(void) {
     if (int e = spgt::encoder_kv_status(false)) return e;       // 40..52: the first half of an encoder layer
     if (int e = spgt::encoder_out_status(false)) return e;      // 60..76: its second half
     if (int e = spgt::conv_status(false)) return e;             // 80..86: the convolution kernel
+    if (int e = spgt::tn_status(false)) return e;               // 90..96: the weight-gradient kernel
     return spgt::ffn_tc_status();               // 21..33: a wait of the fused feed-forward kernel gave up
 }
 
@@ -1097,6 +1136,7 @@ extern "C" int spgt_tc_status_reset(void) {
     if (int e = spgt::encoder_kv_status(true)) return e;
     if (int e = spgt::encoder_out_status(true)) return e;
     if (int e = spgt::conv_status(true)) return e;
+    if (int e = spgt::tn_status(true)) return e;
     return spgt::ffn_tc_status_reset();
 }
 

@@ -49,7 +49,7 @@ class _device:
 
 
 # kernels launched by one call of each entry point (everything else launches one)
-_KERNELS_PER_CALL = {'spgt_batched_skinny_gemm': 2, 'spgt_galerkin_attn_bwd': 2, 'spgt_projpos_bwd_elementwise': 2}
+_KERNELS_PER_CALL = {'spgt_batched_skinny_gemm': 2, 'spgt_galerkin_attn_bwd': 3, 'spgt_projpos_bwd_elementwise': 2}
 LAUNCHES = 0          # running count of kernels launched through this module
 _PROFILE = None       # None, or a dict name -> list of (start_event, end_event) filled while profiling
 
@@ -172,7 +172,7 @@ def projpos_backward(x: Tensor, weight: Tensor, bias: Optional[Tensor], ln_weigh
                      norm_eps: float, num_head: int, dim_head: int, dim_position: int):
     """Gradients of projpos (ln_weight None) or projpos_lnorm with respect to (x, weight, bias, ln_weight, ln_bias) for
     grad_out [B, H, dim_position + dim_head, S].  The element-wise stage (gather, LayerNorm backward, parameter sums) is
-    one kernel; dX = dh W^T and dW = x^T dh reuse the tcgen05 linear and the transpose + split-K skinny GEMM."""
+    one kernel; dX = dh W^T is the tcgen05 linear, dW = x^T dh the weight-gradient kernel."""
     _chk(x, 'input'); _chk(weight, 'weight'); _chk(grad_out, 'grad_out')
     B, S, D = x.shape
     if grad_out.shape != (B, num_head, dim_position + dim_head, S) or D != num_head * dim_head:
@@ -188,9 +188,8 @@ def projpos_backward(x: Tensor, weight: Tensor, bias: Optional[Tensor], ln_weigh
     with _device(x.device):
         _call('spgt_projpos_bwd_elementwise', grad_out.data_ptr(), _p(h), _p(ln_weight), float(norm_eps), dh.data_ptr(), db.data_ptr(),
               _p(dlnw), _p(dlnb), B, S, num_head, dim_head, dim_position, ws.data_ptr(), need, _stream())
-    dx = linear_tc(dh, TcWeight(weight.t().contiguous()), None).view(B, S, D)
-    xT = batched_transpose(x2, [1], [B * S], [D])                       # [1, D, rows]
-    dW = batched_skinny_gemm(xT, dh.view(1, B * S, D), 1.0).view(D, D)
+    dx = linear_tc(dh, TcWeight(weight, transposed=True), None).view(B, S, D)
+    dW, _ = tn_gemm(x2, dh)
     shape = ln_weight.shape if ln_weight is not None else None
     return dx, dW, db, (dlnw.view(shape) if dlnw is not None else None), (dlnb.view(shape) if dlnb is not None else None)
 
@@ -408,13 +407,14 @@ def decoder_head(x: Tensor, w1_kn: Tensor, b1: Tensor, w2: Tensor, b2: float, sc
 class TcWeight:
     """A [K, N] weight prepared for the tcgen05 kernels (tf32 hi/lo planes, K-major, padded)."""
 
-    def __init__(self, w_kn: Tensor):
+    def __init__(self, w_kn: Tensor, transposed: bool = False):
+        """transposed: the argument is [N, K], a torch Linear weight as it is."""
         _chk(w_kn, 'weight')
-        self.K, self.N = w_kn.shape
+        self.K, self.N = reversed(w_kn.shape) if transposed else w_kn.shape
         n = int(lib.spgt_tc_weight_bytes(self.K, self.N))
         self.buf = torch.empty(n, dtype=torch.uint8, device=w_kn.device)
         with _device(w_kn.device):
-            _call('spgt_tc_weight_prepare', w_kn.data_ptr(), w_kn.shape[1], self.K, self.N, self.buf.data_ptr(), n, _stream())
+            _call('spgt_tc_weight_prepare_t' if transposed else 'spgt_tc_weight_prepare', w_kn.data_ptr(), w_kn.shape[1], self.K, self.N, self.buf.data_ptr(), n, _stream())
 
     def data_ptr(self) -> int:
         return self.buf.data_ptr()
@@ -480,6 +480,21 @@ def ffn_tc(x: Tensor, w1: TcWeight, b1: Tensor, w2: TcWeight, b2: Optional[Tenso
         _call('spgt_ffn_tc_fwd', x.data_ptr(), D, w1.data_ptr(), b1.data_ptr(), w2.data_ptr(), _p(b2), _p(residual), D,
               out.data_ptr(), D, rows, D, w1.N, act_code(act), _stream())
     return out
+
+
+def tn_gemm(a: Tensor, b: Tensor, column_sums: bool = False):
+    """(a^T b, column sums of b or None) for a [rows, M], b [rows, N]: weight and bias gradient of a linear layer."""
+    _chk(a, 'a'); _chk(b, 'b')
+    rows, M, N = a.shape[0], a.shape[1], b.shape[1]
+    if b.shape[0] != rows or M % 4 or N % 4:
+        raise ValueError('a and b must be [rows, M] and [rows, N] with M and N multiples of 4')
+    c = torch.empty(M, N, device=a.device, dtype=a.dtype)
+    sums = torch.empty(N, device=a.device, dtype=a.dtype) if column_sums else None
+    need = int(lib.spgt_tn_gemm_workspace_bytes(M, N, rows))
+    ws = torch.empty(need, dtype=torch.uint8, device=a.device)
+    with _device(a.device):
+        _call('spgt_tn_gemm', a.data_ptr(), M, b.data_ptr(), N, c.data_ptr(), N, _p(sums), M, N, rows, ws.data_ptr(), need, _stream(), kernels=2)
+    return c, sums
 
 
 def conv3x3_tc(x: Tensor, cin_off: int, Cin: int, w, bias: Tensor, y: Tensor, cout_off: int, Cout: int, act) -> Tensor:

@@ -62,3 +62,18 @@ def test_conv3x3_shared_memory_operands(B, Hh, Ww, Cin, Cout, act):
     ref = {None: lambda t: t, 'relu': torch.relu, 'silu': silu, 'silu2': lambda t: silu(silu(t))}[act](ref)
     assert rel_l2(y[..., 4:4 + Cout], ref.permute(0, 2, 3, 1)) < TOL
     assert torch.isnan(y[..., :4]).all() and torch.isnan(y[..., 4 + Cout:]).all()
+
+
+# rows: one, around a 32-row block, around the 512-row accumulator chain, many blocks; widths: tails of the 128-wide tiles
+@pytest.mark.parametrize('rows,M,N', [(1, 4, 4), (31, 128, 128), (33, 132, 36), (513, 128, 256), (1000, 256, 128), (7396, 136, 128), (65536, 128, 128), (79524, 32, 128)])
+def test_weight_gradient_gemm(rows, M, N):
+    from spgt_b200 import ops
+    g = torch.Generator().manual_seed(rows)
+    a, b = torch.randn(rows, M, generator=g), torch.randn(rows, N, generator=g)
+    c, s = ops.tn_gemm(a.cuda(), b.cuda(), column_sums=True)
+    assert ops.tc_status() == 0
+    # sums of `rows` products of independent entries: fp32 accumulation errors grow with the square root of their number, as the sums do
+    assert rel_l2(c, a.double().t() @ b.double()) < TOL
+    assert rel_l2(s, b.double().sum(0)) < TOL
+    c2, s2 = ops.tn_gemm(a.cuda(), b.cuda(), column_sums=True)
+    assert torch.equal(c, c2) and torch.equal(s, s2)
