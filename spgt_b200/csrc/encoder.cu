@@ -29,7 +29,7 @@ extern "C" int spgt_encoder_layer_fwd(const spgt_encoder_weights* w, const float
     const size_t need = spgt_encoder_workspace_bytes(B, S);
     if (need == 0) return SPGT_ERR_SHAPE;
     if (workspace_bytes < need) return SPGT_ERR_WORKSPACE;
-    if (!aligned16(x) || !aligned16(pos) || !aligned16(y) || !aligned16(workspace) || !aligned16(w->wkv) || !aligned16(w->wq) || !aligned16(w->wfc) ||
+    if (!aligned16(x) || (reinterpret_cast<uintptr_t>(pos) & 7u) || !aligned16(y) || !aligned16(workspace) || !aligned16(w->wkv) || !aligned16(w->wq) || !aligned16(w->wfc) ||
         (ffn && (!aligned16(w->w1) || !aligned16(w->w2))))
         return SPGT_ERR_ALIGN;
     const EncoderSplit sp = encoder_split(B, S, num_sms());

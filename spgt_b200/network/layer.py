@@ -9,30 +9,52 @@ kernels.
 """
 import torch
 from torch import Tensor
+from torch.nn.modules import module as _hooks
 
 from .. import ops
 
 
 class ParameterWatch:
-    """Tells when a module's parameters are not the ones seen before: tag() differs after a parameter has been written to
-    (an optimizer step bumps the version counters), moved, or replaced, or a submodule has been exchanged.  The tree is walked
-    once, not on every call (Module.parameters() takes longer than the launch it would guard)."""
+    """Tells when a module is not as it was seen before: tag() differs after a parameter has been written to (an optimizer step
+    bumps the version counters), moved, or replaced, a submodule has been exchanged, or an option that kernels are chosen by
+    has been set.  The tree is walked once, not on every call (Module.parameters() takes longer than the launch it would guard)."""
+    OPTIONS = ('activation', 'norm_eps', 'mode', 'structure', 'fused')
 
     def __init__(self):
-        self.tree = None         # (no reference to the module itself: a cycle would keep its memory until a garbage collection)
+        self._tree = None        # one tuple, replaced whole: several threads may share a module
+                                 # (no reference to the module itself: a cycle would keep its memory until a garbage collection)
+
+    def _walk(self, module: torch.nn.Module) -> tuple:
+        modules = list(module.modules())
+        return ([(d, len(d)) for m in modules for d in (m._modules, m._parameters)],
+                [(m._modules, k, c) for m in modules for k, c in m._modules.items()],
+                [(m._parameters, k) for m in modules for k, p in m._parameters.items() if p is not None],
+                [(m.__dict__, k) for m in modules for k in self.OPTIONS if k in m.__dict__],
+                [m.__dict__ for m in modules[1:]])
+
+    def _seen(self, module: torch.nn.Module) -> tuple:
+        tree = self._tree
+        if tree is None or any(len(d) != n for d, n in tree[0]) or any(d[k] is not c for d, k, c in tree[1]):
+            tree = self._tree = self._walk(module)
+        return tree
 
     def tag(self, module: torch.nn.Module) -> tuple:
-        if self.tree is None or any(len(d) != n for d, n in self.sizes) or any(d[k] is not c for d, k, c in self.tree):
-            modules = list(module.modules())
-            self.sizes = [(d, len(d)) for m in modules for d in (m._modules, m._parameters)]
-            self.tree = [(m._modules, k, c) for m in modules for k, c in m._modules.items()]
-            self.slots = [(m._parameters, k) for m in modules for k, p in m._parameters.items() if p is not None]
-        params = [d[k] for d, k in self.slots]
-        return tuple([p._version for p in params] + [p.data_ptr() for p in params])
+        tree = self._seen(module)
+        params = [d[k] for d, k in tree[2]]
+        return tuple([p._version for p in params] + [p.data_ptr() for p in params] + [d[k] for d, k in tree[3]])
 
-    def hold(self) -> list:
+    def observed(self, module: torch.nn.Module) -> bool:
+        """Whether a submodule's call can be told from a call of its kernels: forward hooks, or a forward of its own."""
+        if _hooks._global_forward_hooks or _hooks._global_forward_pre_hooks:
+            return True
+        return any(d['_forward_hooks'] or d['_forward_pre_hooks'] or 'forward' in d for d in self._seen(module)[4])
+
+    def hold(self, module: torch.nn.Module) -> list:
         """Aliases of the parameters' storages: while they are kept, no other tensor can come to lie at these addresses."""
-        return [d[k].detach() for d, k in self.slots]
+        return [d[k].detach() for d, k in self._seen(module)[2]]
+
+    def __deepcopy__(self, memo):
+        return ParameterWatch()
 
 
 class _KernelWeights(torch.nn.Module):
@@ -48,15 +70,24 @@ class _KernelWeights(torch.nn.Module):
         self._kw.clear()
         return super()._apply(fn, *args, **kwargs)
 
+    def __getstate__(self):
+        return {**self.__dict__, '_kw': {}}      # derived layouts (device pointers among them) are not copied with the module
+
     def _cached(self, key, make):
         """Derived layout of the module's weights, rebuilt when a parameter is not the one it was made from."""
         tag = self._watch.tag(self)
         hit = self._kw.get(key)
         if hit is None or hit[0] != tag:
             with torch.no_grad():
-                hit = (tag, make(), self._watch.hold())
+                hit = (tag, make(), self._watch.hold(self))
             self._kw[key] = hit
         return hit[1]
+
+
+def _dense(weight: Tensor) -> Tensor:
+    """A weight that a kernel reads as it is: row-major and 16-byte aligned, copied only where it is not."""
+    w = weight.detach().contiguous()
+    return w if w.data_ptr() % 16 == 0 else w.clone()
 
 
 def _linear_kn(weight: Tensor) -> Tensor:

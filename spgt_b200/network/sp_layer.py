@@ -13,7 +13,7 @@ import torch
 from torch import Tensor
 
 from .. import ops
-from .layer import FeedForward, _KernelWeights, _act, _linear_kn, _linear_tc
+from .layer import FeedForward, _KernelWeights, _act, _dense, _linear_kn, _linear_tc
 
 
 class Sp_GalerkinAttention(_KernelWeights):
@@ -56,12 +56,12 @@ class Sp_GalerkinAttention(_KernelWeights):
     @property
     def fusable(self) -> bool:
         """Whether the fused layer kernels cover these widths."""
-        return self.dim_hidden == 128 and self.num_head == 4 and self.dim_position == 2
+        return self.dim_hidden == 128 and self.num_head == 4 and self.dim_head == 32 and self.dim_position == 2
 
     def fill_native(self, w, ptr) -> None:
         """Device pointers of this layer's weights into a spgt_encoder_weights; `ptr` keeps what it is given alive."""
-        w.wkv, w.wq = ptr(self.kv_weight()), ptr(self.weight_Q.detach())
-        w.wfc, w.bfc = ptr(self.fc_layer.weight.detach()), ptr(self.fc_layer.bias.detach())
+        w.wkv, w.wq = ptr(self.kv_weight()), ptr(_dense(self.weight_Q))
+        w.wfc, w.bfc = ptr(_dense(self.fc_layer.weight)), ptr(self.fc_layer.bias.detach())
         w.bq, w.bk, w.bv = (ptr(b.detach()) for b in (self.bias_Q, self.bias_K, self.bias_V))
         w.lnwk, w.lnbk, w.lnwv, w.lnbv = (ptr(t.detach()) for t in (self.ln_weight_K, self.ln_bias_K, self.ln_weight_V, self.ln_bias_V))
 
@@ -69,7 +69,7 @@ class Sp_GalerkinAttention(_KernelWeights):
         """K and V weights as the fused layer takes them: by head pair K0 K1 V0 V1 | K2 K3 V2 V3, less each head's channel mean (the
         LayerNorm's subtraction, done once on the weights)."""
         def make():
-            centred = lambda w: (h := w.detach().view(-1, self.num_head, self.dim_head)) - h.mean(dim=2, keepdim=True)
+            centred = lambda w: (h := w.detach().reshape(-1, self.num_head, self.dim_head)) - h.mean(dim=2, keepdim=True)
             kv = torch.stack([centred(self.weight_K), centred(self.weight_V)], dim=1).view(-1, 2, 2, 64)      # [128, K | V, pair, 64]
             return ops.TcWeight(kv.transpose(1, 2).reshape(-1, 256).contiguous())
         return self._cached('wkv', make)
@@ -138,7 +138,7 @@ class Sp_EncoderLayer(_KernelWeights):
     def forward(self, X: Tensor, position: Tensor) -> Tensor:
         """X [N,S,D], position [N,S,d_pos] -> X + attention(X) then + ffn(.)  (network/sp_layer.py:94-104)."""
         f = self.ffn_layer
-        if self.fusable:
+        if self.fusable and not self._watch.observed(self):
             plan = self._cached('native', lambda: ops.EncoderPlan(self.fill_native))
             return ops.encoder_layer(plan, X, position, self.attention_layer.norm_eps, f.activation)
         X = self.attention_layer(X, X, X, position, residual=X)
@@ -147,7 +147,8 @@ class Sp_EncoderLayer(_KernelWeights):
     @property
     def fusable(self) -> bool:
         f = self.ffn_layer
-        return (self.attention_layer.fusable and f.layer1.in_features == 128 and f.layer1.out_features == 256
+        return (type(self.attention_layer) is Sp_GalerkinAttention and type(f) is FeedForward and f.fused
+                and self.attention_layer.fusable and f.layer1.in_features == 128 and f.layer1.out_features == 256
                 and f.layer2.out_features == 128)
 
     def forward_train(self, X: Tensor, position: Tensor) -> Tensor:

@@ -8,7 +8,7 @@ from torch import Tensor
 
 from .. import ops
 from .._lib import MAX_LAYERS, DarcyModel
-from .layer import FeedForward, ParameterWatch, _KernelWeights, _linear_kn, _linear_tc
+from .layer import ConvResBlock2D, FeedForward, ParameterWatch, _KernelWeights, _linear_kn, _linear_tc
 from .model import DownScaler2D, UpScaler2D
 from .sp_layer import Sp_EncoderLayer, Sp_SpectralConv2D
 
@@ -165,7 +165,7 @@ class Sp_GalerkinTransformer2D(torch.nn.Module):
         return X
 
     def _forward_fused(self, X: Tensor, position: Tensor, grid: Tensor, taps: dict = None) -> Tensor:
-        plan = self._native_plan(X)
+        plan = None if self._watch.observed(self) else self._native_plan(X)
         if plan is None:
             return self._forward_modules(X, position, grid, taps)
         return ops.darcy_forward(plan, X, position, grid, taps)
@@ -173,10 +173,21 @@ class Sp_GalerkinTransformer2D(torch.nn.Module):
     def _native_plan(self, X: Tensor):
         """The model as the one-call forward takes it, rebuilt when the parameters, the grid or the device are not the ones it was
         made for; None for widths that forward does not cover."""
-        tag = (X.shape[1], X.device, self.normalizer, self.boundary_condition, self._watch.tag(self))
-        if self._plan is None or self._plan[0] != tag:
-            self._plan = (tag, self._build_plan(X), self._watch.hold())
-        return self._plan[1]
+        sizes = [tuple(map(tuple, m.resolution_size)) for m in (self.down_scaler, self.up_scaler)]
+        tag = (X.shape[1], X.device, self.normalizer, self.boundary_condition, sizes, self._watch.tag(self))
+        plan = self._plan                                    # (read once: another thread may replace it)
+        if plan is None or plan[0] != tag:
+            plan = self._plan = (tag, self._build_plan(X), self._watch.hold(self))
+        return plan[1]
+
+    def __getstate__(self):
+        return {**self.__dict__, '_plan': None}              # device pointers are not copied with the module
+
+    def _normalizer_terms(self, r: int, device):
+        affine = self._affine
+        if affine is None or affine[0] != (r, device, self.normalizer):
+            affine = self._affine = ((r, device, self.normalizer), _normalizer_affine(self.normalizer, r, device))
+        return affine[1]
 
     def _apply(self, fn, *args, **kwargs):
         self._plan = self._affine = None
@@ -185,21 +196,15 @@ class Sp_GalerkinTransformer2D(torch.nn.Module):
     def _build_plan(self, X: Tensor):
         r, down, up, dec = X.shape[1], self.down_scaler, self.up_scaler, self.decoder_regressor
         enc = list(self.encoder_mixer.layers)
-        if sum(down.dims) != 128 or not self._native_widths() or max(len(enc), len(dec.layers)) > MAX_LAYERS:
+        if not self._native_widths() or sum(down.dims) != 128 or max(len(enc), len(dec.layers)) > MAX_LAYERS:
             return None
-        size = down.resolution_size
-        if size[0] != (r, r) or size[4] != (r, r) or size[3] != size[1] or any(a != b for a, b in size):
+        size = tuple(map(tuple, down.resolution_size))
+        if size != tuple(map(tuple, up.resolution_size)) or size[0] != (r, r) or size[4] != (r, r) or size[3] != size[1] or any(a != b for a, b in size):
             return None
-        if self._affine is None or self._affine[0] != (r, X.device, self.normalizer):
-            self._affine = ((r, X.device, self.normalizer), _normalizer_affine(self.normalizer, r, X.device))
-        scale, shift, scale_map, shift_map = self._affine[1]
+        scale, shift, scale_map, shift_map = self._normalizer_terms(r, X.device)
         keep = []
 
-        def ptr(t):
-            if t is None:
-                return None
-            keep.append(t)
-            return t.data_ptr()
+        ptr = lambda t: ops.kept_pointer(keep, t)
         m = DarcyModel()
         m.r, m.mid, m.ra, m.n_encoder, m.n_decoder = r, size[1][0], size[2][0], len(enc), len(dec.layers)
         m.d_pos = enc[0].attention_layer.dim_position if enc else dec.dim_position
@@ -224,23 +229,30 @@ class Sp_GalerkinTransformer2D(torch.nn.Module):
         m.fcx_w, m.fcg_w, m.fc_b = ptr(wx), ptr(wg), ptr(dec.spatial_fc_layer.bias.detach())
         for i, layer in enumerate(dec.layers):
             layer.fill_native(m.decoder[i], ptr)
-        m.tables = ptr(ops.spectral_tables(r, m.modes, X.device)) if len(dec.layers) else None
+        m.tables = ptr(ops.spectral_tables(r, m.modes, X.device).view(torch.float32)) if len(dec.layers) else None
         w1, w2, m.b2 = dec.head_weights()
         m.head_w1, m.head_b1, m.head_w2 = ptr(w1), ptr(dec.ffn_layer.layer1.bias.detach()), ptr(w2)
         return ops.DarcyPlan(m, keep)
 
     def _native_widths(self) -> bool:
-        enc, dec, up = self.encoder_mixer.layers, self.decoder_regressor, self.up_scaler
-        return (all(l.fusable for l in enc)
+        """Whether the one-call forward covers this model: its own module types, the widths the kernels are made for, and one
+        activation and epsilon throughout."""
+        enc, dec, down, up = self.encoder_mixer.layers, self.decoder_regressor, self.down_scaler, self.up_scaler
+        if not (type(down) is DownScaler2D and type(up) is UpScaler2D and type(dec) is Sp_DecoderRegressor
+                and all(type(l) is Sp_EncoderLayer for l in enc) and all(type(l) is Sp_SpectralConv2D for l in dec.layers)
+                and all(type(c) is ConvResBlock2D for c in (down.conv0, down.conv1, down.conv2, down.conv3, up.conv))):
+            return False
+        return (all(l.fusable and l.attention_layer.norm_eps == enc[0].attention_layer.norm_eps
+                    and l.ffn_layer.activation == enc[0].ffn_layer.activation for l in enc)
+                and all(c.activation == down.activation for c in (down.conv1, down.conv2, down.conv3))
                 and up.conv.conv_layer.in_channels == 128 and up.conv.conv_layer.out_channels == 128 and dec.in_dim == 128
                 and dec.dim_position == 2 and dec.spatial_fc_layer.out_features == 32 and dec.ffn_layer.layer1.out_features == 128
-                and all(l.structure == 'fused' and l.in_dim == 32 and l.out_dim == 32 for l in dec.layers))
+                and all(l.structure == 'fused' and l.in_dim == 32 and l.out_dim == 32 and l.activation == dec.activation
+                        and l.mode == dec.layers[0].mode for l in dec.layers))
 
     def _forward_modules(self, X: Tensor, position: Tensor, grid: Tensor, taps: dict = None) -> Tensor:
         r = X.shape[1]
-        if self._affine is None or self._affine[0] != (r, X.device, self.normalizer):
-            self._affine = ((r, X.device, self.normalizer), _normalizer_affine(self.normalizer, r, X.device))
-        scale, shift, scale_map, shift_map = self._affine[1]
+        scale, shift, scale_map, shift_map = self._normalizer_terms(r, X.device)
         X = self.down_scaler(X)
         if taps is not None:
             taps['down'] = X

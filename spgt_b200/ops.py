@@ -105,6 +105,12 @@ def _chk(t: Tensor, name: str, dtype=torch.float32) -> Tensor:
     return t
 
 
+def _position(t: Tensor, name: str) -> Tensor:
+    """Node coordinates for the kernels that read a node's two values at once: a copy where they start at an odd value."""
+    _chk(t, name)
+    return t if t.data_ptr() % 8 == 0 else t.clone()
+
+
 def _p(t: Optional[Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
@@ -577,22 +583,30 @@ def spectral_conv2d(x: Tensor, wr_kn: Tensor, br: Tensor, fw0: Tensor, fw1: Tens
 # ---------------------------------------------------------------------------------------------------------
 # encoder layer
 # ---------------------------------------------------------------------------------------------------------
+def kept_pointer(keep: list, t):
+    """Device pointer of a weight (tensor or prepared weight, or None) that `keep` holds from now on."""
+    if t is None:
+        return None
+    if isinstance(t, Tensor):
+        _chk(t, 'weight')
+    keep.append(t)
+    return t.data_ptr()
+
+
 class EncoderPlan:
     """A spgt_encoder_weights with the tensors it points to; `fill` writes the pointers (ptr(tensor) keeps the tensor)."""
 
     def __init__(self, fill):
         self.weights, self.keep, self.need = EncoderWeights(), [], {}
 
-        def ptr(t):
-            self.keep.append(t)
-            return None if t is None else t.data_ptr()
-        fill(self.weights, ptr)
+        fill(self.weights, lambda t: kept_pointer(self.keep, t))
         self.address = ctypes.addressof(self.weights)
 
 
 def encoder_layer(plan: EncoderPlan, x: Tensor, position: Tensor, eps: float, act=None, ffn: bool = True, residual: bool = True) -> Tensor:
     """x [B,S,128], position [B,S,2] -> the encoder layer's output (ffn), or the attention layer's (+ x with residual)."""
-    _chk(x, 'x'); _chk(position, 'position')
+    _chk(x, 'x')
+    position = _position(position, 'position')
     B, S, D = x.shape
     if D != 128 or position.shape != (B, S, 2):
         raise ValueError('x must be [B, S, 128] and position [B, S, 2]')
@@ -630,7 +644,8 @@ def darcy_forward(plan: DarcyPlan, node: Tensor, position: Tensor, grid: Tensor,
     """node [B,r,r,1], position [B,ra,ra,d_pos], grid [B,r,r,2] -> [B,r,r,1]; `taps` receives intermediate tensors."""
     m = plan.model
     B, r, S = node.shape[0], m.r, m.ra * m.ra
-    node, position, grid = _chk(node.contiguous(), 'node'), _chk(position.contiguous(), 'position'), _chk(grid.contiguous(), 'grid')
+    position = _position(position.reshape(B, S, position.size(-1)), 'position')
+    _chk(node, 'node'); _chk(grid, 'grid')
     if node.numel() != B * r * r or position.numel() != B * S * m.d_pos or grid.numel() != 2 * B * r * r:
         raise ValueError('node, position and grid do not match the model\'s grids')
     need, kernels = plan.size(B)

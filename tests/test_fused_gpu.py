@@ -77,3 +77,66 @@ def test_weight_gradient_gemm(rows, M, N):
     assert rel_l2(s, b.double().sum(0)) < TOL
     c2, s2 = ops.tn_gemm(a.cuda(), b.cuda(), column_sums=True)
     assert torch.equal(c, c2) and torch.equal(s, s2)
+
+
+def _model():
+    from spgt_b200.config.config_accessor import get_darcy_config
+    from spgt_b200.dataset.darcy_dataset import GaussNormalizer, meshgrid
+    from spgt_b200.network.sp_model import Sp_GalerkinTransformer2D
+    cfg = get_darcy_config(3, 6, num_frequence_mode=4, clamp_attn=False, fine_resolution=85, num_encoder_layer=2)
+    cfg['target_normalizer'] = GaussNormalizer()
+    torch.manual_seed(5)
+    model = Sp_GalerkinTransformer2D(cfg).cuda().eval()
+    g = torch.Generator().manual_seed(6)
+    expand = lambda m: torch.from_numpy(m).float().expand(3, *m.shape).contiguous().cuda()
+    return model, torch.randn(3, 29, 29, 1, generator=g).cuda(), expand(meshgrid(85, 6)), expand(meshgrid(85, 3))
+
+
+def test_one_call_forward_yields_to_observed_or_changed_modules():
+    import copy
+    model, *args = _model()
+    ref = model(*args)
+    assert torch.equal(copy.deepcopy(model)(*args), ref)           # a copy makes its own plan
+    seen = []
+    handles = [m.register_forward_hook(lambda m, i, o: seen.append(type(m).__name__))
+               for m in (model.encoder_mixer.layers[1].ffn_layer, model.decoder_regressor.layers[0], model.encoder_mixer.layers[0])]
+    assert rel_l2(model(*args), ref) < TOL
+    assert sorted(seen) == ['FeedForward', 'Sp_EncoderLayer', 'Sp_SpectralConv2D']
+    for h in handles:
+        h.remove()
+    assert torch.equal(model(*args), ref)
+
+    class Twice(torch.nn.Module):
+        def __init__(self, inner):
+            super().__init__()
+            self.inner = inner
+
+        def forward(self, x, position):
+            return self.inner(self.inner(x, position), position)
+    plain = model.encoder_mixer.layers[1]
+    model.encoder_mixer.layers[1] = Twice(plain)
+    twice = model(*args)
+    model.encoder_mixer.layers[1] = plain
+    model.encoder_mixer.layers.append(plain)
+    assert rel_l2(twice, model(*args)) < TOL
+    model.encoder_mixer.layers = model.encoder_mixer.layers[:2]
+    for layer in model.encoder_mixer.layers:
+        layer.attention_layer.norm_eps = 0.5                       # an option set after the first forward counts
+    assert rel_l2(model(*args), ref) > 1e-3
+
+
+def test_encoder_layer_takes_any_dense_or_strided_weights_and_positions():
+    layer, g = _layer(3)
+    x, pos = torch.randn(2, 45, 128, generator=g).cuda(), torch.rand(2, 45, 2, generator=g).cuda()
+    layer = layer.cuda()
+    with torch.no_grad():
+        ref = layer(x, pos)
+        shifted = torch.empty(2 * 45 * 2 + 1, device='cuda')[1:].view(2, 45, 2).copy_(pos)
+        assert torch.equal(layer(x, shifted), ref)
+        assert torch.equal(layer(x[1:], pos[1:]), layer(x[1:].clone(), pos[1:].clone()))
+        a = layer.attention_layer
+        a.weight_Q.data = a.weight_Q.data.t().contiguous().t()
+        a.weight_K.data = a.weight_K.data.t().contiguous().t()
+        w = a.fc_layer.weight.data
+        a.fc_layer.weight.data = torch.empty(w.numel() + 1, device='cuda')[1:].view_as(w).copy_(w)
+        assert torch.equal(layer(x, pos), ref)

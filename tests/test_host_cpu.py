@@ -165,3 +165,39 @@ def test_weighted_l2_loss_formulas():
         from SpGT.engine.metric import WeightedL2Loss2D as Ref
         a = Ref(S=r, is_regularization=True, gamma=0.5)(pred, target, None, tgrad, coeff)
         assert all(abs(float(x) - float(y)) < 1e-6 for x, y in zip(a, (loss, reg, metric)))
+
+
+def test_parameter_watch_and_copies():
+    """What the one-call forward is rebuilt for: written, moved or exchanged parameters and modules, and options; observed modules."""
+    import copy
+    from spgt_b200.config.config_accessor import get_darcy_config
+    from spgt_b200.network.sp_model import Sp_GalerkinTransformer2D
+    model = Sp_GalerkinTransformer2D(get_darcy_config(3, 6, num_frequence_mode=4, clamp_attn=False, fine_resolution=85, num_encoder_layer=2))
+    watch, layer = model._watch, model.encoder_mixer.layers[0]
+    tag = watch.tag(model)
+    assert watch.tag(model) == tag and not watch.observed(model)
+    with torch.no_grad():
+        layer.attention_layer.bias_Q.add_(1.0)
+    written = watch.tag(model)
+    assert written != tag
+    layer.attention_layer.norm_eps = 0.25
+    assert watch.tag(model) != written
+    handle = layer.ffn_layer.register_forward_pre_hook(lambda m, i: None)
+    assert watch.observed(model)
+    handle.remove()
+    assert not watch.observed(model)
+    layer.forward = lambda x, position: x
+    assert watch.observed(model)
+    del layer.forward
+    model._plan = (tag, object(), [])
+    model.down_scaler._kw['x'] = (tag, object(), [])
+    other = copy.deepcopy(model)
+    assert other._plan is None and not other.down_scaler._kw and other._watch is not watch and model._plan is not None
+    assert not model._native_widths()                 # one epsilon throughout
+    layer.attention_layer.norm_eps = model.encoder_mixer.layers[1].attention_layer.norm_eps
+    assert model._native_widths()
+    layer.ffn_layer.fused = False
+    assert not model._native_widths()
+    layer.ffn_layer.fused = True
+    model.encoder_mixer.layers[1] = torch.nn.Identity()
+    assert not model._native_widths()
