@@ -21,15 +21,16 @@ class ParameterWatch:
     OPTIONS = ('activation', 'norm_eps', 'mode', 'structure', 'fused')
 
     def __init__(self):
-        self._tree = None        # one tuple, replaced whole: several threads may share a module
-                                 # (no reference to the module itself: a cycle would keep its memory until a garbage collection)
+        # one tuple, replaced whole: several threads may share a module.  It holds neither the module nor its __dict__, which would
+        # be a cycle that keeps the module's memory until a garbage collection
+        self._tree = None
 
     def _walk(self, module: torch.nn.Module) -> tuple:
         modules = list(module.modules())
         return ([(d, len(d)) for m in modules for d in (m._modules, m._parameters)],
                 [(m._modules, k, c) for m in modules for k, c in m._modules.items()],
                 [(m._parameters, k) for m in modules for k, p in m._parameters.items() if p is not None],
-                [(m.__dict__, k) for m in modules for k in self.OPTIONS if k in m.__dict__],
+                [(m.__dict__, k) for m in modules[1:] for k in self.OPTIONS if k in m.__dict__],
                 [m.__dict__ for m in modules[1:]])
 
     def _seen(self, module: torch.nn.Module) -> tuple:
@@ -41,7 +42,8 @@ class ParameterWatch:
     def tag(self, module: torch.nn.Module) -> tuple:
         tree = self._seen(module)
         params = [d[k] for d, k in tree[2]]
-        return tuple([p._version for p in params] + [p.data_ptr() for p in params] + [d[k] for d, k in tree[3]])
+        return tuple([p._version for p in params] + [p.data_ptr() for p in params] + [d[k] for d, k in tree[3]]
+                     + [module.__dict__.get(k) for k in self.OPTIONS])
 
     def observed(self, module: torch.nn.Module) -> bool:
         """Whether a submodule's call can be told from a call of its kernels: forward hooks, or a forward of its own."""

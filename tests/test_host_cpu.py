@@ -201,3 +201,22 @@ def test_parameter_watch_and_copies():
     layer.ffn_layer.fused = True
     model.encoder_mixer.layers[1] = torch.nn.Identity()
     assert not model._native_widths()
+
+
+def test_models_are_freed_without_a_garbage_collection():
+    import gc
+    import weakref
+    from spgt_b200.config.config_accessor import get_darcy_config
+    from spgt_b200.network.sp_model import Sp_GalerkinTransformer2D
+    model = Sp_GalerkinTransformer2D(get_darcy_config(3, 6, num_frequence_mode=4, clamp_attn=False, fine_resolution=85, num_encoder_layer=2))
+    for m in (model, *(m for m in model.modules() if hasattr(m, '_kw'))):
+        m._watch.tag(m)
+        assert not m._watch.observed(m)
+    model._plan = (model._watch.tag(model), None, model._watch.hold(model))
+    seen = [weakref.ref(model), weakref.ref(model.encoder_mixer.layers[0]), weakref.ref(model.up_scaler.conv)]
+    gc.disable()
+    try:
+        del model, m
+        assert all(r() is None for r in seen)
+    finally:
+        gc.enable()
