@@ -14,9 +14,9 @@
 //
 // S1 and S3 run on the persistent tcgen05 GEMM kernel of tc_gemm.cu (3xTF32, operands split on the fly): S1 as the GEMM
 // D[(x, c)][j] over k = y with the prepared image of F1^T as W, S3 as one GEMM per image row over k = (channel | mode) whose
-// W stages are the image of Wr and the image of the row's P block, which S2c writes directly in that layout.
-// For r <= 256 the F3 rows stay in tensor memory as a constant A operand and S3's W-loader warp lays out the row's plain P
-// block itself; larger r streams F3 through the A rings and reads P as a prepared image.
+// W stages are the image of Wr and the row's P block.
+// The F3 rows stay in tensor memory as a constant A operand and S3's W-loader warp lays out the row's plain P block itself.
+// S2a and S2c share the grid rows x of a (ky, sample) between several blocks where there are few (ky, sample) pairs or many rows.
 #include "tc_common.cuh"
 
 namespace spgt {
@@ -24,12 +24,12 @@ namespace spgt {
 // tc_gemm.cu
 int spectral_tc_prepare(const float* w_kn, int ldw, int K, int N, float* img, cudaStream_t st);
 int spectral_fwd_y_tc(const float* x, const float* f1_img, float* y1, int r, int J, int64_t nimg, cudaStream_t st);
-int spectral_inv_y_tc(const float* x, const float* f3, const float* wr_img, const float* p_img, const float* p_plain, int J,
-                      const float* br, float* out, int r, int64_t nimg, int act, cudaStream_t st);
+int spectral_inv_y_tc(const float* x, const float* f3, const float* wr_img, const float* p, int J, const float* br, float* out, int r, int64_t nimg,
+                      int act, cudaStream_t st);
 
 constexpr int SP_C = 32;         // channel width handled by the tensor-core kernels
 constexpr int SP_IMG = 2 * SP_C * TC_BK;   // floats of one W stage image: hi and lo, 32 rows (n) x 32 k each
-constexpr int SP_XMAX = 256;      // largest r the staged S2a / S2c kernels accept (shared-memory budget)
+constexpr int SP_XMAX = 256;      // most grid rows a block of S2a / S2c stages (shared-memory budget)
 __host__ __device__ inline int sp_round_pitch(int n, int rem) {   // smallest p >= n with p % 32 == rem
     int p = (n + 31) / 32 * 32 + rem;
     if (p - 32 >= n) p -= 32;
@@ -38,8 +38,8 @@ __host__ __device__ inline int sp_round_pitch(int n, int rem) {   // smallest p 
 
 struct SpecTables {              // offsets in floats into the table buffer
     int r, m, J, F1P, F3ROWS, KP;
-    int f1t, f3, gr, gi, total;
-    int GA_ROWS, GA_P, ga, GC_ROWS, GC_P, gc;    // zero-padded copies of G in the shared-memory layouts of S2a / S2c (r <= SP_XMAX)
+    int f1t, f3, total;
+    int GA_ROWS, GA_P, ga, GC_ROWS, GC_P, gc;    // G [Re | Im][q][x], zero padded, as S2a / S2c read it
     int f1img, filled;                           // W image of F1^T (written by the weight-preparation kernel); `filled` = floats the table kernel writes
 };
 __host__ __device__ inline SpecTables spec_tables(int r, int m) {
@@ -50,17 +50,11 @@ __host__ __device__ inline SpecTables spec_tables(int r, int m) {
     t.KP = (r + TC_BK - 1) / TC_BK * TC_BK;
     t.f1t = 0;
     t.f3 = t.f1t + r * t.F1P;
-    t.gr = t.f3 + t.F3ROWS * 32;
-    t.gi = t.gr + t.J * r;
-    t.total = (t.gi + t.J * r + 3) / 4 * 4;
     t.GA_ROWS = (2 * t.J + 15) / 16 * 16; t.GA_P = sp_round_pitch((r + 7) / 8 * 8, 4);
     t.GC_ROWS = (2 * t.J + 7) / 8 * 8;    t.GC_P = sp_round_pitch((r + 15) / 16 * 16, 8);
-    t.ga = t.total; t.gc = t.ga;
-    if (r <= SP_XMAX) {
-        t.gc = t.ga + t.GA_ROWS * t.GA_P;
-        t.total = t.gc + t.GC_ROWS * t.GC_P;
-    }
-    t.filled = t.total = (t.total + 3) / 4 * 4;
+    t.ga = (t.f3 + t.F3ROWS * 32 + 3) / 4 * 4;
+    t.gc = t.ga + t.GA_ROWS * t.GA_P;
+    t.filled = t.total = t.gc + t.GC_ROWS * t.GC_P;           // (pitches are multiples of four)
     t.f1img = t.total;
     t.total += 2 * 32 * t.KP;
     return t;
@@ -81,7 +75,7 @@ __global__ void spectral_tables_kernel(float* tab, int r, int m) {
                 sincospi(2.0 * (double)(((int64_t)ky * y) % r) / (double)r, &s, &c);
                 v = (float)((j < m ? c : -s) / (double)r);
             }
-        } else if (i < T.gr) {                                 // F3[y][j]
+        } else if (i < T.f3 + T.F3ROWS * 32) {                 // F3[y][j]
             const int k = i - T.f3;
             const int y = k / 32, j = k % 32;
             if (y < r && j < T.J) {
@@ -91,14 +85,7 @@ __global__ void spectral_tables_kernel(float* tab, int r, int m) {
                 sincospi(2.0 * (double)(((int64_t)ky * y) % r) / (double)r, &s, &c);
                 v = (float)((j < m ? w * c : -w * s) / (double)r);
             }
-        } else if (i < T.gi + T.J * r) {                        // G[q][x] = exp(-2 pi i kx_q x / r)
-            const bool im = i >= T.gi;
-            const int k = i - (im ? T.gi : T.gr);
-            const int q = k / r, x = k % r;
-            double s, c;
-            sincospi(2.0 * (double)(((int64_t)kept_kx(q, r, m) * x) % r) / (double)r, &s, &c);
-            v = (float)(im ? -s : c);
-        } else if (i >= T.ga && r <= SP_XMAX) {                 // padded copies [rows][pitch]: row q' < 2J = (Re | Im) of G
+        } else if (i >= T.ga) {                                 // G[q][x] = exp(-2 pi i kx_q x / r): row q' < 2J = (Re | Im) of G
             const bool c_copy = i >= T.gc;
             const int k = i - (c_copy ? T.gc : T.ga), P = c_copy ? T.GC_P : T.GA_P;
             const int q2 = k / P, x = k % P;
@@ -113,50 +100,10 @@ __global__ void spectral_tables_kernel(float* tab, int r, int m) {
     }
 }
 
-// ------------------------------------------------------------------------------------------------------------
-// S2a: Z[b,q,ky,c] = sum_x G[q,x] * (Y1[b,x,ky,c] + i Y1[b,x,m+ky,c]).   grid (m, B), lane = c, warp = q stride 8.
-// ------------------------------------------------------------------------------------------------------------
+// S2b: O[b,q,ky,o] = sum_i Z[b,q,ky,i] * W[q,ky,i,o].   grid = J*m modes, lane = o, warp = b stride 8.  Z = the sum of `slices`
+// partial results [slice][Re | Im][n], in order.
 __global__ void __launch_bounds__(256)
-spectral_fwd_x_kernel(const float* __restrict__ Y1, const float* __restrict__ tab, float* __restrict__ Zr,
-                      float* __restrict__ Zi, int r, int m) {
-    extern __shared__ __align__(16) float smem[];
-    const SpecTables T = spec_tables(r, m);
-    float* gr = smem; float* gi = smem + T.J * r;
-    for (int i = threadIdx.x; i < 2 * T.J * r; i += blockDim.x) smem[i] = __ldca(tab + T.gr + i);
-    pdl_wait();
-    pdl_launch_next();
-    __syncthreads();
-    const int ky = blockIdx.x; const int64_t b = blockIdx.y;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float zr[4] = {0, 0, 0, 0}, zi[4] = {0, 0, 0, 0};
-    const float* yb = Y1 + b * (int64_t)r * T.J * SP_C + lane;
-#pragma unroll 8
-    for (int x = 0; x < r; ++x) {
-        const float yr = __ldca(yb + ((int64_t)x * T.J + ky) * SP_C);
-        const float yi = __ldca(yb + ((int64_t)x * T.J + m + ky) * SP_C);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int q = warp + 8 * k;
-            if (q < T.J) {
-                const float a = gr[q * r + x], bb = gi[q * r + x];
-                zr[k] = fmaf(a, yr, fmaf(-bb, yi, zr[k]));
-                zi[k] = fmaf(a, yi, fmaf(bb, yr, zi[k]));
-            }
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int q = warp + 8 * k;
-        if (q < T.J) {
-            const int64_t o = ((b * T.J + q) * m + ky) * SP_C + lane;
-            Zr[o] = zr[k]; Zi[o] = zi[k];
-        }
-    }
-}
-
-// S2b: O[b,q,ky,o] = sum_i Z[b,q,ky,i] * W[q,ky,i,o].   grid = J*m modes, lane = o, warp = b stride 8.
-__global__ void __launch_bounds__(256)
-spectral_mix_kernel(const float* __restrict__ Zr, const float* __restrict__ Zi, const float* __restrict__ fw0,
+spectral_mix_kernel(const float* __restrict__ Z, int64_t n, int slices, const float* __restrict__ fw0,
                     const float* __restrict__ fw1, float* __restrict__ Or, float* __restrict__ Oi, int B, int m,
                     const float* __restrict__ wr, float* __restrict__ wr_img) {
     __shared__ float2 w[SP_C * SP_C];
@@ -172,7 +119,9 @@ spectral_mix_kernel(const float* __restrict__ Zr, const float* __restrict__ Zi, 
     const int J = 2 * m;
     for (int b = warp; b < B; b += 8) {
         const int64_t base = (((int64_t)b * J + q) * m + ky) * SP_C;
-        const float zr = __ldca(Zr + base + lane), zi = __ldca(Zi + base + lane);
+        float zr = __ldca(Z + base + lane), zi = __ldca(Z + n + base + lane);
+#pragma unroll 4
+        for (int k = 1; k < slices; ++k) { zr += __ldca(Z + 2 * k * n + base + lane); zi += __ldca(Z + (2 * k + 1) * n + base + lane); }
         float orr = 0.0f, oii = 0.0f;
 #pragma unroll
         for (int i = 0; i < SP_C; ++i) {
@@ -185,80 +134,47 @@ spectral_mix_kernel(const float* __restrict__ Zr, const float* __restrict__ Zi, 
     }
 }
 
-// S2c for large r: P[b,x,ky,o] + i P[b,x,m+ky,o] = sum_q conj(G[q,x]) * O[b,q,ky,o], written into the W stage image of
-// image row (b, x), element (n = o, k = j).   grid (m, B), lane = o, warp = x stride 8.
-__global__ void __launch_bounds__(256)
-spectral_inv_x_kernel(const float* __restrict__ Or, const float* __restrict__ Oi, const float* __restrict__ tab,
-                      float* __restrict__ Pimg, int r, int m) {
-    extern __shared__ __align__(16) float smem[];
-    const SpecTables T = spec_tables(r, m);
-    float* gr = smem; float* gi = smem + T.J * r;
-    for (int i = threadIdx.x; i < 2 * T.J * r; i += blockDim.x) smem[i] = __ldca(tab + T.gr + i);
-    pdl_wait();
-    pdl_launch_next();
-    __syncthreads();
-    const int ky = blockIdx.x; const int64_t b = blockIdx.y;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float orr[32], oii[32];
-#pragma unroll
-    for (int q = 0; q < 32; ++q) {
-        if (q < T.J) {
-            const int64_t o = ((b * T.J + q) * m + ky) * SP_C + lane;
-            orr[q] = __ldca(Or + o); oii[q] = __ldca(Oi + o);
-        } else { orr[q] = 0.0f; oii[q] = 0.0f; }
-    }
-    for (int x = warp; x < r; x += 8) {
-        float pr = 0.0f, pi = 0.0f;
-#pragma unroll
-        for (int q = 0; q < 32; ++q) {
-            if (q < T.J) {
-                const float a = gr[q * r + x], bb = gi[q * r + x];     // conj(G) = a - i bb
-                pr = fmaf(a, orr[q], fmaf(bb, oii[q], pr));
-                pi = fmaf(a, oii[q], fmaf(-bb, orr[q], pi));
-            }
-        }
-        float* img = Pimg + (b * r + x) * (int64_t)SP_IMG;
-        tc_img_store(img, SP_C, lane, ky, pr);
-        tc_img_store(img, SP_C, lane, m + ky, pi);
-    }
-}
-
 // ------------------------------------------------------------------------------------------------------------
-// S2a and S2c on the tensor cores (3xTF32 warp MMA), one CTA per (ky, b), for r <= SP_XMAX.
+// S2a and S2c on the tensor cores (3xTF32 warp MMA), one CTA per (ky, b, slice of `xw` <= SP_XMAX rows x).
 //
 // S2a as a real GEMM:  R[q'][n] = sum_x Gt[q'][x] * Y[x][n],  q' < 2J (rows 0..J-1 = Re G, J..2J-1 = Im G),
 //                      n < 64 (0..31 = Re Y1 = Y1[.., ky, c], 32..63 = Im Y1 = Y1[.., m + ky, c]);
 //                      Zr[q][c] = R[q][c] - R[J+q][32+c],  Zi[q][c] = R[q][32+c] + R[J+q][c].
 // S2c as a real GEMM:  P[x][n] = sum_k Gt[k][x] * Bm[k][n],  k < 2J,
 //                      Bm[q] = (Or[q] | Oi[q]),  Bm[J+q] = (Oi[q] | -Or[q]);  n < 32 -> P[.., ky, :], else P[.., m + ky, :].
-// Both stage the whole G table ([2J][r], zero padded) and their Y1 / O block in shared memory, then every warp
-// owns a slice of the output (S2a: 8 columns, S2c: every eighth 16-row tile); eight warps per CTA.
+// Both stage their slice of the G table ([2J][xw], zero padded) and their Y1 / O block in shared memory, then every warp
+// owns a part of the output (S2a: 8 columns, S2c: every eighth 16-row tile); eight warps per CTA.  S2a leaves one partial Z per
+// slice.  They are bound by latency (load, compute, store once per block).
 // ------------------------------------------------------------------------------------------------------------
 constexpr int SP_YP = 72;         // pitch of the [x][64] / [k][64] B operands, == 8 (mod 32)
 
 
 __global__ void __launch_bounds__(256)
-spectral_fwd_x_mma_kernel(const float* __restrict__ Y1, const float* __restrict__ tab, float* __restrict__ Zr,
-                          float* __restrict__ Zi, int r, int m) {
+spectral_fwd_x_mma_kernel(const float* __restrict__ Y1, const float* __restrict__ tab, float* __restrict__ Z, int64_t zn, int xw, int r, int m) {
     extern __shared__ __align__(16) float smem[];
     const SpecTables T = spec_tables(r, m);
     const int J = T.J, M2 = 2 * J, MT = (M2 + 15) / 16;
-    const int r8 = (r + 7) / 8 * 8;
-    const int GP = sp_round_pitch(r8, 4);                    // G pitch == 4 (mod 32): A fragments conflict-free
+    const int x_begin = blockIdx.z * xw, xn = r - x_begin < xw ? r - x_begin : xw;      // (xw: a multiple of 16)
+    const int r8 = (xn + 7) / 8 * 8;
+    const int GP = sp_round_pitch(xw, 4);                    // G pitch == 4 (mod 32): A fragments conflict-free
     float* gs = smem;                                        // [16*MT][GP]
     float* ys = smem + 16 * MT * GP;                         // [r8][SP_YP]; later R [16*MT][SP_YP]
+    float *Zr = Z + 2 * blockIdx.z * zn, *Zi = Zr + zn;
     const int ky = blockIdx.x; const int64_t b = blockIdx.y;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
-    for (int i = tid; i < 16 * MT * GP / 4; i += 256) cp_async_zfill<16>(gs + 4 * i, tab + T.ga + 4 * i, true);   // padded G, as stored
+    for (int i = tid; i < 16 * MT * (r8 / 4); i += 256) {     // G, zero beyond r and beyond 2J in the table too
+        const int row = i / (r8 / 4), c = i - row * (r8 / 4);
+        cp_async_zfill<16>(gs + row * GP + 4 * c, tab + T.ga + row * T.GA_P + x_begin + 4 * c, true);
+    }
     cp_async_commit();
     pdl_wait();
     pdl_launch_next();
     // Y block: 16 float4 per x (8 from the real row, 8 from the imaginary row)
-    const float* yb = Y1 + b * (int64_t)r * J * SP_C;
+    const float* yb = Y1 + (b * r + x_begin) * (int64_t)J * SP_C;
     for (int i = tid; i < r8 * 16; i += 256) {
         const int x = i >> 4, c4 = i & 15;
-        const bool ok = x < r;
+        const bool ok = x < xn;
         const float* src = yb + ((int64_t)(ok ? x : 0) * J + (c4 < 8 ? ky : m + ky)) * SP_C + (c4 & 7) * 4;
         cp_async_zfill<16>(ys + x * SP_YP + c4 * 4, src, ok);
     }
@@ -323,18 +239,22 @@ spectral_fwd_x_mma_kernel(const float* __restrict__ Y1, const float* __restrict_
 
 __global__ void __launch_bounds__(256)
 spectral_inv_x_mma_kernel(const float* __restrict__ Or, const float* __restrict__ Oi, const float* __restrict__ tab,
-                          float* __restrict__ P, int r, int m) {
+                          float* __restrict__ P, int xw, int r, int m) {
     extern __shared__ __align__(16) float smem[];
     const SpecTables T = spec_tables(r, m);
     const int J = T.J, M2 = 2 * J, K8 = (M2 + 7) / 8 * 8;
-    const int r16 = (r + 15) / 16 * 16;
-    const int GP = sp_round_pitch(r16, 8);                   // G pitch == 8 (mod 32): transposed A fragments conflict-free
+    const int x_begin = blockIdx.z * xw, xn = r - x_begin < xw ? r - x_begin : xw;      // (xw: a multiple of 16)
+    const int r16 = (xn + 15) / 16 * 16;
+    const int GP = sp_round_pitch(xw, 8);                    // G pitch == 8 (mod 32): transposed A fragments conflict-free
     float* gs = smem;                                        // [K8][GP]
     float* bs = smem + K8 * GP;                              // [K8][SP_YP]
     const int ky = blockIdx.x; const int64_t b = blockIdx.y;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
-    for (int i = tid; i < K8 * GP / 4; i += 256) cp_async_zfill<16>(gs + 4 * i, tab + T.gc + 4 * i, true);     // padded G, as stored
+    for (int i = tid; i < K8 * (r16 / 4); i += 256) {
+        const int row = i / (r16 / 4), c = i - row * (r16 / 4);
+        cp_async_zfill<16>(gs + row * GP + 4 * c, tab + T.gc + row * T.GC_P + x_begin + 4 * c, true);
+    }
     cp_async_commit();
     pdl_wait();
     pdl_launch_next();
@@ -351,7 +271,7 @@ spectral_inv_x_mma_kernel(const float* __restrict__ Or, const float* __restrict_
     }
     cp_async_wait<0>();
     __syncthreads();
-    float* pb = P + (b * r) * (int64_t)J * SP_C;
+    float* pb = P + (b * r + x_begin) * (int64_t)J * SP_C;
     for (int mt = warp; mt < r16 / 16; mt += 8) {
         float acc[8][4];
 #pragma unroll
@@ -381,8 +301,8 @@ spectral_inv_x_mma_kernel(const float* __restrict__ Or, const float* __restrict_
         for (int j = 0; j < 8; ++j) {
             const int jrow = (j < 4 ? ky : m + ky), c = (8 * j + 2 * t) & 31;
             const int xa = x0 + g, xb = x0 + g + 8;
-            if (xa < r) *reinterpret_cast<float2*>(pb + ((int64_t)xa * J + jrow) * SP_C + c) = make_float2(acc[j][0], acc[j][1]);
-            if (xb < r) *reinterpret_cast<float2*>(pb + ((int64_t)xb * J + jrow) * SP_C + c) = make_float2(acc[j][2], acc[j][3]);
+            if (xa < xn) *reinterpret_cast<float2*>(pb + ((int64_t)xa * J + jrow) * SP_C + c) = make_float2(acc[j][0], acc[j][1]);
+            if (xb < xn) *reinterpret_cast<float2*>(pb + ((int64_t)xb * J + jrow) * SP_C + c) = make_float2(acc[j][2], acc[j][3]);
         }
     }
 }
@@ -431,14 +351,22 @@ extern "C" int spgt_spectral_launches(int B, int r, int m) {
     return 5 * ceil_div(B, spectral_chunk(r));
 }
 
-// floats of the P blocks of one image row: plain [J][32] for r <= 256, a W stage image for larger r
-static size_t spectral_p_floats(int r, int J) { return r <= 256 ? (size_t)J * SP_C : (size_t)SP_IMG; }
+// Rows per block of the x transforms.  A block per SM at least where r allows slices of 48 rows (below that a block is all latency), at
+// most SP_XMAX rows, and no more slices than their partial Z fit into the P blocks, which are written after they have been read.
+static int spectral_slice_rows(int r, int m, int samples) {
+    int slices = ceil_div(num_sms(), m * samples);
+    if (slices > r / 48) slices = r / 48;
+    if (slices < ceil_div(r, SP_XMAX)) slices = ceil_div(r, SP_XMAX);
+    if (slices > r / (2 * m)) slices = r / (2 * m);
+    return ceil_div(ceil_div(r, slices), 16) * 16;
+}
 
-// workspace layout (floats), sized for one chunk of CH samples: Y1 [CH,r,J,C] | P [CH,r][p_floats] | Zr, Zi, Or, Oi [CH,J,m,C] each | Wr image
+// workspace layout (floats), sized for one chunk of CH samples: Y1 [CH,r,J,C] | P [CH,r,J,C] | Zr, Zi, Or, Oi [CH,J,m,C] each | Wr image;
+// several slices: their partial Z [slice][Re | Im][CH,J,m,C] in the place of P
 extern "C" size_t spgt_spectral_workspace_bytes(int B, int r, int m, int C) {
     if (B <= 0 || C != SP_C || !spectral_shape_ok(r, m)) return 0;
     const size_t J = 2 * (size_t)m, CH = (size_t)(B < spectral_chunk(r) ? B : spectral_chunk(r));
-    return (CH * r * J * C + CH * r * spectral_p_floats(r, (int)J) + (size_t)4 * CH * J * m * C + SP_IMG) * sizeof(float);
+    return (2 * CH * r * J * C + (size_t)4 * CH * J * m * C + SP_IMG) * sizeof(float);
 }
 
 extern "C" int spgt_spectral_conv2d_fwd(const float* x, const float* wr, const float* br, const float* fw0,
@@ -458,18 +386,11 @@ extern "C" int spgt_spectral_conv2d_fwd(const float* x, const float* wr, const f
     if (CH > 65535) return SPGT_ERR_SHAPE;                  // (grid y dimension of the x-transform kernels)
     float* Y1 = (float*)workspace;
     float* P = Y1 + (size_t)CH * r * J * C;
-    float* Zr = P + (size_t)CH * r * spectral_p_floats(r, (int)J);
-    float* Zi = Zr + (size_t)CH * J * m * C;
-    float* Or = Zi + (size_t)CH * J * m * C;
-    float* Oi = Or + (size_t)CH * J * m * C;
-    float* wr_img = Oi + (size_t)CH * J * m * C;
-    const size_t gsmem = (size_t)2 * J * r * sizeof(float);
-    if (gsmem > 200 * 1024) return SPGT_ERR_SHAPE;
-    static SmemOptIn cfg_a, cfg_c, cfg_am, cfg_cm;
-    const bool staged = r <= SP_XMAX;                       // tensor-core S2a / S2c with everything staged in shared memory
-    // Large r: S2c writes W stage images, columns k < 2m only; the k padding must be zero (it meets zero columns of F3, but
-    // 0 * NaN would still spoil the sum), so the images are cleared first.
-    if (!staged && cudaMemsetAsync(P, 0, (size_t)CH * r * SP_IMG * sizeof(float), st) != cudaSuccess) return launch_status();
+    const int64_t zn = (int64_t)CH * J * m * C;
+    float* Z = P + (size_t)CH * r * J * C;
+    float *Or = Z + 2 * zn, *Oi = Or + zn, *wr_img = Oi + zn;
+    if ((size_t)2 * J * r * sizeof(float) > 200 * 1024) return SPGT_ERR_SHAPE;      // (the largest grids the layer takes)
+    static SmemOptIn cfg_a, cfg_c;
     int e;
     const ChainScope chain;
     for (int b0 = 0; b0 < B; b0 += CH) {
@@ -477,29 +398,17 @@ extern "C" int spgt_spectral_conv2d_fwd(const float* x, const float* wr, const f
         const float* xc = x + (size_t)b0 * r * r * C;
         float* yc = y + (size_t)b0 * r * r * C;
         const int64_t nimg = (int64_t)nb * r;
+        const int xw = spectral_slice_rows(r, m, nb), slices = ceil_div(r, xw), MT = ceil_div(2 * (int)J, 16), K8 = ceil_div(2 * (int)J, 8) * 8;
+        float* z = slices > 1 ? P : Z;
+        const size_t smem_a = ((size_t)16 * MT * sp_round_pitch(xw, 4) + (size_t)(xw > 16 * MT ? xw : 16 * MT) * SP_YP) * sizeof(float);
+        const size_t smem_c = ((size_t)K8 * sp_round_pitch(xw, 8) + (size_t)K8 * SP_YP) * sizeof(float);
         if ((e = spectral_fwd_y_tc(xc, tab + T.f1img, Y1, r, (int)J, nimg, st))) return e;
-        if (staged) {
-            const int MT = ceil_div(2 * (int)J, 16), r8 = ceil_div(r, 8) * 8;
-            const size_t smem_a = ((size_t)16 * MT * sp_round_pitch(r8, 4) + (size_t)(r8 > 16 * MT ? r8 : 16 * MT) * SP_YP) * sizeof(float);
-            if ((e = smem_opt_in(spectral_fwd_x_mma_kernel, smem_a, cfg_am))) return e;
-            e = launch_chained(spectral_fwd_x_mma_kernel, dim3(m, nb), 256, smem_a, st, Y1, tab, Zr, Zi, r, m);
-        } else {
-            if ((e = smem_opt_in(spectral_fwd_x_kernel, gsmem, cfg_a))) return e;
-            e = launch_chained(spectral_fwd_x_kernel, dim3(m, nb), 256, gsmem, st, Y1, tab, Zr, Zi, r, m);
-        }
-        if (e) return e;
-        if ((e = launch_chained(spectral_mix_kernel, (unsigned)(J * m), 256, 0, st, Zr, Zi, fw0, fw1, Or, Oi, nb, m, wr, b0 == 0 ? wr_img : nullptr))) return e;
-        if (staged) {
-            const int K8 = ceil_div(2 * (int)J, 8) * 8, r16 = ceil_div(r, 16) * 16;
-            const size_t smem_c = ((size_t)K8 * sp_round_pitch(r16, 8) + (size_t)K8 * SP_YP) * sizeof(float);
-            if ((e = smem_opt_in(spectral_inv_x_mma_kernel, smem_c, cfg_cm))) return e;
-            e = launch_chained(spectral_inv_x_mma_kernel, dim3(m, nb), 256, smem_c, st, Or, Oi, tab, P, r, m);
-        } else {
-            if ((e = smem_opt_in(spectral_inv_x_kernel, gsmem, cfg_c))) return e;
-            e = launch_chained(spectral_inv_x_kernel, dim3(m, nb), 256, gsmem, st, Or, Oi, tab, P, r, m);
-        }
-        if (e) return e;
-        if ((e = spectral_inv_y_tc(xc, tab + T.f3, wr_img, P, P, (int)J, br, yc, r, nimg, act, st))) return e;
+        if ((e = smem_opt_in(spectral_fwd_x_mma_kernel, smem_a, cfg_a))) return e;
+        if ((e = launch_chained(spectral_fwd_x_mma_kernel, dim3(m, nb, slices), 256, smem_a, st, Y1, tab, z, zn, xw, r, m))) return e;
+        if ((e = launch_chained(spectral_mix_kernel, (unsigned)(J * m), 256, 0, st, z, zn, slices, fw0, fw1, Or, Oi, nb, m, wr, b0 == 0 ? wr_img : nullptr))) return e;
+        if ((e = smem_opt_in(spectral_inv_x_mma_kernel, smem_c, cfg_c))) return e;
+        if ((e = launch_chained(spectral_inv_x_mma_kernel, dim3(m, nb, slices), 256, smem_c, st, Or, Oi, tab, P, xw, r, m))) return e;
+        if ((e = spectral_inv_y_tc(xc, tab + T.f3, wr_img, P, (int)J, br, yc, r, nimg, act, st))) return e;
     }
     return SPGT_OK;
 }

@@ -143,66 +143,42 @@ struct TcConv : TcLoaderDefaults {          // 3x3, padding 1, NHWC; k = tap * C
 
 // Spectral layer, inverse transform along y plus the residual linear layer, as one GEMM per image row (b, x):
 //   out[y][o] = sum_i X[y][i] Wr[i][o] + sum_j F3[y][j] P[j][o]            K = 32 channels + 32 (the 2m <= 32 kept modes, zero padded)
-// The GEMM rows of an image row are padded to `upr` units of 256 (two 128-row tiles): GEMM row R lies in unit u = R / 256,
-// image row u / upr, y = (u % upr) * 256 + R % 256.  k-block 0 takes its A rows from X and its W stage from the prepared
-// image of Wr; k-block 1 takes its A rows from the F3 table ([upr * 256][32], zero beyond r and beyond 2m) and its W
-// stage from the image of the row's P block, which the x-transform kernel writes in the W stage layout.
-struct TcSpecInv : TcLoaderDefaults {
-    static constexpr bool W_PER_UNIT = true;
-    const float* x; const float* f3; const float* wr_img; const float* p_img; int r, upr; int rows; int K;
-    __device__ __forceinline__ const float* w_src(const float*, int unit, int kb, int stage_floats) const {
-        return kb == 0 ? wr_img : p_img + (int64_t)(unit / upr) * stage_floats;
-    }
-    __device__ __forceinline__ int64_t out_row(int row) const {
-        const int u = row >> 8, img = u / upr, y = (u - img * upr) * 256 + (row & 255);
-        return (row < rows && y < r) ? (int64_t)img * r + y : -1;
-    }
-    __device__ __forceinline__ int out_valid(int row0) const {
-        const int u = row0 >> 8, img = u / upr, y = (u - img * upr) * 256 + (row0 & 255);
-        return row0 < rows ? r - y : 0;
-    }
-    struct Row { const float* px; const float* pf; bool ok; };
-    struct Kst { int kb; int c4; };
-    __device__ __forceinline__ Row row_state(int row) const {
-        const int u = row >> 8, img = u / upr, y = (u - img * upr) * 256 + (row & 255);
-        Row s; s.ok = row < rows && y < r;
-        s.px = s.ok ? x + ((int64_t)img * r + y) * 32 : x;
-        s.pf = f3 + (int64_t)y * 32;
-        return s;
-    }
-    __device__ __forceinline__ Kst k_state(int kb, int chunk) const { Kst k; k.kb = kb; k.c4 = chunk * 4; return k; }
-    __device__ __forceinline__ const float* ptr(const Row& s, const Kst& k, bool& ok) const {
-        if (k.kb == 0) { ok = s.ok; return s.px + k.c4; }
-        ok = true; return s.pf + k.c4;
-    }
-};
-// The same for r <= 256 (one unit per image row): the F3 rows are the same for every image row, so they are split once
-// and kept in tensor memory as the A operand of k-block 1; only X passes through the raw ring (four stages of 32 KB).
-// The row's P block arrives as plain fp32 [J][32] and is laid out by the W-loader warp.  Tensor memory holds two
-// accumulator buffers, one A stage and the constant block (measured: 222 us for 64 x 211 image rows against 281 us with one
-// accumulator buffer and two A stages).  Image rows are taken from the last to the first: the ones the forward transform
-// read last are the ones still in L2.
+// The rows of an image row are padded to `upr` units of 256 (two 128-row tiles): GEMM row R lies in unit u = R / 256, image row
+// u / upr, y = (u % upr) * 256 + R % 256.  k-block 0 takes its A rows from X and its W stage from the prepared image of Wr; the
+// A rows of k-block 1 are F3 rows ([upr * 256][32], zero beyond r and beyond 2m), the same for every image row: a CTA works on
+// one residue of u modulo upr only (the grid is a multiple of upr), splits its 256 F3 rows once and keeps them in tensor memory;
+// only X passes through the raw ring (stages of 32 KB).  The image row's P block arrives as plain fp32 [J][32] and is laid out by
+// the W-loader warp.  Tensor memory holds two accumulator buffers, one A stage and the constant block (measured: 222 us for
+// 64 x 211 image rows against 281 us with one accumulator buffer and two A stages).  Image rows are taken from the last to the
+// first: the ones the forward transform read last are the ones still in L2.
+// MULTI: r > 256 (upr > 1); the divisions by upr are left out otherwise.
+template <bool MULTI>
 struct TcSpecInvC : TcLoaderDefaults {
     static constexpr bool W_PER_UNIT = true, CONST_A = true, REVERSE_UNITS = true, W_CONVERT = true;     // (W_CONVERT needs 32-wide column tiles: lane = image row)
     static constexpr int RAW_STAGES = 3, W_STAGES = 4, A_STAGES = 1, EPI_GROUPS = 2;
     static constexpr bool RESIDUAL = false, W_TAIL_RESIDENT = true;
-    const float* x; const float* f3; const float* wr_img; const float* p; int J; int r; int rows; int K;
+    const float* x; const float* f3; const float* wr_img; const float* p; int J; int r; int upr; int rows; int K;
+    __device__ __forceinline__ int image(int unit) const { return MULTI ? unit / upr : unit; }
+    __device__ __forceinline__ int first(int unit) const { return MULTI ? (unit % upr) * 256 : 0; }       // y of the unit's first row
     __device__ __forceinline__ const float* w_src(const float*, int, int, int) const { return wr_img; }
-    __device__ __forceinline__ const float* w_plain(int unit) const { return p + (int64_t)unit * J * 32; }
+    __device__ __forceinline__ const float* w_plain(int unit) const { return p + (int64_t)image(unit) * J * 32; }
     __device__ __forceinline__ int w_plain_rows() const { return J; }
     __device__ __forceinline__ int const_ksteps() const { return (J + 7) / 8; }
     __device__ __forceinline__ int64_t out_row(int row) const {
-        const int y = row & 255;
-        return (row < rows && y < r) ? (int64_t)(row >> 8) * r + y : -1;
+        const int u = row >> 8, y = first(u) + (row & 255);
+        return (row < rows && y < r) ? (int64_t)image(u) * r + y : -1;
     }
-    __device__ __forceinline__ int out_valid(int row0) const { return row0 < rows ? r - (row0 & 255) : 0; }
-    __device__ __forceinline__ const float* const_row(int row_in_unit) const { return f3 + (int64_t)row_in_unit * 32; }
+    __device__ __forceinline__ int out_valid(int row0) const { return row0 < rows ? r - first(row0 >> 8) - (row0 & 255) : 0; }
+    // (units are taken in reverse and their number is a multiple of upr: this CTA's residue)
+    __device__ __forceinline__ const float* const_row(int row_in_unit) const {
+        return f3 + (int64_t)((MULTI ? (upr - 1 - (int)blockIdx.x % upr) * 256 : 0) + row_in_unit) * 32;
+    }
     struct Row { const float* px; bool ok; };
     struct Kst { int c4; };
     __device__ __forceinline__ Row row_state(int row) const {
-        const int y = row & 255;
+        const int u = row >> 8, y = first(u) + (row & 255);
         Row s; s.ok = row < rows && y < r;
-        s.px = s.ok ? x + ((int64_t)(row >> 8) * r + y) * 32 : x;
+        s.px = s.ok ? x + ((int64_t)image(u) * r + y) * 32 : x;
         return s;
     }
     __device__ __forceinline__ Kst k_state(int, int chunk) const { Kst k; k.c4 = chunk * 4; return k; }
@@ -994,7 +970,8 @@ static int tc_bn_for(int N, int K) {
 }
 
 template <int BN, int MT, class Loader, int EPI, class EpiParams>
-static int tc_launch(Loader ld, const float* wimg, int kpad, int rows, int n_tiles, const EpiParams& ep, cudaStream_t st) {
+static int tc_launch(Loader ld, const float* wimg, int kpad, int rows, int n_tiles, const EpiParams& ep, cudaStream_t st,
+                     int multiple = 1) {
     static SmemOptIn configured;
     auto kern = tc_gemm_kernel<BN, MT, Loader, EPI, EpiParams>;
     if (int e = smem_opt_in(kern, TcCfg<BN, MT, Loader, EPI>::BYTES, configured)) return e;
@@ -1002,6 +979,8 @@ static int tc_launch(Loader ld, const float* wimg, int kpad, int rows, int n_til
     int per_nt = num_sms() / n_tiles;                 // CTAs per column tile
     if (per_nt < 1) per_nt = 1;
     if (per_nt > m_units) per_nt = m_units;
+    per_nt -= per_nt % multiple;                      // (m_units is a multiple of it, too)
+    if (per_nt < multiple) per_nt = multiple;
     const int grid = per_nt * n_tiles;
     return launch_chained(kern, grid, tc_threads(MT, tc_epi_groups<Loader, MT, BN, EPI>()), TcCfg<BN, MT, Loader, EPI>::BYTES, st, ld, wimg, kpad, rows, n_tiles, m_units, ep);
 }
@@ -1038,22 +1017,17 @@ int spectral_fwd_y_tc(const float* x, const float* f1_img, float* y1, int r, int
     return tc_launch<32, 2, TcSpecFwd, EPI_SPECF, TcSpecFwdEpi>(ld, f1_img, ceil_div(r, TC_BK) * TC_BK, ld.rows, 1, ep, st);
 }
 // out[image row][y][o] = act( X[y][:] Wr + F3[y][:] P[image row] + br[o] ); f3 = [upr * 256][32] table, wr_img = W stage image
-// of Wr.  r <= 256: p_plain = the P blocks as plain fp32 [image row][J][32]; larger r: p_img = one W stage image (2048
-// floats) per image row.
-int spectral_inv_y_tc(const float* x, const float* f3, const float* wr_img, const float* p_img, const float* p_plain, int J,
-                      const float* br, float* out, int r, int64_t nimg, int act, cudaStream_t st) {
+// of Wr, p = the P blocks as plain fp32 [image row][J][32].
+int spectral_inv_y_tc(const float* x, const float* f3, const float* wr_img, const float* p, int J, const float* br, float* out, int r, int64_t nimg,
+                      int act, cudaStream_t st) {
     const int upr = ceil_div(r, 256);
     if (nimg * upr * 256 > 0x7fffffffLL) return SPGT_ERR_SHAPE;
-    TcLinearEpi epc{br, nullptr, 0, out, 32, 32, act};
-    if (upr == 1) {
-        TcSpecInvC ldc;
-        ldc.x = x; ldc.f3 = f3; ldc.wr_img = wr_img; ldc.p = p_plain; ldc.J = J; ldc.r = r; ldc.rows = (int)(nimg * 256); ldc.K = 64;
-        return tc_launch<32, 2, TcSpecInvC, EPI_LINEAR, TcLinearEpi>(ldc, wr_img, 64, ldc.rows, 1, epc, st);
-    }
-    TcSpecInv ld;
-    ld.x = x; ld.f3 = f3; ld.wr_img = wr_img; ld.p_img = p_img; ld.r = r; ld.upr = upr; ld.rows = (int)(nimg * upr * 256); ld.K = 64;
-    TcLinearEpi ep{br, nullptr, 0, out, 32, 32, act};
-    return tc_launch<32, 2, TcSpecInv, EPI_LINEAR, TcLinearEpi>(ld, wr_img, 64, ld.rows, 1, ep, st);
+    const TcLinearEpi ep{br, nullptr, 0, out, 32, 32, act};
+    auto go = [&](auto ld) {
+        ld.x = x; ld.f3 = f3; ld.wr_img = wr_img; ld.p = p; ld.J = J; ld.r = r; ld.upr = upr; ld.rows = (int)(nimg * upr * 256); ld.K = 64;
+        return tc_launch<32, 2, decltype(ld), EPI_LINEAR, TcLinearEpi>(ld, wr_img, 64, ld.rows, 1, ep, st, upr);
+    };
+    return upr == 1 ? go(TcSpecInvC<false>{}) : go(TcSpecInvC<true>{});
 }
 
 // Projection (+ per-head LayerNorm) + position rows of width 128 from plain weights [128][128] (called from gemm.cu): nproj of them.

@@ -140,3 +140,21 @@ def test_encoder_layer_takes_any_dense_or_strided_weights_and_positions():
         w = a.fc_layer.weight.data
         a.fc_layer.weight.data = torch.empty(w.numel() + 1, device='cuda')[1:].view_as(w).copy_(w)
         assert torch.equal(layer(x, pos), ref)
+
+
+# slices of the x transforms: none, one with a remainder, as many as rows or modes allow; grids of one, two and three 256-row units
+@pytest.mark.parametrize('B,r,m', [(1, 2, 1), (1, 95, 12), (1, 97, 12), (1, 256, 16), (2, 257, 16), (2, 421, 15), (3, 513, 3), (1, 600, 16), (20, 150, 8)])
+def test_spectral_layer_slices_and_units(B, r, m):
+    from spgt_b200 import ops
+    g = torch.Generator().manual_seed(r + m)
+    x = torch.randn(B, r, r, 32, generator=g)
+    p = {'residual_layer.weight': torch.randn(32, 32, generator=g) / 6, 'residual_layer.bias': torch.randn(32, generator=g),
+         'fourier_weight.0': torch.randn(m, m, 32, 32, 2, generator=g) / 6, 'fourier_weight.1': torch.randn(m, m, 32, 32, 2, generator=g) / 6}
+    dev = {k: v.cuda() for k, v in p.items()}
+    args = (dev['residual_layer.weight'].t().contiguous(), dev['residual_layer.bias'], dev['fourier_weight.0'], dev['fourier_weight.1'], m, 'silu')
+    y = ops.spectral_conv2d(x.cuda(), *args)
+    assert ops.tc_status() == 0
+    idx = sorted({0, B - 1})
+    ref = O.spectral_conv2d(x[idx].double(), O.to_dtype(p, torch.float64), '', m, 'silu')
+    assert rel_l2(y[idx], ref) < TOL
+    assert torch.equal(y, ops.spectral_conv2d(x.cuda(), *args))
