@@ -19,11 +19,16 @@ constexpr int AB_MAT = AB_TP * AB_TP;
 constexpr int AB_GROUPS = 7, AB_COLS = AB_GROUPS * 16, AB_CP = AB_COLS + 4;      // columns per tile, pitch (an odd number of 16-byte units)
 constexpr int AB_THREADS = 256;                // 7 groups x 36 threads work, all load
 
-// partial [bh][which: T, dT][chunk][36][36]
-__global__ void __launch_bounds__(AB_THREADS)
+// partial [bh][which: T, dT][chunk][36][36].  The next tile's copies are in flight while a tile is multiplied, two blocks per SM: with
+// plain loads between two barriers and one block per SM the kernel waited for memory (batch 16, 4 heads, S = 4096: 302 us, now 70 us).
+// VEC: rows of Q, K, V in 16-byte copies (S a multiple of four, aligned bases), else 4-byte ones; dOut, whose rows are nodes, is
+// transposed by 4-byte copies.  magic = 2^20 / D + 1: i / D = i * magic >> 20 for i < 2^12.
+constexpr int AB_STAGE = 2 * AB_TP * AB_CP;
+template <bool VEC>
+__global__ void __launch_bounds__(AB_THREADS, 2)
 attn_bwd_reduce_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V, const float* __restrict__ dOut,
-                       float* __restrict__ partial, int D, int S, int chunks) {
-    __shared__ __align__(16) float as[AB_TP * AB_CP], bs[AB_TP * AB_CP];
+                       float* __restrict__ partial, int D, int S, int chunks, uint32_t magic) {
+    extern __shared__ __align__(16) float smem[];          // two stages of A rows, B rows
     const int t = threadIdx.x, chunk = blockIdx.x % chunks, which = blockIdx.y;
     const int64_t bh = blockIdx.x / chunks, base = bh * (int64_t)D * S;
     const int tiles = (S + AB_COLS - 1) / AB_COLS;
@@ -31,48 +36,64 @@ attn_bwd_reduce_kernel(const float* __restrict__ Q, const float* __restrict__ K,
     const float* A = (which ? Q : K) + base;
     const float* B = (which ? dOut : V) + base;
     const int g = t / 36, tt = t - g * 36, i0 = tt / 6, j0 = tt - i0 * 6;          // entries (i0 + 6 a, j0 + 6 b)
-    for (int i = t; i < (AB_TP - D) * AB_CP; i += AB_THREADS) { as[D * AB_CP + i] = 0.0f; bs[D * AB_CP + i] = 0.0f; }
-    float acc[6][6] = {};
-    for (int tile = t_begin; tile < t_end; ++tile) {
-        const int s0 = tile * AB_COLS, ns = S - s0 < AB_COLS ? S - s0 : AB_COLS;
-        __syncthreads();
-#pragma unroll 4
-        for (int i = t; i < D * AB_COLS; i += AB_THREADS) {
-            const int r = i / AB_COLS, c = i - r * AB_COLS;
-            as[r * AB_CP + c] = c < ns ? __ldg(A + (int64_t)r * S + s0 + c) : 0.0f;
-            if (!which) bs[r * AB_CP + c] = c < ns ? __ldg(B + (int64_t)r * S + s0 + c) : 0.0f;
-        }
-        if (which)
-#pragma unroll 4
-            for (int i = t; i < D * AB_COLS; i += AB_THREADS) {
-                const int c = i / D, j = i - c * D;
-                bs[j * AB_CP + c] = c < ns ? __ldg(B + (int64_t)s0 * D + i) : 0.0f;
+    for (int i = t; i < (AB_TP - D) * AB_CP; i += AB_THREADS)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) smem[k * AB_TP * AB_CP + D * AB_CP + i] = 0.0f;
+    auto copy_rows = [&](const float* src, float* dst, int s0, int ns) {
+        if constexpr (VEC) {
+            for (int i = t; i < D * (AB_COLS / 4); i += AB_THREADS) {
+                const int r = i / (AB_COLS / 4), c = (i - r * (AB_COLS / 4)) * 4;
+                cp_async_zfill<16>(dst + r * AB_CP + c, c < ns ? src + (int64_t)r * S + s0 + c : src, c < ns);
             }
+        } else {
+            for (int i = t; i < D * AB_COLS; i += AB_THREADS) {
+                const int r = i / AB_COLS, c = i - r * AB_COLS;
+                cp_async_zfill<4>(dst + r * AB_CP + c, c < ns ? src + (int64_t)r * S + s0 + c : src, c < ns);
+            }
+        }
+    };
+    auto load = [&](int tile, int stage) {
+        const int s0 = tile * AB_COLS, ns = S - s0 < AB_COLS ? S - s0 : AB_COLS;
+        float *as = smem + stage * AB_STAGE, *bs = as + AB_TP * AB_CP;
+        copy_rows(A, as, s0, ns);
+        if (!which) copy_rows(B, bs, s0, ns);
+        else
+            for (int i = t; i < D * AB_COLS; i += AB_THREADS) {
+                const int c = (int)(((uint32_t)i * magic) >> 20), j = i - c * D;
+                cp_async_zfill<4>(bs + j * AB_CP + c, c < ns ? B + (int64_t)s0 * D + i : B, c < ns);
+            }
+        cp_async_commit();
+    };
+    float acc[6][6] = {};
+    load(t_begin, 0);
+    for (int tile = t_begin; tile < t_end; ++tile) {
+        const int stage = (tile - t_begin) & 1;
+        if (tile + 1 < t_end) { load(tile + 1, stage ^ 1); cp_async_wait<1>(); } else cp_async_wait<0>();
         __syncthreads();
         if (g < AB_GROUPS) {
-            const float* pa = as + i0 * AB_CP + g * 16;
-            const float* pb = bs + j0 * AB_CP + g * 16;
+            const float* pa = smem + stage * AB_STAGE + i0 * AB_CP + g * 16;
+            const float* pb = smem + stage * AB_STAGE + (AB_TP + j0) * AB_CP + g * 16;
 #pragma unroll
             for (int s = 0; s < 16; s += 4) {
-                float4 a[6], b[6];
+                float4 b[6];
+#pragma unroll
+                for (int e = 0; e < 6; ++e) b[e] = *reinterpret_cast<const float4*>(pb + 6 * e * AB_CP + s);
 #pragma unroll
                 for (int e = 0; e < 6; ++e) {
-                    a[e] = *reinterpret_cast<const float4*>(pa + 6 * e * AB_CP + s);
-                    b[e] = *reinterpret_cast<const float4*>(pb + 6 * e * AB_CP + s);
-                }
-#pragma unroll
-                for (int e = 0; e < 6; ++e)
+                    const float4 a = *reinterpret_cast<const float4*>(pa + 6 * e * AB_CP + s);
 #pragma unroll
                     for (int f = 0; f < 6; ++f) {
-                        acc[e][f] = fmaf(a[e].x, b[f].x, acc[e][f]); acc[e][f] = fmaf(a[e].y, b[f].y, acc[e][f]);
-                        acc[e][f] = fmaf(a[e].z, b[f].z, acc[e][f]); acc[e][f] = fmaf(a[e].w, b[f].w, acc[e][f]);
+                        acc[e][f] = fmaf(a.x, b[f].x, acc[e][f]); acc[e][f] = fmaf(a.y, b[f].y, acc[e][f]);
+                        acc[e][f] = fmaf(a.z, b[f].z, acc[e][f]); acc[e][f] = fmaf(a.w, b[f].w, acc[e][f]);
                     }
+                }
             }
         }
+        __syncthreads();
     }
     // the seven column groups, in order
     float* out = partial + ((bh * 2 + which) * chunks + chunk) * AB_MAT;
-    float* red = as;
+    float* red = smem;
     for (int k = 0; k < AB_GROUPS; ++k) {
         __syncthreads();
         if (g == k)
@@ -157,10 +178,10 @@ attn_bwd_apply_kernel(const float* __restrict__ K, const float* __restrict__ V, 
     multiply(mats, dQ);
 }
 
-// blocks per (batch, head) and matrix: enough for four per SM
+// blocks per (batch, head) and matrix: four waves of two per SM, one tile each at least
 static int attn_bwd_chunks(int64_t BH, int S) {
     const int tiles = ceil_div(S, AB_COLS);
-    int64_t c = ceil_div((int64_t)4 * num_sms(), 2 * BH);
+    int64_t c = (int64_t)8 * num_sms() / (2 * BH);
     if (c > tiles) c = tiles;
     return (int)(c < 1 ? 1 : c);
 }
@@ -191,7 +212,12 @@ extern "C" int spgt_galerkin_attn_bwd(const float* Q, const float* K, const floa
     cudaStream_t st = (cudaStream_t)stream;
     float* partial = (float*)workspace;
     float* sums = partial + BH * 2 * chunks * AB_MAT;
-    attn_bwd_reduce_kernel<<<dim3((unsigned)(BH * chunks), 2), AB_THREADS, 0, st>>>(Q, K, V, d_out, partial, dpk, S, chunks);
+    static SmemOptIn opt_v, opt_s;
+    const bool vec = (S & 3) == 0 && aligned16(Q) && aligned16(K) && aligned16(V);
+    const size_t smem = (size_t)2 * AB_STAGE * sizeof(float);
+    if (int e = vec ? smem_opt_in(attn_bwd_reduce_kernel<true>, smem, opt_v) : smem_opt_in(attn_bwd_reduce_kernel<false>, smem, opt_s)) return e;
+    auto reduce = vec ? attn_bwd_reduce_kernel<true> : attn_bwd_reduce_kernel<false>;
+    reduce<<<dim3((unsigned)(BH * chunks), 2), AB_THREADS, smem, st>>>(Q, K, V, d_out, partial, dpk, S, chunks, (1u << 20) / (uint32_t)dpk + 1);
     if (int e = launch_status()) return e;
     attn_bwd_sum_kernel<<<dim3((unsigned)BH, 2), 256, 0, st>>>(partial, sums, chunks, 1.0f / (float)S);
     if (int e = launch_status()) return e;

@@ -3,11 +3,13 @@
 //
 // The reduction runs over the rows, so both operands are needed K-major with the rows as k: raw blocks of 32 rows arrive row-major
 // (cp.async, padded pitch), and eight warps store them TRANSPOSED - one operand row per matrix column, 32 long - as
-// hi / lo tiles.  Per 8 rows one MMA A_hi x [B_hi | B_lo] (two partial accumulators) and one A_lo x B_hi.  The hi operand is the plain
-// fp32 value (the tensor core reads its upper 19 bits), lo what they leave, rounded.
+// hi / lo tiles.  Per 8 rows one MMA A_hi x [B_hi | B_lo] and one A_lo x B_hi, the latter on top of the B_lo columns.  The hi operand
+// is the plain fp32 value (the tensor core reads its upper 19 bits), lo what they leave, rounded.
 // Bound by shared memory: per 32 rows 512 transposing stores, 64 x 4 read phases and 80 KB of operand reads, about 1300 cycles.
-// Blocks split the rows; every 512 rows the accumulators are added to fp32 registers (an MMA's accumulate step truncates), and
-// the blocks' partial results are added in block order by a second kernel: deterministic.
+// Blocks split the rows; the accumulate step of an MMA truncates towards zero, so the large A_hi B_hi sums
+// have an accumulator of their own and all are added to fp32 registers every 128 rows (with one accumulator and 512 rows the gradients of
+// a training step lay further from fp64 than with fp32 sums: 3.6e-6 against 3.1e-6).  The blocks' partial results are added by a second
+// kernel in an order fixed by their number: deterministic.
 //   warps 0-1 raw loaders (A, B), 2 MMA issuer, 4-11 transposers (A: 4-7, B: 8-11), 12-19 accumulation.
 // Every wait is a bounded mbarrier poll that records a code on expiry.
 #include "tc_common.cuh"
@@ -22,7 +24,7 @@ constexpr int TN_HALF = TN_T * 128, TN_STAGE = 4 * TN_HALF;              // A_hi
 constexpr int TN_OFF_RAW = TN_NS * TN_STAGE, TN_OFF_BAR = TN_OFF_RAW + TN_NR * 2 * TN_RAW;
 constexpr size_t TN_SMEM = TN_OFF_BAR + 256;
 static_assert(TN_SMEM <= 227 * 1024, "shared memory budget");
-constexpr int TN_CHAIN = 16;                                              // blocks of 32 rows per accumulator chain
+constexpr int TN_CHAIN = 4;                                               // blocks of 32 rows per accumulator chain
 
 struct TnParams {
     const float *a, *b;
@@ -104,7 +106,7 @@ __global__ void __launch_bounds__(TN_THREADS, 1) tn_gemm_kernel(const TnParams p
 #pragma unroll
                     for (int k8 = 0; k8 < 4; ++k8) {
                         tc_mma_tf32_ss(d, ah + k8 * 2, b + k8 * 2, idesc2, (k > 0 || k8 > 0) ? 1u : 0u);
-                        tc_mma_tf32_ss(d, al + k8 * 2, b + k8 * 2, idesc1, 1u);
+                        tc_mma_tf32_ss(d + TN_T, al + k8 * 2, b + k8 * 2, idesc1, 1u);
                     }
                     tc_commit(st_empty(s));
                     if (++s == TN_NS) { s = 0; ph ^= 1u; }
@@ -201,19 +203,28 @@ __global__ void __launch_bounds__(TN_THREADS, 1) tn_gemm_kernel(const TnParams p
     }
 }
 
-// C and the column sums: partial results in block order, 64 threads x 4 columns of a row per block row
+// C and the column sums from the partial results.  Eight threads share a result (four columns of a row, or a column sum): thread g adds
+// partial results g, g + 8, ..., and the eight sums are added in order: one thread per result left 16 blocks with 148 serial loads
+// (128 x 128, 65536 rows: 16 us, now 5.5).
 __global__ void __launch_bounds__(256)
 tn_reduce_kernel(const float* __restrict__ partial, const float* __restrict__ colpart, float* __restrict__ C, float* __restrict__ colsum, int ldc,
                  int M, int N, int tiles, int nt, int splits) {
-    const int i = blockIdx.x * 256 + threadIdx.x;           // element of the padded [tiles][128][128 / 4]
-    if (i < tiles * TN_T * (TN_T / 4)) {
+    __shared__ float4 part[8][32];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5, c_blocks = tiles * (TN_T * TN_T / 4 / 32);
+    if ((int)blockIdx.x < c_blocks) {
+        const int i = blockIdx.x * 32 + lane;               // element of the padded [tiles][128][128 / 4]
         const float4* src = reinterpret_cast<const float4*>(partial) + i;
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
-        for (int k = 0; k < splits; ++k) {
+        for (int k = g; k < splits; k += 8) {
             const float4 v = __ldg(src + (int64_t)k * tiles * (TN_T * TN_T / 4));
             s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
         }
+        part[g][lane] = s;
+        __syncthreads();
+        if (g) return;
+#pragma unroll
+        for (int k = 1; k < 8; ++k) { const float4 v = part[k][lane]; s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w; }
         const int c4 = i % (TN_T / 4), r = i / (TN_T / 4) % TN_T, tile = i / (TN_T * TN_T / 4);
         const int row = tile / nt * TN_T + r, col = tile % nt * TN_T + c4 * 4;
         if (row < M) {
@@ -222,14 +233,18 @@ tn_reduce_kernel(const float* __restrict__ partial, const float* __restrict__ co
             for (int e = 0; e < 4; ++e)
                 if (col + e < N) C[(int64_t)row * ldc + col + e] = o[e];
         }
-    } else if (colsum != nullptr) {
-        const int c = i - tiles * TN_T * (TN_T / 4);
-        if (c < N) {
-            float s = 0.0f;
+    } else {
+        const int c = (blockIdx.x - c_blocks) * 32 + lane;   // (colpart has whole 128-column tiles)
+        float s = 0.0f;
+        if (c < N)
 #pragma unroll 8
-            for (int k = 0; k < splits; ++k) s += __ldg(colpart + ((int64_t)k * nt) * TN_T + c);
-            colsum[c] = s;
-        }
+            for (int k = g; k < splits; k += 8) s += __ldg(colpart + ((int64_t)k * nt) * TN_T + c);
+        part[g][lane].x = s;
+        __syncthreads();
+        if (g || c >= N) return;
+#pragma unroll
+        for (int k = 1; k < 8; ++k) s += part[k][lane].x;
+        colsum[c] = s;
     }
 }
 
@@ -270,7 +285,6 @@ extern "C" int spgt_tn_gemm(const float* A, int lda, const float* B, int ldb, fl
     const TnParams p{A, B, partial, colsum ? colpart : nullptr, lda, ldb, M, N, rows, nt};
     tn_gemm_kernel<<<dim3((unsigned)splits, (unsigned)tiles), TN_THREADS, TN_SMEM, (cudaStream_t)stream>>>(p);
     if (int e = launch_status()) return e;
-    const int items = tiles * TN_T * (TN_T / 4) + (colsum ? N : 0);
-    tn_reduce_kernel<<<ceil_div(items, 256), 256, 0, (cudaStream_t)stream>>>(partial, colpart, C, colsum, ldc, M, N, tiles, nt, splits);
+    tn_reduce_kernel<<<tiles * (TN_T * TN_T / 4 / 32) + (colsum ? ceil_div(N, 32) : 0), 256, 0, (cudaStream_t)stream>>>(partial, colpart, C, colsum, ldc, M, N, tiles, nt, splits);
     return launch_status();
 }

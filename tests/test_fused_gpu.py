@@ -158,3 +158,18 @@ def test_spectral_layer_slices_and_units(B, r, m):
     ref = O.spectral_conv2d(x[idx].double(), O.to_dtype(p, torch.float64), '', m, 'silu')
     assert rel_l2(y[idx], ref) < TOL
     assert torch.equal(y, ops.spectral_conv2d(x.cuda(), *args))
+
+
+# columns around the 112-wide tiles, 16-byte and 4-byte copies, several chunks and blocks of several tiles
+@pytest.mark.parametrize('B,H,dpk,S', [(1, 1, 34, 1), (2, 4, 34, 111), (1, 4, 34, 112), (3, 2, 35, 113), (16, 4, 34, 4096), (2, 3, 32, 4097), (80, 4, 34, 225)])
+def test_attention_backward_tiles(B, H, dpk, S):
+    from spgt_b200 import ops
+    g = torch.Generator().manual_seed(S)
+    q, k, v = (torch.randn(B, H, dpk, S, generator=g).cuda() for _ in range(3))
+    dout = torch.randn(B, H, S, dpk, generator=g).cuda()
+    Q, K, V = (t.double().requires_grad_() for t in (q, k, v))
+    want = torch.autograd.grad(Q.transpose(2, 3) @ (K @ V.transpose(2, 3) / S), [Q, K, V], dout.double())
+    got = ops.galerkin_attention_backward(q, k, v, dout)
+    for n, a, b in zip('QKV', got, want):
+        assert rel_l2(a, b) < TOL, n
+    assert all(torch.equal(a, b) for a, b in zip(got, ops.galerkin_attention_backward(q, k, v, dout)))
