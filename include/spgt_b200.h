@@ -348,6 +348,24 @@ size_t spgt_encoder_workspace_bytes(int B, int S);
 int spgt_encoder_layer_fwd(const spgt_encoder_weights* w, const float* x, const float* pos, float* y, int B, int S, float eps, int act, int ffn,
                            int residual, void* workspace, size_t workspace_bytes, spgt_stream_t stream);
 
+/* Encoder layer for training (width 128, 4 heads, 2 position values, feed-forward width 256, ReLU): parameters as the modules keep
+ * them (w* of the projections [128 in][128 out], wfc [128][136], w1 [256][128], w2 [128][256]) and where their gradients go; wqkv
+ * receives the three projections' [3][128][128].  fwd: weight images, projections + LayerNorm and attention, merged heads [B,S,136];
+ * it keeps what bwd needs in `saved`.  bwd: every gradient, from x, the attention, x1 = x + attention wfc + bfc, h = relu(x1 w1 + b1),
+ * dy and the gradients with respect to x1 w1 + b1 (dh), x1 (dx1) and the attention (da).  x, x1, dy, dx1, dx [B,S,128], h, dh [B,S,256],
+ * da [B,S,136], pos [B,S,2].  p->wfc .. p->b2 are not read and may be NULL.  No counterpart as one call in the reference
+ * (network/sp_layer.py:52-104). */
+typedef struct { const float *wq, *bq, *wk, *bk, *wv, *bv, *lnwk, *lnbk, *lnwv, *lnbv, *wfc, *bfc, *w1, *b1, *w2, *b2; } spgt_encoder_params;
+typedef struct { float *wqkv, *bq, *bk, *bv, *lnwk, *lnbk, *lnwv, *lnbv, *wfc, *bfc, *w1, *b1, *w2, *b2; } spgt_encoder_grads;
+size_t spgt_encoder_train_saved_bytes(int B, int S);
+size_t spgt_encoder_train_workspace_bytes(int B, int S);
+int spgt_encoder_train_fwd(const spgt_encoder_params* p, const float* x, const float* pos, float* attention, int B, int S, float eps, void* saved,
+                           size_t saved_bytes, spgt_stream_t stream);
+int spgt_encoder_train_bwd(const spgt_encoder_params* p, const spgt_encoder_grads* g, const float* x, const float* attention,
+                           const float* x1, const float* h, const float* dy, const float* dh, const float* dx1, const float* da, float* dx,
+                           int B, int S, float eps, const void* saved, size_t saved_bytes, void* workspace, size_t workspace_bytes,
+                           spgt_stream_t stream);
+
 /* One spectral layer: as spgt_spectral_conv2d_fwd takes them. */
 typedef struct { const float *wr, *br, *fw0, *fw1; } spgt_spectral_weights;
 

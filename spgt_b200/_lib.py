@@ -98,6 +98,10 @@ SIGNATURES = {
     'spgt_spectral_launches': (_i, [_i, _i, _i]),
     'spgt_encoder_workspace_bytes': (_sz, [_i, _i]),
     'spgt_encoder_layer_fwd': (_i, [_f] * 4 + [_i, _i, _fl, _i, _i, _i, _f, _sz, _st]),
+    'spgt_encoder_train_saved_bytes': (_sz, [_i, _i]),
+    'spgt_encoder_train_workspace_bytes': (_sz, [_i, _i]),
+    'spgt_encoder_train_fwd': (_i, [_f] * 4 + [_i, _i, _fl, _f, _sz, _st]),
+    'spgt_encoder_train_bwd': (_i, [_f] * 11 + [_i, _i, _fl, _f, _sz, _f, _sz, _st]),
     'spgt_darcy_workspace_bytes': (_sz, [_f, _i]),
     'spgt_darcy_launches': (_i, [_f, _i]),
     'spgt_darcy_forward': (_i, [_f] * 5 + [_i, _f, _f, _sz, _st]),

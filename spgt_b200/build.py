@@ -18,7 +18,7 @@ CSRC = os.path.join(PKG, 'csrc')
 INCLUDE = os.path.join(os.path.dirname(PKG), 'include')
 LIB = os.path.join(PKG, 'libspgt_b200.so')
 OBJ = os.path.join(PKG, 'build')
-SOURCES = ['abi.cu', 'datamove.cu', 'attention.cu', 'attention_tc.cu', 'attention_bwd.cu', 'projection_bwd.cu', 'gemm.cu', 'tc_gemm.cu', 'tc_ffn.cu', 'tc_conv.cu', 'tc_tn.cu', 'scaler.cu', 'spectral.cu', 'metric.cu', 'darcy_forward.cu', 'encoder.cu', 'encoder_kv.cu', 'encoder_fold.cu', 'encoder_out.cu', 'darcy_solve.cu']
+SOURCES = ['abi.cu', 'datamove.cu', 'attention.cu', 'attention_tc.cu', 'attention_bwd.cu', 'projection_bwd.cu', 'gemm.cu', 'tc_gemm.cu', 'tc_ffn.cu', 'tc_conv.cu', 'tc_tn.cu', 'scaler.cu', 'spectral.cu', 'metric.cu', 'darcy_forward.cu', 'encoder.cu', 'encoder_kv.cu', 'encoder_fold.cu', 'encoder_out.cu', 'encoder_train.cu', 'darcy_solve.cu']
 NVCC_FLAGS = ['-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo', '-O3', '-std=c++17',
               '-Xcompiler', '-fPIC', '-I', INCLUDE]
 

@@ -9,7 +9,7 @@
 // Both are bound by the values shared memory hands to registers (128 bytes per cycle and SM): with 6 x 6 entries twelve 16-byte
 // reads feed 144 FMAs, with four nodes nine feed 144.  Batch 16, 4 heads, S = 4096: 540 us with five single entries and one
 // node per thread.
-// Layouts as in the forward: Q, K, V, dQ, dK, dV [B*H, dpk, S] (S fastest), dOut [B*H, S, dpk].
+// Layouts as in the forward: Q, K, V, dQ, dK, dV [B*H, dpk, S] (S fastest), dOut [B*H, S, dpk] or, merged heads, [B, S, H * dpk].
 #include "common.cuh"
 
 namespace spgt {
@@ -19,6 +19,14 @@ constexpr int AB_MAT = AB_TP * AB_TP;
 constexpr int AB_GROUPS = 7, AB_COLS = AB_GROUPS * 16, AB_CP = AB_COLS + 4;      // columns per tile, pitch (an odd number of 16-byte units)
 constexpr int AB_THREADS = 256;                // 7 groups x 36 threads work, all load
 
+// Rows of dOut: pitch ld, rows of (batch, head) bh start at `at(bh)`.
+struct AbOut {
+    int ld, H, D, S;                           // merged heads: H > 0, ld = H * D
+    __device__ __forceinline__ int64_t at(int64_t bh) const {
+        return H > 0 ? bh / H * S * ld + bh % H * D : bh * (int64_t)D * S;
+    }
+};
+
 // partial [bh][which: T, dT][chunk][36][36].  The next tile's copies are in flight while a tile is multiplied, two blocks per SM: with
 // plain loads between two barriers and one block per SM the kernel waited for memory (batch 16, 4 heads, S = 4096: 302 us, now 70 us).
 // VEC: rows of Q, K, V in 16-byte copies (S a multiple of four, aligned bases), else 4-byte ones; dOut, whose rows are nodes, is
@@ -27,14 +35,14 @@ constexpr int AB_STAGE = 2 * AB_TP * AB_CP;
 template <bool VEC>
 __global__ void __launch_bounds__(AB_THREADS, 2)
 attn_bwd_reduce_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V, const float* __restrict__ dOut,
-                       float* __restrict__ partial, int D, int S, int chunks, uint32_t magic) {
+                       float* __restrict__ partial, int D, int S, int chunks, uint32_t magic, AbOut od) {
     extern __shared__ __align__(16) float smem[];          // two stages of A rows, B rows
     const int t = threadIdx.x, chunk = blockIdx.x % chunks, which = blockIdx.y;
     const int64_t bh = blockIdx.x / chunks, base = bh * (int64_t)D * S;
     const int tiles = (S + AB_COLS - 1) / AB_COLS;
     const int t_begin = (int)(((int64_t)chunk * tiles) / chunks), t_end = (int)(((int64_t)(chunk + 1) * tiles) / chunks);
     const float* A = (which ? Q : K) + base;
-    const float* B = (which ? dOut : V) + base;
+    const float* B = which ? dOut + od.at(bh) : V + base;
     const int g = t / 36, tt = t - g * 36, i0 = tt / 6, j0 = tt - i0 * 6;          // entries (i0 + 6 a, j0 + 6 b)
     for (int i = t; i < (AB_TP - D) * AB_CP; i += AB_THREADS)
 #pragma unroll
@@ -60,7 +68,7 @@ attn_bwd_reduce_kernel(const float* __restrict__ Q, const float* __restrict__ K,
         else
             for (int i = t; i < D * AB_COLS; i += AB_THREADS) {
                 const int c = (int)(((uint32_t)i * magic) >> 20), j = i - c * D;
-                cp_async_zfill<4>(bs + j * AB_CP + c, c < ns ? B + (int64_t)s0 * D + i : B, c < ns);
+                cp_async_zfill<4>(bs + j * AB_CP + c, c < ns ? B + (int64_t)(s0 + c) * od.ld + j : B, c < ns);
             }
         cp_async_commit();
     };
@@ -131,7 +139,7 @@ constexpr int AP_THREADS = 128;
 template <int AP_NODES>
 __global__ void __launch_bounds__(AP_THREADS, 3)
 attn_bwd_apply_kernel(const float* __restrict__ K, const float* __restrict__ V, const float* __restrict__ dOut, const float* __restrict__ sums,
-                      float* __restrict__ dQ, float* __restrict__ dK, float* __restrict__ dV, int D, int S, int col_tiles) {
+                      float* __restrict__ dQ, float* __restrict__ dK, float* __restrict__ dV, int D, int S, int col_tiles, AbOut od) {
     __shared__ __align__(16) float mats[3 * AB_MAT];       // T | dT | dT transposed
     const int t = threadIdx.x;
     const int64_t bh = blockIdx.x / col_tiles, base = bh * (int64_t)D * S;
@@ -170,11 +178,12 @@ attn_bwd_apply_kernel(const float* __restrict__ K, const float* __restrict__ V, 
     multiply(mats + AB_MAT, dK);
     load_columns(K);
     multiply(mats + 2 * AB_MAT, dV);
+    const float* rows = dOut + od.at(bh);
 #pragma unroll
     for (int n = 0; n < AP_NODES; ++n)
 #pragma unroll
         for (int j = 0; j < AB_TP; ++j)
-            x[j][n] = j < D && s0 + n * AP_THREADS < S ? __ldg(dOut + base + (int64_t)(s0 + n * AP_THREADS) * D + j) : 0.0f;
+            x[j][n] = j < D && s0 + n * AP_THREADS < S ? __ldg(rows + (int64_t)(s0 + n * AP_THREADS) * od.ld + j) : 0.0f;
     multiply(mats, dQ);
 }
 
@@ -196,9 +205,10 @@ extern "C" size_t spgt_galerkin_attn_bwd_workspace_bytes(int B, int H, int dpk, 
     return (size_t)BH * (2 * attn_bwd_chunks(BH, S) + 3) * AB_MAT * sizeof(float);
 }
 
-extern "C" int spgt_galerkin_attn_bwd(const float* Q, const float* K, const float* V, const float* d_out, float* dQ, float* dK,
-                                      float* dV, int B, int H, int dpk, int S, void* workspace, size_t workspace_bytes,
-                                      spgt_stream_t stream) {
+namespace spgt {
+// merged: d_out is [B, S, H * dpk], as the output projection takes it
+int galerkin_attn_bwd(const float* Q, const float* K, const float* V, const float* d_out, float* dQ, float* dK, float* dV, int B, int H, int dpk,
+                      int S, bool merged, void* workspace, size_t workspace_bytes, cudaStream_t st) {
     if (!Q || !K || !V || !d_out || !dQ || !dK || !dV) return SPGT_ERR_NULL;
     if (B <= 0 || H <= 0 || S <= 0 || dpk <= 0 || dpk > AB_MAXD) return SPGT_ERR_SHAPE;
     const int64_t BH = (int64_t)B * H;
@@ -209,7 +219,7 @@ extern "C" int spgt_galerkin_attn_bwd(const float* Q, const float* K, const floa
     const int col_tiles = ceil_div(S, AP_THREADS * nodes);
     if (BH * chunks > 0x7fffffffLL || BH * col_tiles > 0x7fffffffLL) return SPGT_ERR_SHAPE;
     if (!workspace || workspace_bytes < spgt_galerkin_attn_bwd_workspace_bytes(B, H, dpk, S)) return SPGT_ERR_WORKSPACE;
-    cudaStream_t st = (cudaStream_t)stream;
+    const AbOut od{merged ? H * dpk : dpk, merged ? H : 0, dpk, S};
     float* partial = (float*)workspace;
     float* sums = partial + BH * 2 * chunks * AB_MAT;
     static SmemOptIn opt_v, opt_s;
@@ -217,11 +227,18 @@ extern "C" int spgt_galerkin_attn_bwd(const float* Q, const float* K, const floa
     const size_t smem = (size_t)2 * AB_STAGE * sizeof(float);
     if (int e = vec ? smem_opt_in(attn_bwd_reduce_kernel<true>, smem, opt_v) : smem_opt_in(attn_bwd_reduce_kernel<false>, smem, opt_s)) return e;
     auto reduce = vec ? attn_bwd_reduce_kernel<true> : attn_bwd_reduce_kernel<false>;
-    reduce<<<dim3((unsigned)(BH * chunks), 2), AB_THREADS, smem, st>>>(Q, K, V, d_out, partial, dpk, S, chunks, (1u << 20) / (uint32_t)dpk + 1);
+    reduce<<<dim3((unsigned)(BH * chunks), 2), AB_THREADS, smem, st>>>(Q, K, V, d_out, partial, dpk, S, chunks, (1u << 20) / (uint32_t)dpk + 1, od);
     if (int e = launch_status()) return e;
     attn_bwd_sum_kernel<<<dim3((unsigned)BH, 2), 256, 0, st>>>(partial, sums, chunks, 1.0f / (float)S);
     if (int e = launch_status()) return e;
     auto apply = nodes == 4 ? attn_bwd_apply_kernel<4> : nodes == 2 ? attn_bwd_apply_kernel<2> : attn_bwd_apply_kernel<1>;
-    apply<<<(unsigned)(BH * col_tiles), AP_THREADS, 0, st>>>(K, V, d_out, sums, dQ, dK, dV, dpk, S, col_tiles);
+    apply<<<(unsigned)(BH * col_tiles), AP_THREADS, 0, st>>>(K, V, d_out, sums, dQ, dK, dV, dpk, S, col_tiles, od);
     return launch_status();
+}
+}  // namespace spgt
+
+extern "C" int spgt_galerkin_attn_bwd(const float* Q, const float* K, const float* V, const float* d_out, float* dQ, float* dK,
+                                      float* dV, int B, int H, int dpk, int S, void* workspace, size_t workspace_bytes,
+                                      spgt_stream_t stream) {
+    return galerkin_attn_bwd(Q, K, V, d_out, dQ, dK, dV, B, H, dpk, S, false, workspace, workspace_bytes, (cudaStream_t)stream);
 }

@@ -483,13 +483,13 @@ extern "C" int spgt_conv3x3_fwd(const float* x, int cin_pitch, int cin_off, int 
 namespace spgt { int projpos_tc(const float* x, int nproj, const float* const* w, const TcProjEpi& ep, int rows, cudaStream_t st); }      // tc_gemm.cu
 
 static int proj_common(const float* x, int nproj, ProjEpi& ep, int B, int S, int D, int H, int d_head, int d_pos,
-                       cudaStream_t st) {
+                       cudaStream_t st, bool warp_mma = false) {
     if (B <= 0 || S <= 0 || D <= 0 || H <= 0) return SPGT_ERR_SHAPE;
     if (d_head != 32 || D != H * d_head || (D % 128) != 0 || d_pos < 0 || d_pos > 8) return SPGT_ERR_SHAPE;
     const int64_t rows64 = (int64_t)B * S;
     if (rows64 > 0x7fffffffLL / 2) return SPGT_ERR_SHAPE;
     if (d_pos > 0 && !ep.pos) return SPGT_ERR_NULL;
-    if (D == 128) {                                  // (wider models: the warp-MMA kernel below)
+    if (D == 128 && !warp_mma) {                     // (wider models: the warp-MMA kernel below)
         TcProjEpi t = {};
         for (int i = 0; i < nproj; ++i) { t.bias[i] = ep.bias[i]; t.lnw[i] = ep.lnw[i]; t.lnb[i] = ep.lnb[i]; t.out[i] = ep.out[i]; t.invsigma[i] = ep.invsigma[i]; }
         t.pos = ep.pos; t.eps = ep.eps; t.S = S; t.H = H; t.d_pos = d_pos;
@@ -542,6 +542,20 @@ extern "C" int spgt_projpos_qkv_fwd(const float* x, const float* wq, const float
     ep.pos = pos; ep.eps = eps;
     return proj_common(x, 3, ep, B, S, D, H, d_head, d_pos, (cudaStream_t)stream);
 }
+
+// Width 128 on the warp-MMA kernel, whose results the training forward wants (encoder_train.cu).
+namespace spgt {
+int projpos_qkv_mma(const float* x, const float* wq, const float* bq, const float* wk, const float* bk, const float* wv, const float* bv,
+                    const float* lnwk, const float* lnbk, const float* lnwv, const float* lnbv, float eps, const float* pos, float* q, float* k, float* v,
+                    int B, int S, int d_pos, cudaStream_t st) {
+    ProjEpi ep = {};
+    ep.w[0] = wq; ep.bias[0] = bq; ep.out[0] = q;
+    ep.w[1] = wk; ep.bias[1] = bk; ep.lnw[1] = lnwk; ep.lnb[1] = lnbk; ep.out[1] = k;
+    ep.w[2] = wv; ep.bias[2] = bv; ep.lnw[2] = lnwv; ep.lnb[2] = lnbv; ep.out[2] = v;
+    ep.pos = pos; ep.eps = eps;
+    return proj_common(x, 3, ep, B, S, 128, 4, 32, d_pos, st, true);
+}
+}  // namespace spgt
 
 extern "C" int spgt_decoder_head_fwd(const float* x, const float* w1, const float* b1, const float* w2, float b2,
                                      float scale, float shift, const float* scale_map, const float* shift_map,

@@ -17,10 +17,11 @@ namespace spgt {
 
 constexpr int PB_ROWS = 32;      // grid nodes per warp and iteration
 
+// Rows of h and dh have pitches ldh and ldd.
 template <bool LN>
-__global__ void __launch_bounds__(256)
-proj_bwd_kernel(const float* __restrict__ grad_out, const float* __restrict__ h, const float* __restrict__ lnw,
-                float* __restrict__ dh, float* __restrict__ partial, int S, int H, int d_pos, float eps, int tiles_per_sample, int tiles) {
+__device__ __forceinline__ void proj_bwd_body(const float* __restrict__ grad_out, const float* __restrict__ h, int ldh, const float* __restrict__ lnw,
+                                              float* __restrict__ dh, int ldd, float* __restrict__ partial, int S, int H, int d_pos, float eps,
+                                              int tiles_per_sample, int tiles) {
     extern __shared__ float red[];                        // [H][32][33]
     const int D = H * 32, dpk = d_pos + 32;
     const int lane = threadIdx.x & 31, head = threadIdx.x >> 5;
@@ -37,7 +38,7 @@ proj_bwd_kernel(const float* __restrict__ grad_out, const float* __restrict__ h,
         for (int c = 0; c < 32; ++c) g[c] = __ldg(gp + (int64_t)c * S);              // lanes = consecutive nodes
         if constexpr (LN) {
             float v[32], mu = 0.0f, var = 0.0f, m1 = 0.0f, m2 = 0.0f;
-            const float4* hp = reinterpret_cast<const float4*>(h + row * D + head * 32);
+            const float4* hp = reinterpret_cast<const float4*>(h + row * ldh + head * 32);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const float4 q = __ldg(hp + j);
@@ -61,7 +62,7 @@ proj_bwd_kernel(const float* __restrict__ grad_out, const float* __restrict__ h,
 #pragma unroll
             for (int c = 0; c < 32; ++c) g[c] = inv * (g[c] - m1 - v[c] * m2);
         }
-        float4* dp = reinterpret_cast<float4*>(dh + row * D + head * 32);
+        float4* dp = reinterpret_cast<float4*>(dh + row * ldd + head * 32);
 #pragma unroll
         for (int j = 0; j < 8; ++j) dp[j] = make_float4(g[4 * j], g[4 * j + 1], g[4 * j + 2], g[4 * j + 3]);
 #pragma unroll
@@ -84,10 +85,26 @@ proj_bwd_kernel(const float* __restrict__ grad_out, const float* __restrict__ h,
     if (LN) { columns(dw, 1); columns(dbt, 2); }
 }
 
-// 32 columns per block, eight threads per column take every eighth partial sum
+template <bool LN>
 __global__ void __launch_bounds__(256)
-proj_bwd_reduce_kernel(const float* __restrict__ partial, float* __restrict__ db, float* __restrict__ dlnw, float* __restrict__ dlnb,
-                       int D, int nblocks) {
+proj_bwd_kernel(const float* __restrict__ grad_out, const float* __restrict__ h, const float* __restrict__ lnw,
+                float* __restrict__ dh, float* __restrict__ partial, int S, int H, int d_pos, float eps, int tiles_per_sample, int tiles) {
+    proj_bwd_body<LN>(grad_out, h, H * 32, lnw, dh, H * 32, partial, S, H, d_pos, eps, tiles_per_sample, tiles);
+}
+
+// Q, K and V of a layer in one launch (blockIdx.y): dh [rows, 384] = dq | dk | dv, h [rows, 256] = K | V before their LayerNorm
+struct ProjBwdQkv { const float *grad[3], *h, *lnw[3]; float *dh, *partial; };
+__global__ void __launch_bounds__(128)
+proj_bwd_qkv_kernel(const ProjBwdQkv p, int S, int d_pos, float eps, int tiles_per_sample, int tiles) {
+    const int w = blockIdx.y;
+    float* partial = p.partial + (int64_t)w * gridDim.x * 384;
+    if (w == 0) proj_bwd_body<false>(p.grad[0], nullptr, 0, nullptr, p.dh, 384, partial, S, 4, d_pos, eps, tiles_per_sample, tiles);
+    else proj_bwd_body<true>(p.grad[w], p.h + (w - 1) * 128, 256, p.lnw[w], p.dh + w * 128, 384, partial, S, 4, d_pos, eps, tiles_per_sample, tiles);
+}
+
+// 32 columns per block, eight threads per column take every eighth partial sum
+__device__ __forceinline__ void proj_bwd_reduce_body(const float* __restrict__ partial, float* __restrict__ db, float* __restrict__ dlnw,
+                                                     float* __restrict__ dlnb, int D, int nblocks) {
     __shared__ float red[8][33];
     const int c = threadIdx.x & 31, k0 = threadIdx.x >> 5, i = blockIdx.x * 32 + c;
     float s = 0.0f;
@@ -103,9 +120,37 @@ proj_bwd_reduce_kernel(const float* __restrict__ partial, float* __restrict__ db
     }
 }
 
+__global__ void __launch_bounds__(256)
+proj_bwd_reduce_kernel(const float* __restrict__ partial, float* __restrict__ db, float* __restrict__ dlnw, float* __restrict__ dlnb,
+                       int D, int nblocks) {
+    proj_bwd_reduce_body(partial, db, dlnw, dlnb, D, nblocks);
+}
+
+struct ProjBwdQkvOut { float *db[3], *dlnw[3], *dlnb[3]; };
+__global__ void __launch_bounds__(256)
+proj_bwd_reduce_qkv_kernel(const float* __restrict__ partial, const ProjBwdQkvOut o, int nblocks) {
+    const int w = blockIdx.y;
+    if (w == 0 && blockIdx.x >= 4) return;                 // (Q has no LayerNorm)
+    proj_bwd_reduce_body(partial + (int64_t)w * nblocks * 384, o.db[w], o.dlnw[w], o.dlnb[w], 128, nblocks);
+}
+
 static int proj_bwd_blocks(int B, int S, int H) {          // enough warps for eight per SM sub-partition, one tile each at least
     const int64_t tiles = (int64_t)B * ceil_div(S, PB_ROWS), most = (int64_t)num_sms() * (H <= 4 ? 2 : 1);
     return (int)(tiles < most ? tiles : most);
+}
+
+size_t projpos_bwd_qkv_workspace_bytes(int B, int S) { return (size_t)3 * proj_bwd_blocks(B, S, 4) * 384 * sizeof(float); }
+
+// Width 128, four heads.  grad_* [B,4,d_pos+32,S], h [B*S,256] -> dh [B*S,384] and the parameter sums of the three projections.
+int projpos_bwd_qkv(const float* grad_q, const float* grad_k, const float* grad_v, const float* h, const float* lnwk, const float* lnwv, float eps,
+                    float* dh, float* const* db, float* const* dlnw, float* const* dlnb, int B, int S, int d_pos, float* workspace, cudaStream_t st) {
+    const int tps = ceil_div(S, PB_ROWS), blocks = proj_bwd_blocks(B, S, 4);
+    const ProjBwdQkv p{{grad_q, grad_k, grad_v}, h, {nullptr, lnwk, lnwv}, dh, workspace};
+    proj_bwd_qkv_kernel<<<dim3((unsigned)blocks, 3), 128, (size_t)128 * 33 * sizeof(float), st>>>(p, S, d_pos, eps, tps, B * tps);
+    if (int e = launch_status()) return e;
+    const ProjBwdQkvOut o{{db[0], db[1], db[2]}, {nullptr, dlnw[0], dlnw[1]}, {nullptr, dlnb[0], dlnb[1]}};
+    proj_bwd_reduce_qkv_kernel<<<dim3(12, 3), 256, 0, st>>>(workspace, o, blocks);
+    return launch_status();
 }
 
 }  // namespace spgt

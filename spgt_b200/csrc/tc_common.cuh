@@ -206,6 +206,9 @@ __device__ __forceinline__ void tc_img_store(float* stage, int bn, int n, int kk
     stage[off] = __uint_as_float(h);
     stage[bn * TC_BK + off] = __uint_as_float(l2);
 }
+// Weight images to make in one launch.  kind 0: w [K][ldw], 1: w [N][ldw] (transposed), 2: copy N floats.
+struct TcPrepJob { const float* w; float* img; int kind, ldw, K, N, kpad, bn; };
+struct TcPrepJobs { TcPrepJob job[8]; };
 // Store 8 consecutive 32-bit columns of this thread's TMEM lane.
 __device__ __forceinline__ void tc_st8(uint32_t taddr, const uint32_t (&u)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"

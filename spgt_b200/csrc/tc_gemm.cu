@@ -955,6 +955,22 @@ __global__ void tc_weight_prepare_kernel(const float* __restrict__ w, int ldw, i
     }
 }
 
+// The same for several weights in one launch (blockIdx.y); kind 2 copies N floats (a bias that has to lie next to another).
+__global__ void __launch_bounds__(256) tc_weight_prepare_jobs_kernel(const __grid_constant__ TcPrepJobs jobs) {
+    const TcPrepJob& j = jobs.job[blockIdx.y];
+    const int npad = j.kind == 2 ? 0 : (j.N + j.bn - 1) / j.bn * j.bn, total = j.kind == 2 ? j.N : npad * j.kpad, KB = j.kpad / TC_BK;
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
+        if (j.kind == 2) { j.img[i] = __ldg(j.w + i); continue; }
+        const int n = i / j.kpad, k = i - n * j.kpad;
+        const float v = (n < j.N && k < j.K) ? __ldg(j.kind == 1 ? j.w + (int64_t)n * j.ldw + k : j.w + (int64_t)k * j.ldw + n) : 0.0f;
+        tc_img_store(j.img + ((int64_t)(n / j.bn) * KB + k / TC_BK) * (2 * j.bn * TC_BK), j.bn, n % j.bn, k % TC_BK, v);
+    }
+}
+int tc_weight_prepare_jobs(const TcPrepJobs& jobs, int n, cudaStream_t st) {
+    tc_weight_prepare_jobs_kernel<<<dim3(64, (unsigned)n), 256, 0, st>>>(jobs);
+    return launch_status();
+}
+
 // Column tile width.  A 128-wide tile keeps W resident in shared memory only up to K = 128; just above that (the
 // 136-wide merged attention heads) two 64-wide column tiles with W resident beat one 128-wide tile that re-streams W
 // for every row tile, the second read of the rows coming from L2.  At K = 256 the doubled row traffic costs more

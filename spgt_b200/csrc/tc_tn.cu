@@ -28,8 +28,8 @@ constexpr int TN_CHAIN = 4;                                               // blo
 
 struct TnParams {
     const float *a, *b;
-    float *partial, *colsum;            // [split][tile][128][128]; [split][n tile][128] (m tile 0 only), or NULL
-    int lda, ldb, M, N, rows, nt;
+    float *partial, *colsum;            // [split][tile][128][128]; [split][128-column tile of the summed matrix][128], or NULL
+    int lda, ldb, M, N, rows, nt, sum_a;
 };
 
 __global__ void __launch_bounds__(TN_THREADS, 1) tn_gemm_kernel(const TnParams p) {
@@ -155,8 +155,8 @@ __global__ void __launch_bounds__(TN_THREADS, 1) tn_gemm_kernel(const TnParams p
             mbar_arrive(st_full(s));
             if (++s == TN_NS) { s = 0; ph ^= 1u; }
         }
-        // column sums of B: lanes (rows) together
-        if (alive && isb && p.colsum != nullptr && m0 == 0) {
+        // column sums of A or B: lanes (rows) together, by the blocks of the other matrix's first tile
+        if (alive && isb != p.sum_a && p.colsum != nullptr && (p.sum_a ? n0 : m0) == 0) {
             float mine = 0.0f;
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
@@ -165,7 +165,8 @@ __global__ void __launch_bounds__(TN_THREADS, 1) tn_gemm_kernel(const TnParams p
                 for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
                 if (lane == j) mine = t;
             }
-            p.colsum[((int64_t)blockIdx.x * p.nt + tile % p.nt) * TN_T + c0 + lane] = mine;
+            const int ct = p.sum_a ? gridDim.y / p.nt : p.nt, ci = p.sum_a ? tile / p.nt : tile % p.nt;
+            p.colsum[((int64_t)blockIdx.x * ct + ci) * TN_T + c0 + lane] = mine;
         }
     } else if (warp >= 12) {
         // ------------------------------------------ accumulation ------------------------------------------
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(TN_THREADS, 1) tn_gemm_kernel(const TnParams p
 // (128 x 128, 65536 rows: 16 us, now 5.5).
 __global__ void __launch_bounds__(256)
 tn_reduce_kernel(const float* __restrict__ partial, const float* __restrict__ colpart, float* __restrict__ C, float* __restrict__ colsum, int ldc,
-                 int M, int N, int tiles, int nt, int splits) {
+                 int64_t panel, int M, int N, int tiles, int nt, int splits, int sums, int sum_tiles) {
     __shared__ float4 part[8][32];
     const int lane = threadIdx.x & 31, g = threadIdx.x >> 5, c_blocks = tiles * (TN_T * TN_T / 4 / 32);
     if ((int)blockIdx.x < c_blocks) {
@@ -229,19 +230,20 @@ tn_reduce_kernel(const float* __restrict__ partial, const float* __restrict__ co
         const int row = tile / nt * TN_T + r, col = tile % nt * TN_T + c4 * 4;
         if (row < M) {
             const float o[4] = {s.x, s.y, s.z, s.w};
+            float* dst = C + tile % nt * panel + (int64_t)row * ldc + c4 * 4;
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-                if (col + e < N) C[(int64_t)row * ldc + col + e] = o[e];
+                if (col + e < N) dst[e] = o[e];
         }
     } else {
         const int c = (blockIdx.x - c_blocks) * 32 + lane;   // (colpart has whole 128-column tiles)
         float s = 0.0f;
-        if (c < N)
+        if (c < sums)
 #pragma unroll 8
-            for (int k = g; k < splits; k += 8) s += __ldg(colpart + ((int64_t)k * nt) * TN_T + c);
+            for (int k = g; k < splits; k += 8) s += __ldg(colpart + ((int64_t)k * sum_tiles) * TN_T + c);
         part[g][lane].x = s;
         __syncthreads();
-        if (g || c >= N) return;
+        if (g || c >= sums) return;
 #pragma unroll
         for (int k = 1; k < 8; ++k) s += part[k][lane].x;
         colsum[c] = s;
@@ -266,25 +268,36 @@ using namespace spgt;
 
 extern "C" size_t spgt_tn_gemm_workspace_bytes(int M, int N, int rows) {
     if (M <= 0 || N <= 0 || rows <= 0 || M > 4096 || N > 4096) return 0;
-    const size_t tiles = (size_t)ceil_div(M, TN_T) * ceil_div(N, TN_T), splits = (size_t)tn_splits(M, N, rows);
-    return splits * (tiles * TN_T * TN_T + (size_t)ceil_div(N, TN_T) * TN_T) * sizeof(float);
+    const size_t mt = ceil_div(M, TN_T), nt = ceil_div(N, TN_T), splits = (size_t)tn_splits(M, N, rows);
+    return splits * (mt * nt * TN_T * TN_T + (mt > nt ? mt : nt) * TN_T) * sizeof(float);
 }
 
-extern "C" int spgt_tn_gemm(const float* A, int lda, const float* B, int ldb, float* C, int ldc, float* colsum, int M, int N, int rows,
-                            void* workspace, size_t workspace_bytes, spgt_stream_t stream) {
+namespace spgt {
+// sum_a: the column sums are A's [M], not B's [N].  panel: distance between the 128-column panels of C (128: side by side).
+int tn_gemm(const float* A, int lda, const float* B, int ldb, float* C, int ldc, int64_t panel, float* colsum, bool sum_a, int M, int N, int rows,
+            void* workspace, size_t workspace_bytes, cudaStream_t st) {
     if (!A || !B || !C || !workspace) return SPGT_ERR_NULL;
     const size_t need = spgt_tn_gemm_workspace_bytes(M, N, rows);
-    if (need == 0 || lda < M || ldb < N || ldc < N || (lda & 3) || (ldb & 3)) return SPGT_ERR_SHAPE;
+    if (need == 0 || (lda & 3) || (ldb & 3)) return SPGT_ERR_SHAPE;
     if (workspace_bytes < need) return SPGT_ERR_WORKSPACE;
     if (!aligned16(A) || !aligned16(B) || !aligned16(workspace)) return SPGT_ERR_ALIGN;
     static SmemOptIn configured;
     if (int e = smem_opt_in(tn_gemm_kernel, TN_SMEM, configured)) return e;
-    const int nt = ceil_div(N, TN_T), tiles = ceil_div(M, TN_T) * nt, splits = tn_splits(M, N, rows);
+    const int nt = ceil_div(N, TN_T), mt = ceil_div(M, TN_T), tiles = mt * nt, splits = tn_splits(M, N, rows);
     float* partial = (float*)workspace;
     float* colpart = partial + (size_t)splits * tiles * TN_T * TN_T;
-    const TnParams p{A, B, partial, colsum ? colpart : nullptr, lda, ldb, M, N, rows, nt};
-    tn_gemm_kernel<<<dim3((unsigned)splits, (unsigned)tiles), TN_THREADS, TN_SMEM, (cudaStream_t)stream>>>(p);
+    const TnParams p{A, B, partial, colsum ? colpart : nullptr, lda, ldb, M, N, rows, nt, sum_a ? 1 : 0};
+    tn_gemm_kernel<<<dim3((unsigned)splits, (unsigned)tiles), TN_THREADS, TN_SMEM, st>>>(p);
     if (int e = launch_status()) return e;
-    tn_reduce_kernel<<<tiles * (TN_T * TN_T / 4 / 32) + (colsum ? ceil_div(N, 32) : 0), 256, 0, (cudaStream_t)stream>>>(partial, colpart, C, colsum, ldc, M, N, tiles, nt, splits);
+    const int sums = colsum ? (sum_a ? M : N) : 0;
+    tn_reduce_kernel<<<tiles * (TN_T * TN_T / 4 / 32) + ceil_div(sums, 32), 256, 0, st>>>(partial, colpart, C, colsum, ldc, panel, M, N, tiles, nt,
+                                                                                        splits, sums, sum_a ? mt : nt);
     return launch_status();
+}
+}  // namespace spgt
+
+extern "C" int spgt_tn_gemm(const float* A, int lda, const float* B, int ldb, float* C, int ldc, float* colsum, int M, int N, int rows,
+                            void* workspace, size_t workspace_bytes, spgt_stream_t stream) {
+    if (A && B && C && workspace && (lda < M || ldb < N || ldc < N)) return SPGT_ERR_SHAPE;
+    return tn_gemm(A, lda, B, ldb, C, ldc, TN_T, colsum, false, M, N, rows, workspace, workspace_bytes, (cudaStream_t)stream);
 }

@@ -121,6 +121,29 @@ def _attention_forward_train(self, Q: Tensor, K: Tensor, V: Tensor, position: Te
 Sp_GalerkinAttention.forward_train = _attention_forward_train
 
 
+class _EncoderLayerFunction(torch.autograd.Function):
+    """X + attention(X), then + ffn(.): projections and attention in one native call, their backward and all weight gradients in
+    another; the dense layers' products along the layer are plain fp32, whose last bits decide what passes the ReLU."""
+
+    @staticmethod
+    def forward(ctx, x, position, eps, *params):
+        x, params = x.contiguous(), [_dense(p) for p in params]
+        att, saved = ops.encoder_train_forward(x, position.contiguous(), eps, params)
+        linear = torch.nn.functional.linear
+        x1 = x + linear(att, params[10], params[11])
+        h = torch.relu(linear(x1, params[12], params[13]))
+        ctx.save_for_backward(x, att, x1, h, saved, *params)
+        ctx.eps = eps
+        return x1 + linear(h, params[14], params[15])
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, grad_out):
+        x, att, x1, h, saved, *params = ctx.saved_tensors
+        dx, grads = ops.encoder_train_backward(x, att, x1, h, ctx.eps, params, saved, _dense(grad_out))
+        return (dx, None, None, *grads)
+
+
 class Sp_EncoderLayer(_KernelWeights):
     def __init__(self, dim_hidden, num_head, dim_position, norm_eps, attn_droprate, fc_droprate, xavier, diagonal,
                  symmetric, ffn_dim_hidden, ffn_droprate, ffn_activation) -> None:
@@ -152,6 +175,14 @@ class Sp_EncoderLayer(_KernelWeights):
                 and f.layer2.out_features == 128)
 
     def forward_train(self, X: Tensor, position: Tensor) -> Tensor:
+        a, f = self.attention_layer, self.ffn_layer
+        # the fused training layer: its widths and activation, the modules' own linear layers, nothing that watches or alters their calls
+        if (self.fusable and f.activation == 'relu' and X.is_cuda and X.dim() == 3 and X.dtype == torch.float32 and not torch.is_autocast_enabled()
+                and all(type(l) is torch.nn.Linear and l.bias is not None for l in (a.fc_layer, f.layer1, f.layer2))
+                and not self._watch.observed(self)):
+            return _EncoderLayerFunction.apply(
+                X, position, a.norm_eps, a.weight_Q, a.bias_Q, a.weight_K, a.bias_K, a.weight_V, a.bias_V, a.ln_weight_K, a.ln_bias_K,
+                a.ln_weight_V, a.ln_bias_V, a.fc_layer.weight, a.fc_layer.bias, f.layer1.weight, f.layer1.bias, f.layer2.weight, f.layer2.bias)
         X = X + self.attention_layer.forward_train(X, X, X, position)
         return X + self.ffn_layer.forward_train(X)
 

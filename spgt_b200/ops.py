@@ -621,6 +621,48 @@ def encoder_layer(plan: EncoderPlan, x: Tensor, position: Tensor, eps: float, ac
     return y
 
 
+_ENCODER_PARAMS = 16          # wq, bq, wk, bk, wv, bv, lnwk, lnbk, lnwv, lnbv, wfc, bfc, w1, b1, w2, b2
+
+
+def encoder_train_forward(x: Tensor, position: Tensor, eps: float, params: Sequence[Tensor]):
+    """(merged attention [B,S,136], what the layer's backward needs) for x [B,S,128], position [B,S,2] and the layer's 16 parameters."""
+    _chk(x, 'x'); _chk(position, 'position')
+    for p in params:
+        _chk(p, 'parameter')
+    B, S, D = x.shape
+    if D != 128 or position.shape != (B, S, 2) or len(params) != _ENCODER_PARAMS:
+        raise ValueError('x must be [B, S, 128] and position [B, S, 2]')
+    need = int(lib.spgt_encoder_train_saved_bytes(B, S))
+    with _device(x.device):
+        att, saved = torch.empty(B, S, 136, device=x.device, dtype=x.dtype), torch.empty(need // 4, device=x.device, dtype=x.dtype)
+        ptrs = (ctypes.c_void_p * _ENCODER_PARAMS)(*[p.data_ptr() for p in params])
+        _call('spgt_encoder_train_fwd', ptrs, x.data_ptr(), position.data_ptr(), att.data_ptr(), B, S, float(eps), saved.data_ptr(), need, _stream(), kernels=3)
+    return att, saved
+
+
+def encoder_train_backward(x: Tensor, att: Tensor, x1: Tensor, h: Tensor, eps: float, params: Sequence[Tensor], saved: Tensor, grad_out: Tensor):
+    """(dx, [gradient of each parameter]) of a layer from its intermediate values: x1 = x + fc(att), h = relu(layer1(x1))."""
+    _chk(grad_out, 'grad_out')
+    B, S, D = x.shape
+    rows = B * S
+    wfc, w1, w2 = params[10], params[12], params[14]
+    dh = torch.ops.aten.threshold_backward(torch.mm(grad_out.view(rows, D), w2), h.view(rows, 256), 0)
+    dx1 = torch.addmm(grad_out.view(rows, D), dh, w1)
+    da = torch.mm(dx1, wfc)
+    need, kept = int(lib.spgt_encoder_train_workspace_bytes(B, S)), saved.numel() * 4
+    with _device(x.device):
+        dx, dwqkv = torch.empty_like(x), torch.empty(3, 128, 128, device=x.device, dtype=x.dtype)
+        workspace = torch.empty(need, device=x.device, dtype=torch.uint8)
+        wq, wk, wv = dwqkv.unbind(0)
+        grads = [torch.empty_like(p) for p in params[5:]]               # (the first five: wq, bq, wk, bk, wv)
+        bq, bk = torch.empty_like(params[1]), torch.empty_like(params[3])
+        out = (ctypes.c_void_p * 14)(*[t.data_ptr() for t in (dwqkv, bq, bk, *grads)])
+        ptrs = (ctypes.c_void_p * _ENCODER_PARAMS)(*[p.data_ptr() for p in params])
+        _call('spgt_encoder_train_bwd', ptrs, out, x.data_ptr(), att.data_ptr(), x1.data_ptr(), h.data_ptr(), grad_out.data_ptr(), dh.data_ptr(),
+              dx1.data_ptr(), da.data_ptr(), dx.data_ptr(), B, S, float(eps), saved.data_ptr(), kept, workspace.data_ptr(), need, _stream(), kernels=17)
+    return dx, [wq, bq, wk, bk, wv, *grads]
+
+
 # ---------------------------------------------------------------------------------------------------------
 # the whole model
 # ---------------------------------------------------------------------------------------------------------

@@ -173,3 +173,38 @@ def test_attention_backward_tiles(B, H, dpk, S):
     for n, a, b in zip('QKV', got, want):
         assert rel_l2(a, b) < TOL, n
     assert all(torch.equal(a, b) for a, b in zip(got, ops.galerkin_attention_backward(q, k, v, dout)))
+
+
+# one node, ends of a 128-row tile, samples that share tiles, rows around the weight gradients' 32-row blocks and chains
+@pytest.mark.parametrize('B,S', [(1, 1), (1, 127), (2, 129), (3, 171), (4, 1849), (40, 33)])
+def test_encoder_layer_training_gradients(B, S):
+    from spgt_b200 import ops
+    layer, g = _layer(S)
+    x, pos, dy = torch.randn(B, S, 128, generator=g), torch.rand(B, S, 2, generator=g), torch.randn(B, S, 128, generator=g)
+    p = {k: v.detach().double().requires_grad_() for k, v in layer.state_dict().items()}
+    xr = x.double().requires_grad_()
+    cfg = dict(num_head=4, dim_hidden=128, attn_norm_eps=1e-6, acti_encoder_ffn='relu')
+    names = [n for n, _ in layer.named_parameters()]
+    layer = layer.cuda().train()
+    xd = x.cuda().requires_grad_()
+    taps = {}
+    O.encoder_layer(xr, pos.double(), p, '', cfg, taps)
+    x1, linear = taps['post_attn'], torch.nn.functional.linear
+    runs = []
+    for _ in range(2):
+        y = layer.forward_train(xd, pos.cuda())
+        runs.append((y, *torch.autograd.grad(y, [xd] + list(layer.parameters()), dy.cuda())))
+    y = layer.forward_train(xd, pos.cuda())
+    passes = y.grad_fn.saved_tensors[3].cpu() > 0          # a value within rounding of zero may pass the ReLU there and not in float64
+    h = linear(x1, p['ffn_layer.layer1.weight'], p['ffn_layer.layer1.bias']) * passes
+    ref = x1 + linear(h, p['ffn_layer.layer2.weight'], p['ffn_layer.layer2.bias'])
+    want = torch.autograd.grad(ref, [xr] + [p[n] for n in names], dy.double())
+    assert ops.tc_status() == 0 and y.grad_fn.name().startswith('_EncoderLayerFunction')
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
+    assert rel_l2(runs[0][0], ref.detach()) < TOL
+    for n, a, b in zip(['x'] + names, runs[0][1:], want):
+        assert rel_l2(a, b) < 2 * TOL, n
+    handle = layer.ffn_layer.layer1.register_forward_hook(lambda m, i, o: None)      # an observed layer runs op by op
+    y = layer.forward_train(xd, pos.cuda())
+    handle.remove()
+    assert not y.grad_fn.name().startswith('_EncoderLayerFunction') and rel_l2(y, runs[0][0]) < TOL
