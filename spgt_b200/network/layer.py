@@ -105,7 +105,7 @@ def _conv_kn(weight: Tensor) -> Tensor:
 
 def _linear_tc(weight: Tensor) -> 'ops.TcWeight':
     """torch Linear weight [out, in] prepared for the tcgen05 GEMM."""
-    return ops.TcWeight(weight.detach().t().contiguous())
+    return ops.TcWeight(_dense(weight), transposed=True)
 
 
 def _conv_tc(weight: Tensor, bias: Tensor, cin_pad: int, cout_pad: int):

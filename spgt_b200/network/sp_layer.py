@@ -69,9 +69,9 @@ class Sp_GalerkinAttention(_KernelWeights):
         """K and V weights as the fused layer takes them: by head pair K0 K1 V0 V1 | K2 K3 V2 V3, less each head's channel mean (the
         LayerNorm's subtraction, done once on the weights)."""
         def make():
-            centred = lambda w: (h := w.detach().reshape(-1, self.num_head, self.dim_head)) - h.mean(dim=2, keepdim=True)
-            kv = torch.stack([centred(self.weight_K), centred(self.weight_V)], dim=1).view(-1, 2, 2, 64)      # [128, K | V, pair, 64]
-            return ops.TcWeight(kv.transpose(1, 2).reshape(-1, 256).contiguous())
+            w = torch.stack([self.weight_K.detach(), self.weight_V.detach()], dim=1).view(-1, 2, self.num_head, self.dim_head)
+            w = (w - w.mean(dim=3, keepdim=True)).view(-1, 2, 2, 64)                  # [128, K | V, pair, 64]
+            return ops.TcWeight(w.transpose(1, 2).reshape(-1, 256))
         return self._cached('wkv', make)
 
     def forward(self, Q: Tensor, K: Tensor, V: Tensor, position: Tensor, residual: Tensor = None) -> Tensor:
