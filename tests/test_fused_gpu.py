@@ -208,3 +208,16 @@ def test_encoder_layer_training_gradients(B, S):
     y = layer.forward_train(xd, pos.cuda())
     handle.remove()
     assert not y.grad_fn.name().startswith('_EncoderLayerFunction') and rel_l2(y, runs[0][0]) < TOL
+
+
+# ragged segments, one pixel, channel counts that fill a block, divide it unevenly or exceed it
+@pytest.mark.parametrize('B,Hi,Ho,c', [(1, 5, 1, (2, 1, 1)), (2, 77, 43, (42, 42, 44)), (64, 19, 9, (42, 42, 44)), (1, 31, 50, (100, 101, 99)), (3, 8, 8, (5, 6, 9))])
+def test_bilinear_concat3(B, Hi, Ho, c):
+    from spgt_b200 import ops
+    g = torch.Generator().manual_seed(Hi)
+    pad = lambda n: (n + 3) // 4 * 4
+    x = [torch.randn(B, Hi, Hi, pad(n), generator=g) for n in c]
+    y = ops.bilinear_concat3(*[t.cuda() for t in x], *c, Ho, Ho, 'relu')
+    cat = torch.cat([t[..., :n] for t, n in zip(x, c)], dim=-1).permute(0, 3, 1, 2)
+    ref = torch.relu(torch.nn.functional.interpolate(cat, size=(Ho, Ho), mode='bilinear', align_corners=True)).permute(0, 2, 3, 1)
+    assert rel_l2(y, ref) < 1e-6          # (the same fp32 source coordinates, four products and three sums)
