@@ -51,6 +51,13 @@ class ParameterWatch:
             return True
         return any(d['_forward_hooks'] or d['_forward_pre_hooks'] or 'forward' in d for d in self._seen(module)[4])
 
+    def backward_observed(self, *called: torch.nn.Module) -> bool:
+        """Whether hooks wait for the gradients that pass the modules `called`: they fire, and may replace the gradients, only where
+        the modules themselves are called."""
+        if _hooks._global_backward_hooks or _hooks._global_backward_pre_hooks:
+            return True
+        return any(m._backward_hooks or m._backward_pre_hooks for m in called)
+
     def hold(self, module: torch.nn.Module) -> list:
         """Aliases of the parameters' storages: while they are kept, no other tensor can come to lie at these addresses."""
         return [d[k].detach() for d, k in self._seen(module)[2]]

@@ -174,12 +174,19 @@ class Sp_EncoderLayer(_KernelWeights):
                 and self.attention_layer.fusable and f.layer1.in_features == 128 and f.layer1.out_features == 256
                 and f.layer2.out_features == 128)
 
+    def trains_fused(self) -> bool:
+        """Whether the fused training layer stands for this one: its widths and activation, the modules' own linear layers, nothing
+        that watches or alters their calls or the gradients through them."""
+        a, f = self.attention_layer, self.ffn_layer
+        if not self.fusable or f.activation != 'relu':
+            return False
+        linears = (a.fc_layer, f.layer1, f.layer2)
+        return (all(type(l) is torch.nn.Linear and l.bias is not None for l in linears)
+                and not self._watch.observed(self) and not self._watch.backward_observed(*linears))
+
     def forward_train(self, X: Tensor, position: Tensor) -> Tensor:
         a, f = self.attention_layer, self.ffn_layer
-        # the fused training layer: its widths and activation, the modules' own linear layers, nothing that watches or alters their calls
-        if (self.fusable and f.activation == 'relu' and X.is_cuda and X.dim() == 3 and X.dtype == torch.float32 and not torch.is_autocast_enabled()
-                and all(type(l) is torch.nn.Linear and l.bias is not None for l in (a.fc_layer, f.layer1, f.layer2))
-                and not self._watch.observed(self)):
+        if X.is_cuda and X.dim() == 3 and X.dtype == torch.float32 and not torch.is_autocast_enabled() and self.trains_fused():
             return _EncoderLayerFunction.apply(
                 X, position, a.norm_eps, a.weight_Q, a.bias_Q, a.weight_K, a.bias_K, a.weight_V, a.bias_V, a.ln_weight_K, a.ln_bias_K,
                 a.ln_weight_V, a.ln_bias_V, a.fc_layer.weight, a.fc_layer.bias, f.layer1.weight, f.layer1.bias, f.layer2.weight, f.layer2.bias)

@@ -210,6 +210,24 @@ def test_encoder_layer_training_gradients(B, S):
     assert not y.grad_fn.name().startswith('_EncoderLayerFunction') and rel_l2(y, runs[0][0]) < TOL
 
 
+def test_encoder_layer_training_runs_backward_hooks():
+    """Hooks on the linear layers see, and may change, the gradients as they do op by op."""
+    layer, g = _layer(7)
+    layer = layer.cuda().train()
+    x, pos, dy = torch.randn(2, 45, 128, generator=g).cuda().requires_grad_(), torch.rand(2, 45, 2, generator=g).cuda(), torch.randn(2, 45, 128, generator=g).cuda()
+    plain = torch.autograd.grad(layer.forward_train(x, pos), layer.attention_layer.fc_layer.bias, dy)[0]
+    seen = []
+    members = (layer.attention_layer.fc_layer, layer.ffn_layer.layer1, layer.ffn_layer.layer2)
+    handles = [m.register_full_backward_hook(lambda m, gi, go: seen.append(m)) for m in members]
+    handles.append(members[0].register_full_backward_pre_hook(lambda m, go: (2 * go[0],)))
+    hooked = torch.autograd.grad(layer.forward_train(x, pos), [x, members[0].bias], dy)[1]
+    assert {id(m) for m in seen} == {id(m) for m in members}
+    assert rel_l2(hooked, 2 * plain) < TOL
+    for h in handles:
+        h.remove()
+    assert torch.equal(torch.autograd.grad(layer.forward_train(x, pos), members[0].bias, dy)[0], plain)
+
+
 # ragged segments, one pixel, channel counts that fill a block, divide it unevenly or exceed it
 @pytest.mark.parametrize('B,Hi,Ho,c', [(1, 5, 1, (2, 1, 1)), (2, 77, 43, (42, 42, 44)), (64, 19, 9, (42, 42, 44)), (1, 31, 50, (100, 101, 99)), (3, 8, 8, (5, 6, 9))])
 def test_bilinear_concat3(B, Hi, Ho, c):

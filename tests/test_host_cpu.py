@@ -220,3 +220,22 @@ def test_models_are_freed_without_a_garbage_collection():
         assert all(r() is None for r in seen)
     finally:
         gc.enable()
+
+
+def test_fused_training_layer_yields_to_backward_hooks():
+    """Hooks on the gradients of the linear layers fire only where those are called as modules."""
+    from torch.nn.modules import module as hooks
+    from spgt_b200.network.sp_layer import Sp_EncoderLayer
+    layer = Sp_EncoderLayer(128, 4, 2, 1e-6, 0.0, 0.0, 1e-2, 1e-2, False, 256, 0.0, 'relu')
+    members = (layer.attention_layer.fc_layer, layer.ffn_layer.layer1, layer.ffn_layer.layer2)
+    takers = [getattr(m, r) for m in members for r in ('register_full_backward_hook', 'register_full_backward_pre_hook')]
+    takers += [hooks.register_module_full_backward_hook, hooks.register_module_full_backward_pre_hook]
+    assert layer.trains_fused()
+    for register in takers:
+        handle = register(lambda *args: None)
+        assert not layer.trains_fused()
+        handle.remove()
+        assert layer.trains_fused()
+    layer.register_full_backward_hook(lambda *args: None)          # (forward_train does not call these as modules)
+    layer.ffn_layer.register_full_backward_hook(lambda *args: None)
+    assert layer.trains_fused()
