@@ -29,20 +29,22 @@ class ParameterWatch:
         modules = list(module.modules())
         return ([(d, len(d)) for m in modules for d in (m._modules, m._parameters)],
                 [(m._modules, k, c) for m in modules for k, c in m._modules.items()],
-                [(m._parameters, k) for m in modules for k, p in m._parameters.items() if p is not None],
+                [(m._parameters, k) for m in modules for k in m._parameters],
                 [(m.__dict__, k) for m in modules[1:] for k in self.OPTIONS if k in m.__dict__],
                 [m.__dict__ for m in modules[1:]])
 
     def _seen(self, module: torch.nn.Module) -> tuple:
         tree = self._tree
-        if tree is None or any(len(d) != n for d, n in tree[0]) or any(d[k] is not c for d, k, c in tree[1]):
+        if tree is None or any(len(d) != n for d, n in tree[0]) or any(d.get(k, 0) is not c for d, k, c in tree[1]):
             tree = self._tree = self._walk(module)
         return tree
 
     def tag(self, module: torch.nn.Module) -> tuple:
         tree = self._seen(module)
-        params = [d[k] for d, k in tree[2]]
-        return tuple([p._version for p in params] + [p.data_ptr() for p in params] + [d[k] for d, k in tree[3]]
+        if not all(k in d for d, k in tree[2]):           # renamed (pruning, spectral normalisation): as many entries as before
+            tree = self._tree = self._walk(module)
+        params = [d[k] for d, k in tree[2]]               # (None where a bias has been taken out)
+        return tuple([-1 if p is None else p._version for p in params] + [0 if p is None else p.data_ptr() for p in params] + [d.get(k) for d, k in tree[3]]
                      + [module.__dict__.get(k) for k in self.OPTIONS])
 
     def observed(self, module: torch.nn.Module) -> bool:
@@ -60,7 +62,7 @@ class ParameterWatch:
 
     def hold(self, module: torch.nn.Module) -> list:
         """Aliases of the parameters' storages: while they are kept, no other tensor can come to lie at these addresses."""
-        return [d[k].detach() for d, k in self._seen(module)[2]]
+        return [d[k].detach() for d, k in self._seen(module)[2] if d.get(k) is not None]
 
     def __deepcopy__(self, memo):
         return ParameterWatch()

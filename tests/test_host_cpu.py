@@ -239,3 +239,27 @@ def test_fused_training_layer_yields_to_backward_hooks():
     layer.register_full_backward_hook(lambda *args: None)          # (forward_train does not call these as modules)
     layer.ffn_layer.register_full_backward_hook(lambda *args: None)
     assert layer.trains_fused()
+
+
+def test_parameter_watch_follows_renamed_and_removed_parameters():
+    """Pruning and spectral normalisation put another name in a parameter's place, so that a module has as many as before."""
+    from torch.nn.utils import prune, spectral_norm
+    from spgt_b200.network.sp_layer import Sp_EncoderLayer
+    layer = Sp_EncoderLayer(128, 4, 2, 1e-6, 0.0, 0.0, 1e-2, 1e-2, False, 256, 0.0, 'relu')
+    attention, ffn = layer.attention_layer, layer.ffn_layer
+    tags = [layer._watch.tag(layer)]
+    prune.l1_unstructured(attention.fc_layer, 'weight', 0.3)
+    tags.append(layer._watch.tag(layer))
+    spectral_norm(ffn.layer1)
+    tags.append(layer._watch.tag(layer))
+    attention.bias_Q = None
+    tags.append(layer._watch.tag(layer))
+    assert len(set(tags)) == 4 and layer._watch.tag(layer) == tags[-1]
+    names = {n for n, _ in layer.named_parameters()}
+    assert len(layer._watch.hold(layer)) == len(names) == 15
+    with torch.no_grad():
+        attention.fc_layer.weight_orig.add_(1.0)
+    assert layer._watch.tag(layer) != tags[-1]
+    tags.append(layer._watch.tag(layer))
+    attention.bias_Q = torch.nn.Parameter(torch.zeros(128))
+    assert layer._watch.tag(layer) not in tags and len(layer._watch.hold(layer)) == 16
