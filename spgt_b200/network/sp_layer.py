@@ -171,7 +171,8 @@ class Sp_EncoderLayer(_KernelWeights):
     def fusable(self) -> bool:
         f = self.ffn_layer
         return (type(self.attention_layer) is Sp_GalerkinAttention and type(f) is FeedForward and f.fused
-                and self.attention_layer.fusable and f.layer1.in_features == 128 and f.layer1.out_features == 256
+                and self.attention_layer.fusable and type(f.layer1) is torch.nn.Linear and type(f.layer2) is torch.nn.Linear
+                and f.layer1.in_features == 128 and f.layer1.out_features == 256
                 and f.layer2.out_features == 128)
 
     def trains_fused(self) -> bool:

@@ -173,6 +173,8 @@ class Sp_GalerkinTransformer2D(torch.nn.Module):
     def _native_plan(self, X: Tensor):
         """The model as the one-call forward takes it, rebuilt when the parameters, the grid or the device are not the ones it was
         made for; None for widths that forward does not cover."""
+        if not (type(self.down_scaler) is DownScaler2D and type(self.up_scaler) is UpScaler2D):
+            return None
         sizes = [tuple(map(tuple, m.resolution_size)) for m in (self.down_scaler, self.up_scaler)]
         tag = (X.shape[1], X.device, self.normalizer, self.boundary_condition, sizes, self._watch.tag(self))
         plan = self._plan                                    # (read once: another thread may replace it)
@@ -238,9 +240,10 @@ class Sp_GalerkinTransformer2D(torch.nn.Module):
         """Whether the one-call forward covers this model: its own module types, the widths the kernels are made for, and one
         activation and epsilon throughout."""
         enc, dec, down, up = self.encoder_mixer.layers, self.decoder_regressor, self.down_scaler, self.up_scaler
-        if not (type(down) is DownScaler2D and type(up) is UpScaler2D and type(dec) is Sp_DecoderRegressor
+        if not (type(dec) is Sp_DecoderRegressor
                 and all(type(l) is Sp_EncoderLayer for l in enc) and all(type(l) is Sp_SpectralConv2D for l in dec.layers)
-                and all(type(c) is ConvResBlock2D for c in (down.conv0, down.conv1, down.conv2, down.conv3, up.conv))):
+                and all(type(c) is ConvResBlock2D for c in (down.conv0, down.conv1, down.conv2, down.conv3, up.conv))
+                and type(up.conv.conv_layer) is torch.nn.Conv2d and type(dec.spatial_fc_layer) is torch.nn.Linear):
             return False
         return (all(l.fusable and l.attention_layer.norm_eps == enc[0].attention_layer.norm_eps
                     and l.ffn_layer.activation == enc[0].ffn_layer.activation for l in enc)

@@ -113,6 +113,21 @@ def test_one_call_forward_yields_to_observed_or_changed_modules():
 
         def forward(self, x, position):
             return self.inner(self.inner(x, position), position)
+    class Scaler(torch.nn.Module):
+        def __init__(self, inner):
+            super().__init__()
+            self.inner = inner
+
+        def forward(self, x):
+            return self.inner(x)
+
+        def forward_mid(self, x):
+            return self.inner.forward_mid(x)
+    for name in ('down_scaler', 'up_scaler'):
+        inner = getattr(model, name)
+        setattr(model, name, Scaler(inner))
+        assert rel_l2(model(*args), ref) < TOL
+        setattr(model, name, inner)
     plain = model.encoder_mixer.layers[1]
     model.encoder_mixer.layers[1] = Twice(plain)
     twice = model(*args)

@@ -263,3 +263,38 @@ def test_parameter_watch_follows_renamed_and_removed_parameters():
     tags.append(layer._watch.tag(layer))
     attention.bias_Q = torch.nn.Parameter(torch.zeros(128))
     assert layer._watch.tag(layer) not in tags and len(layer._watch.hold(layer)) == 16
+
+
+class _Around(torch.nn.Module):
+    """Another module in a submodule's place, with the calls the model makes and nothing else."""
+
+    def __init__(self, inner):
+        super().__init__()
+        self.inner = inner
+
+    def forward(self, *args, **kwargs):
+        return self.inner(*args, **kwargs)
+
+    def forward_mid(self, X):
+        return self.inner.forward_mid(X)
+
+    def forward_from_mid(self, *args):
+        return self.inner.forward_from_mid(*args)
+
+
+def test_exchanged_submodules_are_not_planned_for():
+    from spgt_b200.config.config_accessor import get_darcy_config
+    from spgt_b200.network.sp_model import Sp_GalerkinTransformer2D
+    X = torch.zeros(1, 29, 29, 1)
+    make = lambda: Sp_GalerkinTransformer2D(get_darcy_config(3, 6, num_frequence_mode=4, clamp_attn=False, fine_resolution=85, num_encoder_layer=2))
+    for path in ('down_scaler', 'up_scaler', 'decoder_regressor', 'encoder_mixer.layers.0', 'encoder_mixer.layers.1.attention_layer',
+                 'encoder_mixer.layers.0.ffn_layer', 'encoder_mixer.layers.0.ffn_layer.layer1', 'encoder_mixer.layers.0.ffn_layer.layer2',
+                 'down_scaler.conv1', 'up_scaler.conv.conv_layer', 'decoder_regressor.spatial_fc_layer', 'decoder_regressor.layers.1'):
+        model = make()
+        parent, _, name = path.rpartition('.')
+        parent = model.get_submodule(parent)
+        setattr(parent, name, _Around(getattr(parent, name)))
+        assert model._native_plan(X) is None, path
+    layer = make().encoder_mixer.layers[0]
+    layer.attention_layer.fc_layer = _Around(layer.attention_layer.fc_layer)
+    assert not layer.trains_fused()
