@@ -105,9 +105,12 @@ def _chk(t: Tensor, name: str, dtype=torch.float32) -> Tensor:
     return t
 
 
-def _position(t: Tensor, name: str) -> Tensor:
-    """Node coordinates for the kernels that read a node's two values at once: a copy where they start at an odd value."""
-    _chk(t, name)
+def _position(t: Tensor, nodes: int) -> Tensor:
+    """Node coordinates for the kernels that read a node's two values at once: the first `nodes` nodes of t [..., 2], whatever its
+    other dimensions; a copy where they start at an odd value."""
+    _chk(t, 'position')
+    if t.shape[-1:] != (2,) or t.numel() < 2 * nodes:
+        raise ValueError(f'position must hold two values for each of {nodes} nodes')
     return t if t.data_ptr() % 8 == 0 else t.clone()
 
 
@@ -606,10 +609,10 @@ class EncoderPlan:
 def encoder_layer(plan: EncoderPlan, x: Tensor, position: Tensor, eps: float, act=None, ffn: bool = True, residual: bool = True) -> Tensor:
     """x [B,S,128], position [B,S,2] -> the encoder layer's output (ffn), or the attention layer's (+ x with residual)."""
     _chk(x, 'x')
-    position = _position(position, 'position')
     B, S, D = x.shape
-    if D != 128 or position.shape != (B, S, 2):
-        raise ValueError('x must be [B, S, 128] and position [B, S, 2]')
+    if D != 128:
+        raise ValueError('x must be [B, S, 128]')
+    position = _position(position, B * S)
     need = plan.need.get((B, S))
     if need is None:
         need = plan.need[(B, S)] = int(lib.spgt_encoder_workspace_bytes(B, S))
@@ -626,12 +629,13 @@ _ENCODER_PARAMS = 16          # wq, bq, wk, bk, wv, bv, lnwk, lnbk, lnwv, lnbv, 
 
 def encoder_train_forward(x: Tensor, position: Tensor, eps: float, params: Sequence[Tensor]):
     """(merged attention [B,S,136], what the layer's backward needs) for x [B,S,128], position [B,S,2] and the layer's 16 parameters."""
-    _chk(x, 'x'); _chk(position, 'position')
+    _chk(x, 'x')
     for p in params:
         _chk(p, 'parameter')
     B, S, D = x.shape
-    if D != 128 or position.shape != (B, S, 2) or len(params) != _ENCODER_PARAMS:
-        raise ValueError('x must be [B, S, 128] and position [B, S, 2]')
+    if D != 128 or len(params) != _ENCODER_PARAMS:
+        raise ValueError('x must be [B, S, 128], with 16 parameters')
+    position = _position(position, B * S)
     need = int(lib.spgt_encoder_train_saved_bytes(B, S))
     with _device(x.device):
         att, saved = torch.empty(B, S, 136, device=x.device, dtype=x.dtype), torch.empty(need // 4, device=x.device, dtype=x.dtype)
@@ -686,7 +690,7 @@ def darcy_forward(plan: DarcyPlan, node: Tensor, position: Tensor, grid: Tensor,
     """node [B,r,r,1], position [B,ra,ra,d_pos], grid [B,r,r,2] -> [B,r,r,1]; `taps` receives intermediate tensors."""
     m = plan.model
     B, r, S = node.shape[0], m.r, m.ra * m.ra
-    position = _position(position.reshape(B, S, position.size(-1)), 'position')
+    position = _position(position.reshape(B, S, position.size(-1)), B * S)
     _chk(node, 'node'); _chk(grid, 'grid')
     if node.numel() != B * r * r or position.numel() != B * S * m.d_pos or grid.numel() != 2 * B * r * r:
         raise ValueError('node, position and grid do not match the model\'s grids')

@@ -140,6 +140,35 @@ def test_one_call_forward_yields_to_observed_or_changed_modules():
     assert rel_l2(model(*args), ref) > 1e-3
 
 
+def test_one_call_forward_yields_to_other_grids():
+    """A grid of other nodes (the regressor is evaluated there), or one with more samples than there are fields."""
+    from spgt_b200.dataset.darcy_dataset import meshgrid
+    model, node, position, grid = _model()
+    ref = model(node, position, grid)
+    assert torch.equal(model(node[:2], position[:2], grid), ref[:2])
+    other = torch.from_numpy(meshgrid(57, 1)).float().expand(3, 57, 57, 2).contiguous()
+    out = model(node, position, other.cuda())
+    cfg = O.default_config(85, 3, 6, 4, 2, 2)
+    cfg['resolution_size'] = [*cfg['resolution_size'][:4], (57, 57)]
+    want = O.model_forward(node.cpu().double(), position.cpu().double(), other.double(), O.to_dtype(model.cpu().state_dict(), torch.float64), cfg)
+    assert rel_l2(out, want) < TOL
+    with pytest.raises((ValueError, RuntimeError)):
+        model.cuda()(node.squeeze(-1), position, grid)          # (the fields have a channel dimension)
+
+
+@pytest.mark.parametrize('training', [False, True])
+def test_encoder_layer_takes_positions_of_any_leading_shape(training):
+    layer, g = _layer(5)
+    layer = layer.cuda().train(training)
+    x, pos = torch.randn(2, 49, 128, generator=g).cuda(), torch.rand(3, 49, 2, generator=g).cuda()
+    run = layer.forward_train if training else layer
+    with torch.no_grad():
+        ref = run(x, pos[:2].contiguous())
+        assert torch.equal(run(x, pos[:2].view(2, 7, 7, 2)), ref) and torch.equal(run(x, pos), ref)
+        with pytest.raises(ValueError):
+            run(x, pos[:1].contiguous())
+
+
 def test_encoder_layer_takes_any_dense_or_strided_weights_and_positions():
     layer, g = _layer(3)
     x, pos = torch.randn(2, 45, 128, generator=g).cuda(), torch.rand(2, 45, 2, generator=g).cuda()
