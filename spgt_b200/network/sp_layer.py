@@ -121,26 +121,45 @@ def _attention_forward_train(self, Q: Tensor, K: Tensor, V: Tensor, position: Te
 Sp_GalerkinAttention.forward_train = _attention_forward_train
 
 
+def _encoder_layer_by_ops(x: Tensor, position: Tensor, eps: float, params) -> Tensor:
+    """The encoder layer (width 128, 4 heads, 2 position values, ReLU) on the single differentiable ops."""
+    from ..extension.bind.galerkin_attention import (multihead_galerkin_attention_cccr_cuda,
+                                                     multihead_projection_layernorm_with_position_rrc_cuda,
+                                                     multihead_projection_with_position_rrc_cuda)
+    wq, bq, wk, bk, wv, bv, lnwk, lnbk, lnwv, lnbv, wfc, bfc, w1, b1, w2, b2 = params
+    linear = torch.nn.functional.linear
+    q = multihead_projection_with_position_rrc_cuda(x, wq, bq, position, 4, 32, 2)
+    k = multihead_projection_layernorm_with_position_rrc_cuda(x, wk, bk, lnwk, lnbk, position, eps, 4, 32, 2)
+    v = multihead_projection_layernorm_with_position_rrc_cuda(x, wv, bv, lnwv, lnbv, position, eps, 4, 32, 2)
+    att = multihead_galerkin_attention_cccr_cuda(q, k, v).transpose(1, 2).reshape(x.shape[0], x.shape[1], 136)
+    x = x + linear(att, wfc, bfc)
+    return x + linear(torch.relu(linear(x, w1, b1)), w2, b2)
+
+
 class _EncoderLayerFunction(torch.autograd.Function):
     """X + attention(X), then + ffn(.): projections and attention in one native call, their backward and all weight gradients in
-    another; the dense layers' products along the layer are plain fp32, whose last bits decide what passes the ReLU."""
+    another; the dense layers' products along the layer are plain fp32, whose last bits decide what passes the ReLU.  A backward
+    pass that is to be differentiated again (create_graph) runs on the single ops, whose gradients carry a graph."""
 
     @staticmethod
     def forward(ctx, x, position, eps, *params):
+        ctx.eps, inputs = eps, (x, position, *params)
         x, params = x.contiguous(), [_dense(p) for p in params]
         att, saved = ops.encoder_train_forward(x, position.contiguous(), eps, params)
         linear = torch.nn.functional.linear
         x1 = x + linear(att, params[10], params[11])
         h = torch.relu(linear(x1, params[12], params[13]))
-        ctx.save_for_backward(x, att, x1, h, saved, *params)
-        ctx.eps = eps
+        ctx.save_for_backward(att, x1, h, saved, *inputs)
         return x1 + linear(h, params[14], params[15])
 
     @staticmethod
-    @torch.autograd.function.once_differentiable
     def backward(ctx, grad_out):
-        x, att, x1, h, saved, *params = ctx.saved_tensors
-        dx, grads = ops.encoder_train_backward(x, att, x1, h, ctx.eps, params, saved, _dense(grad_out))
+        att, x1, h, saved, x, position, *params = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            wanted = [t for t, need in zip((x, *params), (ctx.needs_input_grad[0], *ctx.needs_input_grad[3:])) if need]
+            grads = iter(torch.autograd.grad(_encoder_layer_by_ops(x, position, ctx.eps, params), wanted, grad_out, create_graph=True))
+            return tuple(next(grads) if need else None for need in ctx.needs_input_grad)
+        dx, grads = ops.encoder_train_backward(x.contiguous(), att, x1, h, ctx.eps, [_dense(p) for p in params], saved, _dense(grad_out))
         return (dx, None, None, *grads)
 
 

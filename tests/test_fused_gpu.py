@@ -140,6 +140,27 @@ def test_one_call_forward_yields_to_observed_or_changed_modules():
     assert rel_l2(model(*args), ref) > 1e-3
 
 
+def test_encoder_layer_training_differentiates_twice():
+    """A penalty on one weight's gradient: its own gradients go through the layer's backward and forward pass."""
+    layer, g = _layer(11)
+    x, pos = torch.randn(2, 45, 128, generator=g), torch.rand(2, 45, 2, generator=g)
+    p = {k: v.detach().double().requires_grad_() for k, v in layer.state_dict().items()}
+    cfg = dict(num_head=4, dim_hidden=128, attn_norm_eps=1e-6, acti_encoder_ffn='relu')
+    xr = x.double().requires_grad_()
+
+    def penalty(y, weight):
+        grad, = torch.autograd.grad(y.square().mean(), weight, create_graph=True)
+        return grad.square().sum()
+    w2 = 'ffn_layer.layer2.weight'
+    names = ['attention_layer.weight_K', 'attention_layer.fc_layer.weight', w2]
+    want = torch.autograd.grad(penalty(O.encoder_layer(xr, pos.double(), p, '', cfg), p[w2]), [xr, *(p[n] for n in names)])
+    layer = layer.cuda().train()
+    dev, xd = dict(layer.named_parameters()), x.cuda().requires_grad_()
+    got = torch.autograd.grad(penalty(layer.forward_train(xd, pos.cuda()), dev[w2]), [xd, *(dev[n] for n in names)])
+    for n, a, b in zip(['x'] + names, got, want):
+        assert rel_l2(a, b) < TOL, n
+
+
 def test_one_call_forward_yields_to_other_grids():
     """A grid of other nodes (the regressor is evaluated there), or one with more samples than there are fields."""
     from spgt_b200.dataset.darcy_dataset import meshgrid
@@ -239,7 +260,7 @@ def test_encoder_layer_training_gradients(B, S):
         y = layer.forward_train(xd, pos.cuda())
         runs.append((y, *torch.autograd.grad(y, [xd] + list(layer.parameters()), dy.cuda())))
     y = layer.forward_train(xd, pos.cuda())
-    passes = y.grad_fn.saved_tensors[3].cpu() > 0          # a value within rounding of zero may pass the ReLU there and not in float64
+    passes = y.grad_fn.saved_tensors[2].cpu() > 0          # a value within rounding of zero may pass the ReLU there and not in float64
     h = linear(x1, p['ffn_layer.layer1.weight'], p['ffn_layer.layer1.bias']) * passes
     ref = x1 + linear(h, p['ffn_layer.layer2.weight'], p['ffn_layer.layer2.bias'])
     want = torch.autograd.grad(ref, [xr] + [p[n] for n in names], dy.double())
