@@ -202,6 +202,7 @@ class Sp_EncoderLayer(_KernelWeights):
             return False
         linears = (a.fc_layer, f.layer1, f.layer2)
         return (all(type(l) is torch.nn.Linear and l.bias is not None for l in linears)
+                and all(b is not None for b in (a.bias_Q, a.bias_K, a.bias_V))
                 and not self._watch.observed(self) and not self._watch.backward_observed(*linears))
 
     def forward_train(self, X: Tensor, position: Tensor) -> Tensor:

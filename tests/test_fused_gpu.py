@@ -161,6 +161,18 @@ def test_encoder_layer_training_differentiates_twice():
         assert rel_l2(a, b) < TOL, n
 
 
+def test_encoder_layer_training_without_a_projection_bias():
+    layer, g = _layer(13)
+    x, pos = torch.randn(2, 45, 128, generator=g), torch.rand(2, 45, 2, generator=g)
+    with torch.no_grad():
+        layer.attention_layer.bias_K.zero_()
+    layer = layer.cuda().train()
+    with torch.no_grad():
+        ref = layer.forward_train(x.cuda(), pos.cuda())
+        layer.attention_layer.bias_K = None
+        assert rel_l2(layer.forward_train(x.cuda(), pos.cuda()), ref) < TOL
+
+
 def test_one_call_forward_yields_to_other_grids():
     """A grid of other nodes (the regressor is evaluated there), or one with more samples than there are fields."""
     from spgt_b200.dataset.darcy_dataset import meshgrid
