@@ -88,10 +88,17 @@ __device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) 
     lo = __float_as_uint(x - __uint_as_float(hi));
 }
 
-// Same, with lo also rounded to tf32 (round to nearest) instead of being truncated by the tensor core: two more
-// instructions, unbiased error; used where thousands of products are summed (the K^T V reduction over grid nodes).
+// Same, with lo also rounded to tf32 (round to nearest) instead of being truncated by the tensor core: one more
+// instruction, unbiased error; used where thousands of products are summed (the K^T V reduction over grid nodes).
+// hi comes from the conversion instruction here: the integer rounding turns the NaN that arithmetic makes (0x7fffffff) into a
+// zero, which split_tf32 survives because its lo is that NaN still, while the rounding of lo would lose it there as well.
+__device__ __forceinline__ uint32_t tf32_rna_cvt(float x) {
+    uint32_t r;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+    return r;
+}
 __device__ __forceinline__ void split_tf32_rn(float x, uint32_t& hi, uint32_t& lo) {
-    hi = tf32_rna_bits(x);
+    hi = tf32_rna_cvt(x);
     lo = tf32_rna_bits(x - __uint_as_float(hi));
 }
 

@@ -199,12 +199,11 @@ __host__ __device__ __forceinline__ uint32_t tc_swz(int r, int c) { return (uint
 // One element of a W stage image: the stage holds W_hi then W_lo, each [bn rows (n)][32 k] K-major with the 128-byte
 // swizzle; v = W[k][n], kk = k % 32.  W_lo is rounded to tf32 (the tensor core would truncate it).
 __device__ __forceinline__ void tc_img_store(float* stage, int bn, int n, int kk, float v) {
-    uint32_t h, l, l2;
+    uint32_t h, l;
     split_tf32(v, h, l);
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l2) : "f"(__uint_as_float(l)));
     const int off = (int)(tc_swz(n, kk >> 2) >> 2) + (kk & 3);
     stage[off] = __uint_as_float(h);
-    stage[bn * TC_BK + off] = __uint_as_float(l2);
+    stage[bn * TC_BK + off] = __uint_as_float(tf32_rna_cvt(__uint_as_float(l)));
 }
 // Weight images to make in one launch.  kind 0: w [K][ldw], 1: w [N][ldw] (transposed), 2: copy N floats.
 struct TcPrepJob { const float* w; float* img; int kind, ldw, K, N, kpad, bn; };

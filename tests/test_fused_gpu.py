@@ -316,3 +316,61 @@ def test_bilinear_concat3(B, Hi, Ho, c):
     cat = torch.cat([t[..., :n] for t, n in zip(x, c)], dim=-1).permute(0, 3, 1, 2)
     ref = torch.relu(torch.nn.functional.interpolate(cat, size=(Ho, Ho), mode='bilinear', align_corners=True)).permute(0, 2, 3, 1)
     assert rel_l2(y, ref) < 1e-6          # (the same fp32 source coordinates, four products and three sums)
+
+
+def _with_nan(t, at):
+    """t with a NaN as arithmetic on the GPU makes it (all mantissa bits set)."""
+    t = t.clone()
+    t.view(torch.int32).view(-1)[at] = 0x7fffffff
+    return t
+
+
+# one not-a-number in one operand: the values that depend on it, and no others, are NaN
+@pytest.mark.parametrize('which', ['x', 'weight', 'bias'])
+def test_projection_passes_nan_on(which):
+    from spgt_b200 import ops
+    g = torch.Generator().manual_seed(2)
+    t = {'x': torch.randn(1, 150, 128, generator=g), 'weight': torch.randn(128, 128, generator=g), 'bias': torch.randn(128, generator=g)}
+    t[which] = _with_nan(t[which], 77)
+    out = ops.projpos(*(v.cuda() for v in t.values()), torch.zeros(1, 150, 2).cuda(), 4, 32, 2)[0, :, 2:]
+    want = (t['x'][0] @ t['weight'] + t['bias']).t().reshape(4, 32, 150)
+    assert torch.equal(torch.isnan(out.cpu()), torch.isnan(want))
+
+
+@pytest.mark.parametrize('which', [0, 1, 2])
+def test_attention_passes_nan_on(which):
+    from spgt_b200 import ops
+    g = torch.Generator().manual_seed(3)
+    t = [torch.randn(1, 4, 34, 150, generator=g) for _ in range(3)]
+    t[which] = _with_nan(t[which], 5000)
+    q, k, v = t
+    out = ops.galerkin_attention(*(a.cuda() for a in t))
+    assert torch.equal(torch.isnan(out.cpu()), torch.isnan(q.transpose(2, 3) @ (k @ v.transpose(2, 3))))
+
+
+@pytest.mark.parametrize('r', [40, 260])
+@pytest.mark.parametrize('which', ['x', 'mode', 'residual'])
+def test_spectral_layer_passes_nan_on(r, which):
+    from spgt_b200 import ops
+    g = torch.Generator().manual_seed(4)
+    x, w = torch.randn(2, r, r, 32, generator=g), torch.randn(32, 32, generator=g)
+    fw = [torch.randn(4, 4, 32, 32, 2, generator=g) for _ in range(2)]
+    nan = torch.zeros(2, r, r, 32, dtype=torch.bool)
+    if which == 'x':
+        x, nan[1] = _with_nan(x, r * r * 32 + 100), True
+    elif which == 'mode':
+        fw[1], nan[..., 5] = _with_nan(fw[1], 2 * (32 * 40 + 5)), True
+    else:
+        w, nan[..., 7] = _with_nan(w, 32 * 3 + 7), True
+    out = ops.spectral_conv2d(x.cuda(), w.cuda(), torch.zeros(32).cuda(), fw[0].cuda(), fw[1].cuda(), 4, None)
+    assert torch.equal(torch.isnan(out.cpu()), nan)
+
+
+@pytest.mark.parametrize('which', [0, 1])
+def test_weight_gradient_gemm_passes_nan_on(which):
+    from spgt_b200 import ops
+    g = torch.Generator().manual_seed(6)
+    t = [torch.randn(3000, 128, generator=g), torch.randn(3000, 36, generator=g)]
+    t[which] = _with_nan(t[which], 5000)
+    c, sums = ops.tn_gemm(*(a.cuda() for a in t), column_sums=True)
+    assert torch.equal(torch.isnan(c.cpu()), torch.isnan(t[0].t() @ t[1])) and torch.equal(torch.isnan(sums.cpu()), torch.isnan(t[1].sum(0)))
