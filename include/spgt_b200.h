@@ -353,7 +353,7 @@ int spgt_encoder_layer_fwd(const spgt_encoder_weights* w, const float* x, const 
  * receives the three projections' [3][128][128].  fwd: weight images, projections + LayerNorm and attention, merged heads [B,S,136];
  * it keeps what bwd needs in `saved`.  bwd: every gradient, from x, the attention, x1 = x + attention wfc + bfc, h = relu(x1 w1 + b1),
  * dy and the gradients with respect to x1 w1 + b1 (dh), x1 (dx1) and the attention (da).  x, x1, dy, dx1, dx [B,S,128], h, dh [B,S,256],
- * da [B,S,136], pos [B,S,2].  p->wfc .. p->b2 are not read and may be NULL.  No counterpart as one call in the reference
+ * da [B,S,136], pos [B,S,2].  p->wfc .. p->b2 are not read and may be NULL; g->wfc .. g->b2 may all be NULL: not wanted.  No counterpart as one call in the reference
  * (network/sp_layer.py:52-104). */
 typedef struct { const float *wq, *bq, *wk, *bk, *wv, *bv, *lnwk, *lnbk, *lnwv, *lnbv, *wfc, *bfc, *w1, *b1, *w2, *b2; } spgt_encoder_params;
 typedef struct { float *wqkv, *bq, *bk, *bv, *lnwk, *lnbk, *lnwv, *lnbv, *wfc, *bfc, *w1, *b1, *w2, *b2; } spgt_encoder_grads;

@@ -9,7 +9,7 @@
 // warp-MMA kernel: with the tcgen05 one single hidden values fell on the other side of the ReLU (1e-5 to 2e-4 of a step's gradients).
 // Here: weight images (they change every step; one launch), projections and attention; then attention and LayerNorm backward to
 // dqkv = [dq dk dv], dx = dx1 + dq Wq^T + dk Wk^T + dv Wv^T, one product x^T dqkv for the three projections' weights and one per dense
-// layer, with the bias gradients as its column sums.  LayerNorm's input is recomputed from x.
+// layer (from 128 rows on, below which the caller's fp32 products are closer to fp64), with the bias gradients as its column sums.  LayerNorm's input is recomputed from x.
 // 141 x 141 nodes, batch 4, whole training step: 14.6 -> 10.2 ms.
 #include "tc_common.cuh"
 
@@ -101,8 +101,11 @@ extern "C" int spgt_encoder_train_bwd(const spgt_encoder_params* p, const spgt_e
                                       float* dx, int B, int S, float eps, const void* saved, size_t saved_bytes, void* workspace,
                                       size_t workspace_bytes, spgt_stream_t stream) {
     if (!p || !g || !x || !attention || !x1 || !h || !dy || !dh || !dx1 || !da || !dx || !saved || !workspace || !train_params_ok(p)) return SPGT_ERR_NULL;
-    for (const float* v : {g->wqkv, g->bq, g->bk, g->bv, g->lnwk, g->lnbk, g->lnwv, g->lnbv, g->wfc, g->bfc, g->w1, g->b1, g->w2, g->b2})
+    for (const float* v : {g->wqkv, g->bq, g->bk, g->bv, g->lnwk, g->lnbk, g->lnwv, g->lnbv})
         if (!v) return SPGT_ERR_NULL;
+    const bool dense = g->wfc != nullptr;                  // (all six or none)
+    for (const float* v : {g->bfc, g->w1, g->b1, g->w2, g->b2})
+        if ((v != nullptr) != dense) return SPGT_ERR_NULL;
     if (!train_sizes_ok(B, S)) return SPGT_ERR_SHAPE;
     const TrainSaved t((size_t)B * S);
     const TrainScratch c(B, S);
@@ -116,9 +119,11 @@ extern "C" int spgt_encoder_train_bwd(const spgt_encoder_params* p, const spgt_e
     const cudaStream_t st = (cudaStream_t)stream;
     void* tw = w + c.ws;
     // dense layers: dW = dy^T x as torch keeps it, [out][in]
-    SPGT_TRY(tn_gemm(dy, ET_D, h, ET_F, g->w2, ET_F, 128, g->b2, true, ET_D, ET_F, rows, tw, c.ws_bytes, st));
-    SPGT_TRY(tn_gemm(dh, ET_F, x1, ET_D, g->w1, ET_D, 128, g->b1, true, ET_F, ET_D, rows, tw, c.ws_bytes, st));
-    SPGT_TRY(tn_gemm(dx1, ET_D, attention, ET_A, g->wfc, ET_A, 128, g->bfc, true, ET_D, ET_A, rows, tw, c.ws_bytes, st));
+    if (dense) {
+        SPGT_TRY(tn_gemm(dy, ET_D, h, ET_F, g->w2, ET_F, 128, g->b2, true, ET_D, ET_F, rows, tw, c.ws_bytes, st));
+        SPGT_TRY(tn_gemm(dh, ET_F, x1, ET_D, g->w1, ET_D, 128, g->b1, true, ET_F, ET_D, rows, tw, c.ws_bytes, st));
+        SPGT_TRY(tn_gemm(dx1, ET_D, attention, ET_A, g->wfc, ET_A, 128, g->bfc, true, ET_D, ET_A, rows, tw, c.ws_bytes, st));
+    }
     // attention, LayerNorm, projections
     SPGT_TRY(galerkin_attn_bwd(s + t.q, s + t.k, s + t.v, da, w + c.dq, w + c.dk, w + c.dv, B, 4, 34, S, true, tw, c.ws_bytes, st));
     SPGT_TRY(spgt_linear_tc_fwd(x, ET_D, s + ET_KV, s + ET_BKV, nullptr, ET_F, w + c.hkv, ET_F, rows, ET_D, ET_F, SPGT_ACT_NONE, stream));

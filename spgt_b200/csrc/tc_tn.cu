@@ -3,13 +3,15 @@
 //
 // The reduction runs over the rows, so both operands are needed K-major with the rows as k: raw blocks of 32 rows arrive row-major
 // (cp.async, padded pitch), and eight warps store them TRANSPOSED - one operand row per matrix column, 32 long - as
-// hi / lo tiles.  Per 8 rows one MMA A_hi x [B_hi | B_lo] and one A_lo x B_hi, the latter on top of the B_lo columns.  The hi operand
-// is the plain fp32 value (the tensor core reads its upper 19 bits), lo what they leave, rounded.
-// Bound by shared memory: per 32 rows 512 transposing stores, 64 x 4 read phases and 80 KB of operand reads, about 1300 cycles.
-// Blocks split the rows; the accumulate step of an MMA truncates towards zero, so the large A_hi B_hi sums
-// have an accumulator of their own and all are added to fp32 registers every 128 rows (with one accumulator and 512 rows the gradients of
-// a training step lay further from fp64 than with fp32 sums: 3.6e-6 against 3.1e-6).  The blocks' partial results are added by a second
-// kernel in an order fixed by their number: deterministic.
+// hi / lo tiles, both parts rounded to nearest.  Per 8 rows one MMA A_hi x [B_hi | B_lo] and one A_lo x B_hi, the latter on top of
+// the B_lo columns.
+// What it replaces are fp32 products, so its error has to stay below theirs.  The accumulate step of an MMA truncates towards zero: the
+// large A_hi B_hi sums have an accumulator of their own, and all are added to fp32 registers after every block of 32 rows.  Error
+// relative to fp64 (normal entries, 128 x 256, against the library's fp32 product): 200 rows 1.4e-7 (2.0e-7), 1849 rows 1.4e-7 (2.8e-7),
+// 65536 rows 1.8e-7 (7.7e-7); entries of one sign, 7396 rows 1.3e-7 (1.5e-7).  With sums of 128 rows and a truncated hi part it was 3.5e-7,
+// 3.7e-7, 3.9e-7 and 6.6e-7, above fp32 up to about 4000 rows; the shorter sums and the rounding cost 10 % of the time (7396 rows: 16.8 ->
+// 18.6 us; 65536 rows: 39 -> 45; library product and sum: 70 and 240).  Below 128 rows fp32 is closer (64 rows: 1.1e-7 against 1.3e-7).
+// Blocks split the rows; their partial results are added by a second kernel in an order fixed by their number: deterministic.
 //   warps 0-1 raw loaders (A, B), 2 MMA issuer, 4-11 transposers (A: 4-7, B: 8-11), 12-19 accumulation.
 // Every wait is a bounded mbarrier poll that records a code on expiry.
 #include "tc_common.cuh"
@@ -24,7 +26,6 @@ constexpr int TN_HALF = TN_T * 128, TN_STAGE = 4 * TN_HALF;              // A_hi
 constexpr int TN_OFF_RAW = TN_NS * TN_STAGE, TN_OFF_BAR = TN_OFF_RAW + TN_NR * 2 * TN_RAW;
 constexpr size_t TN_SMEM = TN_OFF_BAR + 256;
 static_assert(TN_SMEM <= 227 * 1024, "shared memory budget");
-constexpr int TN_CHAIN = 4;                                               // blocks of 32 rows per accumulator chain
 
 struct TnParams {
     const float *a, *b;
@@ -52,7 +53,6 @@ __global__ void __launch_bounds__(TN_THREADS, 1) tn_gemm_kernel(const TnParams p
     const int tile = blockIdx.y, m0 = tile / p.nt * TN_T, n0 = tile % p.nt * TN_T;
     const int blocks = (p.rows + TN_ROWS - 1) / TN_ROWS;
     const int k_begin = (int)((int64_t)blockIdx.x * blocks / gridDim.x), n_my = (int)((int64_t)(blockIdx.x + 1) * blocks / gridDim.x) - k_begin;
-    const int chains = (n_my + TN_CHAIN - 1) / TN_CHAIN;
     if (tid == 0) {
         for (int s = 0; s < TN_NR; ++s) { mbar_init(raw_full(s), 64); mbar_init(raw_empty(s), 256); }
         for (int s = 0; s < 2; ++s) { mbar_init(st_full(s), 256); mbar_init(st_empty(s), 1); mbar_init(acc_full(s), 1); mbar_init(acc_empty(s), 256); }
@@ -93,25 +93,21 @@ __global__ void __launch_bounds__(TN_THREADS, 1) tn_gemm_kernel(const TnParams p
         if (tc_elect()) {
             constexpr uint32_t idesc2 = tc_idesc(2 * TN_T), idesc1 = tc_idesc(TN_T);
             uint32_t s = 0, ph = 0;
-            bool alive = true;
-            for (int c = 0; c < chains && alive; ++c) {
-                const uint32_t buf = (uint32_t)(c & 1), d = tmem_base + buf * 256;
-                if (!mbar_wait(acc_empty(buf), (uint32_t)((c >> 1) & 1) ^ 1u, abort_flag, 92, &g_tn_status)) break;
-                const int len = n_my - c * TN_CHAIN < TN_CHAIN ? n_my - c * TN_CHAIN : TN_CHAIN;
-                for (int k = 0; k < len; ++k) {
-                    if (!mbar_wait(st_full(s), ph, abort_flag, 93, &g_tn_status)) { alive = false; break; }
-                    tc_fence_after();
-                    const uint32_t st = smem_base + s * TN_STAGE;
-                    const uint64_t ah = tc_smem_desc(st), al = tc_smem_desc(st + TN_HALF), b = tc_smem_desc(st + 2 * TN_HALF);
+            for (int k = 0; k < n_my; ++k) {
+                const uint32_t buf = (uint32_t)(k & 1), d = tmem_base + buf * 256;
+                if (!mbar_wait(acc_empty(buf), (uint32_t)((k >> 1) & 1) ^ 1u, abort_flag, 92, &g_tn_status)) break;
+                if (!mbar_wait(st_full(s), ph, abort_flag, 93, &g_tn_status)) break;
+                tc_fence_after();
+                const uint32_t st = smem_base + s * TN_STAGE;
+                const uint64_t ah = tc_smem_desc(st), al = tc_smem_desc(st + TN_HALF), b = tc_smem_desc(st + 2 * TN_HALF);
 #pragma unroll
-                    for (int k8 = 0; k8 < 4; ++k8) {
-                        tc_mma_tf32_ss(d, ah + k8 * 2, b + k8 * 2, idesc2, (k > 0 || k8 > 0) ? 1u : 0u);
-                        tc_mma_tf32_ss(d + TN_T, al + k8 * 2, b + k8 * 2, idesc1, 1u);
-                    }
-                    tc_commit(st_empty(s));
-                    if (++s == TN_NS) { s = 0; ph ^= 1u; }
+                for (int k8 = 0; k8 < 4; ++k8) {
+                    tc_mma_tf32_ss(d, ah + k8 * 2, b + k8 * 2, idesc2, k8 > 0 ? 1u : 0u);
+                    tc_mma_tf32_ss(d + TN_T, al + k8 * 2, b + k8 * 2, idesc1, 1u);
                 }
-                if (alive) tc_commit(acc_full(buf));
+                tc_commit(st_empty(s));
+                tc_commit(acc_full(buf));
+                if (++s == TN_NS) { s = 0; ph ^= 1u; }
             }
         }
         __syncwarp();
@@ -140,13 +136,14 @@ __global__ void __launch_bounds__(TN_THREADS, 1) tn_gemm_kernel(const TnParams p
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const float e[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+                uint32_t h[4];
                 float l[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) l[i] = e[i] - __uint_as_float(__float_as_uint(e[i]) & 0xffffe000u);
+                for (int i = 0; i < 4; ++i) { h[i] = tf32_rna_cvt(e[i]); l[i] = e[i] - __uint_as_float(h[i]); }
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int c = 4 * j + i;
-                    *reinterpret_cast<float*>(dst + (c >> 3) * 1024 + coff[c & 7]) = e[i];
+                    *reinterpret_cast<uint32_t*>(dst + (c >> 3) * 1024 + coff[c & 7]) = h[i];
                     *reinterpret_cast<uint32_t*>(dst + TN_HALF + (c >> 3) * 1024 + coff[c & 7]) = __float_as_uint(l[i]) + 0x1000u;
                     sums[c] += e[i];
                 }
@@ -176,9 +173,9 @@ __global__ void __launch_bounds__(TN_THREADS, 1) tn_gemm_kernel(const TnParams p
 #pragma unroll
         for (int j = 0; j < 64; ++j) acc[j] = 0.0f;
         bool alive = true;
-        for (int c = 0; c < chains; ++c) {
-            const uint32_t buf = (uint32_t)(c & 1);
-            if (!mbar_wait(acc_full(buf), (uint32_t)((c >> 1) & 1), abort_flag, 96, &g_tn_status)) { alive = false; break; }
+        for (int k = 0; k < n_my; ++k) {
+            const uint32_t buf = (uint32_t)(k & 1);
+            if (!mbar_wait(acc_full(buf), (uint32_t)((k >> 1) & 1), abort_flag, 96, &g_tn_status)) { alive = false; break; }
             tc_fence_after();
 #pragma unroll
             for (int j = 0; j < 64; j += 16) {

@@ -658,13 +658,19 @@ def encoder_train_backward(x: Tensor, att: Tensor, x1: Tensor, h: Tensor, eps: f
         dx, dwqkv = torch.empty_like(x), torch.empty(3, 128, 128, device=x.device, dtype=x.dtype)
         workspace = torch.empty(need, device=x.device, dtype=torch.uint8)
         wq, wk, wv = dwqkv.unbind(0)
-        grads = [torch.empty_like(p) for p in params[5:]]               # (the first five: wq, bq, wk, bk, wv)
-        bq, bk = torch.empty_like(params[1]), torch.empty_like(params[3])
-        out = (ctypes.c_void_p * 14)(*[t.data_ptr() for t in (dwqkv, bq, bk, *grads)])
+        bq, bk, *grads = (torch.empty_like(p) for p in (params[1], params[3], *params[5:10]))      # (dwqkv: wq, wk, wv)
+        # the dense layers' weight and bias gradients: below 128 rows plain fp32 products are the closer ones (tc_tn.cu)
+        few = rows < 128
+        if few:
+            pairs = [(dy.view(rows, -1), v.view(rows, -1)) for dy, v in ((dx1, att), (dh, x1), (grad_out, h))]
+            dense = [t for dy, v in pairs for t in (torch.mm(dy.t(), v), dy.sum(0))]
+        else:
+            dense = [torch.empty_like(p) for p in params[10:]]
+        out = (ctypes.c_void_p * 14)(*[t.data_ptr() for t in (dwqkv, bq, bk, *grads)], *([None] * 6 if few else [t.data_ptr() for t in dense]))
         ptrs = (ctypes.c_void_p * _ENCODER_PARAMS)(*[p.data_ptr() for p in params])
         _call('spgt_encoder_train_bwd', ptrs, out, x.data_ptr(), att.data_ptr(), x1.data_ptr(), h.data_ptr(), grad_out.data_ptr(), dh.data_ptr(),
-              dx1.data_ptr(), da.data_ptr(), dx.data_ptr(), B, S, float(eps), saved.data_ptr(), kept, workspace.data_ptr(), need, _stream(), kernels=17)
-    return dx, [wq, bq, wk, bk, wv, *grads]
+              dx1.data_ptr(), da.data_ptr(), dx.data_ptr(), B, S, float(eps), saved.data_ptr(), kept, workspace.data_ptr(), need, _stream(), kernels=11 if few else 17)
+    return dx, [wq, bq, wk, bk, wv, *grads, *dense]
 
 
 # ---------------------------------------------------------------------------------------------------------

@@ -64,8 +64,8 @@ def test_conv3x3_shared_memory_operands(B, Hh, Ww, Cin, Cout, act):
     assert torch.isnan(y[..., :4]).all() and torch.isnan(y[..., 4 + Cout:]).all()
 
 
-# rows: one, around a 32-row block, around the 512-row accumulator chain, many blocks; widths: tails of the 128-wide tiles
-@pytest.mark.parametrize('rows,M,N', [(1, 4, 4), (31, 128, 128), (33, 132, 36), (513, 128, 256), (1000, 256, 128), (7396, 136, 128), (65536, 128, 128), (79524, 32, 128)])
+# rows: one, around a 32-row block, around the 256 rows from which two blocks share them, many blocks; widths: tails of the 128-wide tiles
+@pytest.mark.parametrize('rows,M,N', [(1, 4, 4), (31, 128, 128), (33, 132, 36), (257, 128, 256), (1000, 256, 128), (7396, 136, 128), (65536, 128, 128), (79524, 32, 128)])
 def test_weight_gradient_gemm(rows, M, N):
     from spgt_b200 import ops
     g = torch.Generator().manual_seed(rows)
@@ -77,6 +77,20 @@ def test_weight_gradient_gemm(rows, M, N):
     assert rel_l2(s, b.double().sum(0)) < TOL
     c2, s2 = ops.tn_gemm(a.cuda(), b.cuda(), column_sums=True)
     assert torch.equal(c, c2) and torch.equal(s, s2)
+
+
+# the kernel stands in for fp32 products from 128 rows on: no further from fp64 than they are (a tenth more for the scatter of one draw),
+# for entries of both signs and for entries of one, where truncated sums would drift
+@pytest.mark.parametrize('one_sign', [False, True])
+@pytest.mark.parametrize('rows,M,N', [(128, 128, 256), (200, 256, 128), (1849, 128, 136), (7396, 128, 256), (65536, 256, 128)])
+def test_weight_gradient_gemm_is_as_close_as_fp32(rows, M, N, one_sign):
+    from spgt_b200 import ops
+    torch.backends.cuda.matmul.allow_tf32 = False
+    g = torch.Generator().manual_seed(rows)
+    draw = torch.rand if one_sign else torch.randn
+    a, b = draw(rows, M, generator=g).cuda(), draw(rows, N, generator=g).cuda()
+    want = a.double().t() @ b.double()
+    assert rel_l2(ops.tn_gemm(a, b)[0], want) <= 1.1 * rel_l2(a.t() @ b, want)
 
 
 def _model():
