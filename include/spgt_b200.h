@@ -98,7 +98,7 @@ int spgt_galerkin_attn_bwd(const float* Q, const float* K, const float* V, const
  * pre-LayerNorm projection h = x W + b [B*S, H*32] it writes dh [B*S, H*32] (gradient with respect to h) and the parameter
  * gradients db, dlnw, dlnb [H*32] (dlnw, dlnb only with ln_weight != NULL; without LayerNorm dh is the gathered gradient
  * and h may be NULL).  The caller finishes with two GEMMs, dX = dh W^T and dW = x^T dh (spgt_linear_tc_fwd and
- * spgt_batched_transpose + spgt_batched_skinny_gemm).  Replaces the element-wise stages of
+ * spgt_tn_gemm).  Replaces the element-wise stages of
  * multihead_projection[_layernorm]_with_position_rrc_backward (extension/bind/galerkin_attention.cu:26-48, 70-102).
  * Partial sums are added in block order (deterministic).  d_head must be 32, H <= 8. */
 size_t spgt_projpos_bwd_workspace_bytes(int B, int S, int H);

@@ -17,8 +17,8 @@ namespace spgt {
 
 constexpr int PB_ROWS = 32;      // grid nodes per warp and iteration
 
-// Rows of h and dh have pitches ldh and ldd.
-template <bool LN>
+// Rows of h and dh have pitches ldh and ldd.  VEC: they start at 16-byte boundaries.
+template <bool LN, bool VEC = true>
 __device__ __forceinline__ void proj_bwd_body(const float* __restrict__ grad_out, const float* __restrict__ h, int ldh, const float* __restrict__ lnw,
                                               float* __restrict__ dh, int ldd, float* __restrict__ partial, int S, int H, int d_pos, float eps,
                                               int tiles_per_sample, int tiles) {
@@ -38,10 +38,10 @@ __device__ __forceinline__ void proj_bwd_body(const float* __restrict__ grad_out
         for (int c = 0; c < 32; ++c) g[c] = __ldg(gp + (int64_t)c * S);              // lanes = consecutive nodes
         if constexpr (LN) {
             float v[32], mu = 0.0f, var = 0.0f, m1 = 0.0f, m2 = 0.0f;
-            const float4* hp = reinterpret_cast<const float4*>(h + row * ldh + head * 32);
+            const float* hp = h + row * ldh + head * 32;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const float4 q = __ldg(hp + j);
+                const float4 q = VEC ? __ldg(reinterpret_cast<const float4*>(hp) + j) : make_float4(__ldg(hp + 4 * j), __ldg(hp + 4 * j + 1), __ldg(hp + 4 * j + 2), __ldg(hp + 4 * j + 3));
                 v[4 * j] = q.x; v[4 * j + 1] = q.y; v[4 * j + 2] = q.z; v[4 * j + 3] = q.w;
                 mu += (q.x + q.y) + (q.z + q.w);
             }
@@ -62,9 +62,14 @@ __device__ __forceinline__ void proj_bwd_body(const float* __restrict__ grad_out
 #pragma unroll
             for (int c = 0; c < 32; ++c) g[c] = inv * (g[c] - m1 - v[c] * m2);
         }
-        float4* dp = reinterpret_cast<float4*>(dh + row * ldd + head * 32);
+        float* dp = dh + row * ldd + head * 32;
+        if constexpr (VEC) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) dp[j] = make_float4(g[4 * j], g[4 * j + 1], g[4 * j + 2], g[4 * j + 3]);
+            for (int j = 0; j < 8; ++j) reinterpret_cast<float4*>(dp)[j] = make_float4(g[4 * j], g[4 * j + 1], g[4 * j + 2], g[4 * j + 3]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 32; ++c) dp[c] = g[c];
+        }
 #pragma unroll
         for (int c = 0; c < 32; ++c) db[c] += g[c];
     }
@@ -85,11 +90,11 @@ __device__ __forceinline__ void proj_bwd_body(const float* __restrict__ grad_out
     if (LN) { columns(dw, 1); columns(dbt, 2); }
 }
 
-template <bool LN>
+template <bool LN, bool VEC>
 __global__ void __launch_bounds__(256)
 proj_bwd_kernel(const float* __restrict__ grad_out, const float* __restrict__ h, const float* __restrict__ lnw,
                 float* __restrict__ dh, float* __restrict__ partial, int S, int H, int d_pos, float eps, int tiles_per_sample, int tiles) {
-    proj_bwd_body<LN>(grad_out, h, H * 32, lnw, dh, H * 32, partial, S, H, d_pos, eps, tiles_per_sample, tiles);
+    proj_bwd_body<LN, VEC>(grad_out, h, H * 32, lnw, dh, H * 32, partial, S, H, d_pos, eps, tiles_per_sample, tiles);
 }
 
 // Q, K and V of a layer in one launch (blockIdx.y): dh [rows, 384] = dq | dk | dv, h [rows, 256] = K | V before their LayerNorm
@@ -171,10 +176,10 @@ extern "C" int spgt_projpos_bwd_elementwise(const float* grad_out, const float* 
     const int tps = ceil_div(S, PB_ROWS);
     if ((int64_t)B * tps > 0x7fffffffLL) return SPGT_ERR_SHAPE;
     if (!workspace || workspace_bytes < spgt_projpos_bwd_workspace_bytes(B, S, H)) return SPGT_ERR_WORKSPACE;
-    if ((h && !aligned16(h)) || !aligned16(dh)) return SPGT_ERR_ALIGN;
     cudaStream_t st = (cudaStream_t)stream;
     const int D = H * 32, blocks = proj_bwd_blocks(B, S, H);
-    auto kern = ln_weight ? proj_bwd_kernel<true> : proj_bwd_kernel<false>;
+    const bool vec = (!h || aligned16(h)) && aligned16(dh);
+    auto kern = ln_weight ? (vec ? proj_bwd_kernel<true, true> : proj_bwd_kernel<true, false>) : (vec ? proj_bwd_kernel<false, true> : proj_bwd_kernel<false, false>);
     kern<<<(unsigned)blocks, H * 32, (size_t)H * 32 * 33 * sizeof(float), st>>>(grad_out, h, ln_weight, dh, (float*)workspace, S, H, d_pos, eps, tps,
                                                                              B * tps);
     if (int e = launch_status()) return e;

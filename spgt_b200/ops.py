@@ -494,6 +494,7 @@ def ffn_tc(x: Tensor, w1: TcWeight, b1: Tensor, w2: TcWeight, b2: Optional[Tenso
 def tn_gemm(a: Tensor, b: Tensor, column_sums: bool = False):
     """(a^T b, column sums of b or None) for a [rows, M], b [rows, N]: weight and bias gradient of a linear layer."""
     _chk(a, 'a'); _chk(b, 'b')
+    a, b = (t if t.data_ptr() % 16 == 0 else t.clone() for t in (a, b))       # (rows are copied 16 bytes at a time)
     rows, M, N = a.shape[0], a.shape[1], b.shape[1]
     if b.shape[0] != rows or M % 4 or N % 4:
         raise ValueError('a and b must be [rows, M] and [rows, N] with M and N multiples of 4')

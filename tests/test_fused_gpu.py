@@ -79,6 +79,31 @@ def test_weight_gradient_gemm(rows, M, N):
     assert torch.equal(c, c2) and torch.equal(s, s2)
 
 
+@pytest.mark.parametrize('norm', [False, True])
+def test_projection_backward_takes_any_alignment(norm):
+    """x, and h and dh of the element-wise entry point, may start at any float."""
+    from spgt_b200 import ops
+    from spgt_b200._lib import lib
+    g = torch.Generator().manual_seed(9)
+    shifted = lambda t: torch.empty(t.numel() + 1, device='cuda')[1:].view(t.shape).copy_(t)
+    B, S = 2, 70
+    x, w, b, dy = torch.randn(B, S, 128, generator=g).cuda(), torch.randn(128, 128, generator=g).cuda(), torch.randn(128, generator=g).cuda(), torch.randn(B, 4, 34, S, generator=g).cuda()
+    if not norm:
+        want = ops.projpos_backward(x, w, b, None, dy, 0.0, 4, 32, 2)
+        got = ops.projpos_backward(shifted(x), w, b, None, dy, 0.0, 4, 32, 2)
+        assert all(torch.equal(p, q) for p, q in zip(want[:3], got[:3]))
+    h, lnw = torch.randn(B * S, 128, generator=g).cuda(), torch.randn(4, 32, generator=g).cuda() if norm else None
+    need = int(lib.spgt_projpos_bwd_workspace_bytes(B, S, 4))
+    runs = []
+    for place in (torch.clone, shifted):
+        hh, dh, sums, ws = place(h), place(torch.zeros_like(h)), torch.zeros(3, 128, device='cuda'), torch.empty(need, dtype=torch.uint8, device='cuda')
+        code = lib.spgt_projpos_bwd_elementwise(dy.data_ptr(), hh.data_ptr() if norm else None, lnw.data_ptr() if norm else None, 1e-6, dh.data_ptr(), *(s.data_ptr() for s in sums),
+                                                B, S, 4, 32, 2, ws.data_ptr(), need, torch.cuda.current_stream().cuda_stream)
+        assert code == 0
+        runs.append((dh, sums))
+    assert all(torch.equal(p, q) for p, q in zip(*runs))
+
+
 # the kernel stands in for fp32 products from 128 rows on: no further from fp64 than they are (a tenth more for the scatter of one draw),
 # for entries of both signs and for entries of one, where truncated sums would drift
 @pytest.mark.parametrize('one_sign', [False, True])
