@@ -266,8 +266,9 @@ int conv_status(bool reset) {
     return cudaMemcpyFromSymbol(&v, g_conv_status, sizeof(int)) == cudaSuccess ? v : SPGT_ERR_LAUNCH;
 }
 
-// Output channels per block: the two widths of the model's convolutions.  (33 - 48: down-scaler, 42 and 44; else up-scaler.)
-static int conv_bn(int cout) { return cout <= 48 ? 48 : 128; }
+// Output channels per block: the narrowest width that holds them all, because an MMA's time falls with its width.  16 x 106 x 106,
+// 128 -> 52 channels: 124 us with 64, 182 with 128, 157 for the implicit GEMM's 64-wide tile; 64 -> 64: 68, 96 and 90.
+static int conv_bn(int cout) { return cout <= 48 ? 48 : cout <= 64 ? 64 : 128; }
 
 template <int BN> static int conv_launch(const ConvParams& p, cudaStream_t st) {
     static SmemOptIn configured;
@@ -307,5 +308,9 @@ extern "C" int spgt_conv3x3_nhwc_fwd(const float* x, int cin_pitch, int cin_off,
     if (rows * (Ww + CV_TX) > 0x7fffffffLL / 2) return SPGT_ERR_SHAPE;
     if (!aligned16(x) || !aligned16(wprep) || !aligned16(y)) return SPGT_ERR_ALIGN;
     const ConvParams p{x + cin_off, (const float*)wprep, bias, y + cout_off, cin_pitch, Cin, cout_pitch, Cout, B, Hh, Ww, act, ceil_div(Ww, CV_TX), (int)tiles};
-    return conv_bn(Cout) == 48 ? conv_launch<48>(p, (cudaStream_t)stream) : conv_launch<128>(p, (cudaStream_t)stream);
+    switch (conv_bn(Cout)) {
+        case 48: return conv_launch<48>(p, (cudaStream_t)stream);
+        case 64: return conv_launch<64>(p, (cudaStream_t)stream);
+        default: return conv_launch<128>(p, (cudaStream_t)stream);
+    }
 }

@@ -47,7 +47,7 @@ def test_encoder_layer_edges(B, S):
 
 
 @pytest.mark.parametrize('B,Hh,Ww,Cin,Cout,act', [(1, 1, 1, 4, 4, None), (2, 9, 11, 128, 44, 'relu'), (1, 16, 8, 44, 44, 'silu'), (3, 17, 9, 36, 48, 'relu'),
-                                                   (2, 15, 31, 12, 20, None), (1, 20, 17, 128, 128, 'silu2'), (2, 5, 106, 64, 52, 'silu'),
+                                                   (2, 15, 31, 12, 20, None), (3, 17, 9, 36, 64, 'relu'), (20, 77, 77, 44, 56, 'relu'), (1, 20, 17, 128, 128, 'silu2'), (2, 5, 106, 64, 52, 'silu'),
                                                    (4, 106, 106, 128, 128, 'silu2'), (20, 77, 77, 128, 44, 'relu')])
 def test_conv3x3_shared_memory_operands(B, Hh, Ww, Cin, Cout, act):
     from spgt_b200 import ops
