@@ -325,7 +325,8 @@ static int spectral_chunk(int r) {
 
 using namespace spgt;
 
-static bool spectral_shape_ok(int r, int m) { return r >= 2 && m >= 1 && m <= 16 && 2 * m <= r && r <= 4096; }
+// 2 * 2m * r * 4 bytes at most 200 KB: the grids that a whole transform table of fits into shared memory, beyond which nothing is tested
+static bool spectral_shape_ok(int r, int m) { return r >= 2 && m >= 1 && m <= 16 && 2 * m <= r && r <= 4096 && 4 * m * r <= 50 * 1024; }
 
 extern "C" size_t spgt_spectral_tables_bytes(int r, int m) {
     if (!spectral_shape_ok(r, m)) return 0;
@@ -389,7 +390,6 @@ extern "C" int spgt_spectral_conv2d_fwd(const float* x, const float* wr, const f
     const int64_t zn = (int64_t)CH * J * m * C;
     float* Z = P + (size_t)CH * r * J * C;
     float *Or = Z + 2 * zn, *Oi = Or + zn, *wr_img = Oi + zn;
-    if ((size_t)2 * J * r * sizeof(float) > 200 * 1024) return SPGT_ERR_SHAPE;      // (the largest grids the layer takes)
     static SmemOptIn cfg_a, cfg_c;
     int e;
     const ChainScope chain;
