@@ -35,17 +35,24 @@ class ParameterWatch:
 
     def _seen(self, module: torch.nn.Module) -> tuple:
         tree = self._tree
-        if tree is None or any(len(d) != n for d, n in tree[0]) or any(d.get(k, 0) is not c for d, k, c in tree[1]):
-            tree = self._tree = self._walk(module)
+        try:
+            if tree is not None and not any(len(d) != n for d, n in tree[0]) and not any(d[k] is not c for d, k, c in tree[1]):
+                return tree
+        except KeyError:                                  # a submodule under another name: as many entries as before
+            pass
+        tree = self._tree = self._walk(module)
         return tree
 
     def tag(self, module: torch.nn.Module) -> tuple:
         tree = self._seen(module)
-        if not all(k in d for d, k in tree[2]):           # renamed (pruning, spectral normalisation): as many entries as before
+        try:
+            params = [d[k] for d, k in tree[2]]
+            values = [p._version for p in params] + [p.data_ptr() for p in params]
+        except (KeyError, AttributeError):                # renamed (pruning, spectral normalisation), or None in place of a bias
             tree = self._tree = self._walk(module)
-        params = [d[k] for d, k in tree[2]]               # (None where a bias has been taken out)
-        return tuple([-1 if p is None else p._version for p in params] + [0 if p is None else p.data_ptr() for p in params] + [d.get(k) for d, k in tree[3]]
-                     + [module.__dict__.get(k) for k in self.OPTIONS])
+            params = [d[k] for d, k in tree[2]]
+            values = [(0, 0) if p is None else (p._version, p.data_ptr()) for p in params]
+        return tuple(values + [d.get(k) for d, k in tree[3]] + [module.__dict__.get(k) for k in self.OPTIONS])
 
     def observed(self, module: torch.nn.Module) -> bool:
         """Whether a submodule's call can be told from a call of its kernels: forward hooks, or a forward of its own."""
