@@ -283,6 +283,9 @@ int spgt_conv3x3_tc_fwd(const float* x, int cin_pitch, int cin_off, int Cin, con
  * split once per tile instead of once per tap.  w_kn [9 * Cin][ldw], row (ky * 3 + kx) * Cin + c.  bias NULL or [Cout]. */
 size_t spgt_conv3x3_weight_bytes(int Cin, int Cout);
 int spgt_conv3x3_weight_prepare(const float* w_kn, int ldw, int Cin, int Cout, void* out, size_t out_bytes, spgt_stream_t stream);
+/* The same preparation from torch's layout [cout][cin][3][3], zero padded to Cin and Cout channels, and bias [cout] padded to bias_out [Cout]. */
+int spgt_conv3x3_weight_prepare_oihw(const float* w, const float* bias, int cin, int cout, int Cin, int Cout, void* out, size_t out_bytes,
+                                     float* bias_out, spgt_stream_t stream);
 int spgt_conv3x3_nhwc_fwd(const float* x, int cin_pitch, int cin_off, int Cin, const void* wprep, const float* bias, float* y, int cout_pitch,
                           int cout_off, int Cout, int B, int Hh, int Ww, int act, spgt_stream_t stream);
 
@@ -339,6 +342,11 @@ typedef struct {
     const void* w2; const float* b2; /* prepared [256, 128], [128] or NULL */
 } spgt_encoder_weights;
 
+/* The prepared images wkv, w1, w2 of a layer, one after the other (a third of the bytes each), in one launch from the weights as the
+ * modules keep them: wk, wv [128 in][128 out], w1 [256 out][128 in], w2 [128 out][256 in]; w1 and w2 NULL: wkv alone (ffn = 0). */
+size_t spgt_encoder_weights_bytes(int ffn);
+int spgt_encoder_weights_prepare(const float* wk, const float* wv, const float* w1, const float* w2, void* images, size_t bytes,
+                                 spgt_stream_t stream);
 /* Bytes of scratch a layer of B samples of S grid nodes needs (0: unsupported sizes). */
 size_t spgt_encoder_workspace_bytes(int B, int S);
 /* y = a + (ffn ? act(a w1 + b1) w2 + b2 : 0)  with  a = (residual || ffn ? x : 0) + attention(x, pos) wfc + bfc.
@@ -397,6 +405,9 @@ int spgt_darcy_launches(const spgt_darcy_model* model, int B);
  * the up-scaler output before its last interpolation [B,mid,mid,128].  Every launch goes to `stream`; nothing synchronises. */
 int spgt_darcy_forward(const spgt_darcy_model* model, const float* node, const float* position, const float* grid, float* out,
                        int B, float* const* taps, void* workspace, size_t workspace_bytes, spgt_stream_t stream);
+/* The same with the head's second bias read from device memory (head_b2 [1], NULL: model->b2): no copy to the host for a new model. */
+int spgt_darcy_forward_devbias(const spgt_darcy_model* model, const float* head_b2, const float* node, const float* position, const float* grid,
+                               float* out, int B, float* const* taps, void* workspace, size_t workspace_bytes, spgt_stream_t stream);
 
 #ifdef __cplusplus
 }

@@ -88,6 +88,7 @@ SIGNATURES = {
     'spgt_tc_weight_prepare_t': (_i, [_f, _i, _i, _i, _f, _sz, _st]),
     'spgt_conv3x3_weight_bytes': (_sz, [_i, _i]),
     'spgt_conv3x3_weight_prepare': (_i, [_f, _i, _i, _i, _f, _sz, _st]),
+    'spgt_conv3x3_weight_prepare_oihw': (_i, [_f, _f, _i, _i, _i, _i, _f, _sz, _f, _st]),
     'spgt_conv3x3_nhwc_fwd': (_i, [_f, _i, _i, _i, _f, _f, _f, _i, _i, _i, _i, _i, _i, _i, _st]),
     'spgt_projpos_qkv_tc_fwd': (_i, [_f] * 9 + [_fl] + [_f] * 4 + [_i] * 6 + [_st]),
     'spgt_decoder_head_tc_fwd': (_i, [_f, _f, _f, _f, _fl, _fl, _fl, _f, _f, _i, _f, _i, _i, _i, _i, _i, _i, _st]),
@@ -96,6 +97,8 @@ SIGNATURES = {
     'spgt_spectral_workspace_bytes': (_sz, [_i, _i, _i, _i]),
     'spgt_spectral_chunk_samples': (_i, [_i]),
     'spgt_spectral_launches': (_i, [_i, _i, _i]),
+    'spgt_encoder_weights_bytes': (_sz, [_i]),
+    'spgt_encoder_weights_prepare': (_i, [_f] * 5 + [_sz, _st]),
     'spgt_encoder_workspace_bytes': (_sz, [_i, _i]),
     'spgt_encoder_layer_fwd': (_i, [_f] * 4 + [_i, _i, _fl, _i, _i, _i, _f, _sz, _st]),
     'spgt_encoder_train_saved_bytes': (_sz, [_i, _i]),
@@ -105,6 +108,7 @@ SIGNATURES = {
     'spgt_darcy_workspace_bytes': (_sz, [_f, _i]),
     'spgt_darcy_launches': (_i, [_f, _i]),
     'spgt_darcy_forward': (_i, [_f] * 5 + [_i, _f, _f, _sz, _st]),
+    'spgt_darcy_forward_devbias': (_i, [_f] * 6 + [_i, _f, _f, _sz, _st]),
     'spgt_spectral_conv2d_fwd': (_i, [_f, _f, _f, _f, _f, _f, _f, _sz, _f, _i, _i, _i, _i, _i, _st]),
 }
 

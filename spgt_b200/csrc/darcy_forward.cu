@@ -5,6 +5,10 @@
 
 namespace spgt {
 
+int decoder_head_tc(const float* x, const void* w1prep, const float* b1, const float* w2, float b2, const float* b2_dev, float scale, float shift,
+                    const float* scale_map, const float* shift_map, int dirichlet, float* out, int B, int Hh, int Ww, int K, int N1, int act,
+                    cudaStream_t st);      // tc_gemm.cu
+
 static int pad4(int c) { return (c + 3) & ~3; }
 
 // Workspace: the encoder's activations, which outlive the phases, then one region that the phases (down-scaler, encoder layer,
@@ -65,6 +69,12 @@ extern "C" int spgt_darcy_launches(const spgt_darcy_model* m, int B) {
 
 extern "C" int spgt_darcy_forward(const spgt_darcy_model* m, const float* node, const float* position, const float* grid, float* out,
                                   int B, float* const* taps, void* workspace, size_t workspace_bytes, spgt_stream_t stream) {
+    return spgt_darcy_forward_devbias(m, nullptr, node, position, grid, out, B, taps, workspace, workspace_bytes, stream);
+}
+
+extern "C" int spgt_darcy_forward_devbias(const spgt_darcy_model* m, const float* head_b2, const float* node, const float* position,
+                                          const float* grid, float* out, int B, float* const* taps, void* workspace, size_t workspace_bytes,
+                                          spgt_stream_t stream) {
     if (!m || !node || !position || !grid || !out || !workspace) return SPGT_ERR_NULL;
     DarcyPlan p;
     if (!darcy_plan(m, B, p)) return SPGT_ERR_SHAPE;
@@ -110,8 +120,8 @@ extern "C" int spgt_darcy_forward(const spgt_darcy_model* m, const float* node, 
         SPGT_TRY(spgt_spectral_conv2d_fwd(ws + p.y[l & 1], w.wr, w.br, w.fw0, w.fw1, m->tables, ws + p.ws, p.ws_bytes, ws + p.y[(l + 1) & 1], B, r,
                                           32, m->modes, m->act_dec, stream));
     }
-    SPGT_TRY(spgt_decoder_head_tc_fwd(ws + p.y[m->n_decoder & 1], m->head_w1, m->head_b1, m->head_w2, m->b2, m->scale, m->shift, m->scale_map,
-                                      m->shift_map, m->dirichlet, out, B, r, r, 32, 128, m->act_dec, stream));
+    SPGT_TRY(decoder_head_tc(ws + p.y[m->n_decoder & 1], m->head_w1, m->head_b1, m->head_w2, m->b2, head_b2, m->scale, m->shift, m->scale_map,
+                             m->shift_map, m->dirichlet, out, B, r, r, 32, 128, m->act_dec, (cudaStream_t)stream));
 #undef SPGT_TRY
     return SPGT_OK;
 }

@@ -9,11 +9,31 @@ int encoder_fold(const float* partial, const spgt_encoder_weights& w, float* m_i
 int encoder_out(const float* x, const float* m_img, const float* pc, const float* pos, const void* w1, const float* b1, const void* w2,
                 const float* b2, float* y, int B, int S, int act, bool ffn, bool residual, cudaStream_t st);
 
+int tc_weight_prepare_jobs(const TcPrepJobs& jobs, int n, cudaStream_t st);                          // tc_gemm.cu
+
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 }  // namespace spgt
 
 using namespace spgt;
+
+// Images of wkv, w1 and w2, one after the other: each 2 column tiles x 4 k-blocks (w2: 1 x 8) of 2 * 128 * 32 floats.
+constexpr size_t EN_IMAGE = (size_t)8 * 2 * 128 * 32 * sizeof(float);
+
+extern "C" size_t spgt_encoder_weights_bytes(int ffn) { return (ffn ? 3 : 1) * EN_IMAGE; }
+
+extern "C" int spgt_encoder_weights_prepare(const float* wk, const float* wv, const float* w1, const float* w2, void* images, size_t bytes,
+                                            spgt_stream_t stream) {
+    if (!wk || !wv || !images || (w1 != nullptr) != (w2 != nullptr)) return SPGT_ERR_NULL;
+    if (bytes < spgt_encoder_weights_bytes(w1 != nullptr)) return SPGT_ERR_WORKSPACE;
+    if (!aligned16(images)) return SPGT_ERR_ALIGN;
+    float* img = (float*)images;
+    TcPrepJobs jobs;
+    jobs.job[0] = {wk, img, 3, EN_D, EN_D, 2 * EN_D, EN_D, 128, wv};
+    jobs.job[1] = {w1, img + EN_IMAGE / sizeof(float), 1, EN_D, EN_D, 2 * EN_D, EN_D, 128, nullptr};
+    jobs.job[2] = {w2, img + 2 * (EN_IMAGE / sizeof(float)), 1, 2 * EN_D, 2 * EN_D, EN_D, 2 * EN_D, 128, nullptr};
+    return tc_weight_prepare_jobs(jobs, w1 ? 3 : 1, (cudaStream_t)stream);
+}
 
 extern "C" size_t spgt_encoder_workspace_bytes(int B, int S) {
     if (B <= 0 || S <= 0 || (int64_t)B * ceil_div(S, EN_ROWS) > 0x7fffffffLL / EN_ROWS) return 0;

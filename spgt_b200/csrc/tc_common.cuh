@@ -205,8 +205,9 @@ __device__ __forceinline__ void tc_img_store(float* stage, int bn, int n, int kk
     stage[off] = __uint_as_float(h);
     stage[bn * TC_BK + off] = __uint_as_float(tf32_rna_cvt(__uint_as_float(l)));
 }
-// Weight images to make in one launch.  kind 0: w [K][ldw], 1: w [N][ldw] (transposed), 2: copy N floats.
-struct TcPrepJob { const float* w; float* img; int kind, ldw, K, N, kpad, bn; };
+// Weight images to make in one launch.  kind 0: w [K][ldw], 1: w [N][ldw] (transposed), 2: copy N floats, 3: the K / V image of the
+// fused encoder layer from w = Wk and w2 = Wv [128][128]: by head pair K0 K1 V0 V1 | K2 K3 V2 V3, less the mean over each head's channels.
+struct TcPrepJob { const float* w; float* img; int kind, ldw, K, N, kpad, bn; const float* w2; };
 struct TcPrepJobs { TcPrepJob job[8]; };
 // Store 8 consecutive 32-bit columns of this thread's TMEM lane.
 __device__ __forceinline__ void tc_st8(uint32_t taddr, const uint32_t (&u)[8]) {

@@ -260,6 +260,17 @@ __global__ void conv_weight_prepare_kernel(const float* __restrict__ w, int ldw,
     tc_img_store(img + (int64_t)block * (2 * bn * CV_CH), bn, n, kk, v);
 }
 
+// The same from torch's layout [cout][cin][3][3], and the bias zero padded to bout channels.
+__global__ void conv_weight_prepare_oihw_kernel(const float* __restrict__ w, const float* __restrict__ bias, int cin, int cout, int bn,
+                                                float* __restrict__ img, int total, float* __restrict__ bpad, int bout) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < bout) bpad[i] = i < cout ? __ldg(bias + i) : 0.0f;
+    if (i >= total) return;
+    const int kk = i % CV_CH, n = (i / CV_CH) % bn, block = i / (CV_CH * bn), tap = block % 9, c = block / 9 * CV_CH + kk;
+    const float v = n < cout && c < cin ? __ldg(w + ((int64_t)n * cin + c) * 9 + tap) : 0.0f;
+    tc_img_store(img + (int64_t)block * (2 * bn * CV_CH), bn, n, kk, v);
+}
+
 int conv_status(bool reset) {
     int v = 0;
     if (reset) return cudaMemcpyToSymbol(g_conv_status, &v, sizeof(int)) == cudaSuccess ? SPGT_OK : SPGT_ERR_LAUNCH;
@@ -294,6 +305,18 @@ extern "C" int spgt_conv3x3_weight_prepare(const float* w_kn, int ldw, int Cin, 
     if (!aligned16(out)) return SPGT_ERR_ALIGN;
     const int bn = conv_bn(Cout), total = ceil_div(Cin, CV_CH) * 9 * bn * CV_CH;
     conv_weight_prepare_kernel<<<ceil_div(total, 256), 256, 0, (cudaStream_t)stream>>>(w_kn, ldw, Cin, Cout, bn, (float*)out, total);
+    return launch_status();
+}
+
+extern "C" int spgt_conv3x3_weight_prepare_oihw(const float* w, const float* bias, int cin, int cout, int Cin, int Cout, void* out, size_t out_bytes,
+                                                float* bias_out, spgt_stream_t stream) {
+    if (!w || !bias || !out || !bias_out) return SPGT_ERR_NULL;
+    const size_t need = spgt_conv3x3_weight_bytes(Cin, Cout);
+    if (need == 0 || cin <= 0 || cout <= 0 || cin > Cin || cout > Cout) return SPGT_ERR_SHAPE;
+    if (out_bytes < need) return SPGT_ERR_WORKSPACE;
+    if (!aligned16(out)) return SPGT_ERR_ALIGN;
+    const int bn = conv_bn(Cout), total = ceil_div(Cin, CV_CH) * 9 * bn * CV_CH;
+    conv_weight_prepare_oihw_kernel<<<ceil_div(total, 256), 256, 0, (cudaStream_t)stream>>>(w, bias, cin, cout, bn, (float*)out, total, bias_out, Cout);
     return launch_status();
 }
 

@@ -219,6 +219,7 @@ struct TcLinearEpi {
 struct TcHeadEpi {
     const float* b1; const float* w2; float b2, scale, shift; const float* scale_map; const float* shift_map;
     int dirichlet, Hh, Ww, act; float* out;
+    const float* b2_dev;         // b2 on the device, or NULL
 };
 struct TcSpecFwdEpi { float* y1; int J; int64_t nimg; };     // Y1 [image row][J][32 channels]
 enum { EPI_LINEAR = 0, EPI_PROJ = 1, EPI_HEAD = 2, EPI_SPECF = 3 };
@@ -698,11 +699,12 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
                 for (int pp = 0; pp < 8; ++pp)
                     posv[pp] = (pp < ep.d_pos && prow < rows) ? __ldg(ep.pos + (int64_t)prow * ep.d_pos + pp) : 0.0f;
             }
-            float head_sc = 0.0f, head_sh = 0.0f;   // HEAD: this row's de-normalisation and frame flag, prepared ahead in the same way
+            float head_sc = 0.0f, head_sh = 0.0f, head_b2 = 0.0f;   // HEAD: this row's de-normalisation and frame flag, prepared ahead in the same way
             bool head_edge = false;
             if constexpr (EPI == EPI_HEAD) {
                 const int prow = (unit_tile0(ui) + mt_e) * TC_BM + r_in_tile;
                 if (half == 0 && prow < rows) {
+                    head_b2 = ep.b2_dev ? __ldg(ep.b2_dev) : ep.b2;
                     const int prem = prow % (ep.Hh * ep.Ww);
                     head_sc = ep.scale_map ? __ldg(ep.scale_map + prem) : ep.scale;
                     head_sh = ep.shift_map ? __ldg(ep.shift_map + prem) : ep.shift;
@@ -921,7 +923,7 @@ tc_gemm_kernel(Loader ld, const float* __restrict__ wimg, int kpad, int rows, in
                 asm volatile("bar.sync %0, %1;" ::"r"(1 + egroup), "n"(32 * TC_EPI_WARPS) : "memory");   // the eight epilogue warps of this group
                 if (half == 0 && row < rows) {
                     acc += part[r_in_tile];
-                    e.out[row] = head_edge ? 0.0f : (acc + e.b2) * head_sc + head_sh;
+                    e.out[row] = head_edge ? 0.0f : (acc + head_b2) * head_sc + head_sh;
                 }
             }
             if constexpr (!(EPI == EPI_LINEAR && NBUF == 1 && (CPT <= 32 || CS))) {     // (else the LINEAR epilogue has freed the buffer already)
@@ -955,9 +957,22 @@ __global__ void tc_weight_prepare_kernel(const float* __restrict__ w, int ldw, i
     }
 }
 
-// The same for several weights in one launch (blockIdx.y); kind 2 copies N floats (a bias that has to lie next to another).
+// The same for several weights in one launch (blockIdx.y); kind 2 copies N floats (a bias that has to lie next to another), kind 3: a warp
+// per row and head of K or V, a lane per channel.
 __global__ void __launch_bounds__(256) tc_weight_prepare_jobs_kernel(const __grid_constant__ TcPrepJobs jobs) {
     const TcPrepJob& j = jobs.job[blockIdx.y];
+    if (j.kind == 3) {
+        const int lane = threadIdx.x & 31;
+        for (int u = blockIdx.x * 8 + (threadIdx.x >> 5); u < 128 * 8; u += gridDim.x * 8) {
+            const int k = u >> 3, head = (u >> 1) & 3, isv = u & 1, n = (head >> 1) * 128 + isv * 64 + (head & 1) * 32 + lane;
+            const float v = __ldg((isv ? j.w2 : j.w) + k * 128 + head * 32 + lane);
+            float m = v;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+            tc_img_store(j.img + ((n / 128) * 4 + k / TC_BK) * (2 * 128 * TC_BK), 128, n % 128, k % TC_BK, v - m * (1.0f / 32.0f));
+        }
+        return;
+    }
     const int npad = j.kind == 2 ? 0 : (j.N + j.bn - 1) / j.bn * j.bn, total = j.kind == 2 ? j.N : npad * j.kpad, KB = j.kpad / TC_BK;
     for (int i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
         if (j.kind == 2) { j.img[i] = __ldg(j.w + i); continue; }
@@ -1186,10 +1201,11 @@ extern "C" int spgt_projpos_qkv_tc_fwd(const float* x, const void* wprep_qkv, co
     return tc_launch<128, 1, TcDense, EPI_PROJ, TcProjEpi>(ld, (const float*)wprep_qkv, 128, (int)rows64, 3, ep, (cudaStream_t)stream);
 }
 
-extern "C" int spgt_decoder_head_tc_fwd(const float* x, const void* w1prep, const float* b1, const float* w2, float b2,
-                                        float scale, float shift, const float* scale_map, const float* shift_map,
-                                        int dirichlet, float* out, int B, int Hh, int Ww, int K, int N1, int act,
-                                        spgt_stream_t stream) {
+namespace spgt {
+// b2_dev: the second bias on the device, in the place of b2, or NULL
+int decoder_head_tc(const float* x, const void* w1prep, const float* b1, const float* w2, float b2, const float* b2_dev, float scale, float shift,
+                    const float* scale_map, const float* shift_map, int dirichlet, float* out, int B, int Hh, int Ww, int K, int N1, int act,
+                    cudaStream_t st) {
     if (!x || !w1prep || !b1 || !w2 || !out) return SPGT_ERR_NULL;
     if (B <= 0 || Hh <= 0 || Ww <= 0 || K <= 0 || (K & 3) || N1 != 128 || act < 0 || act > 3) return SPGT_ERR_SHAPE;
     const int64_t rows64 = (int64_t)B * Hh * Ww;
@@ -1197,7 +1213,15 @@ extern "C" int spgt_decoder_head_tc_fwd(const float* x, const void* w1prep, cons
     if (!aligned16(x) || !aligned16(w1prep)) return SPGT_ERR_ALIGN;
     TcDense ld;
     ld.x = x; ld.lda = K; ld.rows = (int)rows64; ld.K = K;
-    TcHeadEpi ep{b1, w2, b2, scale, shift, scale_map, shift_map, dirichlet, Hh, Ww, act, out};
+    TcHeadEpi ep{b1, w2, b2, scale, shift, scale_map, shift_map, dirichlet, Hh, Ww, act, out, b2_dev};
     const int kpad = ceil_div(K, TC_BK) * TC_BK;
-    return tc_launch<128, 1, TcDense, EPI_HEAD, TcHeadEpi>(ld, (const float*)w1prep, kpad, (int)rows64, 1, ep, (cudaStream_t)stream);
+    return tc_launch<128, 1, TcDense, EPI_HEAD, TcHeadEpi>(ld, (const float*)w1prep, kpad, (int)rows64, 1, ep, st);
+}
+}  // namespace spgt
+
+extern "C" int spgt_decoder_head_tc_fwd(const float* x, const void* w1prep, const float* b1, const float* w2, float b2,
+                                        float scale, float shift, const float* scale_map, const float* shift_map,
+                                        int dirichlet, float* out, int B, int Hh, int Ww, int K, int N1, int act,
+                                        spgt_stream_t stream) {
+    return decoder_head_tc(x, w1prep, b1, w2, b2, nullptr, scale, shift, scale_map, shift_map, dirichlet, out, B, Hh, Ww, K, N1, act, (cudaStream_t)stream);
 }

@@ -127,13 +127,14 @@ def _linear_tc(weight: Tensor) -> 'ops.TcWeight':
 def _conv_tc(weight: Tensor, bias: Tensor, cin_pad: int, cout_pad: int):
     """Conv2d weight [Cout, Cin, 3, 3] (+ bias) prepared for the tcgen05 implicit GEMM, with input / output channels
     zero-padded to cin_pad / cout_pad (padded outputs come out as act(0))."""
+    if cout_pad <= 128:
+        return ops.ConvWeight.padded(weight.detach().contiguous(), bias.detach().contiguous(), cin_pad, cout_pad)
     cout, cin = weight.shape[:2]
     w = torch.zeros(cout_pad, cin_pad, 3, 3, device=weight.device, dtype=weight.dtype)
     w[:cout, :cin] = weight.detach()
     b = torch.zeros(cout_pad, device=weight.device, dtype=weight.dtype)
     b[:cout] = bias.detach()
-    w = w.permute(2, 3, 1, 0).reshape(9 * cin_pad, cout_pad).contiguous()
-    return (ops.ConvWeight(w, cin_pad) if cout_pad <= 128 else ops.TcWeight(w)), b
+    return ops.TcWeight(w.permute(2, 3, 1, 0).reshape(9 * cin_pad, cout_pad).contiguous()), b
 
 
 class ConvResBlock2D(_KernelWeights):

@@ -58,21 +58,14 @@ class Sp_GalerkinAttention(_KernelWeights):
         """Whether the fused layer kernels cover these widths."""
         return self.dim_hidden == 128 and self.num_head == 4 and self.dim_head == 32 and self.dim_position == 2
 
-    def fill_native(self, w, ptr) -> None:
+    def fill_native(self, w, ptr, images=None) -> None:
         """Device pointers of this layer's weights into a spgt_encoder_weights; `ptr` keeps what it is given alive."""
-        w.wkv, w.wq = ptr(self.kv_weight()), ptr(_dense(self.weight_Q))
+        if images is None:
+            images = self._cached('images', lambda: ops.EncoderImages(_dense(self.weight_K), _dense(self.weight_V)))
+        w.wkv, w.wq = ptr(images), ptr(_dense(self.weight_Q))
         w.wfc, w.bfc = ptr(_dense(self.fc_layer.weight)), ptr(self.fc_layer.bias.detach())
         w.bq, w.bk, w.bv = (ptr(b.detach()) for b in (self.bias_Q, self.bias_K, self.bias_V))
         w.lnwk, w.lnbk, w.lnwv, w.lnbv = (ptr(t.detach()) for t in (self.ln_weight_K, self.ln_bias_K, self.ln_weight_V, self.ln_bias_V))
-
-    def kv_weight(self):
-        """K and V weights as the fused layer takes them: by head pair K0 K1 V0 V1 | K2 K3 V2 V3, less each head's channel mean (the
-        LayerNorm's subtraction, done once on the weights)."""
-        def make():
-            w = torch.stack([self.weight_K.detach(), self.weight_V.detach()], dim=1).view(-1, 2, self.num_head, self.dim_head)
-            w = (w - w.mean(dim=3, keepdim=True)).view(-1, 2, 2, 64)                  # [128, K | V, pair, 64]
-            return ops.TcWeight(w.transpose(1, 2).reshape(-1, 256))
-        return self._cached('wkv', make)
 
     def forward(self, Q: Tensor, K: Tensor, V: Tensor, position: Tensor, residual: Tensor = None) -> Tensor:
         """Q,K,V [N,S,D], position [N,S,d_pos] -> [N,S,D] (+ residual, fused into the output projection).
@@ -173,9 +166,10 @@ class Sp_EncoderLayer(_KernelWeights):
 
     def fill_native(self, w, ptr) -> None:
         a, f = self.attention_layer, self.ffn_layer
-        a.fill_native(w, ptr)
-        w1, w2 = f.tc_weights()
-        w.w1, w.b1, w.w2, w.b2 = ptr(w1), ptr(f.layer1.bias.detach()), ptr(w2), ptr(f.layer2.bias.detach())
+        images = self._cached('images', lambda: ops.EncoderImages(*(_dense(t) for t in (a.weight_K, a.weight_V, f.layer1.weight, f.layer2.weight))))
+        a.fill_native(w, ptr, images)
+        w.w1, w.w2 = images.data_ptr() + images.stride, images.data_ptr() + 2 * images.stride
+        w.b1, w.b2 = ptr(f.layer1.bias.detach()), ptr(f.layer2.bias.detach())
 
     def forward(self, X: Tensor, position: Tensor) -> Tensor:
         """X [N,S,D], position [N,S,d_pos] -> X + attention(X) then + ffn(.)  (network/sp_layer.py:94-104)."""

@@ -50,17 +50,17 @@ class Sp_DecoderRegressor(_KernelWeights):
         self.ffn_layer = FeedForward(dim_spatial_hidden, out_dim, dim_ffn_hidden, droprate, activation)
 
     def head_weights(self):
-        """(first weight as its kernel takes it, second weight [hidden], second bias) of the decoder head."""
+        """(first weight as its kernel takes it, second weight [hidden]) of the decoder head."""
         f = self.ffn_layer
         make = _linear_tc if f.layer1.out_features == 128 else _linear_kn
-        return (self._cached('w1', lambda: make(f.layer1.weight)), self._cached('w2', lambda: f.layer2.weight.detach().reshape(-1).contiguous()),
-                self._cached('b2', lambda: float(f.layer2.bias.detach().reshape(-1)[0])))
+        return self._cached('w1', lambda: make(f.layer1.weight)), self._cached('w2', lambda: f.layer2.weight.detach().reshape(-1).contiguous())
 
     def _spectral_and_head(self, X: Tensor, scale, shift, dirichlet, scale_map=None, shift_map=None) -> Tensor:
         for layer in self.layers:
             X = layer(X)
         f = self.ffn_layer
-        w1, w2, b2 = self.head_weights()
+        w1, w2 = self.head_weights()
+        b2 = self._cached('b2', lambda: float(f.layer2.bias.detach().reshape(-1)[0]))
         if f.layer1.out_features == 128:
             return ops.decoder_head_tc(X, w1, f.layer1.bias.detach(), w2, b2, scale, shift, dirichlet, self.activation,
                                        scale_map, shift_map)
@@ -239,9 +239,9 @@ class Sp_GalerkinTransformer2D(torch.nn.Module):
         for i, layer in enumerate(dec.layers):
             layer.fill_native(m.decoder[i], ptr)
         m.tables = ptr(ops.spectral_tables(r, m.modes, X.device).view(torch.float32)) if len(dec.layers) else None
-        w1, w2, m.b2 = dec.head_weights()
+        w1, w2 = dec.head_weights()
         m.head_w1, m.head_b1, m.head_w2 = ptr(w1), ptr(dec.ffn_layer.layer1.bias.detach()), ptr(w2)
-        return ops.DarcyPlan(m, keep)
+        return ops.DarcyPlan(m, keep, ptr(dec.ffn_layer.layer2.bias.detach()))
 
     def _native_widths(self) -> bool:
         """Whether the one-call forward covers this model: its own module types, the widths the kernels are made for, and one

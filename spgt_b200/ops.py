@@ -436,11 +436,25 @@ class ConvWeight:
         _chk(w_kn, 'weight')
         if w_kn.shape[0] != 9 * Cin:
             raise ValueError('weight must be [9 * Cin, Cout]')
-        self.K, self.N = w_kn.shape
-        n = int(lib.spgt_conv3x3_weight_bytes(Cin, self.N))
-        self.buf = torch.empty(n, dtype=torch.uint8, device=w_kn.device)
+        self._allocate(Cin, w_kn.shape[1], w_kn.device)
         with _device(w_kn.device):
-            _call('spgt_conv3x3_weight_prepare', w_kn.data_ptr(), w_kn.shape[1], Cin, self.N, self.buf.data_ptr(), n, _stream())
+            _call('spgt_conv3x3_weight_prepare', w_kn.data_ptr(), w_kn.shape[1], Cin, self.N, self.buf.data_ptr(), self.buf.numel(), _stream())
+
+    def _allocate(self, Cin: int, Cout: int, device):
+        self.K, self.N = 9 * Cin, Cout
+        self.buf = torch.empty(int(lib.spgt_conv3x3_weight_bytes(Cin, Cout)), dtype=torch.uint8, device=device)
+
+    @classmethod
+    def padded(cls, weight: Tensor, bias: Tensor, Cin: int, Cout: int):
+        """(prepared weight, bias [Cout]) of a torch convolution [cout, cin, 3, 3], zero padded to Cin and Cout channels."""
+        _chk(weight, 'weight'); _chk(bias, 'bias')
+        self = cls.__new__(cls)
+        self._allocate(Cin, Cout, weight.device)
+        b = torch.empty(Cout, dtype=weight.dtype, device=weight.device)
+        with _device(weight.device):
+            _call('spgt_conv3x3_weight_prepare_oihw', weight.data_ptr(), bias.data_ptr(), weight.shape[1], weight.shape[0], Cin, Cout,
+                  self.buf.data_ptr(), self.buf.numel(), b.data_ptr(), _stream())
+        return self, b
 
     def data_ptr(self) -> int:
         return self.buf.data_ptr()
@@ -597,6 +611,23 @@ def kept_pointer(keep: list, t):
     return t.data_ptr()
 
 
+class EncoderImages:
+    """The fused encoder layer's weight images (K / V, and with w1, w2 the feed-forward block's), made in one launch from the weights as
+    the modules keep them."""
+
+    def __init__(self, wk: Tensor, wv: Tensor, w1: Optional[Tensor] = None, w2: Optional[Tensor] = None):
+        for t in (wk, wv) if w1 is None else (wk, wv, w1, w2):
+            _chk(t, 'weight')
+        n = int(lib.spgt_encoder_weights_bytes(int(w1 is not None)))
+        self.buf = torch.empty(n, dtype=torch.uint8, device=wk.device)
+        self.stride = n // (1 if w1 is None else 3)
+        with _device(wk.device):
+            _call('spgt_encoder_weights_prepare', wk.data_ptr(), wv.data_ptr(), _p(w1), _p(w2), self.buf.data_ptr(), n, _stream())
+
+    def data_ptr(self) -> int:
+        return self.buf.data_ptr()
+
+
 class EncoderPlan:
     """A spgt_encoder_weights with the tensors it points to; `fill` writes the pointers (ptr(tensor) keeps the tensor)."""
 
@@ -680,8 +711,9 @@ def encoder_train_backward(x: Tensor, att: Tensor, x1: Tensor, h: Tensor, eps: f
 class DarcyPlan:
     """A spgt_darcy_model with the tensors it points to."""
 
-    def __init__(self, model, keep):
-        self.model, self.keep, self.address = model, keep, ctypes.addressof(model)
+    def __init__(self, model, keep, head_b2: int):
+        """head_b2: device pointer of the decoder head's second bias."""
+        self.model, self.keep, self.address, self.head_b2 = model, keep, ctypes.addressof(model), head_b2
         self.sizes = {}          # batch -> (workspace bytes, kernels launched)
 
     def size(self, B: int):
@@ -712,6 +744,6 @@ def darcy_forward(plan: DarcyPlan, node: Tensor, position: Tensor, grid: Tensor,
             taps.update({f'enc{i}': new(B, S, 128) for i in range(m.n_encoder)}, up_mid=new(B, m.mid, m.mid, 128))
             ptrs = [taps['down'], *(taps[f'enc{i}'] for i in range(m.n_encoder)), taps['up_mid']]
             want = (ctypes.c_void_p * len(ptrs))(*(t.data_ptr() for t in ptrs))
-        _call('spgt_darcy_forward', plan.address, node.data_ptr(), position.data_ptr(), grid.data_ptr(), out.data_ptr(), B, want,
+        _call('spgt_darcy_forward_devbias', plan.address, plan.head_b2, node.data_ptr(), position.data_ptr(), grid.data_ptr(), out.data_ptr(), B, want,
               workspace.data_ptr(), need, _stream(), kernels=kernels)
     return out

@@ -357,6 +357,29 @@ def test_bilinear_concat3(B, Hi, Ho, c):
     assert rel_l2(y, ref) < 1e-6          # (the same fp32 source coordinates, four products and three sums)
 
 
+def test_images_from_the_modules_weights():
+    """Prepared in one launch from the weights as they are: the same bits as from rearranged copies (K / V: but for the rounding of the mean)."""
+    from spgt_b200 import ops
+    g = torch.Generator().manual_seed(8)
+    wk, wv, w1, w2 = (torch.randn(*s, generator=g).cuda() for s in ((128, 128), (128, 128), (256, 128), (128, 256)))
+    images, alone = ops.EncoderImages(wk, wv, w1, w2), ops.EncoderImages(wk, wv)
+    parts = images.buf.view(3, -1)
+    assert torch.equal(parts[0], alone.buf)
+    for part, w in zip(parts[1:], (w1, w2)):
+        assert torch.equal(part, ops.TcWeight(w, transposed=True).buf)
+    w = torch.stack([wk, wv], dim=1).double().view(128, 2, 4, 32)
+    w = (w - w.mean(dim=3, keepdim=True)).view(128, 2, 2, 64).transpose(1, 2).reshape(128, 256)
+    got, want = (t.view(torch.float32).view(2, 4, 2, -1).double().sum(2) for t in (parts[0], ops.TcWeight(w.float()).buf))      # hi + lo
+    assert rel_l2(got, want) < 2e-7                      # one ulp of the mean of 32 values
+    for cin, cout, cin_pad, cout_pad in ((128, 42, 128, 44), (42, 42, 44, 44), (1, 3, 4, 4), (66, 50, 68, 64), (128, 128, 128, 128)):
+        w, b = torch.randn(cout, cin, 3, 3, generator=g).cuda(), torch.randn(cout, generator=g).cuda()
+        pad = torch.zeros(cout_pad, cin_pad, 3, 3, device='cuda')
+        pad[:cout, :cin] = w
+        prepared, bias = ops.ConvWeight.padded(w, b, cin_pad, cout_pad)
+        assert torch.equal(prepared.buf, ops.ConvWeight(pad.permute(2, 3, 1, 0).reshape(9 * cin_pad, cout_pad).contiguous(), cin_pad).buf)
+        assert torch.equal(bias, torch.nn.functional.pad(b, (0, cout_pad - cout)))
+
+
 def _with_nan(t, at):
     """t with a NaN as arithmetic on the GPU makes it (all mantissa bits set)."""
     t = t.clone()
