@@ -37,9 +37,8 @@ METRIC = 'darcy_gt_inference_samples_per_s_211'
 FINE, SUB_NODE, SUB_ATTN, MODES, SEED = 421, 2, 8, 12, 4
 GLOBAL_BATCH = 64
 CPU_SAMPLE = 8                     # samples per forward of the CPU legs (a bounded sample of the 64-sample step)
-# DRAM bytes (read + write) of one launch at batch 64 from the committed ncu summaries of these kernels; they grow in
+# DRAM bytes (read + write) of one spectral layer at batch 64 from the committed ncu summary; they grow in
 # proportion to the batch, so a rank that holds 64/N samples is charged 1/N of them.
-ATTN_TRAFFIC_BYTES_B64 = 343_600_000
 SPECTRAL_TRAFFIC_BYTES_B64 = 1_174_600_000
 
 
@@ -495,23 +494,26 @@ def main():
             ok = ok and abs(float(full[b:e].double().sum()) - float(sums[rk])) <= 1e-9 * abs(float(sums[rk]))   # rank rk's block sits where the global order puts it
         gather_check = 'ok' if ok else 'MISMATCH'
 
-    # ---------------- rooflines of the attention kernel and the spectral layer (separate eager pass) ----------------
-    names = ['spgt_galerkin_attn_fwd', 'spgt_spectral_conv2d_fwd']
+    # ---------------- rooflines of an encoder layer and a spectral layer (separate eager pass, stage by stage) ----------------
+    names = ['spgt_encoder_layer_fwd', 'spgt_spectral_conv2d_fwd']
     with ops.profile_ops(only=names) as prof:
         for _ in range(args.steps):
             model(dev['node'], dev['position'], dev['grid'])
     tm = prof.times_ms()
     peak, peak_kind = measured_peak()
 
-    def roofline(name, kernel, algo_bytes, traffic_b64):
+    def roofline(name, kernel, algo_bytes, traffic_b64, flops=None):
         t = tm.get(name, [])
         avg = sum(t) / max(1, len(t))
         achieved = algo_bytes / (avg * 1e-3) / 1e9 if avg > 0 else None
         return {'kernel': kernel, 'bound': 'hbm', 'achieved': achieved, 'peak': peak, 'peak_kind': peak_kind, 'unit': 'GB/s',
                 'frac': (achieved / peak) if achieved else None,
                 'traffic': (traffic_b64 * B // 64) if traffic_b64 else None, 'algorithmic_bytes': algo_bytes,
-                'avg_launch_ms': avg, 'launches_timed': len(t)}
-    roof_attn = roofline('spgt_galerkin_attn_fwd', 'galerkin_attn_tc_kernel', 4 * B * H * DPK * S * 4, ATTN_TRAFFIC_BYTES_B64)
+                'avg_launch_ms': avg, 'launches_timed': len(t),
+                'tflops': flops / (avg * 1e-3) / 1e12 if flops and avg > 0 else None}
+    # encoder layer: read x and the positions, write y; K and V projections, K^T V, x M, feed-forward (fp32 products, three TF32 products each)
+    roof_enc = roofline('spgt_encoder_layer_fwd', 'encoder layer (encoder_kv, encoder_fold, encoder_out)', B * S * (2 * 128 + 2) * 4, None,
+                        2 * B * S * (2 * 128 * 128 + H * DPK * DPK + 128 * 128 + 2 * 128 * 256))
     # spectral layer: read x once, write y once (fp32, 32 channels) + the complex mode weights; one entry-point call = all its kernels
     roof_spec = roofline('spgt_spectral_conv2d_fwd', 'spectral layer (all kernels of one call)',
                          2 * B * r * r * 32 * 4 + 2 * 2 * MODES * MODES * 32 * 32 * 8, SPECTRAL_TRAFFIC_BYTES_B64)
@@ -559,7 +561,7 @@ def main():
                     'downloads': args.e2e_download,
                     'ms_per_step': e2e_s * 1e3 / args.steps,
                     'collectives_per_step': 0 if world == 1 else 2, 'gather_check': gather_check, 'metric': metric_value},
-            'roofline': roof_attn, 'roofline_spectral': roof_spec, 'cpu_baseline': cpu, 'weak_64_per_gpu': weak,
+            'roofline': roof_enc, 'roofline_spectral': roof_spec, 'cpu_baseline': cpu, 'weak_64_per_gpu': weak,
         }
         print(json.dumps(line), flush=True)
     if world > 1:

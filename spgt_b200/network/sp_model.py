@@ -165,7 +165,7 @@ class Sp_GalerkinTransformer2D(torch.nn.Module):
         return X
 
     def _forward_fused(self, X: Tensor, position: Tensor, grid: Tensor, taps: dict = None) -> Tensor:
-        plan = None if self._watch.observed(self) else self._native_plan(X)
+        plan = None if ops.profiling() or self._watch.observed(self) else self._native_plan(X)
         if plan is None or not self._native_shapes(X, position, grid):
             return self._forward_modules(X, position, grid, taps)
         return ops.darcy_forward(plan, X, position, grid, taps)

@@ -71,6 +71,11 @@ def _call(name: str, *args, kernels: int = None) -> None:
     LAUNCHES += kernels if kernels is not None else _KERNELS_PER_CALL.get(name, 1)
 
 
+def profiling() -> bool:
+    """Whether single entry points are being timed: the model then calls its stages one by one, which launch the same kernels."""
+    return _PROFILE is not None
+
+
 class profile_ops:
     """Context manager: CUDA-event timing around every entry point (or only the named ones) on the current stream.
     After the block (and a synchronize) `times_ms()` gives name -> list of durations."""

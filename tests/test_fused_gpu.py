@@ -212,6 +212,17 @@ def test_encoder_layer_training_without_a_projection_bias():
         assert rel_l2(layer.forward_train(x.cuda(), pos.cuda()), ref) < TOL
 
 
+def test_single_entry_points_can_be_timed():
+    from spgt_b200 import ops
+    model, *args = _model()
+    ref = model(*args)
+    with ops.profile_ops() as profile:
+        out = model(*args)
+    times = profile.times_ms()
+    assert len(times['spgt_encoder_layer_fwd']) == 2 and len(times['spgt_spectral_conv2d_fwd']) == 2 and 'spgt_darcy_forward_devbias' not in times
+    assert rel_l2(out, ref) < TOL and torch.equal(model(*args), ref)
+
+
 def test_one_call_forward_yields_to_other_grids():
     """A grid of other nodes (the regressor is evaluated there), or one with more samples than there are fields."""
     from spgt_b200.dataset.darcy_dataset import meshgrid
