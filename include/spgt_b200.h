@@ -254,7 +254,8 @@ size_t spgt_tn_gemm_workspace_bytes(int M, int N, int rows);
 int spgt_tn_gemm(const float* A, int lda, const float* B, int ldb, float* C, int ldc, float* colsum, int M, int N, int rows,
                  void* workspace, size_t workspace_bytes, spgt_stream_t stream);
 /* 0 if no tensor-core kernel gave up on a bounded wait since the last reset, else the code of the first one that did
- * (GEMM: 1..9; fused feed-forward: 21..34; attention: 101..109; spectral layer: 201..219).  Every wait inside these
+ * (GEMM, the Fourier layer's transforms along y among them: 1..8; fused feed-forward: 21..34; fused encoder layer: 40..54 its
+ * first and 60..76 its last kernel; 3x3 convolution: 80..86; weight gradients: 90..96; attention: 101..110).  Every wait inside these
  * kernels is bounded by two seconds of wall time; a kernel whose wait expires stops waiting, records the code and
  * returns with an incomplete output, so a host loop should read this at its synchronisation points and discard the
  * results when it is not 0.  Synchronises the device.  No counterpart in the reference (its kernels have no waits). */

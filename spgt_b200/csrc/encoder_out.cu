@@ -8,7 +8,8 @@
 //   GEMM 2  A = act(D1 + b1) (warps 4-11),                      D2 128 columns, in D0's place
 // D0 / D2 and D1 swap sides from tile to tile, so that GEMM 0 of the next tile and the last epilogue do not wait for one another.
 // The B operands stream through a ring of 16 KB slots (an image's hi or lo half): 640 KB per tile from L2, 42 B per cycle and SM
-// (measured: L2 delivers at least 79).  Bound by the tensor pipe: 240 MMAs of 64 cycles per tile = 15400 cycles.
+// (measured: L2 delivers at least 79).  The tensor pipe needs 15400 cycles per tile (240 MMAs of 64); measured on its own, 64 x 2809 nodes:
+// 144 us = 21700 cycles for each of at most ten tiles per SM, the pipe 67 % busy: the conversions between the chained GEMMs are in the way.
 //   warps 0-3 x splitters, 4-11 converters / epilogue, 12 x tile loader, 13-14 image loaders (even / odd slots), 15 MMA issuer.
 // Every wait is a bounded mbarrier poll that records a code on expiry.
 #include "encoder_common.cuh"

@@ -5,8 +5,9 @@
 // and a library product plus a reduction per dense layer for the weight and bias gradients.
 // The caller makes the dense layers' forward products and dh = (dy W2^T) [h > 0], dx1 = dy + dh W1^T, da = dx1 Wfc^T in plain fp32: which
 // hidden values pass the ReLU is decided by their last bits, and a chain of 24 products in 3xTF32, whose accumulation truncates,
-// moved a training step's gradients further from fp64 (5.0e-6 against 3.1e-6).  For the same reason the projections run on the
-// warp-MMA kernel: with the tcgen05 one single hidden values fell on the other side of the ReLU (1e-5 to 2e-4 of a step's gradients).
+// moved a training step's gradients further from fp64 (5.0e-6 against 3.1e-6).  The projections stay on the warp-MMA kernel: the
+// tcgen05 one is as close to fp64 (9.1e-7 both before the LayerNorm, 5.0e-7 after it), but its other roundings put other single
+// hidden values on the other side of the ReLU, each worth 1e-5 to 2e-4 of a step's gradients.
 // Here: weight images (they change every step; one launch), projections and attention; then attention and LayerNorm backward to
 // dqkv = [dq dk dv], dx = dx1 + dq Wq^T + dk Wk^T + dv Wv^T, one product x^T dqkv for the three projections' weights and one per dense
 // layer (from 128 rows on, below which the caller's fp32 products are closer to fp64), with the bias gradients as its column sums.  LayerNorm's input is recomputed from x.

@@ -1126,12 +1126,12 @@ extern "C" int spgt_tc_status(void) {
     if (cudaMemcpyFromSymbol(&v, g_tc_status, sizeof(int)) != cudaSuccess) return SPGT_ERR_LAUNCH;
     if (v != 0) return v;
     const int a = spgt::attn_tc_status();
-    if (a != 0) return a > 0 ? 100 + a : a;     // 101..109: a wait of the attention kernel gave up
-    if (int e = spgt::encoder_kv_status(false)) return e;       // 40..52: the first half of an encoder layer
+    if (a != 0) return a > 0 ? 100 + a : a;     // 101..110: a wait of the attention kernel gave up
+    if (int e = spgt::encoder_kv_status(false)) return e;       // 40..54: the first half of an encoder layer
     if (int e = spgt::encoder_out_status(false)) return e;      // 60..76: its second half
     if (int e = spgt::conv_status(false)) return e;             // 80..86: the convolution kernel
     if (int e = spgt::tn_status(false)) return e;               // 90..96: the weight-gradient kernel
-    return spgt::ffn_tc_status();               // 21..33: a wait of the fused feed-forward kernel gave up
+    return spgt::ffn_tc_status();               // 21..34: a wait of the fused feed-forward kernel gave up
 }
 
 extern "C" int spgt_tc_status_reset(void) {

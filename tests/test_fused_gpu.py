@@ -302,8 +302,8 @@ def test_attention_backward_tiles(B, H, dpk, S):
     assert all(torch.equal(a, b) for a, b in zip(got, ops.galerkin_attention_backward(q, k, v, dout)))
 
 
-# one node, ends of a 128-row tile, samples that share tiles, rows around the weight gradients' 32-row blocks and chains
-@pytest.mark.parametrize('B,S', [(1, 1), (1, 127), (2, 129), (3, 171), (4, 1849), (40, 33)])
+# one node, both sides of the 128 rows from which the weight-gradient kernel runs, samples that share its 32-row blocks
+@pytest.mark.parametrize('B,S', [(1, 1), (1, 127), (1, 128), (2, 129), (3, 171), (4, 1849), (40, 33)])
 def test_encoder_layer_training_gradients(B, S):
     from spgt_b200 import ops
     layer, g = _layer(S)
@@ -322,8 +322,13 @@ def test_encoder_layer_training_gradients(B, S):
         y = layer.forward_train(xd, pos.cuda())
         runs.append((y, *torch.autograd.grad(y, [xd] + list(layer.parameters()), dy.cuda())))
     y = layer.forward_train(xd, pos.cuda())
-    passes = y.grad_fn.saved_tensors[2].cpu() > 0          # a value within rounding of zero may pass the ReLU there and not in float64
-    h = linear(x1, p['ffn_layer.layer1.weight'], p['ffn_layer.layer1.bias']) * passes
+    passes = y.grad_fn.saved_tensors[2].cpu() > 0
+    w1 = p['ffn_layer.layer1.weight']
+    pre = linear(x1, w1, p['ffn_layer.layer1.bias'])
+    # a value within rounding of zero may pass the ReLU there and not in float64: x1 is within TOL of its row's norm
+    rounding = TOL * x1.norm(dim=-1, keepdim=True) * w1.norm(dim=1)
+    assert bool(((passes == (pre > 0)) | (pre.abs() < rounding)).all())
+    h = pre * passes
     ref = x1 + linear(h, p['ffn_layer.layer2.weight'], p['ffn_layer.layer2.bias'])
     want = torch.autograd.grad(ref, [xr] + [p[n] for n in names], dy.double())
     assert ops.tc_status() == 0 and y.grad_fn.name().startswith('_EncoderLayerFunction')
