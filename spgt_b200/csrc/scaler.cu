@@ -298,41 +298,53 @@ static int launch_staged(const StagedPlan& p, const float4* x, float4* y, int B,
 }
 
 // y[b,yo,xo,:] = act(bilinear(concat(x1[..., :c1], x2[..., :c2], x3[..., :c3])))  -- the three sources keep their own
-// (padded) channel pitch, the output is dense.  One thread per (pixel, 4 output channels), scalar gathers; an item is a segment of
-// an output row.  (One output channel per thread, whose accesses are 128 bytes wide, was 6 % faster at 64 x 106 x 106 -> 53 x 53, 83.7
-// against 88.3 us, and slower from 2 x 77 to 8 x 106, 15.2 against 11.5 us: four times the index arithmetic.)
+// (padded) channel pitch, the output is dense.  A thread keeps one output channel, so its source, pitch and column are fixed and the
+// lanes of a warp read and write consecutive channels (the sources' boundaries are no multiples of four).  An item is a segment of an
+// output row, C3_U pixels at a time.  On its own the kernel takes 84 us at 64 x 106 x 106 -> 53 x 53 (one thread per four channels: 89;
+// the DRAM traffic alone 72) and 14 at 8 x 106 (11.5): there the fourfold index arithmetic shows.  Inside a forward, where its blocks start
+// under the tail of the convolution before, it is the faster or equal one at every batch: 8 / 16 fields at 211 x 211 take 850 / 1347 us
+// against 852 / 1350.
+constexpr int C3_U = 4;
 __global__ void __launch_bounds__(256)
 bilinear_concat3_kernel(const float* __restrict__ x1, const float* __restrict__ x2, const float* __restrict__ x3, int p1,
-                        int p2, int p3, int c1, int c2, int c3, float4* __restrict__ y, int Hi, int Wi, int Ho, int Wo,
+                        int p2, int p3, int c1, int c2, int c3, float* __restrict__ y, int Hi, int Wi, int Ho, int Wo,
                         int act, int segments, int seg_pixels, int items) {
     pdl_wait();
     pdl_launch_next();
-    const int C4 = (c1 + c2 + c3) / 4;
+    const int C = c1 + c2 + c3, step = (int)blockDim.x < C ? 1 : blockDim.x / C;     // pixels of the block side by side
+    const int px = (int)blockDim.x < C ? 0 : threadIdx.x / C, c_first = threadIdx.x - px * C;
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
         const int row = item / segments, x_begin = (item - row * segments) * seg_pixels;
         const int x_end = x_begin + seg_pixels < Wo ? x_begin + seg_pixels : Wo;
         const int b = row / Ho, yo = row - b * Ho;
         const Tap ty = make_tap(yo, Hi, Ho);
-        const int64_t q0 = ((int64_t)b * Hi + ty.i0) * Wi, q1 = ((int64_t)b * Hi + ty.i1) * Wi;
-        float4* yr = y + (int64_t)row * Wo * C4;
-        for (int e = x_begin * C4 + threadIdx.x; e < x_end * C4; e += blockDim.x) {
-            const int xo = e / C4, cg = e - xo * C4;
-            const Tap tx = make_tap(xo, Wi, Wo);
-            const float w00 = ty.w0 * tx.w0, w01 = ty.w0 * tx.w1, w10 = ty.w1 * tx.w0, w11 = ty.w1 * tx.w1;
-            const int64_t o00 = q0 + tx.i0, o01 = q0 + tx.i1, o10 = q1 + tx.i0, o11 = q1 + tx.i1;
-            float o[4];
+        for (int c = c_first; c < C; c += blockDim.x) {                               // (once, unless there are more channels than threads)
+            const float* src; int pitch;
+            if (c < c1) { src = x1 + c; pitch = p1; }
+            else if (c < c1 + c2) { src = x2 + c - c1; pitch = p2; }
+            else { src = x3 + c - c1 - c2; pitch = p3; }
+            const float* r0 = src + ((int64_t)b * Hi + ty.i0) * Wi * pitch;
+            const float* r1 = src + ((int64_t)b * Hi + ty.i1) * Wi * pitch;
+            float* out = y + (int64_t)row * Wo * C + c;
+            for (int xo = x_begin + px; xo < x_end; xo += C3_U * step) {
+                float v[C3_U][4];
+                Tap tx[C3_U];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                int c = cg * 4 + k;
-                const float* src; int pitch;
-                if (c < c1) { src = x1; pitch = p1; }
-                else if (c < c1 + c2) { src = x2; pitch = p2; c -= c1; }
-                else { src = x3; pitch = p3; c -= c1 + c2; }
-                const float v = __ldca(src + o00 * pitch + c) * w00 + __ldca(src + o01 * pitch + c) * w01 +
-                                __ldca(src + o10 * pitch + c) * w10 + __ldca(src + o11 * pitch + c) * w11;
-                o[k] = apply_act(v, act);
+                for (int u = 0; u < C3_U; ++u) {
+                    const int xu = xo + u * step;
+                    tx[u] = make_tap(xu < x_end ? xu : x_end - 1, Wi, Wo);
+                    const int64_t o0 = (int64_t)tx[u].i0 * pitch, o1 = (int64_t)tx[u].i1 * pitch;
+                    v[u][0] = __ldca(r0 + o0); v[u][1] = __ldca(r0 + o1);
+                    v[u][2] = __ldca(r1 + o0); v[u][3] = __ldca(r1 + o1);
+                }
+#pragma unroll
+                for (int u = 0; u < C3_U; ++u) {
+                    const int xu = xo + u * step;
+                    const float w00 = ty.w0 * tx[u].w0, w01 = ty.w0 * tx[u].w1, w10 = ty.w1 * tx[u].w0, w11 = ty.w1 * tx[u].w1;
+                    const float o = v[u][0] * w00 + v[u][1] * w01 + v[u][2] * w10 + v[u][3] * w11;
+                    if (xu < x_end) out[(int64_t)xu * C] = apply_act(o, act);
+                }
             }
-            yr[e] = make_float4(o[0], o[1], o[2], o[3]);
         }
     }
 }
@@ -365,17 +377,17 @@ extern "C" int spgt_bilinear_concat3_fwd(const float* x1, const float* x2, const
     if (!aligned16(y)) return SPGT_ERR_ALIGN;
     const int64_t rows = (int64_t)B * Ho;
     if (rows > 0x7fffffffLL || (int64_t)Wo * (c1 + c2 + c3) > 0x7fffffffLL) return SPGT_ERR_SHAPE;
-    // Segments of a row.  Four blocks fit on an SM at once; fewer rows than that are cut to fill it (eight pixels of 128 channels keep a
-    // block busy once), rows that would leave a second wave part-empty are halved.  1 x 77 x 77 -> 43 x 43: 6.6 us uncut, 2.9 cut;
-    // 4 x 106 -> 53: 9.0 and 7.2; 16 x 106 -> 53: 28.4 and 25.9; 64 x 31 -> 15, too short to halve: 8.8 and 9.5.
-    const int64_t fit = (int64_t)4 * num_sms();
-    const int pixels = ceil_div(1024, c1 + c2 + c3);
-    int64_t segments = rows <= fit ? fit / rows : (rows < 2 * fit && Wo >= 4 * pixels ? 2 : 1);
-    if (segments > ceil_div(Wo, pixels)) segments = ceil_div(Wo, pixels);
-    const int seg_pixels = ceil_div(Wo, (int)segments);
+    const int C = c1 + c2 + c3, step = C <= 256 ? 256 / C : 1, threads = C <= 256 ? step * C : 256;
+    // segments of a row: as many items as eight blocks per SM take at once (one segment more made a second, nearly empty wave: 8 x 106 -> 53
+    // 15.2 us against 14.0), C3_U pixels per thread at least
+    int64_t segments = (int64_t)8 * num_sms() / rows;
+    if (segments < 1) segments = 1;
+    if (segments > ceil_div(Wo, C3_U * step)) segments = ceil_div(Wo, C3_U * step);
+    const int seg_pixels = ceil_div(ceil_div(Wo, (int)segments), step) * step;
     segments = ceil_div(Wo, seg_pixels);
-    return launch_chained(bilinear_concat3_kernel, grid_for(rows * segments, 1, 8), 256, 0, (cudaStream_t)stream,
-        x1, x2, x3, p1, p2, p3, c1, c2, c3, reinterpret_cast<float4*>(y), Hi, Wi, Ho, Wo, act, (int)segments, seg_pixels, (int)(rows * segments));
+    if (rows * segments > 0x7fffffffLL) return SPGT_ERR_SHAPE;
+    return launch_chained(bilinear_concat3_kernel, grid_for(rows * segments, 1, 8), threads, 0, (cudaStream_t)stream,
+        x1, x2, x3, p1, p2, p3, c1, c2, c3, y, Hi, Wi, Ho, Wo, act, (int)segments, seg_pixels, (int)(rows * segments));
 }
 
 extern "C" int spgt_conv0_down_fwd(const float* node, const float* w, const float* bias, float* y, int B, int Hi, int Wi,
