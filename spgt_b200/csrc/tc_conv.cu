@@ -329,7 +329,7 @@ extern "C" int spgt_conv3x3_nhwc_fwd(const float* x, int cin_pitch, int cin_off,
     if (cin_off + Cin > cin_pitch || cout_off + Cout > cout_pitch || act < 0 || act > 3) return SPGT_ERR_SHAPE;
     if ((Cin & 3) || (cin_off & 3) || (cin_pitch & 3) || (Cout & 3) || (cout_off & 3) || (cout_pitch & 3)) return SPGT_ERR_SHAPE;
     const int64_t rows = (int64_t)B * (Hh + 1), tiles = ceil_div(rows, (int64_t)CV_TY) * ceil_div(Ww, CV_TX);
-    if (rows * (Ww + CV_TX) > 0x7fffffffLL / 2) return SPGT_ERR_SHAPE;
+    if (rows > 0x7fffffffLL - 64 || tiles > 0x7fffffffLL / 2) return SPGT_ERR_SHAPE;      // (rows and tiles are counted in 32 bits)
     if (!aligned16(x) || !aligned16(wprep) || !aligned16(y)) return SPGT_ERR_ALIGN;
     const ConvParams p{x + cin_off, (const float*)wprep, bias, y + cout_off, cin_pitch, Cin, cout_pitch, Cout, B, Hh, Ww, act, ceil_div(Ww, CV_TX), (int)tiles};
     switch (conv_bn(Cout)) {

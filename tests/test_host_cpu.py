@@ -34,6 +34,8 @@ def test_argument_validation_without_gpu():
     for r, m in ((800, 16), (1066, 12), (3200, 4)):
         assert lib.spgt_spectral_tables_bytes(r, m) > 0 and lib.spgt_spectral_workspace_bytes(2, r, m, 32) > 0 and lib.spgt_spectral_launches(2, r, m) > 0
         assert lib.spgt_spectral_tables_bytes(r + 1, m) == 0 and lib.spgt_spectral_workspace_bytes(2, r + 1, m, 32) == 0 and lib.spgt_spectral_launches(2, r + 1, m) == 0
+    # 40 million images of 4 x 4 pixels: within the limits, refused for the alignment of x only
+    assert lib.spgt_conv3x3_nhwc_fwd(20, 4, 0, 4, 16, None, 16, 4, 0, 4, 40_000_000, 4, 4, 0, None) == -3
     assert lib.spgt_spectral_workspace_bytes(8, 211, 12, 32) == (2 * 8 * 211 * 24 * 32 + 4 * 8 * 24 * 12 * 32 + 2048) * 4
     assert lib.spgt_spectral_launches(8, 211, 12) == 5 and lib.spgt_spectral_chunk_samples(211) >= 8
     assert lib.spgt_skinny_gemm_workspace_bytes(32, 32, 1849, 64) % 4 == 0 and lib.spgt_skinny_gemm_workspace_bytes(32, 30, 1849, 64) % 4096 == 0
