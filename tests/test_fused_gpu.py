@@ -288,7 +288,7 @@ def test_spectral_layer_slices_and_units(B, r, m):
 
 
 # columns around the 112-wide tiles, 16-byte and 4-byte copies, several chunks and blocks of several tiles
-@pytest.mark.parametrize('B,H,dpk,S', [(1, 1, 34, 1), (2, 4, 34, 111), (1, 4, 34, 112), (3, 2, 35, 113), (16, 4, 34, 4096), (2, 3, 32, 4097), (80, 4, 34, 225)])
+@pytest.mark.parametrize('B,H,dpk,S', [(1, 1, 34, 1), (2, 4, 34, 111), (1, 4, 34, 112), (3, 2, 35, 113), (16, 4, 34, 4096), (2, 3, 32, 4097), (80, 4, 34, 225), (300, 4, 34, 16), (3, 2, 1, 500), (2, 3, 12, 300), (2, 3, 13, 1000), (1, 2, 24, 63), (1, 2, 25, 130)])
 def test_attention_backward_tiles(B, H, dpk, S):
     from spgt_b200 import ops
     g = torch.Generator().manual_seed(S)
