@@ -72,7 +72,8 @@ class Sp_GalerkinAttention(_KernelWeights):
         When Q, K and V are the same tensor (self-attention) all three projections run in one launch."""
         d = lambda t: t.detach()
         H, dh, dp = self.num_head, self.dim_head, self.dim_position
-        if Q is K and K is V and self.fusable and (residual is None or residual is Q):
+        if (Q is K and K is V and self.fusable and (residual is None or residual is Q)
+                and ops.encoder_fused_pays(Q.shape[0], Q.shape[1], ffn=False)):
             plan = self._cached('native', lambda: ops.EncoderPlan(self.fill_native))
             return ops.encoder_layer(plan, Q, position, self.norm_eps, None, ffn=False, residual=residual is not None)
         if Q is K and K is V and self.dim_hidden == 128:
@@ -174,7 +175,7 @@ class Sp_EncoderLayer(_KernelWeights):
     def forward(self, X: Tensor, position: Tensor) -> Tensor:
         """X [N,S,D], position [N,S,d_pos] -> X + attention(X) then + ffn(.)  (network/sp_layer.py:94-104)."""
         f = self.ffn_layer
-        if self.fusable and not self._watch.observed(self):
+        if self.fusable and not self._watch.observed(self) and ops.encoder_fused_pays(X.shape[0], X.shape[1]):
             plan = self._cached('native', lambda: ops.EncoderPlan(self.fill_native))
             return ops.encoder_layer(plan, X, position, self.attention_layer.norm_eps, f.activation)
         X = self.attention_layer(X, X, X, position, residual=X)

@@ -165,17 +165,23 @@ class Sp_GalerkinTransformer2D(torch.nn.Module):
         return X
 
     def _forward_fused(self, X: Tensor, position: Tensor, grid: Tensor, taps: dict = None) -> Tensor:
-        plan = None if ops.profiling() or self._watch.observed(self) else self._native_plan(X)
-        if plan is None or not self._native_shapes(X, position, grid):
+        if ops.profiling() or self._watch.observed(self) or not self._native_shapes(X, position, grid):
+            plan = None
+        else:
+            plan = self._native_plan(X)
+        if plan is None:
             return self._forward_modules(X, position, grid, taps)
         return ops.darcy_forward(plan, X, position, grid, taps)
 
     def _native_shapes(self, X: Tensor, position: Tensor, grid: Tensor) -> bool:
-        """Whether the inputs are one sample per coordinate set on the model's own grids.  The modules also take a `grid` of other nodes
-        (the regressor is evaluated there) or with more samples than X."""
+        """Whether the inputs are one sample per coordinate set on the model's own grids, and not many samples of few nodes.  The modules
+        also take a `grid` of other nodes (the regressor is evaluated there) or with more samples than X."""
+        if type(self.down_scaler) is not DownScaler2D:
+            return False
         (r, _), _, (ra, _) = self.down_scaler.resolution_size[:3]
         N = X.shape[0]
-        return tuple(X.shape) == (N, r, r, 1) and tuple(grid.shape) == (N, r, r, 2) and position.numel() == N * ra * ra * 2 and position.shape[-1] == 2
+        return (tuple(X.shape) == (N, r, r, 1) and tuple(grid.shape) == (N, r, r, 2) and position.numel() == N * ra * ra * 2
+                and position.shape[-1] == 2 and ops.encoder_fused_pays(N, ra * ra))
 
     def _native_plan(self, X: Tensor):
         """The model as the one-call forward takes it, rebuilt when the parameters, the grid or the device are not the ones it was

@@ -119,6 +119,14 @@ def _position(t: Tensor, nodes: int) -> Tensor:
     return t if t.data_ptr() % 8 == 0 else t.clone()
 
 
+def _coordinates(t: Tensor, nodes: int, dim_position: int) -> Tensor:
+    """Node coordinates [..., dim_position] as the projection kernels read them, one node after the other."""
+    _chk(t, 'position')
+    if t.numel() < nodes * dim_position:
+        raise ValueError(f'position must hold {dim_position} values for each of {nodes} nodes')
+    return t
+
+
 def _p(t: Optional[Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
@@ -128,10 +136,11 @@ def _p(t: Optional[Tensor]) -> Optional[int]:
 # ---------------------------------------------------------------------------------------------------------
 def projpos(x: Tensor, weight: Tensor, bias: Optional[Tensor], position: Tensor, num_head: int, dim_head: int,
             dim_position: int) -> Tensor:
-    _chk(x, 'input'); _chk(weight, 'weight'); _chk(position, 'position')
+    _chk(x, 'input'); _chk(weight, 'weight')
     if bias is not None:
         _chk(bias, 'bias')
     B, S, D = x.shape
+    _coordinates(position, B * S, dim_position)
     out = torch.empty(B, num_head, dim_position + dim_head, S, device=x.device, dtype=x.dtype)
     with _device(x.device):
         _call('spgt_projpos_fwd', x.data_ptr(), weight.data_ptr(), _p(bias), position.data_ptr(), out.data_ptr(),
@@ -142,10 +151,11 @@ def projpos(x: Tensor, weight: Tensor, bias: Optional[Tensor], position: Tensor,
 def projpos_lnorm(x: Tensor, weight: Tensor, bias: Optional[Tensor], ln_weight: Tensor, ln_bias: Tensor,
                   position: Tensor, norm_eps: float, num_head: int, dim_head: int, dim_position: int,
                   return_invsigma: bool = False):
-    _chk(x, 'input'); _chk(weight, 'weight'); _chk(position, 'position'); _chk(ln_weight, 'ln_weight'); _chk(ln_bias, 'ln_bias')
+    _chk(x, 'input'); _chk(weight, 'weight'); _chk(ln_weight, 'ln_weight'); _chk(ln_bias, 'ln_bias')
     if bias is not None:
         _chk(bias, 'bias')
     B, S, D = x.shape
+    _coordinates(position, B * S, dim_position)
     out = torch.empty(B, num_head, dim_position + dim_head, S, device=x.device, dtype=x.dtype)
     inv = torch.empty(B, num_head, S, device=x.device, dtype=x.dtype) if return_invsigma else None
     with _device(x.device):
@@ -156,9 +166,10 @@ def projpos_lnorm(x: Tensor, weight: Tensor, bias: Optional[Tensor], ln_weight: 
 
 
 def projpos_qkv(x, wq, bq, wk, bk, wv, bv, lnwk, lnbk, lnwv, lnbv, eps, position, num_head, dim_head, dim_position):
-    for n, t in (('x', x), ('wq', wq), ('wk', wk), ('wv', wv), ('position', position)):
+    for n, t in (('x', x), ('wq', wq), ('wk', wk), ('wv', wv)):
         _chk(t, n)
     B, S, D = x.shape
+    _coordinates(position, B * S, dim_position)
     q, k, v = (torch.empty(B, num_head, dim_position + dim_head, S, device=x.device, dtype=x.dtype) for _ in range(3))
     with _device(x.device):
         _call('spgt_projpos_qkv_fwd', x.data_ptr(), wq.data_ptr(), _p(bq), wk.data_ptr(), _p(bk), wv.data_ptr(), _p(bv),
@@ -539,8 +550,9 @@ def conv3x3_tc(x: Tensor, cin_off: int, Cin: int, w, bias: Tensor, y: Tensor, co
 
 
 def projpos_qkv_tc(x, wqkv: TcWeight, bq, bk, bv, lnwk, lnbk, lnwv, lnbv, eps, position, num_head, dim_head, dim_position):
-    _chk(x, 'x'); _chk(position, 'position')
+    _chk(x, 'x')
     B, S, D = x.shape
+    _coordinates(position, B * S, dim_position)
     q, k, v = (torch.empty(B, num_head, dim_position + dim_head, S, device=x.device, dtype=x.dtype) for _ in range(3))
     with _device(x.device):
         _call('spgt_projpos_qkv_tc_fwd', x.data_ptr(), wqkv.data_ptr(), _p(bq), _p(bk), _p(bv), lnwk.data_ptr(), lnbk.data_ptr(),
@@ -641,6 +653,16 @@ class EncoderPlan:
 
         fill(self.weights, lambda t: kept_pointer(self.keep, t))
         self.address = ctypes.addressof(self.weights)
+
+
+def encoder_fused_pays(B: int, S: int, ffn: bool = True) -> bool:
+    """Whether the fused encoder kernels are the faster ones for B samples of S nodes.  Their tiles hold rows of one sample and each
+    sample has a matrix of its own, so many samples of few nodes are packed better by the single ops: per sample fused 0.35 + 0.155 us per
+    128-row tile against 0.1 + 0.0022 us per node (attention layer alone 0.36 + 0.094 against 0.1 + 0.0016).  The single ops' launches take
+    108 us (73) of host time, which few samples do not reach.  Calls, us, fused / single: 256 x 128 nodes 151 / 121, 128 x 200 103 / 114,
+    256 x 256 188 / 192; attention layer 128 x 200 84 / 76, 64 x 200 53 / 76, 256 x 390 193 / 219."""
+    tiles = (S + 127) // 128
+    return S >= (250 if ffn else 390) or B * (10 * tiles + (23 if ffn else 38)) <= (7000 if ffn else 7300)
 
 
 def encoder_layer(plan: EncoderPlan, x: Tensor, position: Tensor, eps: float, act=None, ffn: bool = True, residual: bool = True) -> Tensor:

@@ -452,3 +452,31 @@ def test_weight_gradient_gemm_passes_nan_on(which):
     t[which] = _with_nan(t[which], 5000)
     c, sums = ops.tn_gemm(*(a.cuda() for a in t), column_sums=True)
     assert torch.equal(torch.isnan(c.cpu()), torch.isnan(t[0].t() @ t[1])) and torch.equal(torch.isnan(sums.cpu()), torch.isnan(t[1].sum(0)))
+
+
+# both sides of the rule: many samples of few nodes run on the single ops, the same samples a few at a time on the fused kernels
+@pytest.mark.parametrize('B,S,single', [(300, 40, True), (250, 129, True), (100, 129, False), (260, 250, False)])
+def test_encoder_layer_route(B, S, single):
+    from spgt_b200 import ops
+    layer, g = _layer(S)
+    layer = layer.cuda()
+    x, pos = torch.randn(B, S, 128, generator=g).cuda(), torch.rand(B, S, 2, generator=g).cuda()
+    with torch.no_grad():
+        with ops.profile_ops() as profile:
+            y = layer(x, pos)
+        assert ('spgt_encoder_layer_fwd' not in profile.times_ms()) == single
+        assert rel_l2(y[:20], layer(x[:20], pos[:20])) < TOL and rel_l2(y[-20:], layer(x[-20:], pos[-20:])) < TOL
+        with pytest.raises(ValueError):
+            layer(x, pos[:-1])
+    assert ops.tc_status() == 0
+
+
+def test_model_of_many_small_fields_runs_module_by_module():
+    from spgt_b200 import ops
+    model, node, position, grid = _model()                       # 15 x 15 attention nodes
+    times = lambda t: t[torch.arange(200) % 3].contiguous()
+    ref = model(node, position, grid)
+    before = ops.LAUNCHES
+    out = model(times(node), times(position), times(grid))
+    assert rel_l2(out, ref[torch.arange(200) % 3]) < TOL and ops.LAUNCHES > before
+    assert not model._native_shapes(times(node), times(position), times(grid)) and model._native_shapes(node, position, grid)

@@ -304,3 +304,14 @@ def test_exchanged_submodules_are_not_planned_for():
     layer = make().encoder_mixer.layers[0]
     layer.attention_layer.fc_layer = _Around(layer.attention_layer.fc_layer)
     assert not layer.trains_fused()
+
+
+def test_rules_of_the_encoder_route():
+    """Few samples, or enough nodes each: the fused kernels; and no more than one change of route as samples are added."""
+    from spgt_b200 import ops
+    for ffn in (True, False):
+        assert all(ops.encoder_fused_pays(B, S, ffn) for B in (1, 8, 64) for S in (1, 43 * 43, 200, 128, 2809)) and ops.encoder_fused_pays(4096, 512, ffn)
+        assert not ops.encoder_fused_pays(4096, 64, ffn) and not ops.encoder_fused_pays(256, 128, ffn)
+        for S in (1, 128, 129, 249, 389):
+            route = [ops.encoder_fused_pays(B, S, ffn) for B in range(1, 600)]
+            assert route == sorted(route, reverse=True)
