@@ -124,10 +124,10 @@ def _linear_tc(weight: Tensor) -> 'ops.TcWeight':
     return ops.TcWeight(_dense(weight), transposed=True)
 
 
-def _conv_tc(weight: Tensor, bias: Tensor, cin_pad: int, cout_pad: int):
-    """Conv2d weight [Cout, Cin, 3, 3] (+ bias) prepared for the tcgen05 implicit GEMM, with input / output channels
-    zero-padded to cin_pad / cout_pad (padded outputs come out as act(0))."""
-    if cout_pad <= 128:
+def _conv_tc(weight: Tensor, bias: Tensor, cin_pad: int, cout_pad: int, tiles: bool = True):
+    """Conv2d weight [Cout, Cin, 3, 3] (+ bias) prepared for the convolution kernel (`tiles`; up to 128 output channels) or the implicit
+    GEMM, with input / output channels zero-padded to cin_pad / cout_pad (padded outputs come out as act(0))."""
+    if tiles and cout_pad <= 128:
         return ops.ConvWeight.padded(weight.detach().contiguous(), bias.detach().contiguous(), cin_pad, cout_pad)
     cout, cin = weight.shape[:2]
     w = torch.zeros(cout_pad, cin_pad, 3, 3, device=weight.device, dtype=weight.dtype)
@@ -161,13 +161,13 @@ class ConvResBlock2D(_KernelWeights):
         return ops.conv3x3(X, cin_off, w.shape[1], self.kernel_weight(), self.conv_layer.bias.detach(), out, cout_off,
                            w.shape[0], self.activation if act is None else act)
 
-    def tc_weight(self, cin_pad: int, cout_pad: int):
-        return self._cached(('tc', cin_pad, cout_pad), lambda: _conv_tc(self.conv_layer.weight, self.conv_layer.bias, cin_pad, cout_pad))
+    def tc_weight(self, cin_pad: int, cout_pad: int, tiles: bool = True):
+        return self._cached(('tc', cin_pad, cout_pad, tiles), lambda: _conv_tc(self.conv_layer.weight, self.conv_layer.bias, cin_pad, cout_pad, tiles))
 
     def forward_tc(self, X: Tensor, cin_pad: int, cout_pad: int, act=None) -> Tensor:
         """tcgen05 path: X [N,H,W,cin_pad] (channels beyond in_dim must be finite; their weights are zero) ->
         new tensor [N,H,W,cout_pad] whose channels beyond out_dim hold act(0)."""
-        wt, b = self.tc_weight(cin_pad, cout_pad)
+        wt, b = self.tc_weight(cin_pad, cout_pad, ops.conv3x3_tiles_pay(*X.shape[:3], X.device))
         out = torch.empty(*X.shape[:3], cout_pad, device=X.device, dtype=X.dtype)
         return ops.conv3x3_tc(X, 0, cin_pad, wt, b, out, 0, cout_pad, self.activation if act is None else act)
 

@@ -537,6 +537,14 @@ def tn_gemm(a: Tensor, b: Tensor, column_sums: bool = False):
     return c, sums
 
 
+def conv3x3_tiles_pay(B: int, Hh: int, Ww: int, device) -> bool:
+    """Whether the convolution kernel with 8 x 16 pixel tiles and a zero row after each image is the faster one: unless many images are so
+    small that most of a tile's MMAs are padding and there is more than one wave of tiles.  us, tiles / implicit GEMM, 128 -> 128
+    channels: 4096 x 5 x 5 204 / 136, 256 x 9 x 9 56 / 48, 64 x 17 x 17 (no padding to speak of) 40 / 48, 8 x 9 x 9 (one wave) 22 / 43."""
+    tiles = -(-B * (Hh + 1) // 16) * -(-Ww // 8)
+    return 4 * 128 * tiles <= 7 * B * Hh * Ww or tiles <= torch.cuda.get_device_properties(device).multi_processor_count
+
+
 def conv3x3_tc(x: Tensor, cin_off: int, Cin: int, w, bias: Tensor, y: Tensor, cout_off: int, Cout: int, act) -> Tensor:
     """w: a ConvWeight, or a TcWeight (any number of output channels, the general GEMM kernel)."""
     _chk(x, 'x'); _chk(y, 'y'); _chk(bias, 'bias')

@@ -471,6 +471,20 @@ def test_encoder_layer_route(B, S, single):
     assert ops.tc_status() == 0
 
 
+@pytest.mark.parametrize('B,R,general', [(400, 9, True), (2000, 3, True), (8, 9, False), (64, 17, False)])
+def test_convolution_route(B, R, general):
+    from spgt_b200 import ops
+    from spgt_b200.network.layer import ConvResBlock2D
+    torch.manual_seed(R)
+    block = ConvResBlock2D(20, 44, 3, 1, 0.0, 'relu').cuda()
+    x = torch.randn(B, R, R, 20, device='cuda')
+    with torch.no_grad(), ops.profile_ops() as profile:
+        y = block.forward_tc(x, 20, 44)
+    assert ('spgt_conv3x3_tc_fwd' in profile.times_ms()) == general
+    ref = torch.nn.functional.conv2d(x.cpu().permute(0, 3, 1, 2).double(), block.conv_layer.weight.cpu().double(), block.conv_layer.bias.cpu().double(), padding=1)
+    assert rel_l2(y, torch.relu(ref).permute(0, 2, 3, 1).detach()) < TOL
+
+
 def test_model_of_many_small_fields_runs_module_by_module():
     from spgt_b200 import ops
     model, node, position, grid = _model()                       # 15 x 15 attention nodes
