@@ -28,6 +28,12 @@ struct ChainScope {
     ChainScope() { if (before == 0) g_chain = 1; }
     ~ChainScope() { g_chain = before; }
 };
+// Launches inside a ChainPause are ordinary ones, whatever scope it lies in.
+struct ChainPause {
+    const int before = g_chain;
+    explicit ChainPause(bool pause) { if (pause) g_chain = 0; }
+    ~ChainPause() { g_chain = before; }
+};
 template <class... KA, class... A>
 inline int launch_chained(void (*kern)(KA...), dim3 grid, int threads, size_t smem, cudaStream_t st, A&&... args) {
     cudaLaunchConfig_t cfg = {};

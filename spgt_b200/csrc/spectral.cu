@@ -29,6 +29,10 @@ int spectral_inv_y_tc(const float* x, const float* f3, const float* wr_img, cons
 
 constexpr int SP_C = 32;         // channel width handled by the tensor-core kernels
 constexpr int SP_IMG = 2 * SP_C * TC_BK;   // floats of one W stage image: hi and lo, 32 rows (n) x 32 k each
+// Most samples whose kernels are chained.  With more, the blocks of the inverse x transform that wait beside the long mixing kernel cost
+// more than the launch gaps: graph replays of 64 / 96 / 512 samples of 48 x 48 (29 x 29 for 512), us chained 73 / 139 / 305, plain
+// 74 / 101 / 279.
+constexpr int SP_CHAINED = 64;
 constexpr int SP_XMAX = 256;      // most grid rows a block of S2a / S2c stages (shared-memory budget)
 __host__ __device__ inline int sp_round_pitch(int n, int rem) {   // smallest p >= n with p % 32 == rem
     int p = (n + 31) / 32 * 32 + rem;
@@ -393,6 +397,7 @@ extern "C" int spgt_spectral_conv2d_fwd(const float* x, const float* wr, const f
     static SmemOptIn cfg_a, cfg_c;
     int e;
     const ChainScope chain;
+    const ChainPause pause(CH > SP_CHAINED);
     for (int b0 = 0; b0 < B; b0 += CH) {
         const int nb = B - b0 < CH ? B - b0 : CH;
         const float* xc = x + (size_t)b0 * r * r * C;

@@ -270,7 +270,7 @@ def test_encoder_layer_takes_any_dense_or_strided_weights_and_positions():
 
 
 # slices of the x transforms: none, one with a remainder, as many as rows or modes allow; grids of one, two and three 256-row units
-@pytest.mark.parametrize('B,r,m', [(1, 2, 1), (1, 95, 12), (1, 97, 12), (1, 256, 16), (2, 257, 16), (2, 421, 15), (3, 513, 3), (1, 600, 16), (20, 150, 8)])
+@pytest.mark.parametrize('B,r,m', [(1, 2, 1), (1, 95, 12), (1, 97, 12), (1, 256, 16), (2, 257, 16), (2, 421, 15), (3, 513, 3), (1, 600, 16), (20, 150, 8), (70, 40, 5)])
 def test_spectral_layer_slices_and_units(B, r, m):
     from spgt_b200 import ops
     g = torch.Generator().manual_seed(r + m)
