@@ -130,6 +130,11 @@ def _encoder_layer_by_ops(x: Tensor, position: Tensor, eps: float, params) -> Te
     return x + linear(torch.relu(linear(x, w1, b1)), w2, b2)
 
 
+def _as_read(params) -> list:
+    """The parameters as the kernels read them: themselves where they are row-major and 16-byte aligned."""
+    return [p if p.is_contiguous() and p.data_ptr() % 16 == 0 else _dense(p) for p in params]
+
+
 class _EncoderLayerFunction(torch.autograd.Function):
     """X + attention(X), then + ffn(.): projections and attention in one native call, their backward and all weight gradients in
     another; the dense layers' products along the layer are plain fp32, whose last bits decide what passes the ReLU.  A backward
@@ -138,7 +143,7 @@ class _EncoderLayerFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, position, eps, *params):
         ctx.eps, inputs = eps, (x, position, *params)
-        x, params = x.contiguous(), [_dense(p) for p in params]
+        x, params = x.contiguous(), _as_read(params)
         att, saved = ops.encoder_train_forward(x, position.contiguous(), eps, params)
         linear = torch.nn.functional.linear
         x1 = x + linear(att, params[10], params[11])
@@ -153,7 +158,7 @@ class _EncoderLayerFunction(torch.autograd.Function):
             wanted = [t for t, need in zip((x, *params), (ctx.needs_input_grad[0], *ctx.needs_input_grad[3:])) if need]
             grads = iter(torch.autograd.grad(_encoder_layer_by_ops(x, position, ctx.eps, params), wanted, grad_out, create_graph=True))
             return tuple(next(grads) if need else None for need in ctx.needs_input_grad)
-        dx, grads = ops.encoder_train_backward(x.contiguous(), att, x1, h, ctx.eps, [_dense(p) for p in params], saved, _dense(grad_out))
+        dx, grads = ops.encoder_train_backward(x.contiguous(), att, x1, h, ctx.eps, _as_read(params), saved, _dense(grad_out))
         return (dx, None, None, *grads)
 
 
