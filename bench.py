@@ -37,9 +37,10 @@ METRIC = 'darcy_gt_inference_samples_per_s_211'
 FINE, SUB_NODE, SUB_ATTN, MODES, SEED = 421, 2, 8, 12, 4
 GLOBAL_BATCH = 64
 CPU_SAMPLE = 8                     # samples per forward of the CPU legs (a bounded sample of the 64-sample step)
-# DRAM bytes (read + write) of one spectral layer at batch 64 from the committed ncu summary; they grow in
+# DRAM bytes (read + write) of one spectral and one encoder layer at batch 64 from the committed ncu summaries; they grow in
 # proportion to the batch, so a rank that holds 64/N samples is charged 1/N of them.
 SPECTRAL_TRAFFIC_BYTES_B64 = 1_172_100_000
+ENCODER_TRAFFIC_BYTES_B64 = 242_300_000
 
 
 def measured_peak():
@@ -512,7 +513,7 @@ def main():
                 'avg_launch_ms': avg, 'launches_timed': len(t),
                 'tflops': flops / (avg * 1e-3) / 1e12 if flops and avg > 0 else None}
     # encoder layer: read x and the positions, write y; K and V projections, K^T V, x M, feed-forward (fp32 products, three TF32 products each)
-    roof_enc = roofline('spgt_encoder_layer_fwd', 'encoder layer (encoder_kv, encoder_fold, encoder_out)', B * S * (2 * 128 + 2) * 4, None,
+    roof_enc = roofline('spgt_encoder_layer_fwd', 'encoder layer (encoder_kv, encoder_fold, encoder_out)', B * S * (2 * 128 + 2) * 4, ENCODER_TRAFFIC_BYTES_B64,
                         2 * B * S * (2 * 128 * 128 + H * DPK * DPK + 128 * 128 + 2 * 128 * 256))
     # spectral layer: read x once, write y once (fp32, 32 channels) + the complex mode weights; one entry-point call = all its kernels
     roof_spec = roofline('spgt_spectral_conv2d_fwd', 'spectral layer (all kernels of one call)',
